@@ -67,6 +67,7 @@ FS_DEV void integrate_adjoint(const Walls& w, float3 x, float3 v, float3 a, floa
 struct AdjArgs {
   GridDev g;
   NbrList L;
+  ScanXyz q;
   int64_t n;
   fs_model m;
   const float4* xs;    // (x, flags)
@@ -98,7 +99,8 @@ struct AdjArgs {
 // + flags, velocities + mass, mv, (P, R) from the step's rho and pressure,
 // viscosity, cohesion / mass, and ab from the walls / integrator adjoint.
 __global__ void k_adj_prepare(AdjArgs a, float* __restrict__ nu, float* __restrict__ coh, float4* __restrict__ xs,
-                              float4* __restrict__ vs, float* __restrict__ mv, float2* __restrict__ sc2) {
+                              ScanOut q, float4* __restrict__ vs, float* __restrict__ mv,
+                              float2* __restrict__ sc2) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= a.n) return;
   const int32_t i = a.g.perm[s];
@@ -109,6 +111,7 @@ __global__ void k_adj_prepare(AdjArgs a, float* __restrict__ nu, float* __restri
   const float4 x4 = make_float4(x.x, x.y, x.z, pack_pf(pf, w));
   const float mass = m.particle_mass[i];
   xs[s] = x4;
+  scan_put(q, s, x, (pf & PF_ACTIVE) != 0);
   vs[s] = make_float4(v.x, v.y, v.z, mass);
   const float rd = m.rest_density[i];
   mv[s] = rd * (mass / fmaxf(rd, 1.0e-6f));
@@ -179,6 +182,7 @@ FS_DEV PairAdj pair_adjoint(const Cubic& K, float h, float particle_radius, floa
 }
 
 __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
+  extern __shared__ uint2 words[];
   lists_recorded(a.L);
   for_slots(a.n, [&](int64_t s) {
     const float4 xk = a.xs[s];
@@ -206,8 +210,8 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
     const Cubic K(a.h);
     const float h2m = a.h * a.h * kSupportMargin;
     float Pb = 0.f, Rb = 0.f, nub = 0.f;
-    record_list<false>(a.g, a.xs, (int)s, xk, a.h, h2m, a.L);
-    visit<false, true>(a.g, a.xs, (int)s, xk, a.h, h2m, a.L, true, [&](int t, float4 xj) {
+    scan_visit<false>(a.g, a.q, a.xs, (int)s, xk, a.h, h2m, h2m, a.L, words, [](int) { return 0; },
+                      [&](int t, float4 xj, int) {
       const float3 d = make_float3(xk.x - xj.x, xk.y - xj.y, xk.z - xj.z);
       const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
       if (r2 == 0.f) return;  // the forward skips coincident pairs
@@ -271,7 +275,7 @@ __global__ void FS_NB_BOUNDS k_adj_density(AdjArgs a) {
     const Cubic K(a.h);
     float3 xb = make_float3(xr.x, xr.y, xr.z);
     const bool lists_ok = lists_usable(a.L);
-    visit<false, false>(a.g, a.xs, (int)s, xk, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok, [&](int t, float4 xj) {
+    visit<false>(a.g, a.xs, (int)s, xk, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok, [&](int t, float4 xj) {
       const float dx = xk.x - xj.x, dy = xk.y - xj.y, dz = xk.z - xj.z;
       float r, rinv;
       r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
@@ -312,6 +316,7 @@ int fs_wcsph_substep_adjoint(fs_context* c, const fs_model* m, const fs_state* s
   AdjArgs a;
   a.g = grid_view(c);
   a.L = nbr_list(c);
+  a.q = scan_xyz(c);
   a.n = n;
   a.m = *m;
   a.xs = c->xs;
@@ -341,11 +346,11 @@ int fs_wcsph_substep_adjoint(fs_context* c, const fs_model* m, const fs_state* s
   a.walls = make_walls(p->bound_width, p->bound_height, p->bound_length, p->boundary_damping, 0, 0.f, 0.f);
   {
     PassScope ps_(c, P_ADJ_INTEGRATE, st);
-    k_adj_prepare<<<blocks_for(n), kBlock, 0, st>>>(a, c->sc1, c->sc1b, c->xs, c->vs, c->mv, c->sc2);
+    k_adj_prepare<<<blocks_for(n), kBlock, 0, st>>>(a, c->sc1, c->sc1b, c->xs, scan_out(c), c->vs, c->mv, c->sc2);
   }
   {
     PassScope ps_(c, P_ADJ_FORCE, st);
-    k_adj_force<<<nb_blocks(c, n), c->nb_block, 0, st>>>(a);
+    k_adj_force<<<nb_blocks(c, n), c->nb_block, scan_smem(c->nb_block), st>>>(a);
   }
   {
     PassScope ps_(c, P_ADJ_DENSITY, st);

@@ -31,8 +31,8 @@ int reduction_blocks(int64_t n) { return blocks_for(n > 0 ? n : 1, 64); }
 
 // gather of fs_wcsph.cu reused here
 __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
-                                const float* __restrict__ v, float4* __restrict__ xs, float4* __restrict__ vs,
-                                float* __restrict__ mv, uint32_t* status, int nworlds);
+                                const float* __restrict__ v, float4* __restrict__ xs, ScanOut q,
+                                float4* __restrict__ vs, float* __restrict__ mv, uint32_t* status, int nworlds);
 
 namespace {
 
@@ -66,6 +66,7 @@ __global__ void k_gather_scalar(int64_t n, const int32_t* __restrict__ perm, con
 struct DensFactorArgs {
   GridDev g;
   NbrList L;
+  ScanXyz q;
   int64_t n;
   const float4* xs;
   const float4* vs;  // .w = mass
@@ -81,10 +82,11 @@ struct DensFactorArgs {
 
 // Records the neighbour lists of this grid (positions stay fixed for the half
 // step, so every later pass of the half reuses them exactly).
-// 64-register budget (4 resident 256-thread blocks): the compiler's own
-// choice was 48 registers with 52 bytes of spills; 0.306 -> 0.287 ms per
-// launch at 401,856 particles
-__global__ void __launch_bounds__(kNbBlockMax, 4) k_density_factor(DensFactorArgs a) {
+// 85-register budget: the scan and the visit need 72 without spills; with 64
+// (36 bytes of spills) a launch at 401,856 particles takes 0.126 ms, with 72
+// 0.121 (the per-candidate list recorder before took 0.158).
+__global__ void __launch_bounds__(kNbBlockMax, 3) k_density_factor(DensFactorArgs a) {
+  extern __shared__ uint2 words[];
   if (clock_idle(a.clock)) return;
   lists_recorded(a.L);
   for_slots(a.n, [&](int64_t s) {
@@ -99,22 +101,21 @@ __global__ void __launch_bounds__(kNbBlockMax, 4) k_density_factor(DensFactorArg
       return;
     }
     const float h2m = a.h * a.h * kSupportMargin;
-    // the candidate count (no distance test, solver_dfsph.py:163-164) comes from the scan
-    const int cnt = record_list<true>(a.g, a.xs, (int)s, xi, a.h, h2m, a.L);
     const Cubic K(a.h);
     float rho = 0.f, sgx = 0.f, sgy = 0.f, sgz = 0.f, sq = 0.f;
-    visit_with<true, true>(a.g, a.xs, (int)s, xi, a.h, h2m, a.L, true,
-                           [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.vs[t].w)); },
-                           [&](int t, float4 xj, const float2& mm) {  // (rest_density * volume, mass)
+    // the candidate count (no distance test, solver_dfsph.py:163-164) comes from the scan
+    const int cnt = scan_visit<true, true>(a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, words,
+                                           [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.vs[t].w)); },
+                                           [&](int t, float4 xj, const float2& mm) {  // (rest_density * volume, mass)
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
       float r, rinv;
       r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
       rho = fmaf(mm.x, K.w(r), rho);
       const float gsc = mm.y * K.grad_scale(r, rinv);
       const float gx = gsc * dx, gy = gsc * dy, gz = gsc * dz;
-      sgx += gx;
-      sgy += gy;
-      sgz += gz;
+      sgx = __fadd_rn(sgx, gx);  // the sums stay sums (no contraction), whatever surrounds them
+      sgy = __fadd_rn(sgy, gy);
+      sgz = __fadd_rn(sgz, gz);
       sq = fmaf(gx, gx, fmaf(gy, gy, fmaf(gz, gz, sq)));
     });
     const float denom = (sgx * sgx + sgy * sgy + sgz * sgz) + sq;
@@ -160,7 +161,7 @@ __global__ void FS_NB_BOUNDS k_accel_predict(AccelArgs a) {
     const Cubic K(a.h);
     float ax = 0.f, ay = 0.f, az = 0.f;
     const bool lists_ok = a.use_lists && lists_usable(a.L);
-    visit<false, false>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
+    visit<false>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
                         [&](int t, float4 xj) {
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -615,6 +616,7 @@ int run_density_factor(fs_context* c, const fs_model* m, float h, int min_nb, fl
   a.clock = c->clock;
   a.g = grid_view(c);
   a.L = nbr_list(c);
+  a.q = scan_xyz(c);
   a.n = m->n;
   a.xs = c->xs;
   a.vs = c->vs2;
@@ -627,7 +629,7 @@ int run_density_factor(fs_context* c, const fs_model* m, float h, int min_nb, fl
   a.sc2 = c->sc2;
   {
     PassScope ps_(c, P_DFSPH_DENSITY_FACTOR, st);
-    k_density_factor<<<nb_blocks(c, a.n), c->nb_block, 0, st>>>(a);
+    k_density_factor<<<nb_blocks(c, a.n), c->nb_block, scan_smem(c->nb_block), st>>>(a);
   }
   return launch_check("dfsph density/factor");
 }
@@ -729,7 +731,7 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
   if ((rc = grid_build(c, si->particle_q, n, h, st, m->particle_world, c->clock))) return rc;
   {
     PassScope ps_(c, P_GATHER, st);
-    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, si->particle_q, si->particle_qd, c->xs, c->vs,
+    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, si->particle_q, si->particle_qd, c->xs, scan_out(c), c->vs,
                                                     c->mv, c->status, c->nworlds);
   }
   {
@@ -784,7 +786,7 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
   if ((rc = grid_build(c, so->particle_q, n, h, st, m->particle_world, c->clock))) return rc;
   {
     PassScope ps_(c, P_GATHER, st);
-    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, so->particle_q, so->v_star, c->xs, c->vs2, c->mv,
+    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, so->particle_q, so->v_star, c->xs, scan_out(c), c->vs2, c->mv,
                                                     c->status, c->nworlds);
   }
   if ((rc = run_density_factor(c, m, h, p->min_neighbors_for_factor, so->rho, so->factor, so->neighbor_count, st)))
@@ -879,7 +881,7 @@ int fs_dfsph_density_factor(fs_context* c, const fs_model* m, const float* x, fl
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_dfsph_density_factor: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, x, c->xs, c->vs2, c->mv, c->status, c->nworlds);
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, x, c->xs, scan_out(c), c->vs2, c->mv, c->status, c->nworlds);
   return run_density_factor(c, m, h, min_nb, rho, factor, neighbor_count, st);
 }
 
@@ -896,7 +898,7 @@ int fs_dfsph_nonpressure_predict(fs_context* c, const fs_model* m, const float* 
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t n = m->n;
-  k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, c->vs, c->mv, c->status,
+  k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs, c->mv, c->status,
                                                     c->nworlds);
   k_gather_pair<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, rho, nullptr, c->sc2);
   AccelArgs aa;
@@ -926,7 +928,7 @@ int fs_dfsph_divergence(fs_context* c, const fs_model* m, const float* x, const 
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_dfsph_divergence: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v, c->xs, c->vs2, nullptr, c->status, c->nworlds);
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs2, nullptr, c->status, c->nworlds);
   // rho/factor are not needed for the rate itself (mode 1 reads them only for kappa, which is discarded)
   if (cudaMemsetAsync(c->sc2, 0, sizeof(float2) * m->n, st) != cudaSuccess)
     return set_error(FS_ERR_CUDA, "fs_dfsph_divergence: memset");
@@ -940,7 +942,7 @@ int fs_dfsph_correct(fs_context* c, const fs_model* m, const float* x, float* v_
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_dfsph_correct: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v_star, c->xs, c->vs2, nullptr,
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v_star, c->xs, scan_out(c), c->vs2, nullptr,
                                                        c->status, c->nworlds);
   k_gather_pair<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, rho, nullptr, c->sc2);
   k_gather_scalar<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, kappa, c->sc1, nullptr);

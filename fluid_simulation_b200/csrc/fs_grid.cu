@@ -271,6 +271,11 @@ NbrList nbr_list(const fs_context* c) {
   return L;
 }
 
+ScanXyz scan_xyz(const fs_context* c) { return ScanXyz{c->sxyz}; }
+ScanOut scan_out(const fs_context* c) {
+  return ScanOut{c->sxyz, &((ListCtl*)c->nb_ctl)->inactive};
+}
+
 GridDev grid_view(const fs_context* c) {
   GridDev g;
   g.off = c->cell_off;
@@ -506,6 +511,7 @@ static int context_alloc(fs_context* c, int64_t capacity, int64_t ncell) {
       {(void**)&c->skey, sizeof(int32_t) * cap},
       {(void**)&c->scan_part, sizeof(int32_t) * (nb + 1)},
       {(void**)&c->xs, sizeof(float4) * cap},           {(void**)&c->xs2, sizeof(float4) * cap},
+      {(void**)&c->sxyz, sizeof(float) * scan_floats(cap)},
       {(void**)&c->vs, sizeof(float4) * cap},           {(void**)&c->vs2, sizeof(float4) * cap},
       {(void**)&c->mv, sizeof(float) * cap},            {(void**)&c->sc2, sizeof(float2) * cap},
       {(void**)&c->sc1, sizeof(float) * cap},           {(void**)&c->sc1b, sizeof(float) * cap},
@@ -545,7 +551,7 @@ int fs_context_destroy(fs_context* c) {
   DeviceGuard dg(c->device);
   timer_free(c->timer);
   void* ps[] = {c->key, c->slot, c->cell_count, c->cell_off, c->big_cells, c->big_n, c->tmp_ids, c->perm, c->skey, c->scan_part, c->xs, c->xs2,
-                c->vs, c->vs2, c->mv, c->sc2, c->sc1, c->sc1b, c->krm, c->xo_tmp, c->vo_tmp, c->red_part, c->red_cnt,
+                c->sxyz, c->vs, c->vs2, c->mv, c->sc2, c->sc1, c->sc1b, c->krm, c->xo_tmp, c->vo_tmp, c->red_part, c->red_cnt,
                 c->dfsph, c->status, c->tile_stats, c->nb_idx, c->nb_cnt, c->nb_ctl, c->worlds, c->metrics,
                 c->dfsph_worlds, c->pbf_disp};
   for (void* p : ps)

@@ -94,6 +94,7 @@ struct fs_context {
 
   // cell-sorted streams
   float4* xs = nullptr;   // positions + packed flags
+  float* sxyz = nullptr;  // x, y, z of xs in groups of four, for the grid scans
   float4* xs2 = nullptr;  // second position buffer (PBF Jacobi double buffer)
   float4* vs = nullptr;   // velocities + mass
   float4* vs2 = nullptr;  // second velocity buffer (DFSPH v*, PBF x_in)
@@ -163,6 +164,9 @@ struct DeviceGuard {
 };
 
 inline int blocks_for(int64_t n, int b = kBlock) { return (int)((n + b - 1) / b); }
+
+// Floats of a context's scan copy: whole groups of four slots.
+inline int64_t scan_floats(int64_t cap) { return (cap + 3) / 4 * 12; }
 
 // Blocks of a neighbour-kernel launch under the context's tuning.
 inline int nb_blocks(const fs_context* c, int64_t n) {
@@ -586,19 +590,37 @@ FS_DEV int particle_pf(const int32_t* flags, const int32_t* mask, int64_t i) {
   return (act ? PF_ACTIVE : 0) | (dyn ? PF_DYNAMIC : 0);
 }
 
+// The scan copy of the positions (ScanXyz in fs_nbr.cuh): groups of four
+// slots, x[4], y[4], z[4].  An inactive particle lies at kScanFar: its squared
+// distance overflows to +inf.
+constexpr float kScanFar = 1.0e30f;
+struct ScanOut {
+  float* g;
+  int32_t* inactive;  // set when an inactive particle is gathered (ListCtl.inactive)
+};
+FS_DEV void scan_put(const ScanOut& q, int64_t s, float3 p, bool active) {
+  if (!active && q.inactive) *q.inactive = 1;
+  float* o = q.g + (s >> 2) * 12 + (s & 3);
+  o[0] = active ? p.x : kScanFar;
+  o[4] = p.y;
+  o[8] = p.z;
+}
+ScanOut scan_out(const fs_context* c);
+
 // Slot s (particle i = perm[s]) of the cell-order copies that the neighbour
 // loops read: xs = (x, flags + world), vs = (v, mass) when vs, and mv =
 // rest_density * volume with volume = mass / max(rest_density, 1e-6)
 // (compute_particle_volume, solver_wcsph.py:110-116) when mv.  A world index
 // past the model's worlds raises FS_STATUS_BOUNDS.
 FS_DEV void gather_common_slot(int64_t s, int32_t i, const fs_model& m, const float* __restrict__ x,
-                               const float* __restrict__ v, float4* __restrict__ xs, float4* __restrict__ vs,
-                               float* __restrict__ mv, uint32_t* status, int nworlds) {
+                               const float* __restrict__ v, float4* __restrict__ xs, const ScanOut& q,
+                               float4* __restrict__ vs, float* __restrict__ mv, uint32_t* status, int nworlds) {
   const float3 p = ld3(x, i);
   const int pf = particle_pf(m.particle_flags, m.particle_mask, i);
   // batched contexts carry the world in the flags word (queries stay in it)
   const int w = (nworlds > 0 && m.particle_world) ? world_index(m.particle_world[i], nworlds) : 0;
   xs[s] = make_float4(p.x, p.y, p.z, pack_pf(pf, w));
+  scan_put(q, s, p, (pf & PF_ACTIVE) != 0);
   const float mass = m.particle_mass[i];
   if (vs) {
     const float3 u = ld3(v, i);

@@ -3,10 +3,11 @@
 // One thread per cell-sorted slot.  Only ~15 % of a particle's 27-cell grid
 // candidates (the reference's hash_grid_query set) lie inside the support,
 // and every pass of a substep after the first reuses the same grid.  The
-// first pass over a grid therefore records each particle's in-support
-// candidates (plus a skin when positions will move) as a list in the
-// reference's visiting order; later passes iterate those ~35-60 entries
-// instead of ~216 candidates, with all lanes of a warp busy on pair terms.
+// first pass over a grid therefore scans the candidates (scan_visit) and
+// records each particle's in-support ones (plus a skin when positions will
+// move) as a list in the reference's visiting order; later passes iterate
+// those ~35-60 entries instead of ~216 candidates, with all lanes of a warp
+// busy on pair terms.
 #pragma once
 
 #include "fs_internal.cuh"
@@ -108,8 +109,15 @@ constexpr int kNbMax = 192;
 constexpr int64_t kListStride32Max = 0xffffffffLL / kNbMax;
 
 struct ListCtl {
-  int32_t valid;  // lists recorded for the current grid and positions
-  int32_t pad;
+  int32_t valid;     // lists recorded for the current grid and positions
+  int32_t inactive;  // some particle gathered for the current grid is inactive
+};
+
+// The coordinates of the cell-order particles for the grid scans: groups of
+// four slots, x[4], y[4], z[4] (48 bytes, 16-byte aligned); an inactive
+// particle lies far outside any support (kScanFar).
+struct ScanXyz {
+  const float* g;
 };
 
 struct NbrList {
@@ -119,67 +127,282 @@ struct NbrList {
   ListCtl* ctl;
 };
 
-// Records the grid candidates of slot s with r^2 + w <= h2m (self included)
-// in visiting order; returns the active candidates other than s (the DFSPH
-// neighbour count, no distance test) when COUNT.
-//
-// A row range that fits in the list whatever it holds (n + its length <=
-// kNbMax) takes the short loop: no per-candidate capacity test, and the
-// entry offset is 32-bit when the list fits (stride <= kListStride32Max).
-// Other ranges take the checked loop.  Both record the same entries.
+// ------------------------------------------------------------ grid scan --
+// A scan tests ~216 candidates per particle for ~35 hits, so it is bound by
+// the instructions and the L1 data cycles (128 bytes a cycle and SM, with
+// 16-byte records 4 cycles per warp and candidate) of one candidate.  It
+// therefore reads a separate copy of the cell-order coordinates (ScanXyz:
+// 12 bytes a candidate, three 16-byte loads for four), forms r^2 - h2 for two candidates at a time with packed f32x2 operations,
+// and shifts the sign bits into one 32-bit word: 5-6 instructions a candidate
+// where a test with a predicated store and a counter took about 14.  The
+// non-empty words of a particle (9-12) wait in shared memory; its hits are
+// then taken from them in visiting order, so every lane of a warp does pair
+// math in every step, and the list entries of step k leave the warp as one
+// coalesced row (a store at each hit cost one 32-byte sector a hit).
+// B200, against the recorder that tested and stored candidate by candidate:
+// WCSPH density at 4,194,304 particles 1.63 -> 1.00 ms, DFSPH density + factor
+// at 401,856 0.158 -> 0.121, PBF density 0.140 -> 0.106, lambda (mean of one
+// reusing and three scanning launches) 0.136 -> 0.114.  What bounds it now:
+// the L1's data cycles and the latency of its misses (a third of the time is
+// the word loop at about 55 % of the L1's data rate with 28 resident warps).
+// 10 or 16 words instead of 12: density +2 %.
+constexpr int kWords = 12;                 // words per thread between two visits
+constexpr float kScanSlack = 1.000004f;    // the scan takes a few more (never fewer) than the visit's test
+
+using f32x2 = unsigned long long;
+FS_DEV f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+FS_DEV f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+FS_DEV f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Shared memory of a recording launch: words of thread t at smem[w * threads + t].
+inline size_t scan_smem(int threads) { return sizeof(uint2) * kWords * (size_t)threads; }
+
+// Where a particle's scan stands: the next row (z, y), segment j of the row,
+// and the next candidate t of that segment (negative: its first).
+struct ScanPos {
+  int z, y, j, t;
+};
+
+// Writes the slot ranges of the query of slot s, in visiting order
+// (for_each_range's ranges) and cut into pieces of at most 32 candidates
+// (counted from the 16-byte group that holds the first), to words[k * nthr]
+// as (first, end), from pos on until kWords pieces are written or the query
+// is exhausted (live = false); returns their number.  COUNT adds the active
+// candidates other than s (no distance test) to ncand.
 template <bool COUNT>
-FS_DEV int record_list(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, float h2m,
-                       const NbrList& L) {
-  int n = 0, ncand = 0;
-  int32_t* const col = L.idx + s;  // entry k of slot s lives at col[k * stride]
-  const int64_t stride = L.stride;
-  const bool off32 = stride <= kListStride32Max;  // uniform across the launch
-  const uint32_t stride32 = (uint32_t)stride;
-  auto r2_of = [&](float4 xj) {
-    const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    return fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, xj.w)));  // +inf for inactive
-  };
-  auto count = [&](int t, float4 xj) {
-    if (COUNT) ncand += (t != s) ? (__float_as_int(xj.w) & PF_ACTIVE) : 0;
-  };
-  auto checked = [&](int t, float4 xj) {
-    count(t, xj);
-    if (r2_of(xj) <= h2m) {
-      if (n < kNbMax) col[(int64_t)n * stride] = t;
-      ++n;
+FS_DEV int scan_pieces(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, bool inactive,
+                       uint2* words, int nthr, ScanPos& pos, bool& live, int& ncand) {
+  const WorldDev* W = g.worlds ? g.worlds + world_index(world_of(xi), g.nworlds) : nullptr;
+  const QueryBox b = W ? query_box_world(g, *W, xi.x, xi.y, xi.z, h) : query_box_hash(g, xi.x, xi.y, xi.z, h);
+  const int nx = b.x1 - b.x0 + 1;
+  int c0 = b.x0, len1 = nx, nseg = 1;
+  bool slow = false;  // far outside the shifted range: cells clamp, one segment per cell
+  if (!W) {
+    const int xa = b.x0 + (1 << 20);
+    slow = xa < 0;
+    c0 = slow ? 0 : (g.mask_x >= 0 ? (xa & g.mask_x) : xa % g.dim_x);
+    len1 = min(nx, g.dim_x - c0);
+    nseg = slow ? nx : (nx > len1 ? 2 : 1);  // a run that wraps modulo dim_x splits in two
+  }
+  int nw = 0;
+  auto count = [&](int a, int e) {
+    if (inactive) {
+      for (int k = a; k < e; ++k) ncand += (k != s) ? (__float_as_int(__ldg(&xs[k].w)) & PF_ACTIVE) : 0;
+    } else {
+      ncand += (e - a) - ((s >= a && s < e) ? 1 : 0);
     }
   };
-  for_each_range(g, world_of(xi), xi.x, xi.y, xi.z, h, [&](int a, int e) {
-    int t = a;
-    if (off32 && n + (e - a) <= kNbMax) {
-      uint32_t o = (uint32_t)n * stride32;
-      auto fast = [&](int tt, float4 xj) {
-        count(tt, xj);
-        const bool hit = r2_of(xj) <= h2m;
-        if (hit) col[o] = tt;
-        o += hit ? stride32 : 0u;
-        n += hit ? 1 : 0;
-      };
-      for (; t + 4 <= e; t += 4) {  // four independent loads in flight
-        const float4 x0 = __ldg(xs + t), x1 = __ldg(xs + t + 1), x2 = __ldg(xs + t + 2), x3 = __ldg(xs + t + 3);
-        fast(t, x0);
-        fast(t + 1, x1);
-        fast(t + 2, x2);
-        fast(t + 3, x3);
+  const int ny = b.y1 - b.y0 + 1, nz = b.z1 - b.z0 + 1;
+  if (pos.z == INT32_MIN) {
+    pos.z = b.z0, pos.y = b.y0;
+    // The usual query: up to 3 x 3 rows of one segment each, in a world's box
+    // or a hash grid of power-of-two dims.  All their offsets load at once
+    // (one row at a time spent a latency a row and a fifth of the scan).
+    const bool plain = W ? true : (g.mask_y | g.mask_z) >= 0 && nseg == 1 && !slow && min(b.y0, b.z0) >= -(1 << 20);
+    if (plain && nx > 0 && ny <= 3 && nz <= 3) {
+      const int shift = W ? 0 : 1 << 20;
+      const int my = W ? INT32_MAX : g.mask_y, mz = W ? INT32_MAX : g.mask_z;
+      const int sy = W ? W->dims[0] : g.dim_x, sz = sy * (W ? W->dims[1] : g.dim_y);
+      const int32_t* const o = g.off + c0 + (W ? W->base : 0);
+      int a[9], e[9];
+#pragma unroll
+      for (int z = 0; z < 3; ++z)
+#pragma unroll
+        for (int y = 0; y < 3; ++y) {
+          const int row = ((b.z0 + z + shift) & mz) * sz + ((b.y0 + y + shift) & my) * sy;
+          const bool in = z < nz && y < ny;
+          a[z * 3 + y] = in ? __ldg(o + row) : 0;
+          e[z * 3 + y] = in ? __ldg(o + row + nx) : 0;
+        }
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        if (COUNT) count(a[k], e[k]);
+        for (int f = a[k]; f < e[k];) {
+          const int stop = min(e[k], (f & ~3) + 32);
+          if (nw == kWords) {
+            pos.z = b.z0 + k / 3, pos.y = b.y0 + k % 3, pos.t = f;
+            return nw;
+          }
+          words[nw * nthr] = make_uint2((uint32_t)f, (uint32_t)stop);
+          ++nw;
+          f = stop;
+        }
       }
-      for (; t < e; ++t) fast(t, __ldg(xs + t));
-      return;
+      live = false;
+      return nw;
     }
-    for (; t + 4 <= e; t += 4) {
-      const float4 x0 = __ldg(xs + t), x1 = __ldg(xs + t + 1), x2 = __ldg(xs + t + 2), x3 = __ldg(xs + t + 3);
-      checked(t, x0);
-      checked(t + 1, x1);
-      checked(t + 2, x2);
-      checked(t + 3, x3);
+  }
+  if (nx <= 0 || b.y0 > b.y1) pos.z = b.z1 + 1;
+  auto load = [&](int z, int y, int j, int& a, int& e) {
+    const int row = W ? W->base + (z * W->dims[1] + y) * W->dims[0]
+                      : (wrap_axis(z, g.dim_z, g.mask_z) * g.dim_y + wrap_axis(y, g.dim_y, g.mask_y)) * g.dim_x;
+    int first = c0, len = len1;
+    if (j) first = 0, len = nx - len1;
+    if (slow) first = wrap_axis(b.x0 + j, g.dim_x, g.mask_x), len = 1;
+    a = __ldg(g.off + row + first);
+    e = __ldg(g.off + row + first + len);
+  };
+  int a = 0, e = 0;
+  if (pos.z <= b.z1) load(pos.z, pos.y, pos.j, a, e);
+  while (pos.z <= b.z1) {
+    // the next range's offsets load while this one is cut
+    int z = pos.z, y = pos.y, j = pos.j + 1, an = 0, en = 0;
+    if (j == nseg) {
+      j = 0;
+      if (++y > b.y1) y = b.y0, ++z;
     }
-    for (; t < e; ++t) checked(t, __ldg(xs + t));
-  });
-  L.cnt[s] = n <= kNbMax ? n : kNbMax + 1;
+    if (z <= b.z1) load(z, y, j, an, en);
+    int f = pos.t;
+    if (f < 0) {
+      f = a;
+      if (COUNT) count(a, e);
+    }
+    while (f < e) {
+      if (nw == kWords) {
+        pos.t = f;
+        return nw;
+      }
+      const int stop = min(e, (f & ~3) + 32);
+      words[nw * nthr] = make_uint2((uint32_t)f, (uint32_t)stop);
+      ++nw;
+      f = stop;
+    }
+    pos = ScanPos{z, y, j, -1};
+    a = an, e = en;
+  }
+  live = false;
+  return nw;
+}
+
+// Replaces the pieces in `words` by their non-empty hit words (mask, last):
+// bit b set = slot last - b lies within the radius whose square is h2.
+FS_DEV int scan_words(const ScanXyz& q, float4 xi, float h2, uint2* words, int nthr, int np) {
+  const f32x2 nx = pack2(-xi.x, -xi.x), ny = pack2(-xi.y, -xi.y), nz = pack2(-xi.z, -xi.z);
+  const f32x2 nh = pack2(-h2, -h2);
+  int nw = 0;
+  for (int k = 0; k < np; ++k) {
+    const uint2 piece = words[k * nthr];
+    const uint32_t g0 = piece.x >> 2, g1 = (piece.y + 3) >> 2;  // groups of four candidates
+    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(q.g) + (size_t)g0 * 3;
+    uint32_t m = 0;
+#pragma unroll 2  // two groups of loads in flight (density time with 1: +1 to 3 %, with 4: up to +7 %)
+    for (uint32_t i = g0; i < g1; ++i, p += 3) {
+      const ulonglong2 x2 = __ldg(p), y2 = __ldg(p + 1), z2 = __ldg(p + 2);
+      const f32x2 dx0 = add2(x2.x, nx), dx1 = add2(x2.y, nx);
+      const f32x2 dy0 = add2(y2.x, ny), dy1 = add2(y2.y, ny);
+      const f32x2 dz0 = add2(z2.x, nz), dz1 = add2(z2.y, nz);
+      const f32x2 r0 = fma2(dx0, dx0, fma2(dy0, dy0, fma2(dz0, dz0, nh)));
+      const f32x2 r1 = fma2(dx1, dx1, fma2(dy1, dy1, fma2(dz1, dz1, nh)));
+      m = __funnelshift_l((uint32_t)r0, m, 1);  // the sign bit of r^2 - h2: set = within
+      m = __funnelshift_l((uint32_t)(r0 >> 32), m, 1);
+      m = __funnelshift_l((uint32_t)r1, m, 1);
+      m = __funnelshift_l((uint32_t)(r1 >> 32), m, 1);
+    }
+    // slots of the groups outside the piece: before its first, after its last
+    m &= 0xffffffffu >> (32 - 4 * (g1 - g0) + (piece.x & 3));
+    m &= 0xffffffffu << (4 * g1 - piece.y);
+    if (m) {
+      words[nw * nthr] = make_uint2(m, 4 * g1 - 1);
+      ++nw;
+    }
+  }
+  return nw;
+}
+
+// Records the list of slot s (candidates within the radius whose square is
+// h2rec, in visiting order, self included) and calls pair(t, xj, payload) for
+// those that pass visit_with's test at h2m, in the same order; load(t) is
+// issued together with the position gather.  Returns the DFSPH candidate
+// count when COUNT.  More than kNbMax entries mark the list overflowed; the
+// pairs are still all visited here.  REUSE: a particle with reuse >= 0 visits
+// the `reuse` entries its list already holds instead of scanning (in the same
+// loop: lanes that scan and lanes that reuse share the warp's pair math).
+template <bool WITH_SELF, bool COUNT = false, bool REUSE = false, class Load, class Pair>
+FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
+                      float h2rec, float h2m, const NbrList& L, uint2* smem, Load&& load, Pair&& pair,
+                      int reuse = -1) {
+  const int nthr = blockDim.x;
+  uint2* const words = smem + threadIdx.x;
+  const bool inactive = COUNT && L.ctl->inactive;
+  ScanPos pos{INT32_MIN, 0, 0, -1};
+  bool live = true;
+  int n = 0, ncand = 0;
+  int32_t* const col = L.idx + s;
+  auto one = [&](int t, float4 xj, const auto& p) {
+    const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+    if (fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, xj.w))) <= h2m && (WITH_SELF || t != s)) pair(t, xj, p);
+  };
+  const bool scan = !REUSE || reuse < 0;
+  while (live) {
+    int nw = 0;
+    if (scan) {
+      const int np = scan_pieces<COUNT>(g, xs, s, xi, h, inactive, words, nthr, pos, live, ncand);
+      nw = scan_words(q, xi, h2rec * kScanSlack, words, nthr, np);
+    } else {
+      live = false;
+    }
+    int w = 0;
+    uint32_t m = 0, last = 0;
+    auto pop = [&](bool& ok) {
+      if (!m && w < nw) {
+        const uint2 v = words[w * nthr];
+        m = v.x, last = v.y;
+        ++w;
+      }
+      ok = m != 0;
+      const uint32_t hi = 31 - __clz(m);  // ok: the first slot of the word that is left
+      m &= ~(1u << (hi & 31));
+      return ok ? (int)(last - hi) : s;
+    };
+    while (scan ? (m || w < nw) : n < reuse) {
+      bool k0, k1, k2, k3;
+      int t0, t1, t2, t3;
+      if (scan) {
+        t0 = pop(k0), t1 = pop(k1), t2 = pop(k2), t3 = pop(k3);
+      } else {
+        const int32_t* const o = col + (int64_t)n * L.stride;
+        k0 = true, k1 = n + 1 < reuse, k2 = n + 2 < reuse, k3 = n + 3 < reuse;
+        t0 = o[0];
+        t1 = k1 ? o[L.stride] : s;
+        t2 = k2 ? o[2 * L.stride] : s;
+        t3 = k3 ? o[3 * L.stride] : s;
+      }
+      const float4 x0 = __ldg(xs + t0), x1 = __ldg(xs + t1), x2 = __ldg(xs + t2), x3 = __ldg(xs + t3);
+      const auto p0 = load(t0), p1 = load(t1), p2 = load(t2), p3 = load(t3);
+      if (!scan) {
+      } else if (n + 4 <= kNbMax) {
+        int32_t* const o = col + (int64_t)n * L.stride;
+        o[0] = t0;
+        if (k1) o[L.stride] = t1;
+        if (k2) o[2 * L.stride] = t2;
+        if (k3) o[3 * L.stride] = t3;
+      } else {
+        const int tt[4] = {t0, t1, t2, t3};
+        const bool kk[4] = {k0, k1, k2, k3};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (kk[k] && n + k < kNbMax) col[(int64_t)(n + k) * L.stride] = tt[k];
+      }
+      n += (int)k0 + (int)k1 + (int)k2 + (int)k3;
+      one(t0, x0, p0);
+      if (k1) one(t1, x1, p1);
+      if (k2) one(t2, x2, p2);
+      if (k3) one(t3, x3, p3);
+    }
+  }
+  if (scan) L.cnt[s] = n <= kNbMax ? n : kNbMax + 1;
   return ncand;
 }
 
@@ -196,16 +419,14 @@ FS_DEV void scan_grid(const GridDev& g, const float4* __restrict__ xs, int s, fl
 
 // Visits the neighbours of slot s within h2m through its recorded list when
 // lists_ok and the list did not overflow, else by rescanning the grid.
-// FRESH: the list was written by the calling kernel, so entries are read
-// with coherent loads (each thread reads only the entries it wrote).
-template <bool WITH_SELF, bool FRESH, class Pair>
+template <bool WITH_SELF, class Pair>
 FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, float h2m,
                   const NbrList& L, bool lists_ok, Pair&& pair) {
-  const int n = lists_ok ? (FRESH ? L.cnt[s] : __ldg(L.cnt + s)) : kNbMax + 1;
+  const int n = lists_ok ? __ldg(L.cnt + s) : kNbMax + 1;
   const bool use = n <= kNbMax;
   if (use) {
     const int32_t* col = L.idx + s;
-    auto entry = [&](int k) { return FRESH ? col[(int64_t)k * L.stride] : __ldg(col + (int64_t)k * L.stride); };
+    auto entry = [&](int k) { return __ldg(col + (int64_t)k * L.stride); };
     auto one = [&](int t, float4 xj) {
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
       if (fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, xj.w))) <= h2m && (WITH_SELF || t != s)) pair(t, xj);
@@ -235,16 +456,16 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, int s, float4
 // pair(t, xj, payload) is called in the same order and for the same entries
 // as visit() calls pair(t, xj).  Only for lists recorded at the current
 // positions (every entry within h2m except the particle itself), where the
-// early load fetches nothing that visit() would not.  FRESH as in visit().
+// early load fetches nothing that visit() would not.
 // EVICT_FIRST: entries are loaded evict-first (ld.global.cs), leaving the
 // caches to the neighbours' data.  Measured faster for the PBF passes whose
 // lists at most one later pass reads again (delta, non-pressure, XSPH:
 // 1.304 -> 1.287 ms per substep at 401,856 particles); the DFSPH iteration
 // passes, which read the same lists 34 times a substep, were slower with it.
-template <bool WITH_SELF, bool FRESH = false, bool EVICT_FIRST = false, class Load, class Pair>
+template <bool WITH_SELF, bool EVICT_FIRST = false, class Load, class Pair>
 FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, float h2m,
                        const NbrList& L, bool lists_ok, Load&& load, Pair&& pair) {
-  const int n = lists_ok ? (FRESH ? L.cnt[s] : __ldg(L.cnt + s)) : kNbMax + 1;
+  const int n = lists_ok ? __ldg(L.cnt + s) : kNbMax + 1;
   const bool use = n <= kNbMax;
   auto one = [&](int t, float4 xj, const auto& p) {
     const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -253,8 +474,7 @@ FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, int s, f
   if (use) {
     const int32_t* col = L.idx + s;
     auto entry = [&](int k) {
-      return FRESH ? col[(int64_t)k * L.stride]
-                   : (EVICT_FIRST ? __ldcs(col + (int64_t)k * L.stride) : __ldg(col + (int64_t)k * L.stride));
+      return EVICT_FIRST ? __ldcs(col + (int64_t)k * L.stride) : __ldg(col + (int64_t)k * L.stride);
     };
     int k = 0;
     for (; k + 3 < n; k += 4) {
@@ -280,6 +500,7 @@ FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, int s, f
 FS_DEV bool lists_usable(const NbrList& L) { return L.ctl->valid != 0; }
 
 NbrList nbr_list(const fs_context* c);
+ScanXyz scan_xyz(const fs_context* c);
 
 // Marks freshly recorded lists valid (first thread of the recording kernel);
 // a grid build resets the mark.

@@ -23,8 +23,8 @@
 namespace fs {
 
 __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
-                                const float* __restrict__ v, float4* __restrict__ xs, float4* __restrict__ vs,
-                                float* __restrict__ mv, uint32_t* status, int nworlds);
+                                const float* __restrict__ v, float4* __restrict__ xs, ScanOut q,
+                                float4* __restrict__ vs, float* __restrict__ mv, uint32_t* status, int nworlds);
 
 namespace {
 
@@ -49,53 +49,45 @@ __global__ void k_predict(int64_t n, fs_model m, GridDev g, const float* __restr
 // x_in (xin_s, for the velocity update) in one pass over the permutation.
 __global__ void k_gather_pbf(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x_pred,
                              const float* __restrict__ v_pred, const float* __restrict__ x_in, float4* __restrict__ xs,
-                             float4* __restrict__ vs, float* __restrict__ mv, float4* __restrict__ xin_s,
+                             ScanOut q, float4* __restrict__ vs, float* __restrict__ mv, float4* __restrict__ xin_s,
                              uint32_t* status, int nworlds) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const int32_t i = perm[s];
-  gather_common_slot(s, i, m, x_pred, v_pred, xs, vs, mv, status, nworlds);
+  gather_common_slot(s, i, m, x_pred, v_pred, xs, q, vs, mv, status, nworlds);
   const float3 p = ld3(x_in, i);
   xin_s[s] = make_float4(p.x, p.y, p.z, 0.f);
 }
 
 // compute_density (115-141), poly6, self included.  sc2[s] = (rho,
 // mass / max(rho, 1e-6)): the neighbour term of the viscosity and XSPH passes.
-// With `record` it records the neighbour lists that the next pass at the
-// same positions (accel, or XSPH) reuses.  With vout (the final density of a
-// substep) it also writes update_velocity_from_positions (403-416):
+// It records the neighbour lists that the next pass at the same positions
+// (accel, or XSPH) reuses, out to h (1 + skin) where the first lambda pass
+// reuses them too (k_lambda).  With vout (the final density of a substep) it
+// also writes update_velocity_from_positions (403-416):
 // vout[s] = ((x_pred - x_in) / max(dt, 1e-8), m / max(rho, 1e-6)), v_pred
 // for non-dynamic particles.
-__global__ void FS_NB_BOUNDS_PBF k_density(GridDev g, NbrList L, int record, int64_t n,
+__global__ void FS_NB_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, int64_t n,
                                                       const float4* __restrict__ xs, const float4* __restrict__ vs,
                                                       const float* __restrict__ mv, float h, float skin, float* rho,
                                                       float2* __restrict__ sc2, const float4* __restrict__ xin = nullptr,
                                                       float dt = 0.f, float4* __restrict__ vout = nullptr) {
-  if (record) lists_recorded(L);
+  extern __shared__ uint2 words[];
+  lists_recorded(L);
   for_slots(n, [&](int64_t s) {
     const float4 xi = xs[s];
     const int32_t i = g.perm[s];
     float acc = 0.f;
     const float h2m = h * h * kSupportMargin;
     const Poly6Spiky K(h);
-    auto pair = [&](int t, float4 xj) {
-      const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      acc = fmaf(__ldg(mv + t), K.w_r2(fmaf(dx, dx, fmaf(dy, dy, dz * dz))), acc);
-    };
     if (pf_of(xi) & PF_ACTIVE) {
-      if (record) {
-        // entries out to h (1 + skin): the first lambda pass reuses them (k_lambda)
-        const float hr = h * (1.0f + skin);
-        record_list<false>(g, xs, (int)s, xi, h, hr * hr * kSupportMargin, L);
-        visit_with<true, true>(g, xs, (int)s, xi, h, h2m, L, true, [&](int t) { return __ldg(mv + t); },
-                               [&](int t, float4 xj, const float& m) {
-          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-          acc = fmaf(m, K.w_r2(fmaf(dx, dx, fmaf(dy, dy, dz * dz))), acc);
-        });
-      } else {
-        scan_grid<true>(g, xs, (int)s, xi, h, h2m, pair);
-      }
-    } else if (record) {
+      const float hr = h * (1.0f + skin);
+      scan_visit<true>(g, q, xs, (int)s, xi, h, hr * hr * kSupportMargin, h2m, L, words,
+                       [&](int t) { return __ldg(mv + t); }, [&](int t, float4 xj, const float& m) {
+        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+        acc = fmaf(m, K.w_r2(fmaf(dx, dx, fmaf(dy, dy, dz * dz))), acc);
+      });
+    } else {
       L.cnt[s] = 0;
     }
     rho[i] = acc;
@@ -129,6 +121,7 @@ struct AccelArgs {
   Walls walls;
   float* accel;
   float4* xs_out;
+  ScanOut q;                     // xs_out's scan copy (of the particles that move)
   uint32_t* disp_max = nullptr;  // largest |x_out - x| (float bits; null: not tracked)
 };
 
@@ -153,7 +146,7 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
     float ax = 0.f, ay = 0.f, az = 0.f;
     if (gamma != 0.f || mu != 0.f) {
       const bool lists_ok = a.use_lists && lists_usable(a.L);
-      visit_with<false, false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
+      visit_with<false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
                         [&](int t) { return __ldg(a.vs + t); }, [&](int t, float4 xj, const float4& vj) {
         const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
         const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -177,6 +170,7 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
     float3 p = make_float3(xi.x + a.dt * dvx, xi.y + a.dt * dvy, xi.z + a.dt * dvz);
     clamp_position(walls_of(a.walls, a.g, world_of(xi)), p);
     a.xs_out[s] = make_float4(p.x, p.y, p.z, xi.w);
+    scan_put(a.q, s, p, true);
     const float ex = p.x - xi.x, ey = p.y - xi.y, ez = p.z - xi.z;
     dmax = fmaxf(dmax, sqrtf(ex * ex + ey * ey + ez * ez));
   });
@@ -190,7 +184,7 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
 struct LambdaArgs {
   GridDev g;
   NbrList L;
-  int use_lists;
+  ScanXyz q;
   int64_t n;
   const float4* xs;
   const float4* vs;   // .w = mass
@@ -217,6 +211,7 @@ struct LambdaArgs {
 // reproduces the scan's pair sequence exactly.  Particles failing (b), and
 // every particle when (a) fails, scan the grid.
 __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
+  extern __shared__ uint2 words[];
   lists_recorded(a.L);
   const bool reuse_ok = a.xs_rec && __uint_as_float(*a.disp_max) <= a.reuse_limit;
   for_slots(a.n, [&](int64_t s) {
@@ -237,15 +232,15 @@ __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
     int cnt = 0;
     const float h2m = a.h * a.h * kSupportMargin;
     // records the lists the delta pass of this iteration (same positions) reuses
-    const bool reuse = reuse_ok && a.L.cnt[s] <= kNbMax && same_query_cells(a.g, world_of(xi), a.xs_rec[s], xi, a.h);
+    const int listed = reuse_ok ? a.L.cnt[s] : kNbMax + 1;
+    const bool reuse = listed <= kNbMax && same_query_cells(a.g, world_of(xi), a.xs_rec[s], xi, a.h);
     if (a.g.tile_stats && a.xs_rec) {
       const unsigned full = __activemask();
       const unsigned b = __ballot_sync(full, reuse);
       if ((int)(threadIdx.x & 31) == __ffs(full) - 1) atomicAdd(a.g.tile_stats + 2, (unsigned long long)__popc(b));
     }
-    if (!reuse) record_list<false>(a.g, a.xs, (int)s, xi, a.h, h2m, a.L);
-    visit_with<true, true>(a.g, a.xs, (int)s, xi, a.h, h2m, a.L, true, [&](int t) { return __ldg(&a.vs[t].w); },
-                           [&](int t, float4 xj, const float& mj) {
+    scan_visit<true, false, true>(a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, words,
+                                  [&](int t) { return __ldg(&a.vs[t].w); }, [&](int t, float4 xj, const float& mj) {
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
       if (t != (int)s && exact_lt_h(r2, dx, dy, dz, a.h, K.h2)) ++cnt;
@@ -258,7 +253,7 @@ __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
       gx -= gjx;
       gy -= gjy;
       gz -= gjz;
-    });
+    }, reuse ? listed : -1);
     sq = fmaf(gx, gx, fmaf(gy, gy, fmaf(gz, gz, sq)));
     const float ci = fmaxf(rho / rho0 - 1.0f, 0.f);
     const float l = (a.min_nb > 0 && cnt < a.min_nb) ? 0.f : -ci / (sq + a.eps);
@@ -285,6 +280,7 @@ struct DeltaArgs {
   Walls walls;
   float* delta_p;     // API
   float4* xs_out;     // may be null (separate-pass use)
+  ScanOut q;          // xs_out's scan copy (of the particles that move)
 };
 
 // x^n for a small positive integer n by repeated squaring (2 products for
@@ -316,7 +312,7 @@ __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
     const float inv_wdq = scorr ? 1.0f / a.w_dq : 0.f;
     float dx_ = 0.f, dy_ = 0.f, dz_ = 0.f;
     const bool lists_ok = a.use_lists && lists_usable(a.L);
-    visit_with<false, false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
+    visit_with<false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
                       [&](int t) { return __ldg(a.lam_s + t); }, [&](int t, float4 xj, const float2& lj) {
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -345,6 +341,7 @@ __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
       float3 p = make_float3(xi.x + d.x, xi.y + d.y, xi.z + d.z);
       if (a.clamp) clamp_position(walls_of(a.walls, a.g, world_of(xi)), p);
       a.xs_out[s] = make_float4(p.x, p.y, p.z, xi.w);
+      scan_put(a.q, s, p, true);
     }
   });
 }
@@ -380,7 +377,7 @@ __global__ void FS_NB_BOUNDS_PBF k_xsph_final(XsphArgs a) {
         const Poly6Spiky K(a.h);
         float cx = 0.f, cy = 0.f, cz = 0.f;
         const bool lists_ok = a.use_lists && lists_usable(a.L);
-        visit_with<false, false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
+        visit_with<false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
                           [&](int t) { return __ldg(a.vel + t); }, [&](int t, float4 xj, const float4& vj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           // vj = (v, m / max(rho, 1e-6))
@@ -434,8 +431,8 @@ int gather_pbf(fs_context* c, const fs_model* m, const float* x_in, cudaStream_t
   const int64_t n = m->n;
   {
     PassScope ps_(c, P_GATHER, st);
-    k_gather_pbf<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, c->xo_tmp, c->vo_tmp, x_in, c->xs, c->vs, c->mv,
-                                                 c->vs2, c->status, c->nworlds);
+    k_gather_pbf<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, c->xo_tmp, c->vo_tmp, x_in, c->xs, scan_out(c),
+                                                   c->vs, c->mv, c->vs2, c->status, c->nworlds);
   }
   return launch_check("pbf gather");
 }
@@ -487,7 +484,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     return rc;
   {
     PassScope ps_(c, P_PBF_DENSITY, st);
-    k_density<<<nb_blocks(c, n), c->nb_block, 0, st>>>(g, L, 1, n, c->xs, c->vs, c->mv, h, skin, so->rho, c->sc2);
+    k_density<<<nb_blocks(c, n), c->nb_block, scan_smem(c->nb_block), st>>>(g, L, scan_xyz(c), n, c->xs, c->vs, c->mv, h, skin, so->rho, c->sc2);
   }
   AccelArgs aa;
   aa.g = g;
@@ -504,6 +501,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   aa.walls = w;
   aa.accel = accel;
   aa.xs_out = c->xs2;
+  aa.q = scan_out(c);
   aa.disp_max = skin > 0.f ? c->pbf_disp : nullptr;
   {
     PassScope ps_(c, P_PBF_ACCEL, st);
@@ -517,7 +515,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     LambdaArgs la;
     la.g = gi;
     la.L = L;
-    la.use_lists = use_lists;
+    la.q = scan_xyz(c);
     la.n = n;
     la.xs = cur;
     la.vs = c->vs;
@@ -534,7 +532,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     la.reuse_limit = 0.5f * h * (skin - 1.0e-4f);
     {
       PassScope ps_(c, P_PBF_LAMBDA, st);
-      k_lambda<<<nb_blocks(c, n), c->nb_block, 0, st>>>(la);
+      k_lambda<<<nb_blocks(c, n), c->nb_block, scan_smem(c->nb_block), st>>>(la);
     }
     DeltaArgs da;
     da.g = gi;
@@ -554,6 +552,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     da.walls = w;
     da.delta_p = so->delta_p;
     da.xs_out = nxt;
+    da.q = scan_out(c);
     {
       PassScope ps_(c, P_PBF_DELTA, st);
       k_delta<<<nb_blocks(c, n), c->nb_block, 0, st>>>(da);
@@ -579,7 +578,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   {
     // + update_velocity_from_positions into nxt (the other x_pred buffer)
     PassScope ps_(c, P_PBF_DENSITY, st);
-    k_density<<<nb_blocks(c, n), c->nb_block, 0, st>>>(gf, L, 1, n, cur, c->vs, c->mv, h, 0.f, so->rho, c->sc2,
+    k_density<<<nb_blocks(c, n), c->nb_block, scan_smem(c->nb_block), st>>>(gf, L, scan_xyz(c), n, cur, c->vs, c->mv, h, 0.f, so->rho, c->sc2,
                                                        c->vs2, dt, nxt);
   }
   XsphArgs xa;
@@ -625,10 +624,10 @@ int fs_pbf_density(fs_context* c, const fs_model* m, const float* x, float h, fl
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_pbf_density: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, x, c->xs, c->vs, c->mv,
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, x, c->xs, scan_out(c), c->vs, c->mv,
                                                        c->status, c->nworlds);
-  k_density<<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(grid_view(c), nbr_list(c), 0, m->n, c->xs, c->vs, c->mv, h, 0.f,
-                                                                rho, c->sc2);
+  k_density<<<nb_blocks(c, m->n), c->nb_block, scan_smem(c->nb_block), st>>>(
+      grid_view(c), nbr_list(c), scan_xyz(c), m->n, c->xs, c->vs, c->mv, h, 0.f, rho, c->sc2);
   return launch_check("fs_pbf_density");
 }
 
@@ -639,12 +638,12 @@ int fs_pbf_lambda(fs_context* c, const fs_model* m, const float* x_pred, const f
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_pbf_lambda: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, x_pred, c->xs, c->vs, nullptr,
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, x_pred, c->xs, scan_out(c), c->vs, nullptr,
                                                        c->status, c->nworlds);
   LambdaArgs la;
   la.g = grid_view(c);
   la.L = nbr_list(c);
-  la.use_lists = 0;
+  la.q = scan_xyz(c);
   la.n = m->n;
   la.xs = c->xs;
   la.vs = c->vs;
@@ -656,7 +655,7 @@ int fs_pbf_lambda(fs_context* c, const fs_model* m, const float* x_pred, const f
   la.lam = pbf_lambda;
   la.rho = rho;
   la.count = neighbor_count;
-  k_lambda<<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(la);
+  k_lambda<<<nb_blocks(c, m->n), c->nb_block, scan_smem(c->nb_block), st>>>(la);
   return launch_check("fs_pbf_lambda");
 }
 
@@ -668,7 +667,7 @@ int fs_pbf_delta(fs_context* c, const fs_model* m, const float* x_pred, const fl
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_pbf_delta: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, x_pred, c->xs, c->vs, nullptr,
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, x_pred, c->xs, scan_out(c), c->vs, nullptr,
                                                        c->status, c->nworlds);
   k_gather_lambda_mass<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, pbf_lambda, c->vs, c->krm);
   DeltaArgs da;
@@ -689,6 +688,7 @@ int fs_pbf_delta(fs_context* c, const fs_model* m, const float* x_pred, const fl
   da.walls = Walls{};
   da.delta_p = delta_p;
   da.xs_out = nullptr;
+  da.q = ScanOut{};
   k_delta<<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(da);
   return launch_check("fs_pbf_delta");
 }
@@ -700,7 +700,7 @@ int fs_pbf_xsph(fs_context* c, const fs_model* m, const float* x_pred, const flo
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_pbf_xsph: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, v_in, c->xs, c->vs2, nullptr,
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, v_in, c->xs, scan_out(c), c->vs2, nullptr,
                                                        c->status, c->nworlds);
   k_gather_lambda<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, rho, c->sc1);
   k_rho_ratio<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->sc1, c->vs2, c->sc2);

@@ -17,11 +17,11 @@ namespace fs {
 // with volume = mass / max(rest_density, 1e-6) (compute_particle_volume,
 // solver_wcsph.py:110-116).
 __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
-                                const float* __restrict__ v, float4* __restrict__ xs, float4* __restrict__ vs,
-                                float* __restrict__ mv, uint32_t* status, int nworlds) {
+                                const float* __restrict__ v, float4* __restrict__ xs, ScanOut q,
+                                float4* __restrict__ vs, float* __restrict__ mv, uint32_t* status, int nworlds) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  gather_common_slot(s, perm[s], m, x, v, xs, vs, mv, status, nworlds);
+  gather_common_slot(s, perm[s], m, x, v, xs, q, vs, mv, status, nworlds);
 }
 
 // ------------------------------------------------------------- density ----
@@ -31,6 +31,7 @@ __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_
 struct DensityArgs {
   GridDev g;
   NbrList L;
+  ScanXyz q;
   int64_t n;
   const float4* xs;
   const float* mv;
@@ -45,7 +46,11 @@ struct DensityArgs {
   const fs_frame_clock* clock;  // clocked substep: nothing to do once the frame is complete
 };
 
-__global__ void FS_NB_BOUNDS k_wcsph_density(DensityArgs a) {
+// 64-register budget: at the compiler's own 78 registers (no spills, 28
+// resident warps) a launch at 4,194,304 particles takes 1.44 ms, at 64 1.00,
+// at 48 1.07.  Before the word scan (scan_words) it took 1.63.
+__global__ void __launch_bounds__(kNbBlockMax, 4) k_wcsph_density(DensityArgs a) {
+  extern __shared__ uint2 words[];
   if (clock_idle(a.clock)) return;
   lists_recorded(a.L);
   for_slots(a.n, [&](int64_t s) {
@@ -59,11 +64,10 @@ __global__ void FS_NB_BOUNDS k_wcsph_density(DensityArgs a) {
       return;
     }
     const float h2m = a.h * a.h * kSupportMargin;
-    record_list<false>(a.g, a.xs, (int)s, xi, a.h, h2m, a.L);
     const Cubic K(a.h);
     float acc = 0.f;
-    visit_with<true, true>(a.g, a.xs, (int)s, xi, a.h, h2m, a.L, true, [&](int t) { return __ldg(a.mv + t); },
-                           [&](int t, float4 xj, const float& m) {
+    scan_visit<true>(a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, words, [&](int t) { return __ldg(a.mv + t); },
+                     [&](int t, float4 xj, const float& m) {
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
       float r, rinv;
       r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
@@ -117,7 +121,7 @@ __global__ void FS_NB_BOUNDS k_wcsph_force(ForceArgs a) {
     const Cubic K(a.h);
     float ax = 0.f, ay = 0.f, az = 0.f;
     const bool lists_ok = a.use_lists && lists_usable(a.L);
-    visit<false, false>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
+    visit<false>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
                         [&](int t, float4 xj) {
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -176,7 +180,7 @@ int wcsph_gather(fs_context* c, const fs_model* m, const float* x, const float* 
   const int64_t n = m->n;
   {
     PassScope ps_(c, P_GATHER, st);
-    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, c->vs, c->mv, c->status, c->nworlds);
+    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs, c->mv, c->status, c->nworlds);
   }
   return launch_check("wcsph gather");
 }
@@ -187,6 +191,7 @@ int launch_density(fs_context* c, const fs_model* m, float h, int clamp, bool eo
   a.clock = clock;
   a.g = grid_view(c);
   a.L = nbr_list(c);
+  a.q = scan_xyz(c);
   a.n = m->n;
   a.xs = c->xs;
   a.mv = c->mv;
@@ -200,7 +205,7 @@ int launch_density(fs_context* c, const fs_model* m, float h, int clamp, bool eo
   a.sc2 = c->sc2;
   {
     PassScope ps_(c, P_WCSPH_DENSITY, st);
-    k_wcsph_density<<<nb_blocks(c, a.n), c->nb_block, 0, st>>>(a);
+    k_wcsph_density<<<nb_blocks(c, a.n), c->nb_block, scan_smem(c->nb_block), st>>>(a);
   }
   return launch_check("wcsph density");
 }
@@ -301,7 +306,7 @@ int fs_wcsph_density(fs_context* c, const fs_model* m, const float* x, float h, 
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_wcsph_density: build the grid for these points first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, nullptr, c->xs, nullptr, c->mv,
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, nullptr, c->xs, scan_out(c), nullptr, c->mv,
                                                        c->status, c->nworlds);
   return launch_density(c, m, h, clamp_negative, true, rho, pressure, st);
 }

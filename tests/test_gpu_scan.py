@@ -1,0 +1,75 @@
+"""The grid scan at the edges of its tiles: groups of four slots, pieces of 32
+candidates, 12 pieces between two visits, lists of 192 entries; inactive
+candidates, rows that wrap, dims that are no power of two.
+
+Densities against a float64 sum over all pairs: k positive FP32 terms, each a
+few ulp off, summed one after the other, are within (k + 16) 2^-23 of it
+(relative).  DFSPH's neighbour counts (candidates, no distance test) equal the
+oracle's candidate lists."""
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from fluid_simulation_b200.newton_shim import HashGrid, model_from_arrays
+from fluid_simulation_b200.solver import SolverDFSPH, SolverWCSPH
+
+pytestmark = pytest.mark.gpu
+SP = 0.01
+H = 2 * SP
+
+
+def cloud(n, centre, seed):
+    """n points around `centre`, half of them within one cell, the others over 5 h."""
+    rng = np.random.default_rng(seed)
+    near = rng.uniform(0.0, 1.0, (n - n // 2, 3)) * H
+    wide = rng.uniform(-2.5, 2.5, (n // 2, 3)) * H
+    x = np.concatenate([near, wide]) + np.asarray(centre)
+    return x.astype(np.float32)[rng.permutation(n)]
+
+
+def step(cls, x, flags, dims, dev, dt):
+    n = len(x)
+    attrs = dict(particle_mask=0, rest_density=1000.0, surface_tension=0.0, viscosity=0.0)
+    if cls is SolverWCSPH:
+        attrs.update(stiffness=1.0, exponent=1.0)
+    m = model_from_arrays(x, np.zeros_like(x), 1000.0 * SP ** 3, device=dev, flags=flags, radius=0.5 * SP,
+                          attributes=attrs, solver_cls=cls)
+    m.particle_grid = HashGrid(*dims, device=dev)
+    m.particle_grid.reserve(n)
+    solver = cls(m, cls.SphConfig(particle_radius=0.5 * SP, particle_length=SP, smoothing_length_coff=2.0,
+                                  bound_width=1e4, bound_height=1e4, bound_length=1e4))
+    a, b = m.state(), m.state()
+    solver.step(a, b, None, None, dt)
+    torch.cuda.synchronize()
+    return b
+
+
+def density64(x, active):
+    d = np.linalg.norm(x[:, None].astype(np.float64) - x[None].astype(np.float64), axis=2) / np.float64(np.float32(H))
+    k = 8.0 / (np.pi * H ** 3)
+    w = np.where(d <= 0.5, k * (6 * d ** 3 - 6 * d ** 2 + 1), 2 * k * np.clip(1 - d, 0, None) ** 3)
+    w = np.where((d <= 1.0) & active[None], w, 0.0)
+    return np.where(active, 1000.0 * SP ** 3 * w.sum(1), 0.0), int((w > 0).sum(1).max())
+
+
+@pytest.mark.parametrize("dims", [(128, 128, 128), (7, 5, 3)])
+@pytest.mark.parametrize("centre", [(0.31, 0.27, 0.2), (0.0, 0.0, 0.0)])
+@pytest.mark.parametrize("n", [2, 3, 5, 31, 64, 65, 129, 500, 2000])
+def test_scan_edges(n, centre, dims, cuda_device):
+    x = cloud(n, centre, n)
+    flags = np.ones(n, np.int32)
+    flags[::7] = 0
+    if n < 7:
+        flags[:] = 1
+    active = flags == 1
+    want, hits = density64(x, active)
+    got = step(SolverWCSPH, x, flags, dims, cuda_device, 1e-9).sph.rho.cpu().numpy()
+    err = np.abs(got - want).max() / max(want.max(), 1e-30)
+    assert err <= (hits + 16) * 2.0 ** -23, (err, hits)
+    off, cand = oracle.grid_candidates(x, np.float32(H), dims=dims)
+    count = np.array([np.count_nonzero(active[c] & (c != i)) for i, c in
+                      enumerate(np.split(np.asarray(cand), np.asarray(off)[1:-1]))])
+    got = step(SolverDFSPH, x, flags, dims, cuda_device, 1e-9).sph.neighbor_count.cpu().numpy()
+    assert np.array_equal(got, np.where(active, count, 0))
