@@ -181,63 +181,75 @@ FS_DEV PairAdj pair_adjoint(const Cubic& K, float h, float particle_radius, floa
   return o;
 }
 
+// G lanes per particle add up their own pairs' terms, then the lanes' sums
+// (the adjoint's sums have no order to keep).
+template <int G>
 __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
-  extern __shared__ uint2 words[];
+  extern __shared__ uint2 smem[];
   lists_recorded(a.L);
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xk = a.xs[s];
     const int32_t i = a.g.perm[s];
     const int pfk = pf_of(xk);
-    if (!(pfk & PF_ACTIVE)) {  // untouched by the step: identity
-      a.L.cnt[s] = 0;
-      a.xr[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-      st3(a.xbi, i, ld3(a.xbo, i));
-      st3(a.vbi, i, ld3(a.vbo, i));
-      return;
-    }
+    const bool on = live && (pfk & PF_ACTIVE);
     const float4 vk = a.vs[s];
     const float m_k = vk.w;
     const float2 PRk = a.sc2[s];
     const float nu_k = a.nu[s], coh_k = a.coh[s];
     float3 xb = make_float3(0.f, 0.f, 0.f), vb = make_float3(0.f, 0.f, 0.f), abk = make_float3(0.f, 0.f, 0.f);
-    if (pfk & PF_DYNAMIC) {
+    if (pfk & PF_DYNAMIC)
       integrate_adjoint(walls_of(a.walls, a.g, world_of(xk)), xyz(xk), xyz(vk), ld3(a.accel, i), a.dt, ld3(a.xbo, i),
                         ld3(a.vbo, i), xb, vb, abk);
-    } else {
-      xb = ld3(a.xbo, i);
-      vb = ld3(a.vbo, i);
-    }
+    else
+      xb = ld3(a.xbo, i), vb = ld3(a.vbo, i);
+    if (!lead) xb = vb = make_float3(0.f, 0.f, 0.f);  // the lead lane's sums start at the direct terms
     const Cubic K(a.h);
     const float h2m = a.h * a.h * kSupportMargin;
     float Pb = 0.f, Rb = 0.f, nub = 0.f;
-    scan_visit<false>(a.g, a.q, a.xs, (int)s, xk, a.h, h2m, h2m, a.L, words, [](int) { return 0; },
-                      [&](int t, float4 xj, int) {
-      const float3 d = make_float3(xk.x - xj.x, xk.y - xj.y, xk.z - xj.z);
-      const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-      if (r2 == 0.f) return;  // the forward skips coincident pairs
-      const float4 vj = __ldg(a.vs + t);
-      const float2 PRj = __ldg(a.sc2 + t);
-      const float3 u = make_float3(vk.x - vj.x, vk.y - vj.y, vk.z - vj.z);
-      const float Psum = PRk.x + PRj.x;
-      if (pfk & PF_DYNAMIC) {  // term of a_k with neighbour j
-        const PairAdj o = pair_adjoint(K, a.h, a.particle_radius, d, r2, u, abk, nu_k, coh_k, vj.w, PRj.y, Psum);
-        xb = make_float3(xb.x + o.rb.x, xb.y + o.rb.y, xb.z + o.rb.z);
-        vb = make_float3(vb.x + o.ub.x, vb.y + o.ub.y, vb.z + o.ub.z);
-        Pb += o.pb_sum;
-        nub += o.nub;
-      }
-      if (pf_of(xj) & PF_DYNAMIC) {  // term of a_j with neighbour k: d_jk = -d, u_jk = -u
-        const float4 abj4 = __ldg(a.ab + t);
-        const float3 abj = make_float3(abj4.x, abj4.y, abj4.z);
-        const float3 dn = make_float3(-d.x, -d.y, -d.z), un = make_float3(-u.x, -u.y, -u.z);
-        const PairAdj o = pair_adjoint(K, a.h, a.particle_radius, dn, r2, un, abj, __ldg(a.nu + t), __ldg(a.coh + t),
-                                       m_k, PRk.y, Psum);
-        xb = make_float3(xb.x - o.rb.x, xb.y - o.rb.y, xb.z - o.rb.z);
-        vb = make_float3(vb.x - o.ub.x, vb.y - o.ub.y, vb.z - o.ub.z);
-        Pb += o.pb_sum;
-        Rb += o.rb_j;
-      }
-    });
+    scan_sum<G, false, false, false, 0>(
+        a.g, a.q, a.xs, (int)s, xk, a.h, h2m, h2m, a.L, smem, on, -1, [](int) { return 0; },
+        [&](int t, float4 xj, int) {
+          const float3 d = make_float3(xk.x - xj.x, xk.y - xj.y, xk.z - xj.z);
+          const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
+          if (r2 == 0.f) return Terms<0>{};  // the forward skips coincident pairs
+          const float4 vj = __ldg(a.vs + t);
+          const float2 PRj = __ldg(a.sc2 + t);
+          const float3 u = make_float3(vk.x - vj.x, vk.y - vj.y, vk.z - vj.z);
+          const float Psum = PRk.x + PRj.x;
+          if (pfk & PF_DYNAMIC) {  // term of a_k with neighbour j
+            const PairAdj o = pair_adjoint(K, a.h, a.particle_radius, d, r2, u, abk, nu_k, coh_k, vj.w, PRj.y, Psum);
+            xb = make_float3(xb.x + o.rb.x, xb.y + o.rb.y, xb.z + o.rb.z);
+            vb = make_float3(vb.x + o.ub.x, vb.y + o.ub.y, vb.z + o.ub.z);
+            Pb += o.pb_sum;
+            nub += o.nub;
+          }
+          if (pf_of(xj) & PF_DYNAMIC) {  // term of a_j with neighbour k: d_jk = -d, u_jk = -u
+            const float4 abj4 = __ldg(a.ab + t);
+            const float3 abj = make_float3(abj4.x, abj4.y, abj4.z);
+            const float3 dn = make_float3(-d.x, -d.y, -d.z), un = make_float3(-u.x, -u.y, -u.z);
+            const PairAdj o = pair_adjoint(K, a.h, a.particle_radius, dn, r2, un, abj, __ldg(a.nu + t),
+                                           __ldg(a.coh + t), m_k, PRk.y, Psum);
+            xb = make_float3(xb.x - o.rb.x, xb.y - o.rb.y, xb.z - o.rb.z);
+            vb = make_float3(vb.x - o.ub.x, vb.y - o.ub.y, vb.z - o.ub.z);
+            Pb += o.pb_sum;
+            Rb += o.rb_j;
+          }
+          return Terms<0>{};
+        },
+        [](const Terms<0>&) {});
+    if constexpr (G > 1) {
+      xb = make_float3(group_sum<G>(xb.x), group_sum<G>(xb.y), group_sum<G>(xb.z));
+      vb = make_float3(group_sum<G>(vb.x), group_sum<G>(vb.y), group_sum<G>(vb.z));
+      Pb = group_sum<G>(Pb), Rb = group_sum<G>(Rb), nub = group_sum<G>(nub);
+    }
+    if (!lead) return;
+    if (!on) {  // untouched by the step: identity
+      a.L.cnt[s] = 0;
+      a.xr[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+      st3(a.xbi, i, xb);
+      st3(a.vbi, i, vb);
+      return;
+    }
     // P = p / max(rho^2, 1e-6), R = 1 / max(rho, 1e-6), then the EOS
     const float rho = a.rho[i], p = a.pressure[i];
     const float rr = rho * rho;
@@ -265,27 +277,32 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
   });
 }
 
+template <int G>
 __global__ void FS_NB_BOUNDS k_adj_density(AdjArgs a) {
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xk = a.xs[s];
-    if (!(pf_of(xk) & PF_ACTIVE)) return;  // written by the force pass
+    const bool on = live && (pf_of(xk) & PF_ACTIVE);
     const int32_t i = a.g.perm[s];
     const float4 xr = a.xr[s];
     const float mv_k = a.mv[s];
     const Cubic K(a.h);
-    float3 xb = make_float3(xr.x, xr.y, xr.z);
-    const bool lists_ok = lists_usable(a.L);
-    visit<false>(a.g, a.xs, (int)s, xk, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok, [&](int t, float4 xj) {
-      const float dx = xk.x - xj.x, dy = xk.y - xj.y, dz = xk.z - xj.z;
-      float r, rinv;
-      r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
-      const float w = (xr.w * __ldg(a.mv + t) + __ldg(&a.xr[t].w) * mv_k) * K.grad_scale(r, rinv);
-      xb = make_float3(fmaf(w, dx, xb.x), fmaf(w, dy, xb.y), fmaf(w, dz, xb.z));
-    });
-    st3(a.xbi, i, xb);
+    float3 xb = lead ? make_float3(xr.x, xr.y, xr.z) : make_float3(0.f, 0.f, 0.f);
+    list_sum<G, false, false, true, 0>(
+        a.g, a.xs, (int)s, xk, a.h, a.h * a.h * kSupportMargin, a.L, lists_usable(a.L), on,
+        [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.xr[t].w)); },
+        [&](int t, float4 xj, const float2& j) {
+          const float dx = xk.x - xj.x, dy = xk.y - xj.y, dz = xk.z - xj.z;
+          float r, rinv;
+          r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
+          const float w = (xr.w * j.x + j.y * mv_k) * K.grad_scale(r, rinv);
+          xb = make_float3(fmaf(w, dx, xb.x), fmaf(w, dy, xb.y), fmaf(w, dz, xb.z));
+          return Terms<0>{};
+        },
+        [](const Terms<0>&) {});
+    if constexpr (G > 1) xb = make_float3(group_sum<G>(xb.x), group_sum<G>(xb.y), group_sum<G>(xb.z));
+    if (lead && on) st3(a.xbi, i, xb);  // inactive: written by the force pass
   });
 }
-
 
 }  // namespace
 }  // namespace fs
@@ -350,11 +367,11 @@ int fs_wcsph_substep_adjoint(fs_context* c, const fs_model* m, const fs_state* s
   }
   {
     PassScope ps_(c, P_ADJ_FORCE, st);
-    k_adj_force<<<nb_blocks(c, n), c->nb_block, scan_smem(c->nb_block), st>>>(a);
+    FS_NB_LAUNCH(k_adj_force, c, n, nb_group(n), st, true, a);
   }
   {
     PassScope ps_(c, P_ADJ_DENSITY, st);
-    k_adj_density<<<nb_blocks(c, n), c->nb_block, 0, st>>>(a);
+    FS_NB_LAUNCH(k_adj_density, c, n, nb_group(n), st, false, a);
   }
   c->last_stream = st;
   return launch_check("fs_wcsph_substep_adjoint");

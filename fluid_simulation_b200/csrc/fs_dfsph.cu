@@ -25,9 +25,9 @@
 namespace fs {
 
 // Partial-sum slots for the residual reductions: one per block of the
-// smallest block size that launches them (the 64-thread floor leaves room for
-// any block size used here).
-int reduction_blocks(int64_t n) { return blocks_for(n > 0 ? n : 1, 64); }
+// smallest block size that launches them (64 threads, up to 32 lanes a
+// particle: two particles a block).
+int reduction_blocks(int64_t n) { return blocks_for(n > 0 ? n : 1, 2); }
 
 // gather of fs_wcsph.cu reused here
 __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
@@ -85,14 +85,38 @@ struct DensFactorArgs {
 // 85-register budget: the scan and the visit need 72 without spills; with 64
 // (36 bytes of spills) a launch at 401,856 particles takes 0.126 ms, with 72
 // 0.121 (the per-candidate list recorder before took 0.158).
+template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, 3) k_density_factor(DensFactorArgs a) {
-  extern __shared__ uint2 words[];
+  extern __shared__ uint2 smem[];
   if (clock_idle(a.clock)) return;
   lists_recorded(a.L);
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
-    if (!(pf_of(xi) & PF_ACTIVE)) {
+    const bool on = live && (pf_of(xi) & PF_ACTIVE);
+    const float h2m = a.h * a.h * kSupportMargin;
+    const Cubic K(a.h);
+    float rho = 0.f, sgx = 0.f, sgy = 0.f, sgz = 0.f, sq = 0.f;
+    // the candidate count (no distance test, solver_dfsph.py:163-164) comes from the scan
+    const int cnt = scan_sum<G, true, true, false, 5>(
+        a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, -1,
+        [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.vs[t].w)); },
+        [&](int t, float4 xj, const float2& mm) {  // (rest_density * volume, mass)
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          float r, rinv;
+          r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
+          const float gsc = mm.y * K.grad_scale(r, rinv);
+          return Terms<5>{mm.x, K.w(r), gsc * dx, gsc * dy, gsc * dz};
+        },
+        [&](const Terms<5>& u) {
+          rho = fmaf(u.v[0], u.v[1], rho);
+          sgx = __fadd_rn(sgx, u.v[2]);  // sums of the rounded gradients (no contraction), whatever surrounds them
+          sgy = __fadd_rn(sgy, u.v[3]);
+          sgz = __fadd_rn(sgz, u.v[4]);
+          sq = fmaf(u.v[2], u.v[2], fmaf(u.v[3], u.v[3], fmaf(u.v[4], u.v[4], sq)));
+        });
+    if (!lead) return;
+    if (!on) {
       a.rho[i] = 0.f;
       a.factor[i] = 0.f;
       a.count[i] = 0;
@@ -100,25 +124,7 @@ __global__ void __launch_bounds__(kNbBlockMax, 3) k_density_factor(DensFactorArg
       a.L.cnt[s] = 0;
       return;
     }
-    const float h2m = a.h * a.h * kSupportMargin;
-    const Cubic K(a.h);
-    float rho = 0.f, sgx = 0.f, sgy = 0.f, sgz = 0.f, sq = 0.f;
-    // the candidate count (no distance test, solver_dfsph.py:163-164) comes from the scan
-    const int cnt = scan_visit<true, true>(a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, words,
-                                           [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.vs[t].w)); },
-                                           [&](int t, float4 xj, const float2& mm) {  // (rest_density * volume, mass)
-      const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      float r, rinv;
-      r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
-      rho = fmaf(mm.x, K.w(r), rho);
-      const float gsc = mm.y * K.grad_scale(r, rinv);
-      const float gx = gsc * dx, gy = gsc * dy, gz = gsc * dz;
-      sgx = __fadd_rn(sgx, gx);  // the sums stay sums (no contraction), whatever surrounds them
-      sgy = __fadd_rn(sgy, gy);
-      sgz = __fadd_rn(sgz, gz);
-      sq = fmaf(gx, gx, fmaf(gy, gy, fmaf(gz, gz, sq)));
-    });
-    const float denom = (sgx * sgx + sgy * sgy + sgz * sgz) + sq;
+    const float denom = __fadd_rn(norm2(sgx, sgy, sgz), sq);
     const float f = (cnt < a.min_nb || denom < 1.0e-6f) ? 0.f : 1.0f / denom;
     a.rho[i] = rho;
     a.factor[i] = f;
@@ -143,41 +149,49 @@ struct AccelArgs {
   const fs_frame_clock* clock;
 };
 
+template <int G>
 __global__ void FS_NB_BOUNDS k_accel_predict(AccelArgs a) {
   if (clock_idle(a.clock)) return;
   const float dt = a.clock ? a.clock->dt : a.dt;
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const float4 vi = a.vs[s];
     const int32_t i = a.g.perm[s];
-    if (!(pf_of(xi) & PF_DYNAMIC)) {
-      st3(a.accel, i, make_float3(0.f, 0.f, 0.f));
-      a.vstar[s] = make_float4(0.f, 0.f, 0.f, vi.w);
-      return;
-    }
+    const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const float mu10 = 10.f * a.m.viscosity[i];
     const float coh = a.m.surface_tension[i] / vi.w;
     const float visc_den_add = 0.01f * (a.h * a.h);
     const Cubic K(a.h);
     float ax = 0.f, ay = 0.f, az = 0.f;
-    const bool lists_ok = a.use_lists && lists_usable(a.L);
-    visit<false>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
-                        [&](int t, float4 xj) {
-      const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      if (r2 == 0.f) return;  // zero vector d: every term vanishes
-      const float4 vj = __ldg(a.vs + t);
-      const float rho_j = __ldg(&a.sc2[t].x);
-      float r, rinv;
-      r_and_inv(r2, r, rinv);
-      const float wc = coh * vj.w * K.w(fmaxf(r, a.particle_radius));
-      const float vdot = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
-      const float visc = mu10 * __fdividef(vj.w, fmaxf(rho_j, 1.0e-6f)) * __fdividef(vdot, r2 + visc_den_add);
-      const float c = fmaf(visc, K.grad_scale(r, rinv), -wc);
-      ax = fmaf(c, dx, ax);
-      ay = fmaf(c, dy, ay);
-      az = fmaf(c, dz, az);
-    });
+    struct Neighbour {
+      float4 v;
+      float rho;
+    };
+    list_sum<G, false, false, true, 4>(
+        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), live && dyn,
+        [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(&a.sc2[t].x)}; },
+        [&](int t, float4 xj, const Neighbour& j) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          if (r2 == 0.f) return Terms<4>{};  // zero vector d: every term vanishes
+          float r, rinv;
+          r_and_inv(r2, r, rinv);
+          const float wc = coh * j.v.w * K.w(fmaxf(r, a.particle_radius));
+          const float vdot = fmaf(vi.x - j.v.x, dx, fmaf(vi.y - j.v.y, dy, (vi.z - j.v.z) * dz));
+          const float visc = mu10 * __fdividef(j.v.w, fmaxf(j.rho, 1.0e-6f)) * __fdividef(vdot, r2 + visc_den_add);
+          return Terms<4>{fmaf(visc, K.grad_scale(r, rinv), -wc), dx, dy, dz};
+        },
+        [&](const Terms<4>& u) {
+          ax = fmaf(u.v[0], u.v[1], ax);
+          ay = fmaf(u.v[0], u.v[2], ay);
+          az = fmaf(u.v[0], u.v[3], az);
+        });
+    if (!lead) return;
+    if (!dyn) {
+      st3(a.accel, i, make_float3(0.f, 0.f, 0.f));
+      a.vstar[s] = make_float4(0.f, 0.f, 0.f, vi.w);
+      return;
+    }
     const float3 g = gravity_of(a.m, i);
     const float3 acc = make_float3(ax + g.x, ay + g.y, az + g.z);
     st3(a.accel, i, acc);
@@ -306,31 +320,34 @@ __device__ bool last_block(uint32_t* ticket) {
   return am_last;
 }
 
+template <int G>
 __global__ void FS_NB_BOUNDS k_rate(RateArgs a) {
   if (a.ctrl && a.ctrl->done) return;  // uniform across the grid: set by an earlier launch
   if (clock_idle(a.clock)) return;     // uniform: the frame is complete
   const float dt = a.clock ? a.clock->dt : a.dt;
   double term = 0.0;  // this thread's residual terms and dynamic particles
   long long dyn = 0;
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
-    if (world_finished(a.wctl, a.pworld, a.nworlds, i)) return;
+    const bool over = world_finished(a.wctl, a.pworld, a.nworlds, i);
+    if (G == 1 && over) return;
     const int pf = pf_of(xi);
     float d = 0.f;
-    if (pf & PF_ACTIVE) {
-      const float4 vi = a.vstar[s];
-      const Cubic K(a.h);
-      const bool lists_ok = a.use_lists && lists_usable(a.L);
-      visit_with<false>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
-                        [&](int t) { return __ldg(a.vstar + t); }, [&](int t, float4 xj, const float4& vj) {
-        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        float r, rinv;
-        r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
-        const float vdot = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
-        d = fmaf(vj.w * K.grad_scale(r, rinv), vdot, d);
-      });
-    }
+    const float4 vi = a.vstar[s];
+    const Cubic K(a.h);
+    list_sum<G, false, false, false, 2>(
+        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        live && !over && (pf & PF_ACTIVE), [&](int t) { return __ldg(a.vstar + t); },
+        [&](int t, float4 xj, const float4& vj) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          float r, rinv;
+          r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
+          const float vdot = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
+          return Terms<2>{vj.w * K.grad_scale(r, rinv), vdot};
+        },
+        [&](const Terms<2>& u) { d = fmaf(u.v[0], u.v[1], d); });
+    if (!lead || over) return;
     a.d_rho_dt[i] = d;
     const float2 rf = a.sc2[s];
     const bool is_dyn = (pf & PF_DYNAMIC) != 0;
@@ -447,31 +464,38 @@ struct CorrectArgs {
 
 // Four resident 256-thread blocks per SM: a 64-register budget (the compiler
 // otherwise settles at 48 registers and spills; 3.7 % faster measured).
+template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, 4) k_correct(CorrectArgs a) {
   if (a.ctrl && a.ctrl->done) return;
   if (clock_idle(a.clock)) return;
   const float dt = a.clock ? a.clock->dt : a.dt;
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
-    if (world_finished(a.wctl, a.pworld, a.nworlds, i)) return;
-    if (a.kappa_api) a.kappa_api[i] = a.kappa[s];
+    const bool over = world_finished(a.wctl, a.pworld, a.nworlds, i);
+    if (G == 1 && over) return;
     float4 v = a.vstar[s];
-    if (pf_of(xi) & PF_DYNAMIC) {
-      const Cubic K(a.h);
-      const float ci = a.kratio[s].x;
-      float dvx = 0.f, dvy = 0.f, dvz = 0.f;
-      const bool lists_ok = a.use_lists && lists_usable(a.L);
-      visit_with<false>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
-                        [&](int t) { return __ldg(a.kratio + t); }, [&](int t, float4 xj, const float2& kj) {
-        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        float r, rinv;
-        r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
-        const float c = kj.y * (ci + kj.x) * K.grad_scale(r, rinv);
-        dvx = fmaf(c, dx, dvx);
-        dvy = fmaf(c, dy, dvy);
-        dvz = fmaf(c, dz, dvz);
-      });
+    const bool dyn = pf_of(xi) & PF_DYNAMIC;
+    const Cubic K(a.h);
+    const float ci = a.kratio[s].x;
+    float dvx = 0.f, dvy = 0.f, dvz = 0.f;
+    list_sum<G, false, false, false, 4>(
+        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        live && !over && dyn, [&](int t) { return __ldg(a.kratio + t); },
+        [&](int t, float4 xj, const float2& kj) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          float r, rinv;
+          r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
+          return Terms<4>{kj.y * (ci + kj.x) * K.grad_scale(r, rinv), dx, dy, dz};
+        },
+        [&](const Terms<4>& u) {
+          dvx = fmaf(u.v[0], u.v[1], dvx);
+          dvy = fmaf(u.v[0], u.v[2], dvy);
+          dvz = fmaf(u.v[0], u.v[3], dvz);
+        });
+    if (!lead || over) return;
+    if (a.kappa_api) a.kappa_api[i] = a.kappa[s];
+    if (dyn) {
       v.x = v.x - dt * dvx;
       v.y = v.y - dt * dvy;
       v.z = v.z - dt * dvz;
@@ -570,11 +594,12 @@ int run_rate(fs_context* c, const fs_model* m, int mode, int it, float h, float 
   a.nworlds = c->nworlds;
   a.term = per_world ? c->sc1b : nullptr;
   if (per_world && !m->particle_world) return set_error(FS_ERR_INVALID, "dfsph rate: a batched context needs particle_world");
-  if (ctrl && !per_world && nb_blocks(c, a.n) > reduction_blocks(c->capacity))
+  const int group = use_lists ? nb_group(a.n) : 1;  // no list: each thread rescans
+  if (ctrl && !per_world && nb_blocks(c, a.n * group) > reduction_blocks(c->capacity))
     return set_error(FS_ERR_INVALID, "dfsph rate: reduction buffer too small");
   {
     PassScope ps_(c, P_DFSPH_RATE, st, per_world ? 2 : 1);
-    k_rate<<<nb_blocks(c, a.n), c->nb_block, 0, st>>>(a);
+    FS_NB_LAUNCH(k_rate, c, a.n, group, st, false, a);
     if (per_world)
       k_world_residual<<<c->nworlds, kWorldBlock, 0, st>>>(a.g, c->sc1b, c->dfsph_worlds + (ctrl - c->dfsph) * c->nworlds,
                                                            ctrl, it, eta, c->clock);
@@ -605,7 +630,7 @@ int run_correct(fs_context* c, const fs_model* m, float h, float dt, const float
   a.nworlds = c->nworlds;
   {
     PassScope ps_(c, P_DFSPH_CORRECT, st);
-    k_correct<<<nb_blocks(c, a.n), c->nb_block, 0, st>>>(a);
+    FS_NB_LAUNCH(k_correct, c, a.n, use_lists ? nb_group(a.n) : 1, st, false, a);
   }
   return launch_check("dfsph correct");
 }
@@ -629,7 +654,7 @@ int run_density_factor(fs_context* c, const fs_model* m, float h, int min_nb, fl
   a.sc2 = c->sc2;
   {
     PassScope ps_(c, P_DFSPH_DENSITY_FACTOR, st);
-    k_density_factor<<<nb_blocks(c, a.n), c->nb_block, scan_smem(c->nb_block), st>>>(a);
+    FS_NB_LAUNCH(k_density_factor, c, a.n, nb_group(a.n), st, true, a);
   }
   return launch_check("dfsph density/factor");
 }
@@ -759,7 +784,7 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
   aa.clock = c->clock;
   {
     PassScope ps_(c, P_DFSPH_ACCEL, st);
-    k_accel_predict<<<nb_blocks(c, n), c->nb_block, 0, st>>>(aa);
+    FS_NB_LAUNCH(k_accel_predict, c, n, nb_group(n), st, false, aa);
   }
   if ((rc = launch_check("dfsph accel"))) return rc;
   if (p->warm_start) {
@@ -916,7 +941,7 @@ int fs_dfsph_nonpressure_predict(fs_context* c, const fs_model* m, const float* 
   aa.accel = accel;
   aa.vstar = c->vs2;
   aa.clock = nullptr;
-  k_accel_predict<<<nb_blocks(c, n), c->nb_block, 0, st>>>(aa);
+  k_accel_predict<1><<<nb_blocks(c, n), c->nb_block, 0, st>>>(aa);
   k_scatter_xyz<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, c->vs2, v_star);
   return launch_check("fs_dfsph_nonpressure_predict");
 }

@@ -271,6 +271,21 @@ NbrList nbr_list(const fs_context* c) {
   return L;
 }
 
+// Lanes per particle: as many as fill the GPU (148 SMs hold 151,552 threads of
+// these kernels), fewer where the sums, which every lane of a group repeats,
+// outweigh the shorter chain.  Substep times in us, B200:
+//   particles        4,000   8,000   15,000   28,000   38,000   50,000
+//   PBF    1 lane      276     276      287      308      334      306
+//          4 lanes     209     222      231      288      329      406
+//          8 lanes     164     180      207      303      354      430
+//         16 lanes     151     179      250      362      452      552
+//   DFSPH  1 lane      644     662      660      726      728      749
+//          4 lanes     430     453      487      579      655      807
+//          8 lanes     400     409      489      697      814      953
+//         16 lanes     393     481      614      915    1,091    1,345
+// (WCSPH and its adjoint cross over at the same sizes.)
+int nb_group(int64_t n) { return n <= 5000 ? 16 : n <= 14000 ? 8 : n <= 36000 ? 4 : 1; }
+
 ScanXyz scan_xyz(const fs_context* c) { return ScanXyz{c->sxyz}; }
 ScanOut scan_out(const fs_context* c) {
   return ScanOut{c->sxyz, &((ListCtl*)c->nb_ctl)->inactive};

@@ -582,6 +582,10 @@ FS_DEV void st3(float* p, int64_t i, float3 v) {
   p[3 * i + 1] = v.y;
   p[3 * i + 2] = v.z;
 }
+// x^2 + y^2 + z^2 in one fixed order of fused operations, whatever surrounds it.
+FS_DEV float norm2(float x, float y, float z) {
+  return fmaf(z, z, fmaf(x, x, y * y));
+}
 FS_DEV float3 xyz(float4 a) { return make_float3(a.x, a.y, a.z); }
 
 FS_DEV int particle_pf(const int32_t* flags, const int32_t* mask, int64_t i) {

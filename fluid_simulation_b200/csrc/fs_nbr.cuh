@@ -166,9 +166,6 @@ FS_DEV f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   return r;
 }
 
-// Shared memory of a recording launch: words of thread t at smem[w * threads + t].
-inline size_t scan_smem(int threads) { return sizeof(uint2) * kWords * (size_t)threads; }
-
 // Where a particle's scan stands: the next row (z, y), segment j of the row,
 // and the next candidate t of that segment (negative: its first).
 struct ScanPos {
@@ -495,6 +492,274 @@ FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, int s, f
     scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4 xj) { pair(t, xj, load(t)); });
   }
 }
+
+// ------------------------------------------------------ lanes in a group --
+// A small scene leaves most of the GPU idle with one thread per particle, and
+// each thread then walks its candidates and neighbours alone, one memory
+// latency after the other: at 4,079 particles a lambda pass took 28 us with
+// 128 warps for 148 SMs.  G lanes (4, 8 or 16) share a
+// particle instead: each scans every G-th group of four candidates, the hits
+// are compacted in visiting order, each lane evaluates every G-th pair term,
+// and the terms are then added up in visiting order by broadcasting them one
+// after the other, so every sum has the bits of the one-thread form (a lane
+// without a term broadcasts zeros, which change no sum).  What bounds a pass
+// at these sizes is the chain of dependent steps of one warp (load, scan,
+// compact, gather, add up).  nb_group() holds the rule for G.
+//
+// With G > 1 a particle's list is a row (entry k of slot s at
+// idx[s * kNbMax + k], read by its lanes side by side) instead of a column.
+// Every kernel of a context and particle count takes the same G.
+constexpr int kGroupList = 128;  // hits of a particle held in shared memory between two visits
+
+// Shared memory of a recording launch: one thread per particle keeps kWords
+// words at stride `threads`, a group its words and kGroupList hits.
+inline size_t scan_smem(int threads, int group) {
+  const size_t words = sizeof(uint2) * kWords;
+  return group == 1 ? words * threads : (words + sizeof(int32_t) * kGroupList) * (threads / group);
+}
+
+// K floats a pair contributes; the zero value changes no sum.  K = 0: the
+// term adds itself to its lane's own sums, which the caller adds up
+// afterwards (sums without a prescribed order).
+template <int K>
+struct Terms {
+  float v[K] = {};
+};
+template <>
+struct Terms<0> {};
+
+template <int G, int K>
+FS_DEV Terms<K> group_bcast(const Terms<K>& u, int j) {
+  Terms<K> o;
+#pragma unroll
+  for (int k = 0; k < K; ++k) o.v[k] = __shfl_sync(0xffffffffu, u.v[k], j, G);
+  return o;
+}
+
+template <int G, class V>
+FS_DEV V group_sum(V v) {
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, G);
+  return v;
+}
+
+// acc(term) in order for the n entries of the group's particle (n is the same
+// in all its lanes; 0: nothing), entry(k) being the k-th slot.  All lanes of
+// the warp call it together.
+template <int G, bool WITH_SELF, int K, class Entry, class Load, class Term, class Acc>
+FS_DEV void group_visit(const float4* __restrict__ xs, int s, float4 xi, float h2m, int n, Entry&& entry, Load&& load,
+                        Term&& term, Acc&& acc) {
+  const int lane = threadIdx.x & (G - 1);
+  const int nmax = __reduce_max_sync(0xffffffffu, n);
+  // the gathers of the next round are issued before this round's sums
+  int t = lane < n ? entry(lane) : s;
+  float4 xj = __ldg(xs + t);
+  auto p = load(t);
+  for (int k0 = 0; k0 < nmax; k0 += G) {
+    const bool mine = k0 + lane < n;
+    const int t0 = t;
+    const float4 x0 = xj;
+    const auto p0 = p;
+    if (k0 + G + lane < n) {
+      t = entry(k0 + G + lane);
+      xj = __ldg(xs + t);
+      p = load(t);
+    }
+    Terms<K> u;
+    if (mine) {
+      const float dx = xi.x - x0.x, dy = xi.y - x0.y, dz = xi.z - x0.z;
+      if (fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, x0.w))) <= h2m && (WITH_SELF || t0 != s)) u = term(t0, x0, p0);
+    }
+    if constexpr (K > 0) {
+      const int lim = min(G, nmax - k0);
+      for (int j = 0; j < lim; j += 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc(group_bcast<G>(u, j + i));
+      }
+    }
+  }
+}
+
+// scan_visit by the G lanes of a group (`on` and `reuse` are the same in all
+// of them; `on` = false: the particle takes no part).  All lanes of the warp
+// call it together.
+template <int G, bool WITH_SELF, bool COUNT, bool REUSE, int K, class Load, class Term, class Acc>
+FS_DEV int group_scan(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
+                      float h2rec, float h2m, const NbrList& L, void* smem, bool on, int reuse, Load&& load,
+                      Term&& term, Acc&& acc) {
+  constexpr int kIt = kWords * 8 / G;      // groups of four candidates per lane between two visits
+  constexpr int kPk = (kIt + 3) / 4;       // their hit counts, a byte each
+  const int lane = threadIdx.x & (G - 1), grp = threadIdx.x / G;
+  uint2* const words = (uint2*)smem + grp * kWords;
+  int32_t* const list = (int32_t*)((uint2*)smem + (blockDim.x / G) * kWords) + grp * kGroupList;
+  int32_t* const row = L.idx + (int64_t)s * kNbMax;
+  const bool inactive = COUNT && L.ctl->inactive;
+  const float h2 = h2rec * kScanSlack;
+  const f32x2 nx = pack2(-xi.x, -xi.x), ny = pack2(-xi.y, -xi.y), nz = pack2(-xi.z, -xi.z), nh = pack2(-h2, -h2);
+  const bool scan = on && (!REUSE || reuse < 0);
+  ScanPos pos{INT32_MIN, 0, 0, -1};
+  bool live = on;
+  int n = 0, ncand = 0;
+  while (__any_sync(0xffffffffu, live)) {
+    int np = 0;
+    if (live && scan)
+      np = scan_pieces<COUNT>(g, xs, s, xi, h, inactive, words, 1, pos, live, ncand);  // all lanes write the same
+    __syncwarp();
+    uint32_t hit[(kIt + 7) / 8] = {}, pk[kPk] = {};  // four hit bits a round; their counts
+#pragma unroll
+    for (int i = 0; i < kIt; ++i) {
+      const int slot = i * G + lane, piece = slot >> 3;
+      uint32_t nib = 0;
+      if (piece < np) {
+        const uint2 w = words[piece];
+        const uint32_t gi = (w.x >> 2) + (slot & 7);
+        if (gi < (w.y + 3) >> 2) {
+          const ulonglong2* p = reinterpret_cast<const ulonglong2*>(q.g) + (size_t)gi * 3;
+          const ulonglong2 x2 = __ldg(p), y2 = __ldg(p + 1), z2 = __ldg(p + 2);
+          const f32x2 dx0 = add2(x2.x, nx), dx1 = add2(x2.y, nx);
+          const f32x2 dy0 = add2(y2.x, ny), dy1 = add2(y2.y, ny);
+          const f32x2 dz0 = add2(z2.x, nz), dz1 = add2(z2.y, nz);
+          const f32x2 r0 = fma2(dx0, dx0, fma2(dy0, dy0, fma2(dz0, dz0, nh)));
+          const f32x2 r1 = fma2(dx1, dx1, fma2(dy1, dy1, fma2(dz1, dz1, nh)));
+          nib = ((uint32_t)r0 >> 31) | ((uint32_t)(r0 >> 63) << 1) | (((uint32_t)r1 >> 31) << 2) |
+                ((uint32_t)(r1 >> 63) << 3);
+          const int f = (int)w.x - (int)(4 * gi), e = (int)w.y - (int)(4 * gi);  // the piece within this group
+          if (f > 0) nib &= 0xfu << f;
+          if (e < 4) nib &= (1u << e) - 1u;
+        }
+      }
+      hit[i >> 3] |= nib << (4 * (i & 7));
+      pk[i >> 2] += (uint32_t)__popc(nib) << (8 * (i & 3));
+    }
+    // hits before this lane's in each round, and in all lanes
+    uint32_t tot[kPk];
+#pragma unroll
+    for (int k = 0; k < kPk; ++k) {
+      const uint32_t own = pk[k];
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, pk[k], o, G);
+        if (lane >= o) pk[k] += v;
+      }
+      tot[k] = __shfl_sync(0xffffffffu, pk[k], G - 1, G);
+      pk[k] -= own;
+    }
+    int nb = 0;
+#pragma unroll
+    for (int i = 0; i < kIt; ++i) nb += (tot[i >> 2] >> (8 * (i & 3))) & 0xff;
+    if (REUSE && live && !scan) nb = reuse;
+    const int nbmax = __reduce_max_sync(0xffffffffu, nb);
+    for (int w0 = 0; w0 < nbmax; w0 += kGroupList) {
+      if (REUSE && live && !scan) {
+        for (int k = lane; k < kGroupList && w0 + k < nb; k += G) list[k] = row[w0 + k];
+      } else {
+        int base = 0;
+#pragma unroll
+        for (int i = 0; i < kIt; ++i) {
+          uint32_t m = (hit[i >> 3] >> (4 * (i & 7))) & 0xf;
+          int o = base + ((pk[i >> 2] >> (8 * (i & 3))) & 0xff);
+          base += (tot[i >> 2] >> (8 * (i & 3))) & 0xff;
+          if (m) {
+            const int slot = i * G + lane;
+            const int t = (int)(((words[slot >> 3].x >> 2) + (slot & 7)) * 4);
+            for (; m; m &= m - 1, ++o) {
+              const int v = t + __ffs(m) - 1;
+              if (o >= w0 && o < w0 + kGroupList) {
+                list[o - w0] = v;
+                if (n + o < kNbMax) row[n + o] = v;
+              }
+            }
+          }
+        }
+      }
+      __syncwarp();
+      group_visit<G, WITH_SELF, K>(xs, s, xi, h2m, min(max(nb - w0, 0), kGroupList), [&](int k) { return list[k]; },
+                                   load, term, acc);
+      __syncwarp();
+    }
+    n += nb;
+    if (!scan) live = false;
+  }
+  if (scan && lane == 0) L.cnt[s] = n <= kNbMax ? n : kNbMax + 1;
+  return ncand;
+}
+
+// The two neighbour sums of the passes, for one thread (G = 1) or a group of
+// lanes per particle: acc(term(t, xj, load(t))) in visiting order.
+//   scan_sum  scans the grid and records the list (scan_visit, group_scan)
+//   list_sum  iterates the recorded list (visit, visit_with, group_visit),
+//             or rescans where there is none; LAZY: load(t) only after the
+//             distance test (G = 1), where the early load costs registers
+// A particle with on = false takes no part.
+template <int G, bool WITH_SELF, bool COUNT, bool REUSE, int K, class Load, class Term, class Acc>
+FS_DEV int scan_sum(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
+                    float h2rec, float h2m, const NbrList& L, void* smem, bool on, int reuse, Load&& load, Term&& term,
+                    Acc&& acc) {
+  if constexpr (G == 1) {
+    if (!on) return 0;
+    return scan_visit<WITH_SELF, COUNT, REUSE>(
+        g, q, xs, s, xi, h, h2rec, h2m, L, (uint2*)smem, load,
+        [&](int t, float4 xj, const auto& p) { acc(term(t, xj, p)); }, reuse);
+  } else {
+    return group_scan<G, WITH_SELF, COUNT, REUSE, K>(g, q, xs, s, xi, h, h2rec, h2m, L, smem, on, reuse, load, term,
+                                                     acc);
+  }
+}
+
+template <int G, bool WITH_SELF, bool EVICT_FIRST, bool LAZY, int K, class Load, class Term, class Acc>
+FS_DEV void list_sum(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, float h2m,
+                     const NbrList& L, bool lists_ok, bool on, Load&& load, Term&& term, Acc&& acc) {
+  if constexpr (G == 1) {
+    if (!on) return;
+    if constexpr (LAZY)
+      visit<WITH_SELF>(g, xs, s, xi, h, h2m, L, lists_ok, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
+    else
+      visit_with<WITH_SELF, EVICT_FIRST>(g, xs, s, xi, h, h2m, L, lists_ok, load,
+                                         [&](int t, float4 xj, const auto& p) { acc(term(t, xj, p)); });
+  } else {
+    const int n = !on ? 0 : (lists_ok ? __ldg(L.cnt + s) : kNbMax + 1);
+    const bool over = n > kNbMax;
+    const int32_t* const row = L.idx + (int64_t)s * kNbMax;
+    group_visit<G, WITH_SELF, K>(xs, s, xi, h2m, over ? 0 : n, [&](int k) { return __ldg(row + k); }, load, term, acc);
+    if (over && (K > 0 || (threadIdx.x & (G - 1)) == 0))  // each lane adds up the whole sum (K = 0: the first)
+      scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
+  }
+}
+
+// f(s, live, lead) for the slots of this launch: G = 1 as for_slots; else each
+// group of G lanes takes one slot, every lane of the warp calls f (live =
+// false past the last slot) and lead marks the lane that writes.
+template <int G, class F>
+FS_DEV void for_groups(int64_t n, F&& f) {
+  if constexpr (G == 1) {
+    for_slots(n, [&](int64_t s) { f(s, true, true); });
+  } else {
+    const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const bool live = s < n;
+    f(live ? s : n - 1, live, live && (threadIdx.x & (G - 1)) == 0);
+  }
+}
+
+// Lanes per particle of the neighbour kernels for n particles.
+int nb_group(int64_t n);
+
+// Launches KERNEL<G>(args) for n particles at the context's block size.
+#define FS_NB_CASE(KERNEL, G, SMEM, ...)                                                                      \
+  KERNEL<G><<<(unsigned)((n_ * G + c_->nb_block - 1) / c_->nb_block), c_->nb_block,                           \
+              (SMEM) ? scan_smem(c_->nb_block, G) : 0, st_>>>(__VA_ARGS__)
+#define FS_NB_LAUNCH(KERNEL, c, n, group, st, SMEM, ...)                                                      \
+  do {                                                                                                        \
+    const fs_context* c_ = (c);                                                                               \
+    const int64_t n_ = (n);                                                                                   \
+    cudaStream_t st_ = (st);                                                                                  \
+    switch (group) {                                                                                          \
+      case 4: FS_NB_CASE(KERNEL, 4, SMEM, __VA_ARGS__); break;                                                \
+      case 8: FS_NB_CASE(KERNEL, 8, SMEM, __VA_ARGS__); break;                                                \
+      case 16: FS_NB_CASE(KERNEL, 16, SMEM, __VA_ARGS__); break;                                              \
+      default:                                                                                                \
+        KERNEL<1><<<nb_blocks(c_, n_), c_->nb_block, (SMEM) ? scan_smem(c_->nb_block, 1) : 0, st_>>>(__VA_ARGS__); \
+    }                                                                                                         \
+  } while (0)
 
 // Whether lists recorded for the current grid and positions exist.
 FS_DEV bool lists_usable(const NbrList& L) { return L.ctl->valid != 0; }

@@ -67,29 +67,30 @@ __global__ void k_gather_pbf(int64_t n, const int32_t* __restrict__ perm, fs_mod
 // also writes update_velocity_from_positions (403-416):
 // vout[s] = ((x_pred - x_in) / max(dt, 1e-8), m / max(rho, 1e-6)), v_pred
 // for non-dynamic particles.
-__global__ void FS_NB_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, int64_t n,
-                                                      const float4* __restrict__ xs, const float4* __restrict__ vs,
-                                                      const float* __restrict__ mv, float h, float skin, float* rho,
-                                                      float2* __restrict__ sc2, const float4* __restrict__ xin = nullptr,
-                                                      float dt = 0.f, float4* __restrict__ vout = nullptr) {
-  extern __shared__ uint2 words[];
+template <int G>
+__global__ void FS_NB_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, int64_t n, const float4* __restrict__ xs,
+                                           const float4* __restrict__ vs, const float* __restrict__ mv, float h,
+                                           float skin, float* rho, float2* __restrict__ sc2,
+                                           const float4* __restrict__ xin, float dt, float4* __restrict__ vout) {
+  extern __shared__ uint2 smem[];
   lists_recorded(L);
-  for_slots(n, [&](int64_t s) {
+  for_groups<G>(n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = xs[s];
     const int32_t i = g.perm[s];
     float acc = 0.f;
     const float h2m = h * h * kSupportMargin;
     const Poly6Spiky K(h);
-    if (pf_of(xi) & PF_ACTIVE) {
-      const float hr = h * (1.0f + skin);
-      scan_visit<true>(g, q, xs, (int)s, xi, h, hr * hr * kSupportMargin, h2m, L, words,
-                       [&](int t) { return __ldg(mv + t); }, [&](int t, float4 xj, const float& m) {
-        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        acc = fmaf(m, K.w_r2(fmaf(dx, dx, fmaf(dy, dy, dz * dz))), acc);
-      });
-    } else {
-      L.cnt[s] = 0;
-    }
+    const bool on = live && (pf_of(xi) & PF_ACTIVE);
+    const float hr = h * (1.0f + skin);
+    scan_sum<G, true, false, false, 2>(
+        g, q, xs, (int)s, xi, h, hr * hr * kSupportMargin, h2m, L, smem, on, -1, [&](int t) { return __ldg(mv + t); },
+        [&](int t, float4 xj, const float& m) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          return Terms<2>{m, K.w_r2(fmaf(dx, dx, fmaf(dy, dy, dz * dz)))};
+        },
+        [&](const Terms<2>& u) { acc = fmaf(u.v[0], u.v[1], acc); });
+    if (!lead) return;
+    if (!on) L.cnt[s] = 0;
     rho[i] = acc;
     const float4 vi = vs[s];
     const float wgt = vi.w / fmaxf(acc, 1.0e-6f);
@@ -125,16 +126,13 @@ struct AccelArgs {
   uint32_t* disp_max = nullptr;  // largest |x_out - x| (float bits; null: not tracked)
 };
 
+template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
   float dmax = 0.f;
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
-    if (!(pf_of(xi) & PF_DYNAMIC)) {
-      st3(a.accel, i, make_float3(0.f, 0.f, 0.f));
-      a.xs_out[s] = xi;
-      return;
-    }
+    const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const float4 vi = a.vs[s];
     const float mu = a.m.viscosity[i];
     const float gamma = a.m.surface_tension[i];
@@ -144,28 +142,36 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
     const float rp2 = a.particle_radius * a.particle_radius;
     const Poly6Spiky K(a.h);
     float ax = 0.f, ay = 0.f, az = 0.f;
-    if (gamma != 0.f || mu != 0.f) {
-      const bool lists_ok = a.use_lists && lists_usable(a.L);
-      visit_with<false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
-                        [&](int t) { return __ldg(a.vs + t); }, [&](int t, float4 xj, const float4& vj) {
-        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        float c = 0.f;
-        if (gamma != 0.f) c -= coh * vj.w * K.w_r2(fmaxf(r2, rp2));  // W(max(r, r_p))
-        if (mu != 0.f) {
-          const float vdot = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
-          if (vdot != 0.f) {
-            float r, rinv;
-            r_and_inv(r2, r, rinv);
-            c += mu10 * __ldg(&a.sc2[t].y) * __fdividef(vdot, r2 + visc_den_add) * K.grad_scale(r, rinv);
+    const bool on = live && dyn && (gamma != 0.f || mu != 0.f);
+    list_sum<G, false, true, false, 4>(
+        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), on,
+        [&](int t) { return __ldg(a.vs + t); },
+        [&](int t, float4 xj, const float4& vj) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          float c = 0.f;
+          if (gamma != 0.f) c -= coh * vj.w * K.w_r2(fmaxf(r2, rp2));  // W(max(r, r_p))
+          if (mu != 0.f) {
+            const float vdot = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
+            if (vdot != 0.f) {
+              float r, rinv;
+              r_and_inv(r2, r, rinv);
+              c += mu10 * __ldg(&a.sc2[t].y) * __fdividef(vdot, r2 + visc_den_add) * K.grad_scale(r, rinv);
+            }
           }
-        }
-        ax = fmaf(c, dx, ax);
-        ay = fmaf(c, dy, ay);
-        az = fmaf(c, dz, az);
-      });
-    }
+          return Terms<4>{c, dx, dy, dz};
+        },
+        [&](const Terms<4>& u) {
+          ax = fmaf(u.v[0], u.v[1], ax);
+          ay = fmaf(u.v[0], u.v[2], ay);
+          az = fmaf(u.v[0], u.v[3], az);
+        });
+    if (!lead) return;
     st3(a.accel, i, make_float3(ax, ay, az));
+    if (!dyn) {
+      a.xs_out[s] = xi;
+      return;
+    }
     const float dvx = a.dt * ax, dvy = a.dt * ay, dvz = a.dt * az;
     float3 p = make_float3(xi.x + a.dt * dvx, xi.y + a.dt * dvy, xi.z + a.dt * dvz);
     clamp_position(walls_of(a.walls, a.g, world_of(xi)), p);
@@ -210,21 +216,15 @@ struct LambdaArgs {
 // cells as at x_i; visiting that list with the support test at x' then
 // reproduces the scan's pair sequence exactly.  Particles failing (b), and
 // every particle when (a) fails, scan the grid.
+template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
-  extern __shared__ uint2 words[];
+  extern __shared__ uint2 smem[];
   lists_recorded(a.L);
   const bool reuse_ok = a.xs_rec && __uint_as_float(*a.disp_max) <= a.reuse_limit;
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
-    if (!(pf_of(xi) & PF_DYNAMIC)) {
-      a.L.cnt[s] = 0;
-      a.lam_s[s] = make_float2(0.f, a.vs[s].w);
-      if (a.lam) a.lam[i] = 0.f;
-      if (a.rho) a.rho[i] = 0.f;
-      if (a.count) a.count[i] = 0;
-      return;
-    }
+    const bool on = live && (pf_of(xi) & PF_DYNAMIC);
     const float rho0 = fmaxf(a.rest_density[i], 1.0e-6f);
     const float inv_rho0 = 1.0f / rho0;
     const Poly6Spiky K(a.h);
@@ -232,28 +232,42 @@ __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
     int cnt = 0;
     const float h2m = a.h * a.h * kSupportMargin;
     // records the lists the delta pass of this iteration (same positions) reuses
-    const int listed = reuse_ok ? a.L.cnt[s] : kNbMax + 1;
+    const int listed = reuse_ok && on ? a.L.cnt[s] : kNbMax + 1;
     const bool reuse = listed <= kNbMax && same_query_cells(a.g, world_of(xi), a.xs_rec[s], xi, a.h);
     if (a.g.tile_stats && a.xs_rec) {
       const unsigned full = __activemask();
-      const unsigned b = __ballot_sync(full, reuse);
+      const unsigned b = __ballot_sync(full, reuse && lead);
       if ((int)(threadIdx.x & 31) == __ffs(full) - 1) atomicAdd(a.g.tile_stats + 2, (unsigned long long)__popc(b));
     }
-    scan_visit<true, false, true>(a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, words,
-                                  [&](int t) { return __ldg(&a.vs[t].w); }, [&](int t, float4 xj, const float& mj) {
-      const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      if (t != (int)s && exact_lt_h(r2, dx, dy, dz, a.h, K.h2)) ++cnt;
-      float r, rinv;
-      r_and_inv(r2, r, rinv);
-      rho = fmaf(mj, K.w_r2(r2), rho);
-      const float c = -(mj * inv_rho0) * K.grad_scale(r, rinv);
-      const float gjx = c * dx, gjy = c * dy, gjz = c * dz;
-      sq = fmaf(gjx, gjx, fmaf(gjy, gjy, fmaf(gjz, gjz, sq)));
-      gx -= gjx;
-      gy -= gjy;
-      gz -= gjz;
-    }, reuse ? listed : -1);
+    scan_sum<G, true, false, true, 5>(
+        a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, reuse ? listed : -1,
+        [&](int t) { return __ldg(&a.vs[t].w); },
+        [&](int t, float4 xj, const float& mj) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          if (t != (int)s && exact_lt_h(r2, dx, dy, dz, a.h, K.h2)) ++cnt;
+          float r, rinv;
+          r_and_inv(r2, r, rinv);
+          const float c = -(mj * inv_rho0) * K.grad_scale(r, rinv);
+          return Terms<5>{mj, K.w_r2(r2), c * dx, c * dy, c * dz};
+        },
+        [&](const Terms<5>& u) {
+          rho = fmaf(u.v[0], u.v[1], rho);
+          sq = fmaf(u.v[2], u.v[2], fmaf(u.v[3], u.v[3], fmaf(u.v[4], u.v[4], sq)));
+          gx = __fsub_rn(gx, u.v[2]);  // sums of the rounded gradients (no contraction), whatever surrounds them
+          gy = __fsub_rn(gy, u.v[3]);
+          gz = __fsub_rn(gz, u.v[4]);
+        });
+    cnt = group_sum<G>(cnt);
+    if (!lead) return;
+    if (!on) {
+      a.L.cnt[s] = 0;
+      a.lam_s[s] = make_float2(0.f, a.vs[s].w);
+      if (a.lam) a.lam[i] = 0.f;
+      if (a.rho) a.rho[i] = 0.f;
+      if (a.count) a.count[i] = 0;
+      return;
+    }
     sq = fmaf(gx, gx, fmaf(gy, gy, fmaf(gz, gz, sq)));
     const float ci = fmaxf(rho / rho0 - 1.0f, 0.f);
     const float l = (a.min_nb > 0 && cnt < a.min_nb) ? 0.f : -ci / (sq + a.eps);
@@ -294,43 +308,49 @@ FS_DEV float pow_uint(float x, int n) {
   return r;
 }
 
+template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
   // an integral exponent 1..8 (the class default is 4) takes pow_uint
   const int n_int = (a.scorr_n >= 1.f && a.scorr_n <= 8.f && a.scorr_n == rintf(a.scorr_n)) ? (int)a.scorr_n : 0;
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
-    if (!(pf_of(xi) & PF_DYNAMIC)) {
-      st3(a.delta_p, i, make_float3(0.f, 0.f, 0.f));
-      if (a.xs_out) a.xs_out[s] = xi;
-      return;
-    }
+    const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const float rho0 = fmaxf(a.rest_density[i], 1.0e-6f);
     const float li = a.lam_s[s].x;
     const Poly6Spiky K(a.h);
     const bool scorr = a.scorr_k != 0.f && !(a.w_dq <= 1.0e-6f);
     const float inv_wdq = scorr ? 1.0f / a.w_dq : 0.f;
     float dx_ = 0.f, dy_ = 0.f, dz_ = 0.f;
-    const bool lists_ok = a.use_lists && lists_usable(a.L);
-    visit_with<false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
-                      [&](int t) { return __ldg(a.lam_s + t); }, [&](int t, float4 xj, const float2& lj) {
-      const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      float r, rinv;
-      r_and_inv(r2, r, rinv);
-      float sc = 0.f;
-      if (scorr) {
-        const float q = K.w_r2(r2) * inv_wdq;
-        sc = -a.scorr_k * (n_int ? pow_uint(q, n_int) : powf(q, a.scorr_n));
-      }
-      const float c = (li + lj.x + sc) * lj.y * K.grad_scale(r, rinv);
-      dx_ = fmaf(c, dx, dx_);
-      dy_ = fmaf(c, dy, dy_);
-      dz_ = fmaf(c, dz, dz_);
-    });
+    list_sum<G, false, true, false, 4>(
+        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), live && dyn,
+        [&](int t) { return __ldg(a.lam_s + t); },
+        [&](int t, float4 xj, const float2& lj) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          float r, rinv;
+          r_and_inv(r2, r, rinv);
+          float sc = 0.f;
+          if (scorr) {
+            const float q = K.w_r2(r2) * inv_wdq;
+            sc = -a.scorr_k * (n_int ? pow_uint(q, n_int) : powf(q, a.scorr_n));
+          }
+          return Terms<4>{(li + lj.x + sc) * lj.y * K.grad_scale(r, rinv), dx, dy, dz};
+        },
+        [&](const Terms<4>& u) {
+          dx_ = fmaf(u.v[0], u.v[1], dx_);
+          dy_ = fmaf(u.v[0], u.v[2], dy_);
+          dz_ = fmaf(u.v[0], u.v[3], dz_);
+        });
+    if (!lead) return;
+    if (!dyn) {
+      st3(a.delta_p, i, make_float3(0.f, 0.f, 0.f));
+      if (a.xs_out) a.xs_out[s] = xi;
+      return;
+    }
     float3 d = make_float3(dx_ / rho0, dy_ / rho0, dz_ / rho0);
     if (a.max_dp > 0.f) {
-      const float len = sqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
+      const float len = sqrtf(norm2(d.x, d.y, d.z));
       if (len > a.max_dp) {
         const float sc = a.max_dp / fmaxf(len, 1.0e-12f);
         d = make_float3(d.x * sc, d.y * sc, d.z * sc);
@@ -364,31 +384,36 @@ struct XsphArgs {
   float* x_pred_api;   // optional
 };
 
+template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_xsph_final(XsphArgs a) {
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const float4 vi = a.vel[s];
     const int32_t i = a.g.perm[s];
     float3 v = xyz(vi);
     float3 p = xyz(xi);
-    if (a.x_pred_api) st3(a.x_pred_api, i, p);
-    if (pf_of(xi) & PF_DYNAMIC) {
-      if (a.c > 0.f) {
-        const Poly6Spiky K(a.h);
-        float cx = 0.f, cy = 0.f, cz = 0.f;
-        const bool lists_ok = a.use_lists && lists_usable(a.L);
-        visit_with<false, true>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
-                          [&](int t) { return __ldg(a.vel + t); }, [&](int t, float4 xj, const float4& vj) {
+    const bool dyn = pf_of(xi) & PF_DYNAMIC;
+    const Poly6Spiky K(a.h);
+    float cx = 0.f, cy = 0.f, cz = 0.f;
+    list_sum<G, false, true, false, 4>(
+        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        live && dyn && a.c > 0.f, [&](int t) { return __ldg(a.vel + t); },
+        [&](int t, float4 xj, const float4& vj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           // vj = (v, m / max(rho, 1e-6))
           // (m_j / max(rho_j, 1e-6)) W(r), the ratio from the final density pass
           const float w = vj.w * K.w_r2(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
-          cx = fmaf(vj.x - vi.x, w, cx);
-          cy = fmaf(vj.y - vi.y, w, cy);
-          cz = fmaf(vj.z - vi.z, w, cz);
+          return Terms<4>{w, vj.x - vi.x, vj.y - vi.y, vj.z - vi.z};
+        },
+        [&](const Terms<4>& u) {
+          cx = fmaf(u.v[1], u.v[0], cx);
+          cy = fmaf(u.v[2], u.v[0], cy);
+          cz = fmaf(u.v[3], u.v[0], cz);
         });
-        v = make_float3(fmaf(a.c, cx, vi.x), fmaf(a.c, cy, vi.y), fmaf(a.c, cz, vi.z));
-      }
+    if (!lead) return;
+    if (a.x_pred_api) st3(a.x_pred_api, i, p);
+    if (dyn) {
+      if (a.c > 0.f) v = make_float3(fmaf(a.c, cx, vi.x), fmaf(a.c, cy, vi.y), fmaf(a.c, cz, vi.z));
       if (a.bounds) apply_walls(walls_of(a.walls, a.g, world_of(xi)), p, v);
     }
     if (a.x_out) st3(a.x_out, i, p);
@@ -474,6 +499,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   // neighbour lists: density -> accel, lambda -> delta, final density -> XSPH
   const NbrList L = nbr_list(c);
   const int use_lists = 1;
+  const int group = nb_group(n);
   // the first density records its lists out to h (1 + skin) so that the first
   // lambda pass can reuse them instead of scanning the grid (k_lambda).  The
   // non-pressure update between the two moves particles by dt^2 |a|: at most
@@ -484,7 +510,8 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     return rc;
   {
     PassScope ps_(c, P_PBF_DENSITY, st);
-    k_density<<<nb_blocks(c, n), c->nb_block, scan_smem(c->nb_block), st>>>(g, L, scan_xyz(c), n, c->xs, c->vs, c->mv, h, skin, so->rho, c->sc2);
+    FS_NB_LAUNCH(k_density, c, n, group, st, true, g, L, scan_xyz(c), n, c->xs, c->vs, c->mv, h, skin, so->rho, c->sc2,
+                 nullptr, 0.f, nullptr);
   }
   AccelArgs aa;
   aa.g = g;
@@ -505,7 +532,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   aa.disp_max = skin > 0.f ? c->pbf_disp : nullptr;
   {
     PassScope ps_(c, P_PBF_ACCEL, st);
-    k_accel_apply<<<nb_blocks(c, n), c->nb_block, 0, st>>>(aa);
+    FS_NB_LAUNCH(k_accel_apply, c, n, group, st, false, aa);
   }
   if ((rc = launch_check("pbf accel"))) return rc;
   float4* cur = c->xs2;
@@ -532,7 +559,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     la.reuse_limit = 0.5f * h * (skin - 1.0e-4f);
     {
       PassScope ps_(c, P_PBF_LAMBDA, st);
-      k_lambda<<<nb_blocks(c, n), c->nb_block, scan_smem(c->nb_block), st>>>(la);
+      FS_NB_LAUNCH(k_lambda, c, n, group, st, true, la);
     }
     DeltaArgs da;
     da.g = gi;
@@ -555,7 +582,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     da.q = scan_out(c);
     {
       PassScope ps_(c, P_PBF_DELTA, st);
-      k_delta<<<nb_blocks(c, n), c->nb_block, 0, st>>>(da);
+      FS_NB_LAUNCH(k_delta, c, n, group, st, false, da);
     }
     if ((rc = launch_check("pbf iteration"))) return rc;
     float4* t = cur;
@@ -578,8 +605,8 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   {
     // + update_velocity_from_positions into nxt (the other x_pred buffer)
     PassScope ps_(c, P_PBF_DENSITY, st);
-    k_density<<<nb_blocks(c, n), c->nb_block, scan_smem(c->nb_block), st>>>(gf, L, scan_xyz(c), n, cur, c->vs, c->mv, h, 0.f, so->rho, c->sc2,
-                                                       c->vs2, dt, nxt);
+    FS_NB_LAUNCH(k_density, c, n, group, st, true, gf, L, scan_xyz(c), n, cur, c->vs, c->mv, h, 0.f, so->rho, c->sc2,
+                 c->vs2, dt, nxt);
   }
   XsphArgs xa;
   xa.g = gf;
@@ -598,7 +625,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   xa.x_pred_api = x_pred;
   {
     PassScope ps_(c, P_PBF_XSPH, st);
-    k_xsph_final<<<nb_blocks(c, n), c->nb_block, 0, st>>>(xa);
+    FS_NB_LAUNCH(k_xsph_final, c, n, group, st, false, xa);
   }
   c->last_stream = st;
   return launch_check("pbf final");
@@ -626,8 +653,8 @@ int fs_pbf_density(fs_context* c, const fs_model* m, const float* x, float h, fl
   cudaStream_t st = (cudaStream_t)stream;
   k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, x, c->xs, scan_out(c), c->vs, c->mv,
                                                        c->status, c->nworlds);
-  k_density<<<nb_blocks(c, m->n), c->nb_block, scan_smem(c->nb_block), st>>>(
-      grid_view(c), nbr_list(c), scan_xyz(c), m->n, c->xs, c->vs, c->mv, h, 0.f, rho, c->sc2);
+  FS_NB_LAUNCH(k_density, c, m->n, nb_group(m->n), st, true, grid_view(c), nbr_list(c), scan_xyz(c), m->n, c->xs,
+               c->vs, c->mv, h, 0.f, rho, c->sc2, nullptr, 0.f, nullptr);
   return launch_check("fs_pbf_density");
 }
 
@@ -655,7 +682,7 @@ int fs_pbf_lambda(fs_context* c, const fs_model* m, const float* x_pred, const f
   la.lam = pbf_lambda;
   la.rho = rho;
   la.count = neighbor_count;
-  k_lambda<<<nb_blocks(c, m->n), c->nb_block, scan_smem(c->nb_block), st>>>(la);
+  FS_NB_LAUNCH(k_lambda, c, m->n, nb_group(m->n), st, true, la);
   return launch_check("fs_pbf_lambda");
 }
 
@@ -689,7 +716,7 @@ int fs_pbf_delta(fs_context* c, const fs_model* m, const float* x_pred, const fl
   da.delta_p = delta_p;
   da.xs_out = nullptr;
   da.q = ScanOut{};
-  k_delta<<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(da);
+  k_delta<1><<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(da);  // no list: each thread rescans
   return launch_check("fs_pbf_delta");
 }
 
@@ -719,7 +746,7 @@ int fs_pbf_xsph(fs_context* c, const fs_model* m, const float* x_pred, const flo
   xa.x_out = nullptr;
   xa.v_out = v_out;
   xa.x_pred_api = nullptr;
-  k_xsph_final<<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(xa);
+  k_xsph_final<1><<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(xa);
   return launch_check("fs_pbf_xsph");
 }
 

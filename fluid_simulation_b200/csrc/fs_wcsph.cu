@@ -49,30 +49,35 @@ struct DensityArgs {
 // 64-register budget: at the compiler's own 78 registers (no spills, 28
 // resident warps) a launch at 4,194,304 particles takes 1.44 ms, at 64 1.00,
 // at 48 1.07.  Before the word scan (scan_words) it took 1.63.
+template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, 4) k_wcsph_density(DensityArgs a) {
-  extern __shared__ uint2 words[];
+  extern __shared__ uint2 smem[];
   if (clock_idle(a.clock)) return;
   lists_recorded(a.L);
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
-    if (!(pf_of(xi) & PF_ACTIVE)) {
+    const bool on = live && (pf_of(xi) & PF_ACTIVE);
+    const float h2m = a.h * a.h * kSupportMargin;
+    const Cubic K(a.h);
+    float acc = 0.f;
+    scan_sum<G, true, false, false, 2>(
+        a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, -1, [&](int t) { return __ldg(a.mv + t); },
+        [&](int t, float4 xj, const float& m) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          float r, rinv;
+          r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
+          return Terms<2>{m, K.w(r)};
+        },
+        [&](const Terms<2>& u) { acc = fmaf(u.v[0], u.v[1], acc); });
+    if (!lead) return;
+    if (!on) {
       a.rho[i] = 0.f;
       a.pressure[i] = 0.f;
       a.sc2[s] = make_float2(0.f, 0.f);
       a.L.cnt[s] = 0;
       return;
     }
-    const float h2m = a.h * a.h * kSupportMargin;
-    const Cubic K(a.h);
-    float acc = 0.f;
-    scan_visit<true>(a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, words, [&](int t) { return __ldg(a.mv + t); },
-                     [&](int t, float4 xj, const float& m) {
-      const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      float r, rinv;
-      r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
-      acc = fmaf(m, K.w(r), acc);
-    });
     float p = a.stiffness[i] * (powf(acc / fmaxf(a.rest_density[i], 1.0e-6f), a.exponent[i]) - 1.0f);
     if (a.clamp) p = fmaxf(p, 0.f);
     a.rho[i] = acc;
@@ -101,48 +106,56 @@ struct ForceArgs {
   const fs_frame_clock* clock;  // clocked substep: dt from the clock, nothing to do once the frame is complete
 };
 
+template <int G>
 __global__ void FS_NB_BOUNDS k_wcsph_force(ForceArgs a) {
   if (clock_idle(a.clock)) return;
   const float dt = a.clock ? a.clock->dt : a.dt;
-  for_slots(a.n, [&](int64_t s) {
+  for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const float4 vi = a.vs[s];
     const int32_t i = a.g.perm[s];
-    if (!(pf_of(xi) & PF_DYNAMIC)) {
-      st3(a.accel, i, make_float3(0.f, 0.f, 0.f));
-      st3(a.v_out, i, xyz(vi));
-      st3(a.x_out, i, xyz(xi));
-      return;
-    }
+    const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const float dp_i = a.sc2[s].x;
     const float mu10 = 10.f * a.m.viscosity[i];
     const float coh = a.m.surface_tension[i] / vi.w;
     const float visc_den_add = 0.01f * (a.h * a.h);
     const Cubic K(a.h);
     float ax = 0.f, ay = 0.f, az = 0.f;
-    const bool lists_ok = a.use_lists && lists_usable(a.L);
-    visit<false>(a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, lists_ok,
-                        [&](int t, float4 xj) {
-      const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      if (r2 == 0.f) return;  // coincident particles: every term carries the zero vector d
-      const float4 vj = __ldg(a.vs + t);
-      const float2 rj = __ldg(a.sc2 + t);  // (p_j / rho_j^2, 1 / rho_j)
-      float r, rinv;
-      r_and_inv(r2, r, rinv);
-      const float m_j = vj.w;
-      // cohesion -gamma/m_i m_j W(max(r, r_p)) d
-      const float wc = coh * m_j * K.w(fmaxf(r, a.particle_radius));
-      // viscosity 10 mu (m_j / rho_j) (v_ij . d) / (r^2 + 0.01 h^2) grad W
-      const float vdot = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
-      const float visc = mu10 * m_j * rj.y * __fdividef(vdot, r2 + visc_den_add);
-      // pressure -m_j (p_i / rho_i^2 + p_j / rho_j^2) grad W
-      const float pres = -m_j * (dp_i + rj.x);
-      const float c = fmaf(visc + pres, K.grad_scale(r, rinv), -wc);
-      ax = fmaf(c, dx, ax);
-      ay = fmaf(c, dy, ay);
-      az = fmaf(c, dz, az);
-    });
+    struct Neighbour {
+      float4 v;
+      float2 r;  // (p_j / rho_j^2, 1 / rho_j)
+    };
+    list_sum<G, false, false, true, 4>(
+        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), live && dyn,
+        [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(a.sc2 + t)}; },
+        [&](int t, float4 xj, const Neighbour& j) {
+          const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          if (r2 == 0.f) return Terms<4>{};  // coincident particles: every term carries the zero vector d
+          float r, rinv;
+          r_and_inv(r2, r, rinv);
+          const float m_j = j.v.w;
+          // cohesion -gamma/m_i m_j W(max(r, r_p)) d
+          const float wc = coh * m_j * K.w(fmaxf(r, a.particle_radius));
+          // viscosity 10 mu (m_j / rho_j) (v_ij . d) / (r^2 + 0.01 h^2) grad W
+          const float vdot = fmaf(vi.x - j.v.x, dx, fmaf(vi.y - j.v.y, dy, (vi.z - j.v.z) * dz));
+          const float visc = mu10 * m_j * j.r.y * __fdividef(vdot, r2 + visc_den_add);
+          // pressure -m_j (p_i / rho_i^2 + p_j / rho_j^2) grad W
+          const float pres = -m_j * (dp_i + j.r.x);
+          return Terms<4>{fmaf(visc + pres, K.grad_scale(r, rinv), -wc), dx, dy, dz};
+        },
+        [&](const Terms<4>& u) {
+          ax = fmaf(u.v[0], u.v[1], ax);
+          ay = fmaf(u.v[0], u.v[2], ay);
+          az = fmaf(u.v[0], u.v[3], az);
+        });
+    if (!lead) return;
+    if (!dyn) {
+      st3(a.accel, i, make_float3(0.f, 0.f, 0.f));
+      st3(a.v_out, i, xyz(vi));
+      st3(a.x_out, i, xyz(xi));
+      return;
+    }
     const float3 g = gravity_of(a.m, i);
     const float3 acc = make_float3(ax + g.x, ay + g.y, az + g.z);
     st3(a.accel, i, acc);
@@ -205,7 +218,7 @@ int launch_density(fs_context* c, const fs_model* m, float h, int clamp, bool eo
   a.sc2 = c->sc2;
   {
     PassScope ps_(c, P_WCSPH_DENSITY, st);
-    k_wcsph_density<<<nb_blocks(c, a.n), c->nb_block, scan_smem(c->nb_block), st>>>(a);
+    FS_NB_LAUNCH(k_wcsph_density, c, a.n, nb_group(a.n), st, true, a);
   }
   return launch_check("wcsph density");
 }
@@ -231,7 +244,7 @@ int launch_force(fs_context* c, const fs_model* m, const fs_wcsph_params* p, flo
   a.v_out = v_out;
   {
     PassScope ps_(c, P_WCSPH_FORCE, st);
-    k_wcsph_force<<<nb_blocks(c, a.n), c->nb_block, 0, st>>>(a);
+    FS_NB_LAUNCH(k_wcsph_force, c, a.n, use_lists ? nb_group(a.n) : 1, st, false, a);  // no list: each thread rescans
   }
   return launch_check("wcsph force");
 }

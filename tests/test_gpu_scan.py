@@ -5,7 +5,11 @@ candidates, rows that wrap, dims that are no power of two.
 Densities against a float64 sum over all pairs: k positive FP32 terms, each a
 few ulp off, summed one after the other, are within (k + 16) 2^-23 of it
 (relative).  DFSPH's neighbour counts (candidates, no distance test) equal the
-oracle's candidate lists."""
+oracle's candidate lists.
+
+Small scenes give several lanes to a particle (16, 8, 4 or 1 by the particle
+count): a scene stepped together with particles far away from it, whose number
+moves the count across those limits, keeps every bit of its step alone."""
 
 import numpy as np
 import pytest
@@ -13,7 +17,7 @@ import torch
 
 import oracle
 from fluid_simulation_b200.newton_shim import HashGrid, model_from_arrays
-from fluid_simulation_b200.solver import SolverDFSPH, SolverWCSPH
+from fluid_simulation_b200.solver import SolverDFSPH, SolverPBF, SolverWCSPH
 
 pytestmark = pytest.mark.gpu
 SP = 0.01
@@ -73,3 +77,46 @@ def test_scan_edges(n, centre, dims, cuda_device):
                       enumerate(np.split(np.asarray(cand), np.asarray(off)[1:-1]))])
     got = step(SolverDFSPH, x, flags, dims, cuda_device, 1e-9).sph.neighbor_count.cpu().numpy()
     assert np.array_equal(got, np.where(active, count, 0))
+
+
+def block(n, corner, seed):
+    """n particles of a jittered lattice at rest spacing, moving."""
+    side = int(np.ceil(n ** (1.0 / 3.0)))
+    k = np.arange(n)
+    g = np.stack([k // side ** 2, k // side % side, k % side], 1)
+    rng = np.random.default_rng(seed)
+    x = (g + rng.uniform(-0.2, 0.2, g.shape)) * SP + np.asarray(corner)
+    return x.astype(np.float32), rng.normal(0.0, 0.1, x.shape).astype(np.float32)
+
+
+@pytest.mark.parametrize("total", [4999, 5001, 14000, 14001, 36000, 36001])
+@pytest.mark.parametrize("kind", ["wcsph", "dfsph", "pbf"])
+def test_lanes_per_particle_change_no_bit(kind, total, cuda_device):
+    cls = dict(wcsph=SolverWCSPH, dfsph=SolverDFSPH, pbf=SolverPBF)[kind]
+    base = dict(particle_radius=0.5 * SP, particle_length=SP, smoothing_length_coff=2.0, bound_width=0.6,
+                bound_height=0.6, bound_length=0.5, boundary_damping=0.0)
+    attrs = dict(particle_mask=0, rest_density=1000.0, surface_tension=0.01, viscosity=0.005)
+    if kind == "wcsph":
+        cfg, dt = cls.SphConfig(**base), 1e-4
+        attrs.update(stiffness=2.5e5, exponent=7.0)
+    elif kind == "dfsph":  # no early end: the residual is a mean over all particles
+        cfg, dt = cls.SphConfig(max_rho_iterations=3, max_vel_iterations=4, warm_start=False, eta_density=-1.0,
+                                eta_divergence=-1.0, **base), 1e-3
+    else:
+        cfg, dt = cls.PbfConfig(max_iterations=3, lambda_epsilon=100.0, max_delta_position=0.25 * SP, xsph_c=0.05,
+                                scorr_k=1e-4, **base), 1e-3
+    n = 2500
+    x, v = block(n, (-0.55, -0.55, 0.02), 1)
+    x2, v2 = block(total - n, (-0.2, -0.2, 0.02), 2)
+
+    def run(x, v):
+        m = model_from_arrays(x, v, 1000.0 * SP ** 3, device=cuda_device, radius=0.5 * SP, attributes=attrs,
+                              solver_cls=cls)
+        s = cls(m, cfg)
+        a, b = m.state(), m.state()
+        s.step(a, b, None, None, dt)
+        return dict(vars(b.sph), x=b.particle_q, v=b.particle_qd, accel=s._particle_accel)
+
+    alone, both = run(x, v), run(np.concatenate([x, x2]), np.concatenate([v, v2]))
+    for name, t in alone.items():
+        assert torch.equal(t, both[name][:n]), name
