@@ -14,7 +14,7 @@
 //   pres_ij = -m_j (P_i + P_j),                   grad W(d) = gs(r) d
 //   u' = v + dt a;  x' = x + dt u';  walls(x', u')
 // Given the adjoints of the outputs (xb', vb') the three passes compute:
-//   prepare    elementwise: cell-order copies of the step's data, and
+//   gather     (in the grid build) cell-order copies of the step's data, and
 //              walls^T and the integrator -> ab_i
 //   force      per particle k, both sides of every pair (k, j): its own term
 //              of a_k (weights ab_k) and its term in a_j (weights ab_j), so
@@ -25,7 +25,7 @@
 //   density    xb_k += sum_j (rhob_k mv_j + rhob_j mv_k) gs(r) d_kj
 // The force pass records the neighbour lists of the step's positions; the
 // density pass reuses them.
-#include "fs_nbr.cuh"
+#include "fs_build.cuh"
 
 namespace fs {
 
@@ -95,38 +95,42 @@ struct AdjArgs {
   Walls walls;
 };
 
-// Cell-order copies of what the adjoint passes read (one kernel): positions
+// Cell-order copies of what the adjoint passes read (gathered by the grid
+// build's last kernel): positions
 // + flags, velocities + mass, mv, (P, R) from the step's rho and pressure,
 // viscosity, cohesion / mass, and ab from the walls / integrator adjoint.
-__global__ void k_adj_prepare(AdjArgs a, float* __restrict__ nu, float* __restrict__ coh, float4* __restrict__ xs,
-                              ScanOut q, float4* __restrict__ vs, float* __restrict__ mv,
-                              float2* __restrict__ sc2) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= a.n) return;
-  const int32_t i = a.g.perm[s];
-  const fs_model& m = a.m;
-  const float3 x = ld3(a.xin, i), v = ld3(a.vin, i);
-  const int pf = particle_pf(m.particle_flags, m.particle_mask, i);
-  const int w = (a.g.nworlds > 0 && m.particle_world) ? world_index(m.particle_world[i], a.g.nworlds) : 0;
-  const float4 x4 = make_float4(x.x, x.y, x.z, pack_pf(pf, w));
-  const float mass = m.particle_mass[i];
-  xs[s] = x4;
-  scan_put(q, s, x, (pf & PF_ACTIVE) != 0);
-  vs[s] = make_float4(v.x, v.y, v.z, mass);
-  const float rd = m.rest_density[i];
-  mv[s] = rd * (mass / fmaxf(rd, 1.0e-6f));
-  const float r = a.rho[i];
-  sc2[s] = make_float2(a.pressure[i] / fmaxf(r * r, 1.0e-6f), 1.0f / fmaxf(r, 1.0e-6f));
-  nu[s] = m.viscosity[i];
-  coh[s] = m.surface_tension[i] / mass;
-  float3 ab = make_float3(0.f, 0.f, 0.f);
-  if (pf & PF_DYNAMIC) {
-    float3 xb, vb;
-    integrate_adjoint(walls_of(a.walls, a.g, w), x, v, ld3(a.accel, i), a.dt, ld3(a.xbo, i), ld3(a.vbo, i), xb, vb,
-                      ab);
+struct AdjGather {
+  AdjArgs a;
+  float *nu, *coh;
+  float4* xs;
+  ScanOut q;
+  float4* vs;
+  float* mv;
+  float2* sc2;
+  FS_DEV void operator()(int64_t s, int32_t i) const {
+    const fs_model& m = a.m;
+    const float3 x = ld3(a.xin, i), v = ld3(a.vin, i);
+    const int pf = particle_pf(m.particle_flags, m.particle_mask, i);
+    const int w = (a.g.nworlds > 0 && m.particle_world) ? world_index(m.particle_world[i], a.g.nworlds) : 0;
+    const float mass = m.particle_mass[i];
+    xs[s] = make_float4(x.x, x.y, x.z, pack_pf(pf, w));
+    scan_put(q, s, x, (pf & PF_ACTIVE) != 0);
+    vs[s] = make_float4(v.x, v.y, v.z, mass);
+    const float rd = m.rest_density[i];
+    mv[s] = rd * (mass / fmaxf(rd, 1.0e-6f));
+    const float r = a.rho[i];
+    sc2[s] = make_float2(a.pressure[i] / fmaxf(r * r, 1.0e-6f), 1.0f / fmaxf(r, 1.0e-6f));
+    nu[s] = m.viscosity[i];
+    coh[s] = m.surface_tension[i] / mass;
+    float3 ab = make_float3(0.f, 0.f, 0.f);
+    if (pf & PF_DYNAMIC) {
+      float3 xb, vb;
+      integrate_adjoint(walls_of(a.walls, a.g, w), x, v, ld3(a.accel, i), a.dt, ld3(a.xbo, i), ld3(a.vbo, i), xb, vb,
+                        ab);
+    }
+    a.ab[s] = make_float4(ab.x, ab.y, ab.z, 0.f);
   }
-  a.ab[s] = make_float4(ab.x, ab.y, ab.z, 0.f);
-}
+};
 
 // d (c d) / d(d) applied to ab:  rb = c ab + (ab . d) dc/dd, and the
 // velocity adjoint ub of the pair, for the term of a_i with neighbour j.
@@ -329,7 +333,6 @@ int fs_wcsph_substep_adjoint(fs_context* c, const fs_model* m, const fs_state* s
   const int64_t n = m->n;
   const float h = p->smoothing_length;
   int rc;
-  if ((rc = grid_build(c, si->particle_q, n, h * c->cell_ratio, st, m->particle_world))) return rc;
   AdjArgs a;
   a.g = grid_view(c);
   a.L = nbr_list(c);
@@ -361,10 +364,10 @@ int fs_wcsph_substep_adjoint(fs_context* c, const fs_model* m, const fs_state* s
   a.dt = p->dt;
   a.clamp = p->clamp_negative_pressure;
   a.walls = make_walls(p->bound_width, p->bound_height, p->bound_length, p->boundary_damping, 0, 0.f, 0.f);
-  {
-    PassScope ps_(c, P_ADJ_INTEGRATE, st);
-    k_adj_prepare<<<blocks_for(n), kBlock, 0, st>>>(a, c->sc1, c->sc1b, c->xs, scan_out(c), c->vs, c->mv, c->sc2);
-  }
+  if ((rc = grid_build(c, n, h * c->cell_ratio, st, m->particle_world, nullptr, KeyPositions{si->particle_q},
+                       AdjGather{a, c->sc1, c->sc1b, c->xs, scan_out(c), c->vs, c->mv, c->sc2})))
+    return rc;
+  a.g = grid_view(c);
   {
     PassScope ps_(c, P_ADJ_FORCE, st);
     FS_NB_LAUNCH(k_adj_force, c, n, nb_group(n), st, true, a);

@@ -13,20 +13,21 @@
 // individually rounded operations (no contraction into FMAs), as the
 // reference's float32 expression does, so the result equals the reference's
 // bit for bit.
-#include "fs_internal.cuh"
+#include "fs_build.cuh"
 
 namespace fs {
 namespace {
 
 // positions (original order) into cell order, with the active bit in .w
-__global__ void k_sep_gather(int64_t n, const int32_t* __restrict__ perm, const float* __restrict__ x,
-                             const int32_t* __restrict__ flags, float4* __restrict__ xs) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const int32_t i = perm[s];
-  const float3 p = ld3(x, i);
-  xs[s] = make_float4(p.x, p.y, p.z, pack_pf((flags[i] & 1) ? PF_ACTIVE : 0));
-}
+struct SepGather {
+  const float* x;
+  const int32_t* flags;
+  float4* xs;
+  FS_DEV void operator()(int64_t s, int32_t i) const {
+    const float3 p = ld3(x, i);
+    xs[s] = make_float4(p.x, p.y, p.z, pack_pf((flags[i] & 1) ? PF_ACTIVE : 0));
+  }
+};
 
 struct SepArgs {
   GridDev g;
@@ -127,11 +128,8 @@ int fs_apic_separation(fs_context* c, float* x, const int32_t* flags, int64_t n,
               hiz = p->bound_hi[2] - p->wall_margin;
   int rc;
   for (int it = 0; it < iters; ++it) {
-    if ((rc = grid_build(c, x, n, p->query_radius, st, nullptr))) return rc;
-    {
-      PassScope ps_(c, P_GATHER, st);
-      k_sep_gather<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, x, flags, c->xs);
-    }
+    if ((rc = grid_build(c, n, p->query_radius, st, nullptr, nullptr, KeyPositions{x}, SepGather{x, flags, c->xs})))
+      return rc;
     SepArgs a;
     a.g = grid_view(c);
     a.n = n;

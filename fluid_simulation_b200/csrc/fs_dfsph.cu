@@ -20,7 +20,7 @@
 // worlds are done.  Each scene iterates exactly as it would alone.
 #include <algorithm>
 
-#include "fs_nbr.cuh"
+#include "fs_build.cuh"
 
 namespace fs {
 
@@ -512,21 +512,28 @@ __global__ void k_kappa_ratio(int64_t n, const float* __restrict__ kappa, const 
   if (s < n) kratio[s] = make_float2(kappa[s] / fmaxf(sc2[s].x, 1.0e-6f), vm[s].w);
 }
 
-// integrate_positions (341-353); also publishes v* in original order.
-__global__ void k_integrate(int64_t n, const int32_t* __restrict__ perm, const float4* __restrict__ xs,
-                            const float4* __restrict__ vstar, float dt, float* x_out, float* vstar_api,
-                            const fs_frame_clock* clock) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n || clock_idle(clock)) return;
-  if (clock) dt = clock->dt;
-  const float4 xi = xs[s];
-  const float4 v = vstar[s];
-  const int32_t i = perm[s];
-  float3 p = xyz(xi);
-  if (pf_of(xi) & PF_DYNAMIC) p = make_float3(xi.x + v.x * dt, xi.y + v.y * dt, xi.z + v.z * dt);
-  st3(x_out, i, p);
-  st3(vstar_api, i, xyz(v));
-}
+// The second grid build's positions: integrate_positions (341-353) of the
+// particle in slot t of the first grid, made in the key pass; also publishes
+// v* in original order.
+struct KeyIntegrate {
+  const int32_t* perm;
+  const float4 *xs, *vstar;
+  float dt;
+  float *x_out, *vstar_api;
+  const fs_frame_clock* clock;
+  FS_DEV void reset() const {}
+  FS_DEV float3 position(int64_t t, int64_t& i) const {
+    const float step = clock ? clock->dt : dt;
+    const float4 xi = xs[t];
+    const float4 v = vstar[t];
+    i = perm[t];
+    float3 p = xyz(xi);
+    if (pf_of(xi) & PF_DYNAMIC) p = make_float3(xi.x + v.x * step, xi.y + v.y * step, xi.z + v.z * step);
+    st3(x_out, i, p);
+    st3(vstar_api, i, xyz(v));
+    return p;
+  }
+};
 
 // copy v* -> particle_qd then apply_bounds (407-442, unconditional damping);
 // batched contexts apply each world's own tank.
@@ -753,18 +760,11 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
       (rc = check_cuda(cudaMemsetAsync(c->dfsph_worlds, 0, sizeof(DfsphWorld) * 2 * c->nworlds, st), "dfsph reset")))
     return rc;
   // ---- first half: positions x_in
-  if ((rc = grid_build(c, si->particle_q, n, h, st, m->particle_world, c->clock))) return rc;
-  {
-    PassScope ps_(c, P_GATHER, st);
-    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, si->particle_q, si->particle_qd, c->xs, scan_out(c), c->vs,
-                                                    c->mv, c->status, c->nworlds);
-  }
-  {
-    // density/factor reads masses from vs2.w: fill it from vs (v_in, mass) first
-    if ((rc = check_cuda(cudaMemcpyAsync(c->vs2, c->vs, sizeof(float4) * n, cudaMemcpyDeviceToDevice, st),
-                         "dfsph copy")))
-      return rc;
-  }
+  // (vs2, too: density/factor reads its masses there)
+  if ((rc = grid_build(c, n, h, st, m->particle_world, c->clock, KeyPositions{si->particle_q},
+                       CommonGather{*m, si->particle_q, si->particle_qd, c->xs, scan_out(c), c->vs, c->vs2, c->mv,
+                                    c->status, c->nworlds})))
+    return rc;
   if ((rc = run_density_factor(c, m, h, p->min_neighbors_for_factor, so->rho, so->factor, so->neighbor_count, st)))
     return rc;
   AccelArgs aa;
@@ -801,19 +801,12 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
       return rc;
     if ((rc = run_correct(c, m, h, dt, c->sc1, c->krm, so->kappa, nullptr, c->dfsph + 0, st))) return rc;
   }
-  {
-    PassScope ps_(c, P_DFSPH_INTEGRATE, st);
-    k_integrate<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, c->xs, c->vs2, dt, so->particle_q, so->v_star,
-                                                   c->clock);
-  }
-  if ((rc = launch_check("dfsph integrate"))) return rc;
   // ---- second half: positions x_out
-  if ((rc = grid_build(c, so->particle_q, n, h, st, m->particle_world, c->clock))) return rc;
-  {
-    PassScope ps_(c, P_GATHER, st);
-    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, so->particle_q, so->v_star, c->xs, scan_out(c), c->vs2, c->mv,
-                                                    c->status, c->nworlds);
-  }
+  if ((rc = grid_build(c, n, h, st, m->particle_world, c->clock,
+                       KeyIntegrate{c->perm, c->xs, c->vs2, dt, so->particle_q, so->v_star, c->clock},
+                       CommonGather{*m, so->particle_q, so->v_star, c->xs, scan_out(c), c->vs2, nullptr, c->mv,
+                                    c->status, c->nworlds})))
+    return rc;
   if ((rc = run_density_factor(c, m, h, p->min_neighbors_for_factor, so->rho, so->factor, so->neighbor_count, st)))
     return rc;
   if (p->warm_start) {

@@ -4,15 +4,15 @@
 // Result (identical to a stable radix sort of (cell key, particle id)):
 //   perm[s]      original index of the particle in sorted slot s
 //   off[c]       first slot of cell c; off[c+1] one past its last slot
-// Algorithm (O(N) + O(cells) HBM traffic, deterministic):
+// Algorithm (O(N) + O(cells) HBM traffic, deterministic; fs_build.cuh):
 //   1. keys:    cell key per particle, arrival slot by atomicAdd on the cell count
-//   2. scan:    exclusive prefix of the counts (tile sums, then a down-sweep
-//               in which each tile adds up the sums before it)
+//   2. scan:    exclusive prefix of the counts, each tile adding up the sums of
+//               the tiles before it
 //   3. scatter: tmp[off[key] + arrival] = i        (order inside a cell arbitrary)
 //   4. rank:    slot = off[key] + #{j in cell : j < i}; perm[slot] = i, for
-//               cells of up to kSmallCell particles
-//   5. crowded cells: one block sorts each cell's ids (fs_sort.cuh)
-// Steps 4-5 restore ascending original index inside each cell, which is the
+//               cells of up to kSmallCell particles; a more crowded cell's ids
+//               are sorted by one block (fs_sort.cuh)
+// Step 4 restores ascending original index inside each cell, which is the
 // order warp's stable radix sort produces, so results do not depend on the
 // order in which atomics were served; the work is O(N) at any occupancy.
 // Non-finite positions are not binned into a cell: they take the extra key
@@ -22,95 +22,29 @@
 #include <cstdio>
 #include <cstring>
 
-#include "fs_nbr.cuh"
-#include "fs_sort.cuh"
+#include "fs_build.cuh"
 
 namespace fs {
 
 namespace {
 
-constexpr int kScanThreads = 512;
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;  // 4096 cells per block
-
 // A thread's kScanItems consecutive counts: two 16-byte loads when all lie
-// below m (base is a multiple of 8, the arrays come from cudaMalloc).
-__device__ __forceinline__ void load_items(const int32_t* __restrict__ in, int64_t base, int64_t m,
-                                           int32_t (&v)[kScanItems]) {
+// below m (base is a multiple of 8, the arrays come from cudaMalloc).  The
+// counts that are not zero are cleared for the next build.
+__device__ __forceinline__ void take_items(int32_t* in, int64_t base, int64_t m, int32_t (&v)[kScanItems]) {
   static_assert(kScanItems == 8, "two int4 per thread");
   if (base + kScanItems <= m) {
-    const int4 a = __ldg(reinterpret_cast<const int4*>(in + base));
-    const int4 b = __ldg(reinterpret_cast<const int4*>(in + base) + 1);
+    int4* const p = reinterpret_cast<int4*>(in + base);
+    const int4 a = p[0], b = p[1], zero = make_int4(0, 0, 0, 0);
+    if (a.x | a.y | a.z | a.w) p[0] = zero;
+    if (b.x | b.y | b.z | b.w) p[1] = zero;
     v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
   } else {
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) v[k] = base + k < m ? in[base + k] : 0;
-  }
-}
-
-__global__ void k_cell_keys(int64_t n, const float* __restrict__ x, float inv, int dim_x, int dim_y, int dim_z,
-                            int rounding, int32_t discard, int32_t* __restrict__ key, int32_t* __restrict__ slot,
-                            int32_t* __restrict__ count, int32_t* big_n, uint32_t* status,
-                            const fs_frame_clock* clock) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || clock_idle(clock)) return;
-  if (i == 0) *big_n = 0;  // crowded cells of this build, counted by k_rank
-  const float px = x[3 * i], py = x[3 * i + 1], pz = x[3 * i + 2];
-  int k = discard;
-  if (!(isfinite(px) && isfinite(py) && isfinite(pz))) {
-    atomicOr(status, FS_STATUS_NONFINITE);
-  } else {
-    GridDev g;
-    g.dim_x = dim_x;
-    g.dim_y = dim_y;
-    g.dim_z = dim_z;
-    g.mask_x = g.mask_y = g.mask_z = -1;
-    k = phys_cell(g, to_cell(__fmul_rn(px, inv), rounding), to_cell(__fmul_rn(py, inv), rounding),
-                  to_cell(__fmul_rn(pz, inv), rounding));
-  }
-  key[i] = k;
-  slot[i] = atomicAdd(count + k, 1);
-}
-
-// Batched contexts: key = (world, cell) as the world's base + its local cell.
-__global__ void k_cell_keys_worlds(int64_t n, const float* __restrict__ x, const int32_t* __restrict__ world,
-                                   const WorldDev* __restrict__ worlds, int nworlds, float inv, int32_t discard,
-                                   int32_t* __restrict__ key, int32_t* __restrict__ slot,
-                                   int32_t* __restrict__ count, int32_t* big_n, uint32_t* status,
-                                   const fs_frame_clock* clock) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || clock_idle(clock)) return;
-  if (i == 0) *big_n = 0;
-  const float px = x[3 * i], py = x[3 * i + 1], pz = x[3 * i + 2];
-  const int w = world[i];
-  if (w < 0 || w >= nworlds) atomicOr(status, FS_STATUS_BOUNDS);
-  int k = discard;
-  if (!(isfinite(px) && isfinite(py) && isfinite(pz)))
-    atomicOr(status, FS_STATUS_NONFINITE);
-  else
-    k = world_cell_key(worlds[world_index(w, nworlds)], inv, px, py, pz);
-  key[i] = k;
-  slot[i] = atomicAdd(count + k, 1);
-}
-
-// phase 1: per-tile sums
-__global__ void k_scan_reduce(const int32_t* __restrict__ in, int64_t m, int32_t* __restrict__ part,
-                              const fs_frame_clock* clock) {
-  if (clock_idle(clock)) return;
-  __shared__ int32_t warp_sums[kScanThreads / 32];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
-  int32_t v[kScanItems];
-  load_items(in, base, m, v);
-  int32_t s = 0;
-#pragma unroll
-  for (int k = 0; k < kScanItems; ++k) s += v[k];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int32_t v = threadIdx.x < kScanThreads / 32 ? warp_sums[threadIdx.x] : 0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (threadIdx.x == 0) part[blockIdx.x] = v;
+    for (int k = 0; k < kScanItems; ++k) {
+      v[k] = base + k < m ? in[base + k] : 0;
+      if (v[k]) in[base + k] = 0;
+    }
   }
 }
 
@@ -143,19 +77,31 @@ __device__ int32_t block_exclusive_scan(int32_t v, int32_t* total) {
   return res;
 }
 
-// phase 2: scan inside tiles, offset by the sum of the preceding tiles
-// counts (each block adds up part[0 .. blockIdx.x) itself: at most a few
-// thousand integers, exact in any order); out has m + 1 entries
-__global__ void k_scan_down(const int32_t* __restrict__ in, int64_t m, const int32_t* __restrict__ part,
-                            int32_t* __restrict__ out, const fs_frame_clock* clock) {
+// Copies of the tile sums: enough to spread the atomics of a large key pass
+// (at 401,856 particles it takes 23 us with one copy, 13 with eight; at 20,000
+// one copy is as fast), few enough that the blocks of the scan, each adding up
+// all sums before its own, read little (at most 8 x 600 words).
+int tile_copies_max(int ntiles) { return ntiles <= 600 ? 8 : ntiles <= 1200 ? 4 : ntiles <= 2048 ? 2 : 1; }
+int tile_copies(int ntiles, int64_t n) { return n < 60000 ? 1 : tile_copies_max(ntiles); }
+
+// Scan inside tiles, offset by the sum of the preceding tiles' counts (each
+// block adds up the copies of part[0 .. blockIdx.x) itself: at most a few
+// thousand integers, exact in any order); out has m + 1 entries.  (One launch with
+// tiles that publish their sums and poll for those before them: 15.3 us at
+// 128^3 cells for this one's 7, the polling of a few lines by every block.)
+__global__ void __launch_bounds__(kScanThreads) k_scan(int32_t* __restrict__ in, int64_t m,
+                                                       const int32_t* __restrict__ part, int copies,
+                                                       int32_t* __restrict__ out, const fs_frame_clock* clock) {
   if (clock_idle(clock)) return;
   int32_t before = 0;
-  for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x) before += __ldcg(part + k);
-  int32_t prefix = 0;
-  block_exclusive_scan(before, &prefix);
+  for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x)
+#pragma unroll 8
+    for (int c = 0; c < copies; ++c) before += __ldcg(part + c * gridDim.x + k);
   const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
   int32_t v[kScanItems];
-  load_items(in, base, m, v);
+  take_items(in, base, m, v);
+  int32_t prefix = 0;
+  block_exclusive_scan(before, &prefix);
   int32_t s = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) s += v[k];
@@ -178,52 +124,14 @@ __global__ void k_scan_down(const int32_t* __restrict__ in, int64_t m, const int
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[m] = prefix + tile;
 }
 
+// Also clears the tile sums for the next build (the scan has read them).
 __global__ void k_scatter(int64_t n, const int32_t* __restrict__ key, const int32_t* __restrict__ slot,
-                          const int32_t* __restrict__ off, int32_t* __restrict__ tmp, const fs_frame_clock* clock) {
+                          const int32_t* __restrict__ off, int32_t* __restrict__ tmp, int32_t* tile_sum, int nsums,
+                          const fs_frame_clock* clock) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || clock_idle(clock)) return;
-  tmp[off[key[i]] + slot[i]] = (int32_t)i;
-}
-
-__global__ void k_rank(int64_t n, const int32_t* __restrict__ key, const int32_t* __restrict__ off,
-                       const int32_t* __restrict__ tmp, int32_t* __restrict__ perm, int32_t* __restrict__ skey,
-                       int32_t* big_cells, int32_t* big_n, const fs_frame_clock* clock) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n || clock_idle(clock)) return;
-  const int32_t i = tmp[s];
-  const int32_t c = key[i];
-  const int32_t a = off[c], b = off[c + 1];
-  if (b - a > kSmallCell) {  // crowded: sorted by k_big_sort
-    if (s == a) big_cells[atomicAdd(big_n, 1)] = c;
-    return;
-  }
-  int32_t rank = 0;
-  for (int32_t t = a; t < b; ++t) rank += tmp[t] < i ? 1 : 0;
-  perm[a + rank] = i;
-  skey[a + rank] = c;
-}
-
-// The crowded cells listed by k_rank, one block each (grid-stride over the
-// list): ids sorted ascending, then perm / skey written.
-__global__ void __launch_bounds__(kSortThreads) k_big_sort(int64_t n, const int32_t* __restrict__ off,
-                                                           int32_t* tmp, int32_t* perm, int32_t* skey,
-                                                           const int32_t* __restrict__ big_cells,
-                                                           const int32_t* __restrict__ big_n,
-                                                           const fs_frame_clock* clock) {
-  extern __shared__ int32_t sort_smem[];
   if (clock_idle(clock)) return;
-  const int nbig = *big_n;
-  const int bits = id_bits(n);
-  for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
-    const int32_t c = big_cells[b];
-    const int32_t a = off[c], len = off[c + 1] - a;
-    int32_t* sorted = block_sort_ids(tmp + a, perm + a, len, bits, sort_smem);
-    for (int k = threadIdx.x; k < len; k += blockDim.x) {
-      perm[a + k] = sorted[k];  // same element when sorted == perm + a
-      skey[a + k] = c;
-    }
-    __syncthreads();
-  }
+  for (int64_t k = i; k < nsums; k += (int64_t)gridDim.x * blockDim.x) tile_sum[k] = 0;
+  if (i < n) tmp[off[key[i]] + slot[i]] = (int32_t)i;
 }
 
 __global__ void k_tables(int64_t n, int64_t ncell, const int32_t* __restrict__ perm, const int32_t* __restrict__ key,
@@ -233,7 +141,7 @@ __global__ void k_tables(int64_t n, int64_t ncell, const int32_t* __restrict__ p
   if (t < n) {
     const int32_t i = perm[t];
     if (point_ids) point_ids[t] = i;
-    if (point_cells) point_cells[t] = key[i];  // == skey[t]
+    if (point_cells) point_cells[t] = key[i];
   }
   if (t < ncell) {
     if (cell_starts) cell_starts[t] = off[t];
@@ -259,8 +167,6 @@ __global__ void k_candidates(GridDev g, const float* __restrict__ q, const int32
 }  // namespace
 
 int scan_blocks(int64_t m) { return (int)((m + kScanTile - 1) / kScanTile); }
-
-constexpr int kBigSortBlocks = 148;  // one per SM
 
 NbrList nbr_list(const fs_context* c) {
   NbrList L;
@@ -295,7 +201,6 @@ GridDev grid_view(const fs_context* c) {
   GridDev g;
   g.off = c->cell_off;
   g.perm = c->perm;
-  g.skey = c->skey;
   g.dim_x = c->grid.dim_x;
   g.dim_y = c->grid.dim_y;
   g.dim_z = c->grid.dim_z;
@@ -311,47 +216,61 @@ GridDev grid_view(const fs_context* c) {
   return g;
 }
 
-int grid_build(fs_context* c, const float* x, int64_t n, float radius, cudaStream_t st, const int32_t* world,
-               const fs_frame_clock* clock) {
-  if (n < 0 || (n > 0 && !x) || !(radius > 0.f)) return set_error(FS_ERR_INVALID, "grid_build: bad arguments");
+int grid_prepare(fs_context* c, int64_t n, float radius, const int32_t* world, const fs_frame_clock* clock,
+                 KeyArgs* a) {
+  if (n < 0 || !(radius > 0.f)) return set_error(FS_ERR_INVALID, "grid_build: bad arguments");
   if (c->worlds && n > 0 && !world)
     return set_error(FS_ERR_INVALID, "grid_build: a batched context needs particle_world");
   if (n > c->capacity) return set_error(FS_ERR_CAPACITY, "grid_build: n=%lld > capacity=%lld", (long long)n,
                                         (long long)c->capacity);
-  const float inv = 1.0f / radius;
-  PassScope ps_(c, P_GRID, st, n > 0 ? 6 : 2);
+  a->g = grid_view(c);
+  a->g.inv = 1.0f / radius;
+  a->world = world;
+  a->discard = (int32_t)c->ncell;  // the bucket after the cells
+  a->key = c->key;
+  a->slot = c->slot;
+  a->count = c->cell_count;
+  a->tile_sum = c->scan_part;
+  a->ntiles = scan_blocks(c->ncell + 1);
+  a->copies = tile_copies(a->ntiles, n);
+  a->status = c->status;
+  a->ctl = (ListCtl*)c->nb_ctl;
+  a->clock = clock;
+  return FS_OK;
+}
+
+void grid_scan_scatter(fs_context* c, int64_t n, cudaStream_t st, const fs_frame_clock* clock) {
   // ncell + 1 buckets: the cells, then the non-finite positions
   const int64_t nbucket = c->ncell + 1;
-  const int32_t discard = (int32_t)c->ncell;
-  int rc = check_cuda(cudaMemsetAsync(c->cell_count, 0, sizeof(int32_t) * nbucket, st), "memset cell counts");
-  if (rc) return rc;
-  // a new grid invalidates recorded neighbour lists
-  rc = check_cuda(cudaMemsetAsync(c->nb_ctl, 0, sizeof(ListCtl), st), "memset list control");
-  if (rc) return rc;
-  if (n > 0 && c->worlds)
-    k_cell_keys_worlds<<<blocks_for(n), kBlock, 0, st>>>(n, x, world, c->worlds, c->nworlds, inv, discard, c->key,
-                                                         c->slot, c->cell_count, c->big_n, c->status, clock);
-  else if (n > 0)
-    k_cell_keys<<<blocks_for(n), kBlock, 0, st>>>(n, x, inv, c->grid.dim_x, c->grid.dim_y, c->grid.dim_z,
-                                                   c->grid.rounding, discard, c->key, c->slot, c->cell_count, c->big_n,
-                                                   c->status, clock);
-  const int nb = scan_blocks(nbucket);
-  k_scan_reduce<<<nb, kScanThreads, 0, st>>>(c->cell_count, nbucket, c->scan_part, clock);
-  k_scan_down<<<nb, kScanThreads, 0, st>>>(c->cell_count, nbucket, c->scan_part, c->cell_off, clock);
-  if (n > 0) {
-    k_scatter<<<blocks_for(n), kBlock, 0, st>>>(n, c->key, c->slot, c->cell_off, c->tmp_ids, clock);
-    k_rank<<<blocks_for(n), kBlock, 0, st>>>(n, c->key, c->cell_off, c->tmp_ids, c->perm, c->skey, c->big_cells,
-                                             c->big_n, clock);
-    // a few blocks, each taking crowded cells from the list (none: they return at once)
-    k_big_sort<<<kBigSortBlocks, kSortThreads, kSortSmemBytes, st>>>(n, c->cell_off, c->tmp_ids, c->perm, c->skey,
-                                                                      c->big_cells, c->big_n, clock);
-  }
-  rc = launch_check("grid_build");
+  const int nb = scan_blocks(nbucket), copies = tile_copies(nb, n);
+  k_scan<<<nb, kScanThreads, 0, st>>>(c->cell_count, nbucket, c->scan_part, copies, c->cell_off, clock);
+  if (n > 0)
+    k_scatter<<<blocks_for(n), kBlock, 0, st>>>(n, c->key, c->slot, c->cell_off, c->tmp_ids, c->scan_part,
+                                                    nb * copies, clock);
+}
+
+int grid_finish(fs_context* c, int64_t n, float radius, cudaStream_t st) {
+  int rc = launch_check("grid_build");
   if (rc) return rc;
   c->built_n = n;
-  c->built_inv = inv;
+  c->built_inv = 1.0f / radius;
   c->last_stream = st;
   return FS_OK;
+}
+
+// The build of a caller's positions, with nothing gathered.
+static int grid_build_positions(fs_context* c, const float* x, int64_t n, float radius, cudaStream_t st,
+                                const int32_t* world) {
+  if (n > 0 && !x) return set_error(FS_ERR_INVALID, "grid_build: bad arguments");
+  if (n > 0) return grid_build(c, n, radius, st, world, nullptr, KeyPositions{x}, NoGather{});
+  KeyArgs a;
+  int rc = grid_prepare(c, n, radius, world, nullptr, &a);
+  if (rc) return rc;
+  PassScope ps_(c, P_GRID, st, 1);
+  rc = check_cuda(cudaMemsetAsync(c->nb_ctl, 0, sizeof(ListCtl), st), "memset list control");
+  if (rc) return rc;
+  grid_scan_scatter(c, 0, st, nullptr);  // the counts are zero: so are the offsets
+  return grid_finish(c, n, radius, st);
 }
 
 }  // namespace fs
@@ -521,10 +440,8 @@ static int context_alloc(fs_context* c, int64_t capacity, int64_t ncell) {
   } allocs[] = {
       {(void**)&c->key, sizeof(int32_t) * cap},         {(void**)&c->slot, sizeof(int32_t) * cap},
       {(void**)&c->cell_count, sizeof(int32_t) * (ncell + 1)}, {(void**)&c->cell_off, sizeof(int32_t) * (ncell + 2)},
-      {(void**)&c->big_cells, sizeof(int32_t) * max_big_cells(cap)}, {(void**)&c->big_n, sizeof(int32_t)},
       {(void**)&c->tmp_ids, sizeof(int32_t) * cap},     {(void**)&c->perm, sizeof(int32_t) * cap},
-      {(void**)&c->skey, sizeof(int32_t) * cap},
-      {(void**)&c->scan_part, sizeof(int32_t) * (nb + 1)},
+      {(void**)&c->scan_part, sizeof(int32_t) * nb * tile_copies_max(nb)},
       {(void**)&c->xs, sizeof(float4) * cap},           {(void**)&c->xs2, sizeof(float4) * cap},
       {(void**)&c->sxyz, sizeof(float) * scan_floats(cap)},
       {(void**)&c->vs, sizeof(float4) * cap},           {(void**)&c->vs2, sizeof(float4) * cap},
@@ -552,6 +469,9 @@ static int context_alloc(fs_context* c, int64_t capacity, int64_t ncell) {
   if (!rc) rc = check_cuda(cudaMemset(c->dfsph, 0, sizeof(DfsphDev) * 2), "fs_context_create: memset");
   if (!rc) rc = check_cuda(cudaMemset(c->tile_stats, 0, sizeof(unsigned long long) * 8), "fs_context_create: memset");
   if (!rc) rc = check_cuda(cudaMemset(c->nb_ctl, 0, sizeof(ListCtl)), "fs_context_create: memset");
+  // zero between grid builds: each build clears what it counted
+  if (!rc) rc = check_cuda(cudaMemset(c->cell_count, 0, sizeof(int32_t) * (ncell + 1)), "fs_context_create: memset");
+  if (!rc) rc = check_cuda(cudaMemset(c->scan_part, 0, sizeof(int32_t) * nb * tile_copies_max(nb)), "fs_context_create: memset");
   if (rc) {
     fs_context_destroy(c);
     return rc;
@@ -565,7 +485,7 @@ int fs_context_destroy(fs_context* c) {
   if (!c) return FS_OK;
   DeviceGuard dg(c->device);
   timer_free(c->timer);
-  void* ps[] = {c->key, c->slot, c->cell_count, c->cell_off, c->big_cells, c->big_n, c->tmp_ids, c->perm, c->skey, c->scan_part, c->xs, c->xs2,
+  void* ps[] = {c->key, c->slot, c->cell_count, c->cell_off, c->tmp_ids, c->perm, c->scan_part, c->xs, c->xs2,
                 c->sxyz, c->vs, c->vs2, c->mv, c->sc2, c->sc1, c->sc1b, c->krm, c->xo_tmp, c->vo_tmp, c->red_part, c->red_cnt,
                 c->dfsph, c->status, c->tile_stats, c->nb_idx, c->nb_cnt, c->nb_ctl, c->worlds, c->metrics,
                 c->dfsph_worlds, c->pbf_disp};
@@ -581,7 +501,7 @@ int fs_grid_build(fs_context* c, const float* x, int64_t n, float radius, fs_str
   if (!c) return set_error(FS_ERR_INVALID, "fs_grid_build: null context");
   if (c->worlds) return set_error(FS_ERR_INVALID, "fs_grid_build: batched context, use fs_grid_build_worlds");
   DeviceGuard dg(c->device);
-  return grid_build(c, x, n, radius, (cudaStream_t)stream, nullptr);
+  return grid_build_positions(c, x, n, radius, (cudaStream_t)stream, nullptr);
 }
 
 int fs_grid_build_worlds(fs_context* c, const float* x, const int32_t* world, int64_t n, float radius,
@@ -589,7 +509,7 @@ int fs_grid_build_worlds(fs_context* c, const float* x, const int32_t* world, in
   if (!c) return set_error(FS_ERR_INVALID, "fs_grid_build_worlds: null context");
   if (!c->worlds) return set_error(FS_ERR_INVALID, "fs_grid_build_worlds: not a batched context");
   DeviceGuard dg(c->device);
-  return grid_build(c, x, n, radius, (cudaStream_t)stream, world);
+  return grid_build_positions(c, x, n, radius, (cudaStream_t)stream, world);
 }
 
 int fs_grid_tables(fs_context* c, int32_t* point_ids, int32_t* point_cells, int32_t* cell_starts,

@@ -62,7 +62,6 @@ struct GridDev {
   int32_t nworlds = 0;
   const int32_t* off;   // [ncell + 1] exclusive prefix of cell occupancy (hash-key order)
   const int32_t* perm;  // [n] sorted slot -> original particle index (warp's point_ids)
-  const int32_t* skey;  // [n] cell key of each sorted slot (warp's point_cells)
   int32_t dim_x, dim_y, dim_z, rounding;
   int32_t mask_x, mask_y, mask_z;  // dim - 1 when the dim is a power of two, else -1
   float inv;            // 1 / cell width, float32 as warp
@@ -83,14 +82,11 @@ struct fs_context {
   // grid build
   int32_t* key = nullptr;        // [cap] cell key of original particle i
   int32_t* slot = nullptr;       // [cap] arrival slot inside the cell
-  int32_t* cell_count = nullptr; // [ncell + 1]; the last bucket holds non-finite positions
+  int32_t* cell_count = nullptr; // [ncell + 1]; the last bucket holds non-finite positions (zero between builds)
   int32_t* cell_off = nullptr;   // [ncell + 2]
   int32_t* tmp_ids = nullptr;    // [cap] unordered-in-cell ids
-  int32_t* big_cells = nullptr;  // [max_big_cells(cap)] cells too crowded to rank in place
-  int32_t* big_n = nullptr;      // [1] how many
   int32_t* perm = nullptr;       // [cap] sorted slot -> original index
-  int32_t* skey = nullptr;       // [cap] cell key of each sorted slot
-  int32_t* scan_part = nullptr;  // [scan blocks + 1]
+  int32_t* scan_part = nullptr;  // [copies][scan blocks] occupancy of each tile of cells (zero between builds)
 
   // cell-sorted streams
   float4* xs = nullptr;   // positions + packed flags
@@ -197,13 +193,6 @@ struct PassScope {
     if (slot >= 0) cudaEventRecord(c->timer.ev[2 * slot + 1], st);
   }
 };
-
-// grid build (fs_grid.cu)
-// world: particle_world of the model (required by batched contexts, unused otherwise)
-// clock (optional): a device-side frame clock; its kernels do nothing while
-// clock->active == 0 (the frame is complete).
-int grid_build(fs_context* c, const float* x, int64_t n, float radius, cudaStream_t st, const int32_t* world,
-               const fs_frame_clock* clock = nullptr);
 
 // Whether a kernel of a clocked substep has work (no clock: always).
 __device__ __forceinline__ bool clock_idle(const fs_frame_clock* clock) { return clock && !clock->active; }

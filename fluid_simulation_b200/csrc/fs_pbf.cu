@@ -1,8 +1,9 @@
 // PBF substep on B200 (replaces SolverPBF.step, solver_pbf.py:676-954).
 //
-//   predict   v_pred = v + dt g; x_pred = x + dt v_pred; position bounds  (original order)
-//   grid build(x_pred)          -- the only build unless rebuild_grid_each_iteration
-//   gather    x_pred, v_pred, x_in, mass, flags -> cell order          (one pass)
+//   grid build(x_pred)          -- the only build unless rebuild_grid_each_iteration;
+//             its first kernel predicts (v_pred = v + dt g; x_pred = x + dt v_pred;
+//             position bounds; original order), its last gathers x_pred, v_pred,
+//             x_in, mass, flags into cell order
 //   density   (poly6)
 //   accel     non-pressure (PBF variant) + apply_non_pressure_prediction + bounds -> x_pred'
 //   repeat max_iterations:
@@ -12,7 +13,7 @@
 //   xsph      XSPH viscosity, copy to state_out, apply_bounds      (fused)
 // As in the reference, the candidate set of every pass after the build is the
 // one binned at build time, queried from the particle's current position.
-#include "fs_nbr.cuh"
+#include "fs_build.cuh"
 
 // The PBF neighbour kernels run fastest with a 64-register budget (1024
 // resident threads per SM, no spills): measured 3 % faster per substep on
@@ -29,35 +30,56 @@ __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_
 namespace {
 
 // predict_velocity_with_gravity (193-208) + predict_positions (212-224) +
-// apply_position_bounds (367-399); original order.
-__global__ void k_predict(int64_t n, fs_model m, GridDev g, const float* __restrict__ x, const float* __restrict__ v,
-                          float dt, Walls walls, float* __restrict__ x_pred, float* __restrict__ v_pred) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float3 p = ld3(x, i), u = ld3(v, i);
-  if (particle_pf(m.particle_flags, m.particle_mask, i) & PF_DYNAMIC) {
-    const float3 gv = gravity_of(m, i);
-    u = make_float3(u.x + dt * gv.x, u.y + dt * gv.y, u.z + dt * gv.z);
-    p = make_float3(p.x + dt * u.x, p.y + dt * u.y, p.z + dt * u.z);
-    clamp_position(walls_of_particle(walls, g, m, i), p);
+// apply_position_bounds (367-399) of particle i; original order.
+struct Predict {
+  fs_model m;
+  GridDev g;
+  const float *x, *v;
+  float dt;
+  Walls walls;
+  float *x_pred, *v_pred;
+  FS_DEV float3 operator()(int64_t i) const {
+    float3 p = ld3(x, i), u = ld3(v, i);
+    if (particle_pf(m.particle_flags, m.particle_mask, i) & PF_DYNAMIC) {
+      const float3 gv = gravity_of(m, i);
+      u = make_float3(u.x + dt * gv.x, u.y + dt * gv.y, u.z + dt * gv.z);
+      p = make_float3(p.x + dt * u.x, p.y + dt * u.y, p.z + dt * u.z);
+      clamp_position(walls_of_particle(walls, g, m, i), p);
+    }
+    st3(x_pred, i, p);
+    st3(v_pred, i, u);
+    return p;
   }
-  st3(x_pred, i, p);
-  st3(v_pred, i, u);
+};
+
+__global__ void k_predict(int64_t n, Predict predict) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) predict(i);
 }
 
+// The grid build's positions: the prediction, made in the key pass.
+struct KeyPredict {
+  Predict predict;
+  uint32_t* disp;  // the displacement since the lists' recording: none yet
+  FS_DEV void reset() const { *disp = 0; }
+  FS_DEV float3 position(int64_t t, int64_t& i) const {
+    i = t;
+    return predict(t);
+  }
+};
+
 // The common gather of x_pred / v_pred plus the substep's input positions
-// x_in (xin_s, for the velocity update) in one pass over the permutation.
-__global__ void k_gather_pbf(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x_pred,
-                             const float* __restrict__ v_pred, const float* __restrict__ x_in, float4* __restrict__ xs,
-                             ScanOut q, float4* __restrict__ vs, float* __restrict__ mv, float4* __restrict__ xin_s,
-                             uint32_t* status, int nworlds) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const int32_t i = perm[s];
-  gather_common_slot(s, i, m, x_pred, v_pred, xs, q, vs, mv, status, nworlds);
-  const float3 p = ld3(x_in, i);
-  xin_s[s] = make_float4(p.x, p.y, p.z, 0.f);
-}
+// x_in (xin_s, for the velocity update).
+struct PbfGather {
+  CommonGather common;
+  const float* x_in;
+  float4* xin_s;
+  FS_DEV void operator()(int64_t s, int32_t i) const {
+    common(s, i);
+    const float3 p = ld3(x_in, i);
+    xin_s[s] = make_float4(p.x, p.y, p.z, 0.f);
+  }
+};
 
 // compute_density (115-141), poly6, self included.  sc2[s] = (rho,
 // mass / max(rho, 1e-6)): the neighbour term of the viscosity and XSPH passes.
@@ -452,14 +474,10 @@ __global__ void k_gather_lambda_mass(int64_t n, const int32_t* __restrict__ perm
   if (s < n) out[s] = make_float2(lam[perm[s]], vs[s].w);
 }
 
-int gather_pbf(fs_context* c, const fs_model* m, const float* x_in, cudaStream_t st) {
-  const int64_t n = m->n;
-  {
-    PassScope ps_(c, P_GATHER, st);
-    k_gather_pbf<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, c->xo_tmp, c->vo_tmp, x_in, c->xs, scan_out(c),
-                                                   c->vs, c->mv, c->vs2, c->status, c->nworlds);
-  }
-  return launch_check("pbf gather");
+PbfGather pbf_gather(fs_context* c, const fs_model* m, const float* x_in) {
+  return PbfGather{CommonGather{*m, c->xo_tmp, c->vo_tmp, c->xs, scan_out(c), c->vs, nullptr, c->mv, c->status,
+                                c->nworlds},
+                   x_in, c->vs2};
 }
 
 }  // namespace
@@ -487,14 +505,10 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   const Walls w = make_walls(p->bound_width, p->bound_height, p->bound_length, p->boundary_damping, 2,
                              p->particle_radius, p->boundary_epsilon);
   int rc;
-  {
-    PassScope ps_(c, P_PBF_PREDICT, st);
-    k_predict<<<blocks_for(n), kBlock, 0, st>>>(n, *m, grid_view(c), si->particle_q, si->particle_qd, dt, w, c->xo_tmp,
-                                                c->vo_tmp);
-  }
-  if ((rc = launch_check("pbf predict"))) return rc;
-  if ((rc = grid_build(c, c->xo_tmp, n, h, st, m->particle_world))) return rc;
-  if ((rc = gather_pbf(c, m, si->particle_q, st))) return rc;
+  const Predict predict{*m, grid_view(c), si->particle_q, si->particle_qd, dt, w, c->xo_tmp, c->vo_tmp};
+  if ((rc = grid_build(c, n, h, st, m->particle_world, nullptr, KeyPredict{predict, c->pbf_disp},
+                       pbf_gather(c, m, si->particle_q))))
+    return rc;
   const GridDev g = grid_view(c);
   // neighbour lists: density -> accel, lambda -> delta, final density -> XSPH
   const NbrList L = nbr_list(c);
@@ -506,8 +520,6 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   // 0.003 h in the 401,856-particle dam break, well inside the default
   // 0.02 h skin (+6 % list entries).
   const float skin = (!p->rebuild_grid_each_iteration && p->max_iterations > 0) ? c->list_skin : 0.f;
-  if (skin > 0.f && (rc = check_cuda(cudaMemsetAsync(c->pbf_disp, 0, sizeof(uint32_t), st), "pbf reset")))
-    return rc;
   {
     PassScope ps_(c, P_PBF_DENSITY, st);
     FS_NB_LAUNCH(k_density, c, n, group, st, true, g, L, scan_xyz(c), n, c->xs, c->vs, c->mv, h, skin, so->rho, c->sc2,
@@ -594,8 +606,9 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
         PassScope ps_(c, P_GATHER, st);
         k_scatter_x<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, cur, c->xo_tmp);
       }
-      if ((rc = grid_build(c, c->xo_tmp, n, h, st, m->particle_world))) return rc;
-      if ((rc = gather_pbf(c, m, si->particle_q, st))) return rc;
+      if ((rc = grid_build(c, n, h, st, m->particle_world, nullptr, KeyPositions{c->xo_tmp},
+                           pbf_gather(c, m, si->particle_q))))
+        return rc;
       cur = c->xs;
       nxt = c->xs2;
     }
@@ -641,7 +654,7 @@ int fs_pbf_predict(fs_context* c, const fs_model* m, const float* x, const float
   cudaStream_t st = (cudaStream_t)stream;
   const Walls w = make_walls(p->bound_width, p->bound_height, p->bound_length, p->boundary_damping, 2,
                              p->particle_radius, p->boundary_epsilon);
-  k_predict<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, *m, grid_view(c), x, v, p->dt, w, x_pred, v_pred);
+  k_predict<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, Predict{*m, grid_view(c), x, v, p->dt, w, x_pred, v_pred});
   return launch_check("fs_pbf_predict");
 }
 

@@ -2,13 +2,13 @@
 //
 // Pass structure (one thread per cell-sorted slot; neighbour reads are
 // contiguous slot ranges of the cell-sorted streams):
-//   grid build(x_in)                       -- fs_grid.cu
-//   gather    x_in, v_in, mass, flags      -> xs, vs, mv     (cell order)
+//   grid build(x_in)                       -- fs_build.cuh; its last kernel gathers
+//             x_in, v_in, mass, flags      -> xs, vs, mv     (cell order)
 //   density   rho, p (EOS)                 -> sc2 (cell order) + rho/pressure (original order)
 //   force     pressure + viscosity + cohesion + gravity, then
 //             integrate_velocity, integrate_positions and apply_bounds fused
 //             -> accel, particle_qd, particle_q (original order)
-#include "fs_nbr.cuh"
+#include "fs_build.cuh"
 
 namespace fs {
 
@@ -198,6 +198,14 @@ int wcsph_gather(fs_context* c, const fs_model* m, const float* x, const float* 
   return launch_check("wcsph gather");
 }
 
+// The grid of the substep's input positions, gathered into cell order.
+static int wcsph_build(fs_context* c, const fs_model* m, const fs_state* si, float h, cudaStream_t st,
+                       const fs_frame_clock* clock) {
+  return grid_build(c, m->n, h * c->cell_ratio, st, m->particle_world, clock, KeyPositions{si->particle_q},
+                    CommonGather{*m, si->particle_q, si->particle_qd, c->xs, scan_out(c), c->vs, nullptr, c->mv,
+                                 c->status, c->nworlds});
+}
+
 int launch_density(fs_context* c, const fs_model* m, float h, int clamp, bool eos, float* rho, float* pressure,
                    cudaStream_t st, const fs_frame_clock* clock = nullptr) {
   DensityArgs a;
@@ -278,8 +286,7 @@ int fs_wcsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_st
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   const float h = p->smoothing_length;
-  if ((rc = grid_build(c, si->particle_q, m->n, h * c->cell_ratio, st, m->particle_world))) return rc;
-  if ((rc = wcsph_gather(c, m, si->particle_q, si->particle_qd, st))) return rc;
+  if ((rc = wcsph_build(c, m, si, h, st, nullptr))) return rc;
   if ((rc = launch_density(c, m, h, p->clamp_negative_pressure, true, so->rho, so->pressure, st))) return rc;
   return launch_force(c, m, p, accel, so->particle_q, so->particle_qd, st, true);
 }
@@ -297,8 +304,7 @@ int fs_wcsph_substep_clocked(fs_context* c, const fs_model* m, const fs_state* s
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   const float h = p->smoothing_length;
-  if ((rc = grid_build(c, si->particle_q, m->n, h * c->cell_ratio, st, m->particle_world, clock))) return rc;
-  if ((rc = wcsph_gather(c, m, si->particle_q, si->particle_qd, st))) return rc;
+  if ((rc = wcsph_build(c, m, si, h, st, clock))) return rc;
   if ((rc = launch_density(c, m, h, p->clamp_negative_pressure, true, so->rho, so->pressure, st, clock))) return rc;
   if ((rc = launch_force(c, m, p, accel, so->particle_q, so->particle_qd, st, true, clock))) return rc;
   {
