@@ -190,6 +190,7 @@ FS_DEV PairAdj pair_adjoint(const Cubic& K, float h, float particle_radius, floa
 template <int G>
 __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
   extern __shared__ uint2 smem[];
+  grid_begin();
   lists_recorded(a.L);
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xk = a.xs[s];
@@ -283,6 +284,7 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
 
 template <int G>
 __global__ void FS_NB_BOUNDS k_adj_density(AdjArgs a) {
+  grid_begin();
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xk = a.xs[s];
     const bool on = live && (pf_of(xk) & PF_ACTIVE);

@@ -40,7 +40,8 @@ struct SepArgs {
 
 // accumulate_particle_separation
 __global__ void k_sep_accumulate(SepArgs a) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t s = thread_id();
   if (s >= a.n) return;
   const float4 xi = a.xs[s];
   const int32_t i = a.g.perm[s];
@@ -95,7 +96,8 @@ FS_DEV float clamp_ref(float v, float lo, float hi) {  // min(max(v, lo), hi) wi
 // apply_particle_separation_delta
 __global__ void k_sep_apply(int64_t n, const int32_t* __restrict__ flags, const float* __restrict__ delta, float lox,
                             float loy, float loz, float hix, float hiy, float hiz, float* __restrict__ x) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t i = thread_id();
   if (i >= n || !(flags[i] & 1)) return;
   const float3 p = ld3(x, i), d = ld3(delta, i);
   st3(x, i, make_float3(clamp_ref(__fadd_rn(p.x, d.x), lox, hix), clamp_ref(__fadd_rn(p.y, d.y), loy, hiy),
@@ -145,8 +147,8 @@ int fs_apic_separation(fs_context* c, float* x, const int32_t* flags, int64_t n,
     a.delta = delta;
     {
       PassScope ps_(c, P_APIC_SEPARATION, st, 2);
-      k_sep_accumulate<<<blocks_for(n), kBlock, 0, st>>>(a);
-      k_sep_apply<<<blocks_for(n), kBlock, 0, st>>>(n, flags, delta, lox, loy, loz, hix, hiy, hiz, x);
+      launch(k_sep_accumulate, blocks_for(n), kBlock, 0, st, a);
+      launch(k_sep_apply, blocks_for(n), kBlock, 0, st, n, flags, delta, lox, loy, loz, hix, hiy, hiz, x);
     }
     if ((rc = launch_check("fs_apic_separation"))) return rc;
   }

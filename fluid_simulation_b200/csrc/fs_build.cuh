@@ -74,7 +74,8 @@ struct CommonGather {
 
 template <class Key>
 __global__ void k_cell_keys(int64_t n, Key source, KeyArgs a) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t t = thread_id();
   if (t == 0) {
     source.reset();
     a.ctl->valid = 0;  // a new grid invalidates recorded neighbour lists
@@ -122,10 +123,11 @@ __global__ void __launch_bounds__(kRankThreads) k_rank(int64_t n, const int32_t*
   __shared__ int32_t smem[kSortSmemInts];
   __shared__ int32_t crowded[kRankThreads / kSmallCell + 1];
   __shared__ int ncrowded;
+  grid_begin();
   if (clock_idle(clock)) return;
   if (threadIdx.x == 0) ncrowded = 0;
   __syncthreads();
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t s = thread_id();
   if (s < n) {
     const int32_t i = tmp[s];
     const int32_t c = key[i];
@@ -171,9 +173,9 @@ int grid_build(fs_context* c, int64_t n, float radius, cudaStream_t st, const in
   int rc = grid_prepare(c, n, radius, world, clock, &a);
   if (rc) return rc;
   PassScope ps_(c, P_GRID, st, 4);
-  k_cell_keys<<<blocks_for(n), kBlock, sizeof(int32_t) * a.ntiles, st>>>(n, source, a);
+  launch(k_cell_keys<Key>, blocks_for(n), kBlock, sizeof(int32_t) * a.ntiles, st, n, source, a);
   grid_scan_scatter(c, n, st, clock);
-  k_rank<<<blocks_for(n, kRankThreads), kRankThreads, 0, st>>>(n, c->key, c->cell_off, c->tmp_ids, c->perm, gather,
+  launch(k_rank<Gather>, blocks_for(n, kRankThreads), kRankThreads, 0, st, n, c->key, c->cell_off, c->tmp_ids, c->perm, gather,
                                                                clock);
   return grid_finish(c, n, radius, st);
 }

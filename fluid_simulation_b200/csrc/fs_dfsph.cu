@@ -54,7 +54,8 @@ __global__ void k_gather_pair(int64_t n, const int32_t* __restrict__ perm, const
 
 __global__ void k_gather_scalar(int64_t n, const int32_t* __restrict__ perm, const float* __restrict__ a,
                                 float* __restrict__ out, float* __restrict__ copy_to) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t s = thread_id();
   if (s >= n) return;
   const int32_t i = perm[s];
   const float v = a[i];
@@ -88,6 +89,7 @@ struct DensFactorArgs {
 template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, 3) k_density_factor(DensFactorArgs a) {
   extern __shared__ uint2 smem[];
+  grid_begin();
   if (clock_idle(a.clock)) return;
   lists_recorded(a.L);
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
@@ -151,6 +153,7 @@ struct AccelArgs {
 
 template <int G>
 __global__ void FS_NB_BOUNDS k_accel_predict(AccelArgs a) {
+  grid_begin();
   if (clock_idle(a.clock)) return;
   const float dt = a.clock ? a.clock->dt : a.dt;
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
@@ -322,6 +325,7 @@ __device__ bool last_block(uint32_t* ticket) {
 
 template <int G>
 __global__ void FS_NB_BOUNDS k_rate(RateArgs a) {
+  grid_begin();
   if (a.ctrl && a.ctrl->done) return;  // uniform across the grid: set by an earlier launch
   if (clock_idle(a.clock)) return;     // uniform: the frame is complete
   const float dt = a.clock ? a.clock->dt : a.dt;
@@ -388,6 +392,7 @@ constexpr int kWorldBlock = 512;  // threads per world of the residual pass
 __global__ void __launch_bounds__(kWorldBlock) k_world_residual(GridDev g, const float* __restrict__ term,
                                                                 DfsphWorld* wctl, DfsphDev* gctl, int it, float eta,
                                                                 const fs_frame_clock* clock) {
+  grid_begin();
   if (gctl->done || clock_idle(clock)) return;
   const int w = blockIdx.x;
   DfsphWorld& W = wctl[w];
@@ -466,6 +471,7 @@ struct CorrectArgs {
 // otherwise settles at 48 registers and spills; 3.7 % faster measured).
 template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, 4) k_correct(CorrectArgs a) {
+  grid_begin();
   if (a.ctrl && a.ctrl->done) return;
   if (clock_idle(a.clock)) return;
   const float dt = a.clock ? a.clock->dt : a.dt;
@@ -508,7 +514,8 @@ __global__ void __launch_bounds__(kNbBlockMax, 4) k_correct(CorrectArgs a) {
 // kappa / max(rho, 1e-6) of gathered kappas (warm start, separate pass)
 __global__ void k_kappa_ratio(int64_t n, const float* __restrict__ kappa, const float2* __restrict__ sc2,
                               const float4* __restrict__ vm, float2* __restrict__ kratio) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t s = thread_id();
   if (s < n) kratio[s] = make_float2(kappa[s] / fmaxf(sc2[s].x, 1.0e-6f), vm[s].w);
 }
 
@@ -539,7 +546,8 @@ struct KeyIntegrate {
 // batched contexts apply each world's own tank.
 __global__ void k_final(int64_t n, GridDev g, const float4* __restrict__ xs, const float4* __restrict__ vstar,
                         Walls walls, float* x_out, float* v_out, float* vstar_api, const fs_frame_clock* clock) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t s = thread_id();
   if (s >= n || clock_idle(clock)) return;
   const float4 xi = xs[s];
   const float4 v4 = vstar[s];
@@ -608,7 +616,7 @@ int run_rate(fs_context* c, const fs_model* m, int mode, int it, float h, float 
     PassScope ps_(c, P_DFSPH_RATE, st, per_world ? 2 : 1);
     FS_NB_LAUNCH(k_rate, c, a.n, group, st, false, a);
     if (per_world)
-      k_world_residual<<<c->nworlds, kWorldBlock, 0, st>>>(a.g, c->sc1b, c->dfsph_worlds + (ctrl - c->dfsph) * c->nworlds,
+      launch(k_world_residual, c->nworlds, kWorldBlock, 0, st, a.g, c->sc1b, c->dfsph_worlds + (ctrl - c->dfsph) * c->nworlds,
                                                            ctrl, it, eta, c->clock);
   }
   return launch_check("dfsph rate");
@@ -680,7 +688,8 @@ namespace {
 // A clocked substep after its frame is complete: state_out = state_in for
 // every field both states give.
 __global__ void k_idle_copy_dfsph(int64_t n, const fs_frame_clock* clock, fs_state si, fs_state so) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t i = thread_id();
   if (i >= n || !clock_idle(clock)) return;
   st3(so.particle_q, i, ld3(si.particle_q, i));
   st3(so.particle_qd, i, ld3(si.particle_qd, i));
@@ -726,7 +735,7 @@ int fs_dfsph_substep_clocked(fs_context* c, const fs_model* m, const fs_state* s
   cudaStream_t st = (cudaStream_t)stream;
   {
     PassScope ps_(c, P_OTHER, st);
-    k_idle_copy_dfsph<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, clock, *si, *so);
+    launch(k_idle_copy_dfsph, blocks_for(m->n), kBlock, 0, st, m->n, clock, *si, *so);
   }
   return launch_check("fs_dfsph_substep_clocked");
 }
@@ -790,8 +799,8 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
   if (p->warm_start) {
     {
       PassScope ps_(c, P_GATHER, st, 2);
-      k_gather_scalar<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, si->kappa, c->sc1, nullptr);
-      k_kappa_ratio<<<blocks_for(n), kBlock, 0, st>>>(n, c->sc1, c->sc2, c->vs2, c->krm);
+      launch(k_gather_scalar, blocks_for(n), kBlock, 0, st, n, c->perm, si->kappa, c->sc1, nullptr);
+      launch(k_kappa_ratio, blocks_for(n), kBlock, 0, st, n, c->sc1, c->sc2, c->vs2, c->krm);
     }
     if ((rc = run_correct(c, m, h, dt, c->sc1, c->krm, so->kappa, nullptr, nullptr, st))) return rc;
   }
@@ -812,8 +821,8 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
   if (p->warm_start) {
     {
       PassScope ps_(c, P_GATHER, st, 2);
-      k_gather_scalar<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, si->kappa_v, c->sc1, nullptr);
-      k_kappa_ratio<<<blocks_for(n), kBlock, 0, st>>>(n, c->sc1, c->sc2, c->vs2, c->krm);
+      launch(k_gather_scalar, blocks_for(n), kBlock, 0, st, n, c->perm, si->kappa_v, c->sc1, nullptr);
+      launch(k_kappa_ratio, blocks_for(n), kBlock, 0, st, n, c->sc1, c->sc2, c->vs2, c->krm);
     }
     if ((rc = run_correct(c, m, h, dt, c->sc1, c->krm, so->kappa_v, nullptr, nullptr, st))) return rc;
   }
@@ -826,7 +835,7 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
   const Walls w = make_walls(p->bound_width, p->bound_height, p->bound_length, p->boundary_damping, 1, 0.f, 0.f);
   {
     PassScope ps_(c, P_DFSPH_FINAL, st);
-    k_final<<<blocks_for(n), kBlock, 0, st>>>(n, grid_view(c), c->xs, c->vs2, w, so->particle_q, so->particle_qd,
+    launch(k_final, blocks_for(n), kBlock, 0, st, n, grid_view(c), c->xs, c->vs2, w, so->particle_q, so->particle_qd,
                                               so->v_star, c->clock);
   }
   c->last_stream = st;
@@ -934,7 +943,7 @@ int fs_dfsph_nonpressure_predict(fs_context* c, const fs_model* m, const float* 
   aa.accel = accel;
   aa.vstar = c->vs2;
   aa.clock = nullptr;
-  k_accel_predict<1><<<nb_blocks(c, n), c->nb_block, 0, st>>>(aa);
+  launch(k_accel_predict<1>, nb_blocks(c, n), c->nb_block, 0, st, aa);
   k_scatter_xyz<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, c->vs2, v_star);
   return launch_check("fs_dfsph_nonpressure_predict");
 }
@@ -963,10 +972,10 @@ int fs_dfsph_correct(fs_context* c, const fs_model* m, const float* x, float* v_
   k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v_star, c->xs, scan_out(c), c->vs2, nullptr,
                                                        c->status, c->nworlds);
   k_gather_pair<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, rho, nullptr, c->sc2);
-  k_gather_scalar<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, kappa, c->sc1, nullptr);
+  launch(k_gather_scalar, blocks_for(m->n), kBlock, 0, st, m->n, c->perm, kappa, c->sc1, nullptr);
   {
     PassScope ps_(c, P_GATHER, st);
-    k_kappa_ratio<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->sc1, c->sc2, c->vs2, c->krm);
+    launch(k_kappa_ratio, blocks_for(m->n), kBlock, 0, st, m->n, c->sc1, c->sc2, c->vs2, c->krm);
   }
   return run_correct(c, m, h, dt, c->sc1, c->krm, nullptr, v_star, nullptr, st, false);
 }

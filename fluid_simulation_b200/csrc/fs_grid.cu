@@ -92,6 +92,7 @@ int tile_copies(int ntiles, int64_t n) { return n < 60000 ? 1 : tile_copies_max(
 __global__ void __launch_bounds__(kScanThreads) k_scan(int32_t* __restrict__ in, int64_t m,
                                                        const int32_t* __restrict__ part, int copies,
                                                        int32_t* __restrict__ out, const fs_frame_clock* clock) {
+  grid_begin();
   if (clock_idle(clock)) return;
   int32_t before = 0;
   for (int k = threadIdx.x; k < (int)blockIdx.x; k += blockDim.x)
@@ -128,7 +129,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(int32_t* __restrict__ in,
 __global__ void k_scatter(int64_t n, const int32_t* __restrict__ key, const int32_t* __restrict__ slot,
                           const int32_t* __restrict__ off, int32_t* __restrict__ tmp, int32_t* tile_sum, int nsums,
                           const fs_frame_clock* clock) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t i = thread_id();
   if (clock_idle(clock)) return;
   for (int64_t k = i; k < nsums; k += (int64_t)gridDim.x * blockDim.x) tile_sum[k] = 0;
   if (i < n) tmp[off[key[i]] + slot[i]] = (int32_t)i;
@@ -243,9 +245,9 @@ void grid_scan_scatter(fs_context* c, int64_t n, cudaStream_t st, const fs_frame
   // ncell + 1 buckets: the cells, then the non-finite positions
   const int64_t nbucket = c->ncell + 1;
   const int nb = scan_blocks(nbucket), copies = tile_copies(nb, n);
-  k_scan<<<nb, kScanThreads, 0, st>>>(c->cell_count, nbucket, c->scan_part, copies, c->cell_off, clock);
+  launch(k_scan, nb, kScanThreads, 0, st, c->cell_count, nbucket, c->scan_part, copies, c->cell_off, clock);
   if (n > 0)
-    k_scatter<<<blocks_for(n), kBlock, 0, st>>>(n, c->key, c->slot, c->cell_off, c->tmp_ids, c->scan_part,
+    launch(k_scatter, blocks_for(n), kBlock, 0, st, n, c->key, c->slot, c->cell_off, c->tmp_ids, c->scan_part,
                                                     nb * copies, clock);
 }
 

@@ -31,7 +31,8 @@ FS_DEV float block_max(float v) {
 // their bit patterns, so the cross-block maximum is an integer atomicMax.
 __global__ void k_norm_maxima(const float* __restrict__ v, int64_t nv, const float* __restrict__ a, int64_t na,
                               float* out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t i = thread_id();
   const float sv = i < nv ? sq_or_inf(ld3(v, i)) : 0.f;
   const float sa = i < na ? sq_or_inf(ld3(a, i)) : 0.f;
   const float bv = block_max(sv);
@@ -65,6 +66,7 @@ __global__ void k_clock_start(fs_frame_clock* c, double frame_dt) {
 // 185-196) on the device, in double precision as the Python harness
 // evaluates it; maxima[] were just reduced from the current state.
 __global__ void k_clock_rule(fs_frame_clock* c, fs_cfl_rule r) {
+  grid_begin();
   if (c->fault) {
     c->active = 0;
     return;
@@ -118,7 +120,7 @@ int fs_norm_maxima(const float* v, int64_t nv, const float* a, int64_t na, float
   if (rc) return rc;
   const int64_t m = nv > na ? nv : na;
   if (m == 0) return FS_OK;
-  k_norm_maxima<<<blocks_for(m), kBlock, 0, st>>>(v, nv, a, na, out);
+  launch(k_norm_maxima, blocks_for(m), kBlock, 0, st, v, nv, a, na, out);
   return launch_check("fs_norm_maxima");
 }
 
@@ -149,8 +151,8 @@ int fs_frame_clock_advance(fs_frame_clock* clock, const fs_cfl_rule* rule, const
   int rc = check_cuda(cudaMemsetAsync(clock->maxima, 0, sizeof(clock->maxima), st), "fs_frame_clock_advance: memset");
   if (rc) return rc;
   const int64_t m = nv > na ? nv : na;
-  if (m > 0) k_norm_maxima<<<blocks_for(m), kBlock, 0, st>>>(v, nv, accel, na, clock->maxima);
-  k_clock_rule<<<1, 1, 0, st>>>(clock, *rule);
+  if (m > 0) launch(k_norm_maxima, blocks_for(m), kBlock, 0, st, v, nv, accel, na, clock->maxima);
+  launch(k_clock_rule, 1, 1, 0, st, clock, *rule);
   return launch_check("fs_frame_clock_advance");
 }
 

@@ -734,7 +734,7 @@ FS_DEV void for_groups(int64_t n, F&& f) {
   if constexpr (G == 1) {
     for_slots(n, [&](int64_t s) { f(s, true, true); });
   } else {
-    const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+    const int64_t s = thread_id() / G;
     const bool live = s < n;
     f(live ? s : n - 1, live, live && (threadIdx.x & (G - 1)) == 0);
   }
@@ -745,8 +745,8 @@ int nb_group(int64_t n);
 
 // Launches KERNEL<G>(args) for n particles at the context's block size.
 #define FS_NB_CASE(KERNEL, G, SMEM, ...)                                                                      \
-  KERNEL<G><<<(unsigned)((n_ * G + c_->nb_block - 1) / c_->nb_block), c_->nb_block,                           \
-              (SMEM) ? scan_smem(c_->nb_block, G) : 0, st_>>>(__VA_ARGS__)
+  launch(KERNEL<G>, (unsigned)((n_ * G + c_->nb_block - 1) / c_->nb_block), c_->nb_block,                     \
+         (SMEM) ? scan_smem(c_->nb_block, G) : 0, st_, __VA_ARGS__)
 #define FS_NB_LAUNCH(KERNEL, c, n, group, st, SMEM, ...)                                                      \
   do {                                                                                                        \
     const fs_context* c_ = (c);                                                                               \
@@ -757,7 +757,8 @@ int nb_group(int64_t n);
       case 8: FS_NB_CASE(KERNEL, 8, SMEM, __VA_ARGS__); break;                                                \
       case 16: FS_NB_CASE(KERNEL, 16, SMEM, __VA_ARGS__); break;                                              \
       default:                                                                                                \
-        KERNEL<1><<<nb_blocks(c_, n_), c_->nb_block, (SMEM) ? scan_smem(c_->nb_block, 1) : 0, st_>>>(__VA_ARGS__); \
+        launch(KERNEL<1>, nb_blocks(c_, n_), c_->nb_block, (SMEM) ? scan_smem(c_->nb_block, 1) : 0, st_,      \
+               __VA_ARGS__);                                                                                 \
     }                                                                                                         \
   } while (0)
 

@@ -95,6 +95,7 @@ __global__ void FS_NB_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, int6
                                            float skin, float* rho, float2* __restrict__ sc2,
                                            const float4* __restrict__ xin, float dt, float4* __restrict__ vout) {
   extern __shared__ uint2 smem[];
+  grid_begin();
   lists_recorded(L);
   for_groups<G>(n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = xs[s];
@@ -150,6 +151,7 @@ struct AccelArgs {
 
 template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
+  grid_begin();
   float dmax = 0.f;
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
@@ -241,6 +243,7 @@ struct LambdaArgs {
 template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
   extern __shared__ uint2 smem[];
+  grid_begin();
   lists_recorded(a.L);
   const bool reuse_ok = a.xs_rec && __uint_as_float(*a.disp_max) <= a.reuse_limit;
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
@@ -332,6 +335,7 @@ FS_DEV float pow_uint(float x, int n) {
 
 template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
+  grid_begin();
   // an integral exponent 1..8 (the class default is 4) takes pow_uint
   const int n_int = (a.scorr_n >= 1.f && a.scorr_n <= 8.f && a.scorr_n == rintf(a.scorr_n)) ? (int)a.scorr_n : 0;
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
@@ -408,6 +412,7 @@ struct XsphArgs {
 
 template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_xsph_final(XsphArgs a) {
+  grid_begin();
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const float4 vi = a.vel[s];
@@ -445,7 +450,8 @@ __global__ void FS_NB_BOUNDS_PBF k_xsph_final(XsphArgs a) {
 
 __global__ void k_scatter_x(int64_t n, const int32_t* __restrict__ perm, const float4* __restrict__ xs,
                             float* __restrict__ x) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t s = thread_id();
   if (s >= n) return;
   st3(x, perm[s], xyz(xs[s]));
 }
@@ -604,7 +610,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
       // x_pred back to original order, rebuild, regather (v_pred/x_in follow)
       {
         PassScope ps_(c, P_GATHER, st);
-        k_scatter_x<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, cur, c->xo_tmp);
+        launch(k_scatter_x, blocks_for(n), kBlock, 0, st, n, c->perm, cur, c->xo_tmp);
       }
       if ((rc = grid_build(c, n, h, st, m->particle_world, nullptr, KeyPositions{c->xo_tmp},
                            pbf_gather(c, m, si->particle_q))))
@@ -729,7 +735,7 @@ int fs_pbf_delta(fs_context* c, const fs_model* m, const float* x_pred, const fl
   da.delta_p = delta_p;
   da.xs_out = nullptr;
   da.q = ScanOut{};
-  k_delta<1><<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(da);  // no list: each thread rescans
+  launch(k_delta<1>, nb_blocks(c, m->n), c->nb_block, 0, st, da);  // no list: each thread rescans
   return launch_check("fs_pbf_delta");
 }
 
@@ -759,7 +765,7 @@ int fs_pbf_xsph(fs_context* c, const fs_model* m, const float* x_pred, const flo
   xa.x_out = nullptr;
   xa.v_out = v_out;
   xa.x_pred_api = nullptr;
-  k_xsph_final<1><<<nb_blocks(c, m->n), c->nb_block, 0, st>>>(xa);
+  launch(k_xsph_final<1>, nb_blocks(c, m->n), c->nb_block, 0, st, xa);
   return launch_check("fs_pbf_xsph");
 }
 

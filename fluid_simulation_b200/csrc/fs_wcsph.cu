@@ -52,6 +52,7 @@ struct DensityArgs {
 template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, 4) k_wcsph_density(DensityArgs a) {
   extern __shared__ uint2 smem[];
+  grid_begin();
   if (clock_idle(a.clock)) return;
   lists_recorded(a.L);
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
@@ -108,6 +109,7 @@ struct ForceArgs {
 
 template <int G>
 __global__ void FS_NB_BOUNDS k_wcsph_force(ForceArgs a) {
+  grid_begin();
   if (clock_idle(a.clock)) return;
   const float dt = a.clock ? a.clock->dt : a.dt;
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
@@ -181,7 +183,8 @@ __global__ void k_gather_ratios(int64_t n, const int32_t* __restrict__ perm, con
 __global__ void k_idle_copy(int64_t n, const fs_frame_clock* clock, const float* __restrict__ x_in,
                             const float* __restrict__ v_in, const float* __restrict__ rho_in,
                             const float* __restrict__ p_in, float* x_out, float* v_out, float* rho_out, float* p_out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_begin();
+  const int64_t i = thread_id();
   if (i >= n || !clock_idle(clock)) return;
   st3(x_out, i, ld3(x_in, i));
   st3(v_out, i, ld3(v_in, i));
@@ -309,7 +312,7 @@ int fs_wcsph_substep_clocked(fs_context* c, const fs_model* m, const fs_state* s
   if ((rc = launch_force(c, m, p, accel, so->particle_q, so->particle_qd, st, true, clock))) return rc;
   {
     PassScope ps_(c, P_OTHER, st);
-    k_idle_copy<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, clock, si->particle_q, si->particle_qd, si->rho,
+    launch(k_idle_copy, blocks_for(m->n), kBlock, 0, st, m->n, clock, si->particle_q, si->particle_qd, si->rho,
                                                      si->pressure, so->particle_q, so->particle_qd, so->rho,
                                                      so->pressure);
   }
