@@ -294,7 +294,7 @@ __global__ void FS_NB_BOUNDS k_adj_density(AdjArgs a) {
     const Cubic K(a.h);
     float3 xb = lead ? make_float3(xr.x, xr.y, xr.z) : make_float3(0.f, 0.f, 0.f);
     list_sum<G, false, false, true, 0>(
-        a.g, a.xs, (int)s, xk, a.h, a.h * a.h * kSupportMargin, a.L, lists_usable(a.L), on,
+        a.g, a.xs, a.xs, (int)s, xk, a.h, a.h * a.h * kSupportMargin, a.L, lists_usable(a.L), on,
         [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.xr[t].w)); },
         [&](int t, float4 xj, const float2& j) {
           const float dx = xk.x - xj.x, dy = xk.y - xj.y, dz = xk.z - xj.z;

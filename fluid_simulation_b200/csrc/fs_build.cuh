@@ -56,19 +56,18 @@ struct NoGather {
   FS_DEV void operator()(int64_t, int32_t) const {}
 };
 
-// What the neighbour loops read (gather_common_slot); vs2: a second copy of vs.
+// What the neighbour loops read (gather_common_slot).
 struct CommonGather {
   fs_model m;
   const float *x, *v;
   float4* xs;
   ScanOut q;
-  float4 *vs, *vs2;
-  float* mv;
+  float4* vs;
+  float *mv, *ms;
   uint32_t* status;
   int nworlds;
   FS_DEV void operator()(int64_t s, int32_t i) const {
-    gather_common_slot(s, i, m, x, v, xs, q, vs, mv, status, nworlds);
-    if (vs2) vs2[s] = vs[s];
+    gather_common_slot(s, i, m, x, v, xs, q, vs, mv, ms, status, nworlds);
   }
 };
 
@@ -78,8 +77,7 @@ __global__ void k_cell_keys(int64_t n, Key source, KeyArgs a) {
   const int64_t t = thread_id();
   if (t == 0) {
     source.reset();
-    a.ctl->valid = 0;  // a new grid invalidates recorded neighbour lists
-    a.ctl->inactive = 0;
+    *a.ctl = ListCtl{};  // a new grid invalidates recorded neighbour lists
   }
   if (clock_idle(a.clock)) return;
   // Lattice-ordered particles run along z, whose cells lie tiles apart: every

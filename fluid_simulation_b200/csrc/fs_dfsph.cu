@@ -32,15 +32,16 @@ int reduction_blocks(int64_t n) { return blocks_for(n > 0 ? n : 1, 2); }
 // gather of fs_wcsph.cu reused here
 __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
                                 const float* __restrict__ v, float4* __restrict__ xs, ScanOut q,
-                                float4* __restrict__ vs, float* __restrict__ mv, uint32_t* status, int nworlds);
+                                float4* __restrict__ vs, float* __restrict__ mv, float* __restrict__ ms,
+                                uint32_t* status, int nworlds);
 
 namespace {
 
-// xyz of a cell-order float4 stream into an original-order [n][3] array
-__global__ void k_scatter_xyz(int64_t n, const int32_t* __restrict__ perm, const float4* __restrict__ in,
-                              float* __restrict__ out) {
+// a packed cell-order velocity (xv.w, vyz) into an original-order [n][3] array
+__global__ void k_scatter_velocity(int64_t n, const int32_t* __restrict__ perm, const float4* __restrict__ xv,
+                                   const float2* __restrict__ vyz, float* __restrict__ out) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < n) st3(out, perm[s], xyz(in[s]));
+  if (s < n) st3(out, perm[s], make_float3(xv[s].w, vyz[s].x, vyz[s].y));
 }
 
 // (a[i], b[i]) of original order into cell order
@@ -70,7 +71,7 @@ struct DensFactorArgs {
   ScanXyz q;
   int64_t n;
   const float4* xs;
-  const float4* vs;  // .w = mass
+  const float* ms;   // mass
   const float* mv;
   float h;
   int min_nb;
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(kNbBlockMax, 3) k_density_factor(DensFactorArg
     // the candidate count (no distance test, solver_dfsph.py:163-164) comes from the scan
     const int cnt = scan_sum<G, true, true, false, 5>(
         a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, -1,
-        [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.vs[t].w)); },
+        [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(a.ms + t)); },
         [&](int t, float4 xj, const float2& mm) {  // (rest_density * volume, mass)
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           float r, rinv;
@@ -142,12 +143,14 @@ struct AccelArgs {
   int use_lists;
   int64_t n;
   const float4* xs;
-  const float4* vs;
+  const float4* vs;  // (v, mass)
+  const float* ms;
   const float2* sc2;
   fs_model m;
   float h, particle_radius, dt;
   float* accel;
-  float4* vstar;     // cell order (v*, mass)
+  float4* xv;        // cell order (x, y, z, v*_x)
+  float2* vyz;       // cell order (v*_y, v*_z)
   const fs_frame_clock* clock;
 };
 
@@ -171,8 +174,8 @@ __global__ void FS_NB_BOUNDS k_accel_predict(AccelArgs a) {
       float rho;
     };
     list_sum<G, false, false, true, 4>(
-        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), live && dyn,
-        [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(&a.sc2[t].x)}; },
+        a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        live && dyn, [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(&a.sc2[t].x)}; },
         [&](int t, float4 xj, const Neighbour& j) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -192,13 +195,15 @@ __global__ void FS_NB_BOUNDS k_accel_predict(AccelArgs a) {
     if (!lead) return;
     if (!dyn) {
       st3(a.accel, i, make_float3(0.f, 0.f, 0.f));
-      a.vstar[s] = make_float4(0.f, 0.f, 0.f, vi.w);
+      a.xv[s] = make_float4(xi.x, xi.y, xi.z, 0.f);
+      a.vyz[s] = make_float2(0.f, 0.f);
       return;
     }
     const float3 g = gravity_of(a.m, i);
     const float3 acc = make_float3(ax + g.x, ay + g.y, az + g.z);
     st3(a.accel, i, acc);
-    a.vstar[s] = make_float4(vi.x + dt * acc.x, vi.y + dt * acc.y, vi.z + dt * acc.z, vi.w);
+    a.xv[s] = make_float4(xi.x, xi.y, xi.z, vi.x + dt * acc.x);
+    a.vyz[s] = make_float2(vi.y + dt * acc.y, vi.z + dt * acc.z);
   });
 }
 
@@ -211,7 +216,9 @@ struct RateArgs {
   GridDev g;
   int64_t n;
   const float4* xs;
-  const float4* vstar;      // (v*, mass)
+  const float4* xv;         // (x, y, z, v*_x) and
+  const float2* vyz;        // (v*_y, v*_z): what a pair gathers
+  const float* ms;          // mass
   const float2* sc2;        // (rho, factor)
   const float* rest_density;
   float h, dt, max_kappa, eta;
@@ -219,7 +226,7 @@ struct RateArgs {
   float* d_rho_dt;          // API
   float* rho_star;          // API (mode 0)
   float* kappa_new;         // cell order candidate kappa
-  float2* kratio_new;       // cell order (kappa / max(rho, 1e-6), mass): what the correction gathers per neighbour
+  float4* rec_new;          // cell order (x, y, z, kappa / max(rho, 1e-6)): what the correction gathers per neighbour
   NbrList L;
   int use_lists;
   DfsphDev* ctrl;           // null: separate-pass use, no residual
@@ -329,6 +336,11 @@ __global__ void FS_NB_BOUNDS k_rate(RateArgs a) {
   if (a.ctrl && a.ctrl->done) return;  // uniform across the grid: set by an earlier launch
   if (clock_idle(a.clock)) return;     // uniform: the frame is complete
   const float dt = a.clock ? a.clock->dt : a.dt;
+  const Masses<G> mass(a.ms, a.L.ctl);
+  struct Neighbour {
+    float2 v;
+    float m;
+  };
   double term = 0.0;  // this thread's residual terms and dynamic particles
   long long dyn = 0;
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
@@ -338,17 +350,17 @@ __global__ void FS_NB_BOUNDS k_rate(RateArgs a) {
     if (G == 1 && over) return;
     const int pf = pf_of(xi);
     float d = 0.f;
-    const float4 vi = a.vstar[s];
+    const float4 vi = make_float4(a.xv[s].w, a.vyz[s].x, a.vyz[s].y, 0.f);
     const Cubic K(a.h);
     list_sum<G, false, false, false, 2>(
-        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
-        live && !over && (pf & PF_ACTIVE), [&](int t) { return __ldg(a.vstar + t); },
-        [&](int t, float4 xj, const float4& vj) {
+        a.g, a.xs, a.xv, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        live && !over && (pf & PF_ACTIVE), [&](int t) { return Neighbour{__ldg(a.vyz + t), mass(t)}; },
+        [&](int t, float4 xj, const Neighbour& j) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           float r, rinv;
           r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
-          const float vdot = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
-          return Terms<2>{vj.w * K.grad_scale(r, rinv), vdot};
+          const float vdot = fmaf(vi.x - xj.w, dx, fmaf(vi.y - j.v.x, dy, (vi.z - j.v.y) * dz));
+          return Terms<2>{j.m * K.grad_scale(r, rinv), vdot};
         },
         [&](const Terms<2>& u) { d = fmaf(u.v[0], u.v[1], d); });
     if (!lead || over) return;
@@ -371,7 +383,7 @@ __global__ void FS_NB_BOUNDS k_rate(RateArgs a) {
     }
     if (a.kappa_new) {
       a.kappa_new[s] = kap;
-      a.kratio_new[s] = make_float2(kap / fmaxf(rf.x, 1.0e-6f), a.vstar[s].w);
+      a.rec_new[s] = make_float4(xi.x, xi.y, xi.z, kap / fmaxf(rf.x, 1.0e-6f));
     }
     if (a.term) a.term[s] = tv;
     if (is_dyn) {
@@ -452,9 +464,11 @@ struct CorrectArgs {
   GridDev g;
   int64_t n;
   const float4* xs;
-  float4* vstar;          // in/out (own slot only)
+  float4* xv;             // (x, y, z, v*_x), in/out (own slot only)
+  float2* vyz;            // (v*_y, v*_z), in/out (own slot only)
+  const float* ms;        // mass
   const float* kappa;     // cell order (committed to the API array)
-  const float2* kratio;   // cell order (kappa / max(rho, 1e-6), mass): one gather per neighbour
+  const float4* rec;      // cell order (x, y, z, kappa / max(rho, 1e-6)): one gather per neighbour
   float h, dt;
   float* kappa_api;       // commit kappa to the API array (may be null)
   float* vstar_api;       // optional original-order v* output
@@ -475,24 +489,24 @@ __global__ void __launch_bounds__(kNbBlockMax, 4) k_correct(CorrectArgs a) {
   if (a.ctrl && a.ctrl->done) return;
   if (clock_idle(a.clock)) return;
   const float dt = a.clock ? a.clock->dt : a.dt;
+  const Masses<G> mass(a.ms, a.L.ctl);
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
     const bool over = world_finished(a.wctl, a.pworld, a.nworlds, i);
     if (G == 1 && over) return;
-    float4 v = a.vstar[s];
+    float3 v = make_float3(a.xv[s].w, a.vyz[s].x, a.vyz[s].y);
     const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const Cubic K(a.h);
-    const float ci = a.kratio[s].x;
+    const float ci = a.rec[s].w;
     float dvx = 0.f, dvy = 0.f, dvz = 0.f;
     list_sum<G, false, false, false, 4>(
-        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
-        live && !over && dyn, [&](int t) { return __ldg(a.kratio + t); },
-        [&](int t, float4 xj, const float2& kj) {
+        a.g, a.xs, a.rec, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        live && !over && dyn, mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           float r, rinv;
           r_and_inv(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), r, rinv);
-          return Terms<4>{kj.y * (ci + kj.x) * K.grad_scale(r, rinv), dx, dy, dz};
+          return Terms<4>{mj * (ci + xj.w) * K.grad_scale(r, rinv), dx, dy, dz};
         },
         [&](const Terms<4>& u) {
           dvx = fmaf(u.v[0], u.v[1], dvx);
@@ -505,26 +519,50 @@ __global__ void __launch_bounds__(kNbBlockMax, 4) k_correct(CorrectArgs a) {
       v.x = v.x - dt * dvx;
       v.y = v.y - dt * dvy;
       v.z = v.z - dt * dvz;
-      a.vstar[s] = v;
+      a.xv[s] = make_float4(xi.x, xi.y, xi.z, v.x);
+      a.vyz[s] = make_float2(v.y, v.z);
     }
-    if (a.vstar_api) st3(a.vstar_api, i, xyz(v));
+    if (a.vstar_api) st3(a.vstar_api, i, v);
   });
 }
 
-// kappa / max(rho, 1e-6) of gathered kappas (warm start, separate pass)
+// (x, y, z, kappa / max(rho, 1e-6)) of gathered kappas (warm start, separate pass)
 __global__ void k_kappa_ratio(int64_t n, const float* __restrict__ kappa, const float2* __restrict__ sc2,
-                              const float4* __restrict__ vm, float2* __restrict__ kratio) {
+                              const float4* __restrict__ xs, float4* __restrict__ rec) {
   grid_begin();
   const int64_t s = thread_id();
-  if (s < n) kratio[s] = make_float2(kappa[s] / fmaxf(sc2[s].x, 1.0e-6f), vm[s].w);
+  if (s < n) rec[s] = make_float4(xs[s].x, xs[s].y, xs[s].z, kappa[s] / fmaxf(sc2[s].x, 1.0e-6f));
 }
+
+// (x, y, z, v_x) and (v_y, v_z) of gathered positions and velocities (separate passes)
+__global__ void k_pack_velocity(int64_t n, const float4* __restrict__ xs, const float4* __restrict__ vs,
+                                float4* __restrict__ xv, float2* __restrict__ vyz) {
+  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n) return;
+  xv[s] = make_float4(xs[s].x, xs[s].y, xs[s].z, vs[s].x);
+  vyz[s] = make_float2(vs[s].y, vs[s].z);
+}
+
+// The second half's gather: what the neighbour loops read, v* packed for them.
+struct VstarGather {
+  CommonGather common;
+  float4* xv;
+  float2* vyz;
+  FS_DEV void operator()(int64_t s, int32_t i) const {
+    common(s, i);
+    const float3 x = ld3(common.x, i), v = ld3(common.v, i);
+    xv[s] = make_float4(x.x, x.y, x.z, v.x);
+    vyz[s] = make_float2(v.y, v.z);
+  }
+};
 
 // The second grid build's positions: integrate_positions (341-353) of the
 // particle in slot t of the first grid, made in the key pass; also publishes
 // v* in original order.
 struct KeyIntegrate {
   const int32_t* perm;
-  const float4 *xs, *vstar;
+  const float4 *xs, *xv;
+  const float2* vyz;
   float dt;
   float *x_out, *vstar_api;
   const fs_frame_clock* clock;
@@ -532,27 +570,26 @@ struct KeyIntegrate {
   FS_DEV float3 position(int64_t t, int64_t& i) const {
     const float step = clock ? clock->dt : dt;
     const float4 xi = xs[t];
-    const float4 v = vstar[t];
+    const float3 v = make_float3(xv[t].w, vyz[t].x, vyz[t].y);
     i = perm[t];
     float3 p = xyz(xi);
     if (pf_of(xi) & PF_DYNAMIC) p = make_float3(xi.x + v.x * step, xi.y + v.y * step, xi.z + v.z * step);
     st3(x_out, i, p);
-    st3(vstar_api, i, xyz(v));
+    st3(vstar_api, i, v);
     return p;
   }
 };
 
 // copy v* -> particle_qd then apply_bounds (407-442, unconditional damping);
 // batched contexts apply each world's own tank.
-__global__ void k_final(int64_t n, GridDev g, const float4* __restrict__ xs, const float4* __restrict__ vstar,
-                        Walls walls, float* x_out, float* v_out, float* vstar_api, const fs_frame_clock* clock) {
+__global__ void k_final(int64_t n, GridDev g, const float4* __restrict__ xs, const float4* __restrict__ xv,
+                        const float2* __restrict__ vyz, Walls walls, float* x_out, float* v_out, float* vstar_api, const fs_frame_clock* clock) {
   grid_begin();
   const int64_t s = thread_id();
   if (s >= n || clock_idle(clock)) return;
   const float4 xi = xs[s];
-  const float4 v4 = vstar[s];
   const int32_t i = g.perm[s];
-  float3 p = xyz(xi), v = xyz(v4);
+  float3 p = xyz(xi), v = make_float3(xv[s].w, vyz[s].x, vyz[s].y);
   st3(vstar_api, i, v);
   if (pf_of(xi) & PF_DYNAMIC) apply_walls(walls_of(walls, g, world_of(xi)), p, v);
   st3(x_out, i, p);
@@ -578,7 +615,7 @@ __global__ void k_residual(int64_t n, const int32_t* __restrict__ flags, const i
 }
 
 int run_rate(fs_context* c, const fs_model* m, int mode, int it, float h, float dt, float max_kappa, float eta,
-             float* d_rho_dt, float* rho_star, float* kappa_new, float2* kratio_new, DfsphDev* ctrl,
+             float* d_rho_dt, float* rho_star, float* kappa_new, float4* rec_new, DfsphDev* ctrl,
              cudaStream_t st, bool use_lists = true) {
   RateArgs a;
   a.clock = c->clock;
@@ -587,7 +624,9 @@ int run_rate(fs_context* c, const fs_model* m, int mode, int it, float h, float 
   a.use_lists = use_lists ? 1 : 0;
   a.n = m->n;
   a.xs = c->xs;
-  a.vstar = c->vs2;
+  a.xv = c->xs2;
+  a.vyz = (const float2*)c->vo_tmp;
+  a.ms = c->mass;
   a.sc2 = c->sc2;
   a.rest_density = m->rest_density;
   a.h = h;
@@ -599,7 +638,7 @@ int run_rate(fs_context* c, const fs_model* m, int mode, int it, float h, float 
   a.d_rho_dt = d_rho_dt;
   a.rho_star = rho_star;
   a.kappa_new = kappa_new;
-  a.kratio_new = kratio_new;
+  a.rec_new = rec_new;
   a.ctrl = ctrl;
   a.red_part = c->red_part;
   a.red_cnt = c->red_cnt;
@@ -622,7 +661,7 @@ int run_rate(fs_context* c, const fs_model* m, int mode, int it, float h, float 
   return launch_check("dfsph rate");
 }
 
-int run_correct(fs_context* c, const fs_model* m, float h, float dt, const float* kappa, const float2* kratio,
+int run_correct(fs_context* c, const fs_model* m, float h, float dt, const float* kappa, const float4* rec,
                 float* kappa_api, float* vstar_api, const DfsphDev* ctrl, cudaStream_t st, bool use_lists = true) {
   CorrectArgs a;
   a.clock = c->clock;
@@ -631,9 +670,11 @@ int run_correct(fs_context* c, const fs_model* m, float h, float dt, const float
   a.use_lists = use_lists ? 1 : 0;
   a.n = m->n;
   a.xs = c->xs;
-  a.vstar = c->vs2;
+  a.xv = c->xs2;
+  a.vyz = (float2*)c->vo_tmp;
+  a.ms = c->mass;
   a.kappa = kappa;
-  a.kratio = kratio;
+  a.rec = rec;
   a.h = h;
   a.dt = dt;
   a.kappa_api = kappa_api;
@@ -659,7 +700,7 @@ int run_density_factor(fs_context* c, const fs_model* m, float h, int min_nb, fl
   a.q = scan_xyz(c);
   a.n = m->n;
   a.xs = c->xs;
-  a.vs = c->vs2;
+  a.ms = c->mass;
   a.mv = c->mv;
   a.h = h;
   a.min_nb = min_nb;
@@ -769,9 +810,8 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
       (rc = check_cuda(cudaMemsetAsync(c->dfsph_worlds, 0, sizeof(DfsphWorld) * 2 * c->nworlds, st), "dfsph reset")))
     return rc;
   // ---- first half: positions x_in
-  // (vs2, too: density/factor reads its masses there)
   if ((rc = grid_build(c, n, h, st, m->particle_world, c->clock, KeyPositions{si->particle_q},
-                       CommonGather{*m, si->particle_q, si->particle_qd, c->xs, scan_out(c), c->vs, c->vs2, c->mv,
+                       CommonGather{*m, si->particle_q, si->particle_qd, c->xs, scan_out(c), c->vs, c->mv, c->mass,
                                     c->status, c->nworlds})))
     return rc;
   if ((rc = run_density_factor(c, m, h, p->min_neighbors_for_factor, so->rho, so->factor, so->neighbor_count, st)))
@@ -783,13 +823,15 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
   aa.n = n;
   aa.xs = c->xs;
   aa.vs = c->vs;
+  aa.ms = c->mass;
   aa.sc2 = c->sc2;
   aa.m = *m;
   aa.h = h;
   aa.particle_radius = p->particle_radius;
   aa.dt = dt;
   aa.accel = accel;
-  aa.vstar = c->vs2;
+  aa.xv = c->xs2;
+  aa.vyz = (float2*)c->vo_tmp;
   aa.clock = c->clock;
   {
     PassScope ps_(c, P_DFSPH_ACCEL, st);
@@ -800,21 +842,23 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
     {
       PassScope ps_(c, P_GATHER, st, 2);
       launch(k_gather_scalar, blocks_for(n), kBlock, 0, st, n, c->perm, si->kappa, c->sc1, nullptr);
-      launch(k_kappa_ratio, blocks_for(n), kBlock, 0, st, n, c->sc1, c->sc2, c->vs2, c->krm);
+      launch(k_kappa_ratio, blocks_for(n), kBlock, 0, st, n, c->sc1, c->sc2, c->xs, c->rec);
     }
-    if ((rc = run_correct(c, m, h, dt, c->sc1, c->krm, so->kappa, nullptr, nullptr, st))) return rc;
+    if ((rc = run_correct(c, m, h, dt, c->sc1, c->rec, so->kappa, nullptr, nullptr, st))) return rc;
   }
   for (int it = 0; it < p->max_rho_iterations; ++it) {
     if ((rc = run_rate(c, m, 0, it, h, dt, p->max_kappa, p->eta_density, so->d_rho_dt, so->rho_star, c->sc1,
-                       c->krm, c->dfsph + 0, st)))
+                       c->rec, c->dfsph + 0, st)))
       return rc;
-    if ((rc = run_correct(c, m, h, dt, c->sc1, c->krm, so->kappa, nullptr, c->dfsph + 0, st))) return rc;
+    if ((rc = run_correct(c, m, h, dt, c->sc1, c->rec, so->kappa, nullptr, c->dfsph + 0, st))) return rc;
   }
   // ---- second half: positions x_out
   if ((rc = grid_build(c, n, h, st, m->particle_world, c->clock,
-                       KeyIntegrate{c->perm, c->xs, c->vs2, dt, so->particle_q, so->v_star, c->clock},
-                       CommonGather{*m, so->particle_q, so->v_star, c->xs, scan_out(c), c->vs2, nullptr, c->mv,
-                                    c->status, c->nworlds})))
+                       KeyIntegrate{c->perm, c->xs, c->xs2, (const float2*)c->vo_tmp, dt, so->particle_q, so->v_star,
+                                    c->clock},
+                       VstarGather{CommonGather{*m, so->particle_q, so->v_star, c->xs, scan_out(c), nullptr, c->mv,
+                                                c->mass, c->status, c->nworlds},
+                                   c->xs2, (float2*)c->vo_tmp})))
     return rc;
   if ((rc = run_density_factor(c, m, h, p->min_neighbors_for_factor, so->rho, so->factor, so->neighbor_count, st)))
     return rc;
@@ -822,20 +866,20 @@ int dfsph_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_state
     {
       PassScope ps_(c, P_GATHER, st, 2);
       launch(k_gather_scalar, blocks_for(n), kBlock, 0, st, n, c->perm, si->kappa_v, c->sc1, nullptr);
-      launch(k_kappa_ratio, blocks_for(n), kBlock, 0, st, n, c->sc1, c->sc2, c->vs2, c->krm);
+      launch(k_kappa_ratio, blocks_for(n), kBlock, 0, st, n, c->sc1, c->sc2, c->xs, c->rec);
     }
-    if ((rc = run_correct(c, m, h, dt, c->sc1, c->krm, so->kappa_v, nullptr, nullptr, st))) return rc;
+    if ((rc = run_correct(c, m, h, dt, c->sc1, c->rec, so->kappa_v, nullptr, nullptr, st))) return rc;
   }
   for (int it = 0; it < p->max_vel_iterations; ++it) {
     if ((rc = run_rate(c, m, 1, it, h, dt, p->max_kappa_v, p->eta_divergence, so->d_rho_dt, nullptr, c->sc1,
-                       c->krm, c->dfsph + 1, st)))
+                       c->rec, c->dfsph + 1, st)))
       return rc;
-    if ((rc = run_correct(c, m, h, dt, c->sc1, c->krm, so->kappa_v, nullptr, c->dfsph + 1, st))) return rc;
+    if ((rc = run_correct(c, m, h, dt, c->sc1, c->rec, so->kappa_v, nullptr, c->dfsph + 1, st))) return rc;
   }
   const Walls w = make_walls(p->bound_width, p->bound_height, p->bound_length, p->boundary_damping, 1, 0.f, 0.f);
   {
     PassScope ps_(c, P_DFSPH_FINAL, st);
-    launch(k_final, blocks_for(n), kBlock, 0, st, n, grid_view(c), c->xs, c->vs2, w, so->particle_q, so->particle_qd,
+    launch(k_final, blocks_for(n), kBlock, 0, st, n, grid_view(c), c->xs, c->xs2, (const float2*)c->vo_tmp, w, so->particle_q, so->particle_qd,
                                               so->v_star, c->clock);
   }
   c->last_stream = st;
@@ -908,7 +952,7 @@ int fs_dfsph_density_factor(fs_context* c, const fs_model* m, const float* x, fl
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_dfsph_density_factor: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, x, c->xs, scan_out(c), c->vs2, c->mv, c->status, c->nworlds);
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, x, c->xs, scan_out(c), c->vs2, c->mv, c->mass, c->status, c->nworlds);
   return run_density_factor(c, m, h, min_nb, rho, factor, neighbor_count, st);
 }
 
@@ -925,8 +969,7 @@ int fs_dfsph_nonpressure_predict(fs_context* c, const fs_model* m, const float* 
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t n = m->n;
-  k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs, c->mv, c->status,
-                                                    c->nworlds);
+  k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs, c->mv, c->mass, c->status, c->nworlds);
   k_gather_pair<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, rho, nullptr, c->sc2);
   AccelArgs aa;
   aa.g = grid_view(c);
@@ -935,16 +978,18 @@ int fs_dfsph_nonpressure_predict(fs_context* c, const fs_model* m, const float* 
   aa.n = n;
   aa.xs = c->xs;
   aa.vs = c->vs;
+  aa.ms = c->mass;
   aa.sc2 = c->sc2;
   aa.m = *m;
   aa.h = h;
   aa.particle_radius = particle_radius;
   aa.dt = dt;
   aa.accel = accel;
-  aa.vstar = c->vs2;
+  aa.xv = c->xs2;
+  aa.vyz = (float2*)c->vo_tmp;
   aa.clock = nullptr;
   launch(k_accel_predict<1>, nb_blocks(c, n), c->nb_block, 0, st, aa);
-  k_scatter_xyz<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, c->vs2, v_star);
+  k_scatter_velocity<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, c->xs2, (const float2*)c->vo_tmp, v_star);
   return launch_check("fs_dfsph_nonpressure_predict");
 }
 
@@ -955,7 +1000,8 @@ int fs_dfsph_divergence(fs_context* c, const fs_model* m, const float* x, const 
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_dfsph_divergence: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs2, nullptr, c->status, c->nworlds);
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs2, nullptr, c->mass, c->status, c->nworlds);
+  k_pack_velocity<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->xs, c->vs2, c->xs2, (float2*)c->vo_tmp);
   // rho/factor are not needed for the rate itself (mode 1 reads them only for kappa, which is discarded)
   if (cudaMemsetAsync(c->sc2, 0, sizeof(float2) * m->n, st) != cudaSuccess)
     return set_error(FS_ERR_CUDA, "fs_dfsph_divergence: memset");
@@ -970,14 +1016,15 @@ int fs_dfsph_correct(fs_context* c, const fs_model* m, const float* x, float* v_
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v_star, c->xs, scan_out(c), c->vs2, nullptr,
-                                                       c->status, c->nworlds);
+                                                       c->mass, c->status, c->nworlds);
+  k_pack_velocity<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->xs, c->vs2, c->xs2, (float2*)c->vo_tmp);
   k_gather_pair<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, rho, nullptr, c->sc2);
   launch(k_gather_scalar, blocks_for(m->n), kBlock, 0, st, m->n, c->perm, kappa, c->sc1, nullptr);
   {
     PassScope ps_(c, P_GATHER, st);
-    launch(k_kappa_ratio, blocks_for(m->n), kBlock, 0, st, m->n, c->sc1, c->sc2, c->vs2, c->krm);
+    launch(k_kappa_ratio, blocks_for(m->n), kBlock, 0, st, m->n, c->sc1, c->sc2, c->xs, c->rec);
   }
-  return run_correct(c, m, h, dt, c->sc1, c->krm, nullptr, v_star, nullptr, st, false);
+  return run_correct(c, m, h, dt, c->sc1, c->rec, nullptr, v_star, nullptr, st, false);
 }
 
 int fs_dfsph_residual(fs_context* c, const fs_model* m, const float* a, const float* b, double* out,

@@ -196,7 +196,7 @@ int nb_group(int64_t n) { return n <= 5000 ? 16 : n <= 14000 ? 8 : n <= 36000 ? 
 
 ScanXyz scan_xyz(const fs_context* c) { return ScanXyz{c->sxyz}; }
 ScanOut scan_out(const fs_context* c) {
-  return ScanOut{c->sxyz, &((ListCtl*)c->nb_ctl)->inactive};
+  return ScanOut{c->sxyz, (ListCtl*)c->nb_ctl};
 }
 
 GridDev grid_view(const fs_context* c) {
@@ -449,7 +449,7 @@ static int context_alloc(fs_context* c, int64_t capacity, int64_t ncell) {
       {(void**)&c->vs, sizeof(float4) * cap},           {(void**)&c->vs2, sizeof(float4) * cap},
       {(void**)&c->mv, sizeof(float) * cap},            {(void**)&c->sc2, sizeof(float2) * cap},
       {(void**)&c->sc1, sizeof(float) * cap},           {(void**)&c->sc1b, sizeof(float) * cap},
-      {(void**)&c->krm, sizeof(float2) * cap},
+      {(void**)&c->mass, sizeof(float) * cap},          {(void**)&c->rec, sizeof(float4) * cap},
       {(void**)&c->xo_tmp, sizeof(float) * 3 * cap},    {(void**)&c->vo_tmp, sizeof(float) * 3 * cap},
       {(void**)&c->red_part, sizeof(double) * rb},      {(void**)&c->red_cnt, sizeof(int64_t) * rb},
       {(void**)&c->dfsph, sizeof(DfsphDev) * 2},         {(void**)&c->status, sizeof(uint32_t)},
@@ -488,7 +488,7 @@ int fs_context_destroy(fs_context* c) {
   DeviceGuard dg(c->device);
   timer_free(c->timer);
   void* ps[] = {c->key, c->slot, c->cell_count, c->cell_off, c->tmp_ids, c->perm, c->scan_part, c->xs, c->xs2,
-                c->sxyz, c->vs, c->vs2, c->mv, c->sc2, c->sc1, c->sc1b, c->krm, c->xo_tmp, c->vo_tmp, c->red_part, c->red_cnt,
+                c->sxyz, c->vs, c->vs2, c->mv, c->sc2, c->sc1, c->sc1b, c->mass, c->rec, c->xo_tmp, c->vo_tmp, c->red_part, c->red_cnt,
                 c->dfsph, c->status, c->tile_stats, c->nb_idx, c->nb_cnt, c->nb_ctl, c->worlds, c->metrics,
                 c->dfsph_worlds, c->pbf_disp};
   for (void* p : ps)

@@ -34,6 +34,12 @@ struct DfsphWorld {   // batched contexts: one world's decisions in one half of 
   double residual;    // its last residual (mean over its dynamic particles)
 };
 
+struct ListCtl {        // notes on the current grid's lists and gather (cleared by a build)
+  int32_t valid;       // lists recorded for the current grid and positions
+  int32_t inactive;    // some gathered particle is inactive
+  int32_t mixed_mass;  // the gathered particles' masses differ
+};
+
 // Passes for the per-pass CUDA-event timer (fs_timer_*) and launch counter.
 enum Pass {
   P_GRID = 0, P_GATHER, P_WCSPH_DENSITY, P_WCSPH_FORCE, P_DFSPH_DENSITY_FACTOR, P_DFSPH_ACCEL, P_DFSPH_RATE,
@@ -98,7 +104,9 @@ struct fs_context {
   float2* sc2 = nullptr;  // per-slot scalar pair (rho, p) / (rho, factor)
   float* sc1 = nullptr;   // per-slot scalar (kappa / lambda)
   float* sc1b = nullptr;  // per-slot scalar (second)
-  float2* krm = nullptr;  // per-slot (kappa / rho, mass) for the DFSPH correction, (lambda, mass) for PBF's delta
+  float* mass = nullptr;  // per-slot mass
+  float4* rec = nullptr;  // per-slot (x, y, z, value): kappa / rho for the DFSPH correction, lambda for PBF's delta,
+                          // p / rho^2 for the WCSPH force
   float* xo_tmp = nullptr;  // [cap*3] original-order scratch positions (PBF x_pred)
   float* vo_tmp = nullptr;  // [cap*3] original-order scratch velocities (PBF v_pred)
 
@@ -626,10 +634,10 @@ FS_DEV int particle_pf(const int32_t* flags, const int32_t* mask, int64_t i) {
 constexpr float kScanFar = 1.0e30f;
 struct ScanOut {
   float* g;
-  int32_t* inactive;  // set when an inactive particle is gathered (ListCtl.inactive)
+  ListCtl* ctl;  // notes of the gather (may be null)
 };
 FS_DEV void scan_put(const ScanOut& q, int64_t s, float3 p, bool active) {
-  if (!active && q.inactive) *q.inactive = 1;
+  if (!active && q.ctl) q.ctl->inactive = 1;
   float* o = q.g + (s >> 2) * 12 + (s & 3);
   o[0] = active ? p.x : kScanFar;
   o[4] = p.y;
@@ -638,13 +646,14 @@ FS_DEV void scan_put(const ScanOut& q, int64_t s, float3 p, bool active) {
 ScanOut scan_out(const fs_context* c);
 
 // Slot s (particle i = perm[s]) of the cell-order copies that the neighbour
-// loops read: xs = (x, flags + world), vs = (v, mass) when vs, and mv =
-// rest_density * volume with volume = mass / max(rest_density, 1e-6)
+// loops read: xs = (x, flags + world), ms = mass when ms, vs = (v, mass) when vs, and
+// mv = rest_density * volume with volume = mass / max(rest_density, 1e-6)
 // (compute_particle_volume, solver_wcsph.py:110-116) when mv.  A world index
 // past the model's worlds raises FS_STATUS_BOUNDS.
 FS_DEV void gather_common_slot(int64_t s, int32_t i, const fs_model& m, const float* __restrict__ x,
                                const float* __restrict__ v, float4* __restrict__ xs, const ScanOut& q,
-                               float4* __restrict__ vs, float* __restrict__ mv, uint32_t* status, int nworlds) {
+                               float4* __restrict__ vs, float* __restrict__ mv, float* __restrict__ ms,
+                               uint32_t* status, int nworlds) {
   const float3 p = ld3(x, i);
   const int pf = particle_pf(m.particle_flags, m.particle_mask, i);
   // batched contexts carry the world in the flags word (queries stay in it)
@@ -652,6 +661,10 @@ FS_DEV void gather_common_slot(int64_t s, int32_t i, const fs_model& m, const fl
   xs[s] = make_float4(p.x, p.y, p.z, pack_pf(pf, w));
   scan_put(q, s, p, (pf & PF_ACTIVE) != 0);
   const float mass = m.particle_mass[i];
+  if (ms) {
+    ms[s] = mass;
+    if (mass != m.particle_mass[0]) q.ctl->mixed_mass = 1;
+  }
   if (vs) {
     const float3 u = ld3(v, i);
     vs[s] = make_float4(u.x, u.y, u.z, mass);

@@ -108,9 +108,30 @@ constexpr int kNbMax = 192;
 // Entry offsets k * stride (k < kNbMax) fit 32 bits up to this stride (capacity).
 constexpr int64_t kListStride32Max = 0xffffffffLL / kNbMax;
 
-struct ListCtl {
-  int32_t valid;     // lists recorded for the current grid and positions
-  int32_t inactive;  // some particle gathered for the current grid is inactive
+// The mass that the pair terms read for each neighbour.  Particles of one
+// fluid mostly share one: the gather notes whether they do (ListCtl), and then
+// no pair loads it.  The list passes are held by the L1's data cycles (a
+// gather of 16 bytes takes a warp about 12, of 4 bytes 4), so that a load
+// saved counts: with the records of a pass (the position and one value) the
+// gathers of a pair went from 32 to 24 bytes in the DFSPH rate, from 24 to 16
+// in its correction and PBF's delta, 40 to 32 in PBF's non-pressure pass.
+// B200, 401,856 particles, us a launch: rate 71 -> 65, correction 50 -> 46,
+// delta 51 -> 46, non-pressure 85 -> 73, lambda 115 -> 110.  (Not so the WCSPH
+// force, 40 -> 32 bytes: 1 % for what its density pass then writes.)  With
+// several lanes per particle the latency of the note itself would count: the
+// mass is always loaded.
+template <int G>
+struct Masses {
+  const float* p;
+  float first = 0.f;
+  bool mixed = true;
+  FS_DEV Masses(const float* p_, const ListCtl* ctl) : p(p_) {
+    if (G > 1) return;
+    mixed = ctl->mixed_mass != 0;
+    // no thread index orders this load behind grid_begin(): it stays where it is written
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(first) : "l"(p_) : "memory");
+  }
+  FS_DEV float operator()(int t) const { return mixed ? __ldg(p + t) : first; }
 };
 
 // The coordinates of the cell-order particles for the grid scans: groups of
@@ -416,9 +437,11 @@ FS_DEV void scan_grid(const GridDev& g, const float4* __restrict__ xs, int s, fl
 
 // Visits the neighbours of slot s within h2m through its recorded list when
 // lists_ok and the list did not overflow, else by rescanning the grid.
+// rec: the record gathered with each neighbour, its position and one value
+// (xs itself, or a pass's own); pair(t, rec[t]).
 template <bool WITH_SELF, class Pair>
-FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, float h2m,
-                  const NbrList& L, bool lists_ok, Pair&& pair) {
+FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s, float4 xi,
+                  float h, float h2m, const NbrList& L, bool lists_ok, Pair&& pair) {
   const int n = lists_ok ? __ldg(L.cnt + s) : kNbMax + 1;
   const bool use = n <= kNbMax;
   if (use) {
@@ -426,12 +449,12 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, int s, float4
     auto entry = [&](int k) { return __ldg(col + (int64_t)k * L.stride); };
     auto one = [&](int t, float4 xj) {
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      if (fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, xj.w))) <= h2m && (WITH_SELF || t != s)) pair(t, xj);
+      if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= h2m && (WITH_SELF || t != s)) pair(t, xj);
     };
     int k = 0;
     for (; k + 3 < n; k += 4) {  // four independent gathers in flight
       const int t0 = entry(k), t1 = entry(k + 1), t2 = entry(k + 2), t3 = entry(k + 3);
-      const float4 x0 = __ldg(xs + t0), x1 = __ldg(xs + t1), x2 = __ldg(xs + t2), x3 = __ldg(xs + t3);
+      const float4 x0 = __ldg(rec + t0), x1 = __ldg(rec + t1), x2 = __ldg(rec + t2), x3 = __ldg(rec + t3);
       one(t0, x0);
       one(t1, x1);
       one(t2, x2);
@@ -439,10 +462,10 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, int s, float4
     }
     for (; k < n; ++k) {
       const int t0 = entry(k);
-      one(t0, __ldg(xs + t0));
+      one(t0, __ldg(rec + t0));
     }
   } else {
-    scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, pair);
+    scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { pair(t, __ldg(rec + t)); });
   }
 }
 
@@ -460,13 +483,13 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, int s, float4
 // 1.304 -> 1.287 ms per substep at 401,856 particles); the DFSPH iteration
 // passes, which read the same lists 34 times a substep, were slower with it.
 template <bool WITH_SELF, bool EVICT_FIRST = false, class Load, class Pair>
-FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, float h2m,
-                       const NbrList& L, bool lists_ok, Load&& load, Pair&& pair) {
+FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s,
+                       float4 xi, float h, float h2m, const NbrList& L, bool lists_ok, Load&& load, Pair&& pair) {
   const int n = lists_ok ? __ldg(L.cnt + s) : kNbMax + 1;
   const bool use = n <= kNbMax;
   auto one = [&](int t, float4 xj, const auto& p) {
     const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    if (fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, xj.w))) <= h2m && (WITH_SELF || t != s)) pair(t, xj, p);
+    if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= h2m && (WITH_SELF || t != s)) pair(t, xj, p);
   };
   if (use) {
     const int32_t* col = L.idx + s;
@@ -476,7 +499,7 @@ FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, int s, f
     int k = 0;
     for (; k + 3 < n; k += 4) {
       const int t0 = entry(k), t1 = entry(k + 1), t2 = entry(k + 2), t3 = entry(k + 3);
-      const float4 x0 = __ldg(xs + t0), x1 = __ldg(xs + t1), x2 = __ldg(xs + t2), x3 = __ldg(xs + t3);
+      const float4 x0 = __ldg(rec + t0), x1 = __ldg(rec + t1), x2 = __ldg(rec + t2), x3 = __ldg(rec + t3);
       const auto p0 = load(t0), p1 = load(t1), p2 = load(t2), p3 = load(t3);
       one(t0, x0, p0);
       one(t1, x1, p1);
@@ -485,11 +508,11 @@ FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, int s, f
     }
     for (; k < n; ++k) {
       const int t0 = entry(k);
-      const float4 x0 = __ldg(xs + t0);
+      const float4 x0 = __ldg(rec + t0);
       one(t0, x0, load(t0));
     }
   } else {
-    scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4 xj) { pair(t, xj, load(t)); });
+    scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { pair(t, __ldg(rec + t), load(t)); });
   }
 }
 
@@ -547,13 +570,13 @@ FS_DEV V group_sum(V v) {
 // in all its lanes; 0: nothing), entry(k) being the k-th slot.  All lanes of
 // the warp call it together.
 template <int G, bool WITH_SELF, int K, class Entry, class Load, class Term, class Acc>
-FS_DEV void group_visit(const float4* __restrict__ xs, int s, float4 xi, float h2m, int n, Entry&& entry, Load&& load,
+FS_DEV void group_visit(const float4* __restrict__ rec, int s, float4 xi, float h2m, int n, Entry&& entry, Load&& load,
                         Term&& term, Acc&& acc) {
   const int lane = threadIdx.x & (G - 1);
   const int nmax = __reduce_max_sync(0xffffffffu, n);
   // the gathers of the next round are issued before this round's sums
   int t = lane < n ? entry(lane) : s;
-  float4 xj = __ldg(xs + t);
+  float4 xj = __ldg(rec + t);
   auto p = load(t);
   for (int k0 = 0; k0 < nmax; k0 += G) {
     const bool mine = k0 + lane < n;
@@ -562,13 +585,13 @@ FS_DEV void group_visit(const float4* __restrict__ xs, int s, float4 xi, float h
     const auto p0 = p;
     if (k0 + G + lane < n) {
       t = entry(k0 + G + lane);
-      xj = __ldg(xs + t);
+      xj = __ldg(rec + t);
       p = load(t);
     }
     Terms<K> u;
     if (mine) {
       const float dx = xi.x - x0.x, dy = xi.y - x0.y, dz = xi.z - x0.z;
-      if (fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, x0.w))) <= h2m && (WITH_SELF || t0 != s)) u = term(t0, x0, p0);
+      if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= h2m && (WITH_SELF || t0 != s)) u = term(t0, x0, p0);
     }
     if constexpr (K > 0) {
       const int lim = min(G, nmax - k0);
@@ -707,22 +730,23 @@ FS_DEV int scan_sum(const GridDev& g, const ScanXyz& q, const float4* __restrict
 }
 
 template <int G, bool WITH_SELF, bool EVICT_FIRST, bool LAZY, int K, class Load, class Term, class Acc>
-FS_DEV void list_sum(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, float h2m,
-                     const NbrList& L, bool lists_ok, bool on, Load&& load, Term&& term, Acc&& acc) {
+FS_DEV void list_sum(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s, float4 xi,
+                     float h, float h2m, const NbrList& L, bool lists_ok, bool on, Load&& load, Term&& term,
+                     Acc&& acc) {
   if constexpr (G == 1) {
     if (!on) return;
     if constexpr (LAZY)
-      visit<WITH_SELF>(g, xs, s, xi, h, h2m, L, lists_ok, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
+      visit<WITH_SELF>(g, xs, rec, s, xi, h, h2m, L, lists_ok, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
     else
-      visit_with<WITH_SELF, EVICT_FIRST>(g, xs, s, xi, h, h2m, L, lists_ok, load,
+      visit_with<WITH_SELF, EVICT_FIRST>(g, xs, rec, s, xi, h, h2m, L, lists_ok, load,
                                          [&](int t, float4 xj, const auto& p) { acc(term(t, xj, p)); });
   } else {
     const int n = !on ? 0 : (lists_ok ? __ldg(L.cnt + s) : kNbMax + 1);
     const bool over = n > kNbMax;
     const int32_t* const row = L.idx + (int64_t)s * kNbMax;
-    group_visit<G, WITH_SELF, K>(xs, s, xi, h2m, over ? 0 : n, [&](int k) { return __ldg(row + k); }, load, term, acc);
+    group_visit<G, WITH_SELF, K>(rec, s, xi, h2m, over ? 0 : n, [&](int k) { return __ldg(row + k); }, load, term, acc);
     if (over && (K > 0 || (threadIdx.x & (G - 1)) == 0))  // each lane adds up the whole sum (K = 0: the first)
-      scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
+      scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { acc(term(t, __ldg(rec + t), load(t))); });
   }
 }
 

@@ -25,7 +25,8 @@ namespace fs {
 
 __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
                                 const float* __restrict__ v, float4* __restrict__ xs, ScanOut q,
-                                float4* __restrict__ vs, float* __restrict__ mv, uint32_t* status, int nworlds);
+                                float4* __restrict__ vs, float* __restrict__ mv, float* __restrict__ ms,
+                                uint32_t* status, int nworlds);
 
 namespace {
 
@@ -81,8 +82,8 @@ struct PbfGather {
   }
 };
 
-// compute_density (115-141), poly6, self included.  sc2[s] = (rho,
-// mass / max(rho, 1e-6)): the neighbour term of the viscosity and XSPH passes.
+// compute_density (115-141), poly6, self included.  vs[s].w becomes
+// mass / max(rho, 1e-6), the neighbour term of the viscosity pass.
 // It records the neighbour lists that the next pass at the same positions
 // (accel, or XSPH) reuses, out to h (1 + skin) where the first lambda pass
 // reuses them too (k_lambda).  With vout (the final density of a substep) it
@@ -91,8 +92,8 @@ struct PbfGather {
 // for non-dynamic particles.
 template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, int64_t n, const float4* __restrict__ xs,
-                                           const float4* __restrict__ vs, const float* __restrict__ mv, float h,
-                                           float skin, float* rho, float2* __restrict__ sc2,
+                                           float4* __restrict__ vs, const float* __restrict__ mv,
+                                           const float* __restrict__ ms, float h, float skin, float* rho,
                                            const float4* __restrict__ xin, float dt, float4* __restrict__ vout) {
   extern __shared__ uint2 smem[];
   grid_begin();
@@ -116,8 +117,8 @@ __global__ void FS_NB_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, int6
     if (!on) L.cnt[s] = 0;
     rho[i] = acc;
     const float4 vi = vs[s];
-    const float wgt = vi.w / fmaxf(acc, 1.0e-6f);
-    sc2[s] = make_float2(acc, wgt);
+    const float wgt = ms[s] / fmaxf(acc, 1.0e-6f);
+    if (!vout) vs[s] = make_float4(vi.x, vi.y, vi.z, wgt);
     if (vout) {
       float3 u = xyz(vi);  // non-dynamic: v_pred == v_in
       if (pf_of(xi) & PF_DYNAMIC) {
@@ -138,8 +139,8 @@ struct AccelArgs {
   int use_lists;
   int64_t n;
   const float4* xs;
-  const float4* vs;
-  const float2* sc2;
+  const float4* vs;  // (v, mass / max(rho, 1e-6))
+  const float* ms;
   fs_model m;
   float h, particle_radius, dt;
   Walls walls;
@@ -153,6 +154,11 @@ template <int G>
 __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
   grid_begin();
   float dmax = 0.f;
+  const Masses<G> mass(a.ms, a.L.ctl);
+  struct Neighbour {
+    float4 v;
+    float m;
+  };
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
@@ -160,7 +166,7 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
     const float4 vi = a.vs[s];
     const float mu = a.m.viscosity[i];
     const float gamma = a.m.surface_tension[i];
-    const float coh = gamma / vi.w;
+    const float coh = gamma / a.ms[s];
     const float mu10 = 10.f * mu;
     const float visc_den_add = 0.01f * (a.h * a.h);
     const float rp2 = a.particle_radius * a.particle_radius;
@@ -168,19 +174,19 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
     float ax = 0.f, ay = 0.f, az = 0.f;
     const bool on = live && dyn && (gamma != 0.f || mu != 0.f);
     list_sum<G, false, true, false, 4>(
-        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), on,
-        [&](int t) { return __ldg(a.vs + t); },
-        [&](int t, float4 xj, const float4& vj) {
+        a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), on,
+        [&](int t) { return Neighbour{__ldg(a.vs + t), mass(t)}; },
+        [&](int t, float4 xj, const Neighbour& j) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
           float c = 0.f;
-          if (gamma != 0.f) c -= coh * vj.w * K.w_r2(fmaxf(r2, rp2));  // W(max(r, r_p))
+          if (gamma != 0.f) c -= coh * j.m * K.w_r2(fmaxf(r2, rp2));  // W(max(r, r_p))
           if (mu != 0.f) {
-            const float vdot = fmaf(vi.x - vj.x, dx, fmaf(vi.y - vj.y, dy, (vi.z - vj.z) * dz));
+            const float vdot = fmaf(vi.x - j.v.x, dx, fmaf(vi.y - j.v.y, dy, (vi.z - j.v.z) * dz));
             if (vdot != 0.f) {
               float r, rinv;
               r_and_inv(r2, r, rinv);
-              c += mu10 * __ldg(&a.sc2[t].y) * __fdividef(vdot, r2 + visc_den_add) * K.grad_scale(r, rinv);
+              c += mu10 * j.v.w * __fdividef(vdot, r2 + visc_den_add) * K.grad_scale(r, rinv);
             }
           }
           return Terms<4>{c, dx, dy, dz};
@@ -217,11 +223,11 @@ struct LambdaArgs {
   ScanXyz q;
   int64_t n;
   const float4* xs;
-  const float4* vs;   // .w = mass
+  const float* ms;    // mass
   const float* rest_density;
   float h, eps;
   int min_nb;
-  float2* lam_s;      // cell order (lambda, mass): what the delta pass gathers per neighbour
+  float4* rec;        // cell order (x, y, z, lambda): what the delta pass gathers per neighbour
   float* lam;         // API
   float* rho;         // API
   int32_t* count;     // API
@@ -245,6 +251,7 @@ __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
   extern __shared__ uint2 smem[];
   grid_begin();
   lists_recorded(a.L);
+  const Masses<G> mass(a.ms, a.L.ctl);
   const bool reuse_ok = a.xs_rec && __uint_as_float(*a.disp_max) <= a.reuse_limit;
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
@@ -266,8 +273,7 @@ __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
     }
     scan_sum<G, true, false, true, 5>(
         a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, reuse ? listed : -1,
-        [&](int t) { return __ldg(&a.vs[t].w); },
-        [&](int t, float4 xj, const float& mj) {
+        mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
           if (t != (int)s && exact_lt_h(r2, dx, dy, dz, a.h, K.h2)) ++cnt;
@@ -287,7 +293,7 @@ __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
     if (!lead) return;
     if (!on) {
       a.L.cnt[s] = 0;
-      a.lam_s[s] = make_float2(0.f, a.vs[s].w);
+      a.rec[s] = make_float4(xi.x, xi.y, xi.z, 0.f);
       if (a.lam) a.lam[i] = 0.f;
       if (a.rho) a.rho[i] = 0.f;
       if (a.count) a.count[i] = 0;
@@ -296,7 +302,7 @@ __global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
     sq = fmaf(gx, gx, fmaf(gy, gy, fmaf(gz, gz, sq)));
     const float ci = fmaxf(rho / rho0 - 1.0f, 0.f);
     const float l = (a.min_nb > 0 && cnt < a.min_nb) ? 0.f : -ci / (sq + a.eps);
-    a.lam_s[s] = make_float2(l, a.vs[s].w);
+    a.rec[s] = make_float4(xi.x, xi.y, xi.z, l);
     if (a.lam) a.lam[i] = l;
     if (a.rho) a.rho[i] = rho;
     if (a.count) a.count[i] = cnt;
@@ -311,8 +317,8 @@ struct DeltaArgs {
   int use_lists;
   int64_t n;
   const float4* xs;
-  const float4* vs;   // .w = mass
-  const float2* lam_s;  // (lambda, mass), one gather per neighbour
+  const float* ms;    // mass
+  const float4* rec;  // (x, y, z, lambda), one gather per neighbour
   const float* rest_density;
   float h, scorr_k, scorr_n, w_dq, max_dp;
   int clamp;
@@ -338,20 +344,20 @@ __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
   grid_begin();
   // an integral exponent 1..8 (the class default is 4) takes pow_uint
   const int n_int = (a.scorr_n >= 1.f && a.scorr_n <= 8.f && a.scorr_n == rintf(a.scorr_n)) ? (int)a.scorr_n : 0;
+  const Masses<G> mass(a.ms, a.L.ctl);
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xi = a.xs[s];
     const int32_t i = a.g.perm[s];
     const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const float rho0 = fmaxf(a.rest_density[i], 1.0e-6f);
-    const float li = a.lam_s[s].x;
+    const float li = a.rec[s].w;
     const Poly6Spiky K(a.h);
     const bool scorr = a.scorr_k != 0.f && !(a.w_dq <= 1.0e-6f);
     const float inv_wdq = scorr ? 1.0f / a.w_dq : 0.f;
     float dx_ = 0.f, dy_ = 0.f, dz_ = 0.f;
     list_sum<G, false, true, false, 4>(
-        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), live && dyn,
-        [&](int t) { return __ldg(a.lam_s + t); },
-        [&](int t, float4 xj, const float2& lj) {
+        a.g, a.xs, a.rec, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        live && dyn, mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
           float r, rinv;
@@ -361,7 +367,7 @@ __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
             const float q = K.w_r2(r2) * inv_wdq;
             sc = -a.scorr_k * (n_int ? pow_uint(q, n_int) : powf(q, a.scorr_n));
           }
-          return Terms<4>{(li + lj.x + sc) * lj.y * K.grad_scale(r, rinv), dx, dy, dz};
+          return Terms<4>{(li + xj.w + sc) * mj * K.grad_scale(r, rinv), dx, dy, dz};
         },
         [&](const Terms<4>& u) {
           dx_ = fmaf(u.v[0], u.v[1], dx_);
@@ -401,7 +407,6 @@ struct XsphArgs {
   int64_t n;
   const float4* xs;
   const float4* vel;   // (v, m / max(rho, 1e-6)) cell order
-  const float2* sc2;   // rho
   float h, c;
   Walls walls;
   int bounds;          // fused apply_bounds (substep) or not (separate pass)
@@ -423,7 +428,7 @@ __global__ void FS_NB_BOUNDS_PBF k_xsph_final(XsphArgs a) {
     const Poly6Spiky K(a.h);
     float cx = 0.f, cy = 0.f, cz = 0.f;
     list_sum<G, false, true, false, 4>(
-        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn && a.c > 0.f, [&](int t) { return __ldg(a.vel + t); },
         [&](int t, float4 xj, const float4& vj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -462,26 +467,22 @@ __global__ void k_gather_lambda(int64_t n, const int32_t* __restrict__ perm, con
   if (s < n) out[s] = a[perm[s]];
 }
 
-// (rho, mass / max(rho, 1e-6)) from a cell-order density and the mass in
-// vel.w; vel.w then holds the ratio (XSPH's neighbour weight)
-__global__ void k_rho_ratio(int64_t n, const float* __restrict__ rho, float4* __restrict__ vel,
-                            float2* __restrict__ out) {
+// vel.w: mass / max(rho, 1e-6) (XSPH's neighbour weight) from a cell-order
+// density and the mass that is there
+__global__ void k_rho_ratio(int64_t n, const float* __restrict__ rho, float4* __restrict__ vel) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const float ratio = vel[s].w / fmaxf(rho[s], 1.0e-6f);
-  out[s] = make_float2(rho[s], ratio);
-  vel[s].w = ratio;
+  if (s < n) vel[s].w = vel[s].w / fmaxf(rho[s], 1.0e-6f);
 }
 
-// (lambda[i], mass) of original order into cell order (mass from the gathered vs.w)
-__global__ void k_gather_lambda_mass(int64_t n, const int32_t* __restrict__ perm, const float* __restrict__ lam,
-                                     const float4* __restrict__ vs, float2* __restrict__ out) {
+// (x, y, z, lambda[i]) in cell order
+__global__ void k_gather_lambda_rec(int64_t n, const int32_t* __restrict__ perm, const float* __restrict__ lam,
+                                    const float4* __restrict__ xs, float4* __restrict__ rec) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < n) out[s] = make_float2(lam[perm[s]], vs[s].w);
+  if (s < n) rec[s] = make_float4(xs[s].x, xs[s].y, xs[s].z, lam[perm[s]]);
 }
 
 PbfGather pbf_gather(fs_context* c, const fs_model* m, const float* x_in) {
-  return PbfGather{CommonGather{*m, c->xo_tmp, c->vo_tmp, c->xs, scan_out(c), c->vs, nullptr, c->mv, c->status,
+  return PbfGather{CommonGather{*m, c->xo_tmp, c->vo_tmp, c->xs, scan_out(c), c->vs, c->mv, c->mass, c->status,
                                 c->nworlds},
                    x_in, c->vs2};
 }
@@ -528,7 +529,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   const float skin = (!p->rebuild_grid_each_iteration && p->max_iterations > 0) ? c->list_skin : 0.f;
   {
     PassScope ps_(c, P_PBF_DENSITY, st);
-    FS_NB_LAUNCH(k_density, c, n, group, st, true, g, L, scan_xyz(c), n, c->xs, c->vs, c->mv, h, skin, so->rho, c->sc2,
+    FS_NB_LAUNCH(k_density, c, n, group, st, true, g, L, scan_xyz(c), n, c->xs, c->vs, c->mv, c->mass, h, skin, so->rho,
                  nullptr, 0.f, nullptr);
   }
   AccelArgs aa;
@@ -538,7 +539,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   aa.n = n;
   aa.xs = c->xs;
   aa.vs = c->vs;
-  aa.sc2 = c->sc2;
+  aa.ms = c->mass;
   aa.m = *m;
   aa.h = h;
   aa.particle_radius = p->particle_radius;
@@ -563,12 +564,12 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     la.q = scan_xyz(c);
     la.n = n;
     la.xs = cur;
-    la.vs = c->vs;
+    la.ms = c->mass;
     la.rest_density = m->rest_density;
     la.h = h;
     la.eps = p->lambda_epsilon;
     la.min_nb = p->min_neighbors_for_lambda;
-    la.lam_s = c->krm;
+    la.rec = c->rec;
     la.lam = so->pbf_lambda;
     la.rho = so->rho;
     la.count = so->neighbor_count;
@@ -585,8 +586,8 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
     da.use_lists = use_lists;
     da.n = n;
     da.xs = cur;
-    da.vs = c->vs;
-    da.lam_s = c->krm;
+    da.ms = c->mass;
+    da.rec = c->rec;
     da.rest_density = m->rest_density;
     da.h = h;
     da.scorr_k = p->scorr_k;
@@ -624,7 +625,7 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   {
     // + update_velocity_from_positions into nxt (the other x_pred buffer)
     PassScope ps_(c, P_PBF_DENSITY, st);
-    FS_NB_LAUNCH(k_density, c, n, group, st, true, gf, L, scan_xyz(c), n, cur, c->vs, c->mv, h, 0.f, so->rho, c->sc2,
+    FS_NB_LAUNCH(k_density, c, n, group, st, true, gf, L, scan_xyz(c), n, cur, c->vs, c->mv, c->mass, h, 0.f, so->rho,
                  c->vs2, dt, nxt);
   }
   XsphArgs xa;
@@ -634,7 +635,6 @@ int fs_pbf_substep(fs_context* c, const fs_model* m, const fs_state* si, fs_stat
   xa.n = n;
   xa.xs = cur;
   xa.vel = nxt;
-  xa.sc2 = c->sc2;
   xa.h = h;
   xa.c = p->xsph_c;
   xa.walls = w;
@@ -671,9 +671,9 @@ int fs_pbf_density(fs_context* c, const fs_model* m, const float* x, float h, fl
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, x, c->xs, scan_out(c), c->vs, c->mv,
-                                                       c->status, c->nworlds);
+                                                       c->mass, c->status, c->nworlds);
   FS_NB_LAUNCH(k_density, c, m->n, nb_group(m->n), st, true, grid_view(c), nbr_list(c), scan_xyz(c), m->n, c->xs,
-               c->vs, c->mv, h, 0.f, rho, c->sc2, nullptr, 0.f, nullptr);
+               c->vs, c->mv, c->mass, h, 0.f, rho, nullptr, 0.f, nullptr);
   return launch_check("fs_pbf_density");
 }
 
@@ -685,19 +685,19 @@ int fs_pbf_lambda(fs_context* c, const fs_model* m, const float* x_pred, const f
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, x_pred, c->xs, scan_out(c), c->vs, nullptr,
-                                                       c->status, c->nworlds);
+                                                       c->mass, c->status, c->nworlds);
   LambdaArgs la;
   la.g = grid_view(c);
   la.L = nbr_list(c);
   la.q = scan_xyz(c);
   la.n = m->n;
   la.xs = c->xs;
-  la.vs = c->vs;
+  la.ms = c->mass;
   la.rest_density = m->rest_density;
   la.h = p->smoothing_length;
   la.eps = p->lambda_epsilon;
   la.min_nb = p->min_neighbors_for_lambda;
-  la.lam_s = c->krm;
+  la.rec = c->rec;
   la.lam = pbf_lambda;
   la.rho = rho;
   la.count = neighbor_count;
@@ -714,16 +714,16 @@ int fs_pbf_delta(fs_context* c, const fs_model* m, const float* x_pred, const fl
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, x_pred, c->xs, scan_out(c), c->vs, nullptr,
-                                                       c->status, c->nworlds);
-  k_gather_lambda_mass<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, pbf_lambda, c->vs, c->krm);
+                                                       c->mass, c->status, c->nworlds);
+  k_gather_lambda_rec<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, pbf_lambda, c->xs, c->rec);
   DeltaArgs da;
   da.g = grid_view(c);
   da.L = nbr_list(c);
   da.use_lists = 0;
   da.n = m->n;
   da.xs = c->xs;
-  da.vs = c->vs;
-  da.lam_s = c->krm;
+  da.ms = c->mass;
+  da.rec = c->rec;
   da.rest_density = m->rest_density;
   da.h = p->smoothing_length;
   da.scorr_k = p->scorr_k;
@@ -747,9 +747,9 @@ int fs_pbf_xsph(fs_context* c, const fs_model* m, const float* x_pred, const flo
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, v_in, c->xs, scan_out(c), c->vs2, nullptr,
-                                                       c->status, c->nworlds);
+                                                       c->mass, c->status, c->nworlds);
   k_gather_lambda<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, rho, c->sc1);
-  k_rho_ratio<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->sc1, c->vs2, c->sc2);
+  k_rho_ratio<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->sc1, c->vs2);
   XsphArgs xa;
   xa.g = grid_view(c);
   xa.L = nbr_list(c);
@@ -757,7 +757,6 @@ int fs_pbf_xsph(fs_context* c, const fs_model* m, const float* x_pred, const flo
   xa.n = m->n;
   xa.xs = c->xs;
   xa.vel = c->vs2;
-  xa.sc2 = c->sc2;
   xa.h = h;
   xa.c = xsph_c;
   xa.walls = Walls{};

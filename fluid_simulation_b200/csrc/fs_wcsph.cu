@@ -18,10 +18,11 @@ namespace fs {
 // solver_wcsph.py:110-116).
 __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
                                 const float* __restrict__ v, float4* __restrict__ xs, ScanOut q,
-                                float4* __restrict__ vs, float* __restrict__ mv, uint32_t* status, int nworlds) {
+                                float4* __restrict__ vs, float* __restrict__ mv, float* __restrict__ ms,
+                                uint32_t* status, int nworlds) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  gather_common_slot(s, perm[s], m, x, v, xs, q, vs, mv, status, nworlds);
+  gather_common_slot(s, perm[s], m, x, v, xs, q, vs, mv, ms, status, nworlds);
 }
 
 // ------------------------------------------------------------- density ----
@@ -128,8 +129,8 @@ __global__ void FS_NB_BOUNDS k_wcsph_force(ForceArgs a) {
       float2 r;  // (p_j / rho_j^2, 1 / rho_j)
     };
     list_sum<G, false, false, true, 4>(
-        a.g, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), live && dyn,
-        [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(a.sc2 + t)}; },
+        a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
+        live && dyn, [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(a.sc2 + t)}; },
         [&](int t, float4 xj, const Neighbour& j) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
           const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -196,7 +197,7 @@ int wcsph_gather(fs_context* c, const fs_model* m, const float* x, const float* 
   const int64_t n = m->n;
   {
     PassScope ps_(c, P_GATHER, st);
-    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs, c->mv, c->status, c->nworlds);
+    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs, c->mv, c->mass, c->status, c->nworlds);
   }
   return launch_check("wcsph gather");
 }
@@ -205,7 +206,7 @@ int wcsph_gather(fs_context* c, const fs_model* m, const float* x, const float* 
 static int wcsph_build(fs_context* c, const fs_model* m, const fs_state* si, float h, cudaStream_t st,
                        const fs_frame_clock* clock) {
   return grid_build(c, m->n, h * c->cell_ratio, st, m->particle_world, clock, KeyPositions{si->particle_q},
-                    CommonGather{*m, si->particle_q, si->particle_qd, c->xs, scan_out(c), c->vs, nullptr, c->mv,
+                    CommonGather{*m, si->particle_q, si->particle_qd, c->xs, scan_out(c), c->vs, c->mv, nullptr,
                                  c->status, c->nworlds});
 }
 
@@ -329,7 +330,7 @@ int fs_wcsph_density(fs_context* c, const fs_model* m, const float* x, float h, 
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, nullptr, c->xs, scan_out(c), nullptr, c->mv,
-                                                       c->status, c->nworlds);
+                                                       c->mass, c->status, c->nworlds);
   return launch_density(c, m, h, clamp_negative, true, rho, pressure, st);
 }
 

@@ -89,34 +89,56 @@ def block(n, corner, seed):
     return x.astype(np.float32), rng.normal(0.0, 0.1, x.shape).astype(np.float32)
 
 
-@pytest.mark.parametrize("total", [4999, 5001, 14000, 14001, 36000, 36001])
-@pytest.mark.parametrize("kind", ["wcsph", "dfsph", "pbf"])
-def test_lanes_per_particle_change_no_bit(kind, total, cuda_device):
-    cls = dict(wcsph=SolverWCSPH, dfsph=SolverDFSPH, pbf=SolverPBF)[kind]
+def config(kind, cls):
+    """Config, time step and model attributes with every pass at work; DFSPH never ends early (its residual is a mean
+    over all particles)."""
     base = dict(particle_radius=0.5 * SP, particle_length=SP, smoothing_length_coff=2.0, bound_width=0.6,
                 bound_height=0.6, bound_length=0.5, boundary_damping=0.0)
     attrs = dict(particle_mask=0, rest_density=1000.0, surface_tension=0.01, viscosity=0.005)
     if kind == "wcsph":
-        cfg, dt = cls.SphConfig(**base), 1e-4
         attrs.update(stiffness=2.5e5, exponent=7.0)
-    elif kind == "dfsph":  # no early end: the residual is a mean over all particles
-        cfg, dt = cls.SphConfig(max_rho_iterations=3, max_vel_iterations=4, warm_start=False, eta_density=-1.0,
-                                eta_divergence=-1.0, **base), 1e-3
-    else:
-        cfg, dt = cls.PbfConfig(max_iterations=3, lambda_epsilon=100.0, max_delta_position=0.25 * SP, xsph_c=0.05,
-                                scorr_k=1e-4, **base), 1e-3
+        return cls.SphConfig(**base), 1e-4, attrs
+    if kind == "dfsph":
+        return cls.SphConfig(max_rho_iterations=3, max_vel_iterations=4, warm_start=False, eta_density=-1.0,
+                             eta_divergence=-1.0, **base), 1e-3, attrs
+    return cls.PbfConfig(max_iterations=3, lambda_epsilon=100.0, max_delta_position=0.25 * SP, xsph_c=0.05,
+                         scorr_k=1e-4, **base), 1e-3, attrs
+
+
+def run_step(kind, x, v, mass, dev):
+    cls = dict(wcsph=SolverWCSPH, dfsph=SolverDFSPH, pbf=SolverPBF)[kind]
+    cfg, dt, attrs = config(kind, cls)
+    m = model_from_arrays(x, v, mass, device=dev, radius=0.5 * SP, attributes=attrs, solver_cls=cls)
+    s = cls(m, cfg)
+    a, b = m.state(), m.state()
+    s.step(a, b, None, None, dt)
+    return dict(vars(b.sph), x=b.particle_q, v=b.particle_qd, accel=s._particle_accel)
+
+
+@pytest.mark.parametrize("n", [3000, 40000])
+@pytest.mark.parametrize("kind", ["wcsph", "dfsph", "pbf"])
+def test_particles_of_another_mass_far_away_change_no_bit(kind, n, cuda_device):
+    """One mass for all is not loaded for each neighbour; one far particle of another mass has them all loaded."""
+    x, v = block(n, (-0.55, -0.55, 0.02), 1)
+    far = np.array([[0.55, 0.55, 0.9]], np.float32)
+    mass = 1000.0 * SP ** 3
+    same = run_step(kind, np.concatenate([x, far]), np.concatenate([v, 0 * far]), mass, cuda_device)
+    masses = np.full(n + 1, mass, np.float32)
+    masses[n] *= 2.0
+    mixed = run_step(kind, np.concatenate([x, far]), np.concatenate([v, 0 * far]), masses, cuda_device)
+    for name, t in same.items():
+        assert torch.equal(t[:n], mixed[name][:n]), name
+
+
+@pytest.mark.parametrize("total", [4999, 5001, 14000, 14001, 36000, 36001])
+@pytest.mark.parametrize("kind", ["wcsph", "dfsph", "pbf"])
+def test_lanes_per_particle_change_no_bit(kind, total, cuda_device):
     n = 2500
     x, v = block(n, (-0.55, -0.55, 0.02), 1)
     x2, v2 = block(total - n, (-0.2, -0.2, 0.02), 2)
 
-    def run(x, v):
-        m = model_from_arrays(x, v, 1000.0 * SP ** 3, device=cuda_device, radius=0.5 * SP, attributes=attrs,
-                              solver_cls=cls)
-        s = cls(m, cfg)
-        a, b = m.state(), m.state()
-        s.step(a, b, None, None, dt)
-        return dict(vars(b.sph), x=b.particle_q, v=b.particle_qd, accel=s._particle_accel)
-
-    alone, both = run(x, v), run(np.concatenate([x, x2]), np.concatenate([v, v2]))
+    mass = 1000.0 * SP ** 3
+    alone = run_step(kind, x, v, mass, cuda_device)
+    both = run_step(kind, np.concatenate([x, x2]), np.concatenate([v, v2]), mass, cuda_device)
     for name, t in alone.items():
         assert torch.equal(t, both[name][:n]), name
