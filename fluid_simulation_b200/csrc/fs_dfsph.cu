@@ -331,7 +331,7 @@ __device__ bool last_block(uint32_t* ticket) {
 }
 
 template <int G>
-__global__ void FS_NB_BOUNDS k_rate(RateArgs a) {
+__global__ void __launch_bounds__(kNbBlockMax, 4) k_rate(RateArgs a) {
   grid_begin();
   if (a.ctrl && a.ctrl->done) return;  // uniform across the grid: set by an earlier launch
   if (clock_idle(a.clock)) return;     // uniform: the frame is complete

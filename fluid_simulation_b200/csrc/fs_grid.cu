@@ -182,17 +182,18 @@ NbrList nbr_list(const fs_context* c) {
 // Lanes per particle: as many as fill the GPU (148 SMs hold 151,552 threads of
 // these kernels), fewer where the sums, which every lane of a group repeats,
 // outweigh the shorter chain.  Substep times in us, B200:
-//   particles        4,000   8,000   15,000   28,000   38,000   50,000
-//   PBF    1 lane      276     276      287      308      334      306
-//          4 lanes     209     222      231      288      329      406
-//          8 lanes     164     180      207      303      354      430
-//         16 lanes     151     179      250      362      452      552
-//   DFSPH  1 lane      644     662      660      726      728      749
-//          4 lanes     430     453      487      579      655      807
-//          8 lanes     400     409      489      697      814      953
-//         16 lanes     393     481      614      915    1,091    1,345
-// (WCSPH and its adjoint cross over at the same sizes.)
-int nb_group(int64_t n) { return n <= 5000 ? 16 : n <= 14000 ? 8 : n <= 36000 ? 4 : 1; }
+//   particles        4,000   7,500   14,000   30,000   38,000   46,000
+//   PBF    1 lane      218     221      227      239      269      273
+//          4 lanes     132     135      145      218      263      294
+//          8 lanes     104     115      135      253      299      353
+//         16 lanes      93     129      177      322      394      460
+//   DFSPH  1 lane      495     513      536      556      587      599
+//          4 lanes     301     311      328      446      521      644
+//          8 lanes     278     296      346      579      657      804
+//         16 lanes     265     325      481      792      962    1,119
+// (WCSPH and its adjoint cross over at the same sizes; two lanes are slower
+// than one or four throughout, but for DFSPH between 38,000 and 50,000.)
+int nb_group(int64_t n) { return n <= 6000 ? 16 : n <= 14000 ? 8 : n <= 38000 ? 4 : 1; }
 
 ScanXyz scan_xyz(const fs_context* c) { return ScanXyz{c->sxyz}; }
 ScanOut scan_out(const fs_context* c) {

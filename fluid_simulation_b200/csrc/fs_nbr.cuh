@@ -196,10 +196,10 @@ struct ScanPos {
 // Writes the slot ranges of the query of slot s, in visiting order
 // (for_each_range's ranges) and cut into pieces of at most 32 candidates
 // (counted from the 16-byte group that holds the first), to words[k * nthr]
-// as (first, end), from pos on until kWords pieces are written or the query
+// as (first, end), from pos on until CAP pieces are written or the query
 // is exhausted (live = false); returns their number.  COUNT adds the active
 // candidates other than s (no distance test) to ncand.
-template <bool COUNT>
+template <bool COUNT, int CAP>
 FS_DEV int scan_pieces(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, bool inactive,
                        uint2* words, int nthr, ScanPos& pos, bool& live, int& ncand) {
   const WorldDev* W = g.worlds ? g.worlds + world_index(world_of(xi), g.nworlds) : nullptr;
@@ -249,7 +249,7 @@ FS_DEV int scan_pieces(const GridDev& g, const float4* __restrict__ xs, int s, f
         if (COUNT) count(a[k], e[k]);
         for (int f = a[k]; f < e[k];) {
           const int stop = min(e[k], (f & ~3) + 32);
-          if (nw == kWords) {
+          if (nw == CAP) {
             pos.z = b.z0 + k / 3, pos.y = b.y0 + k % 3, pos.t = f;
             return nw;
           }
@@ -288,7 +288,7 @@ FS_DEV int scan_pieces(const GridDev& g, const float4* __restrict__ xs, int s, f
       if (COUNT) count(a, e);
     }
     while (f < e) {
-      if (nw == kWords) {
+      if (nw == CAP) {
         pos.t = f;
         return nw;
       }
@@ -304,35 +304,50 @@ FS_DEV int scan_pieces(const GridDev& g, const float4* __restrict__ xs, int s, f
   return nw;
 }
 
-// Replaces the pieces in `words` by their non-empty hit words (mask, last):
-// bit b set = slot last - b lies within the radius whose square is h2.
+// A particle's position and squared radius (negative), doubled for the packed
+// operations of the scan.
+struct ScanQuery {
+  f32x2 nx, ny, nz, nh;
+  FS_DEV ScanQuery(float4 xi, float h2)
+      : nx(pack2(-xi.x, -xi.x)), ny(pack2(-xi.y, -xi.y)), nz(pack2(-xi.z, -xi.z)), nh(pack2(-h2, -h2)) {}
+};
+
+// The hit word of the piece [first, end), not empty, at most 32 slots from the
+// group of four that holds the first: bit b set = slot last - b is within.
+FS_DEV uint32_t scan_word(const ScanXyz& q, const ScanQuery& o, uint32_t first, uint32_t end, uint32_t& last) {
+  const uint32_t g0 = first >> 2, g1 = (end + 3) >> 2;
+  const ulonglong2* p = reinterpret_cast<const ulonglong2*>(q.g) + (size_t)g0 * 3;
+  uint32_t m = 0;
+#pragma unroll 2  // two groups of loads in flight (density time with 1: +1 to 3 %, with 4: up to +7 %)
+  for (uint32_t i = g0; i < g1; ++i, p += 3) {
+    const ulonglong2 x2 = __ldg(p), y2 = __ldg(p + 1), z2 = __ldg(p + 2);
+    const f32x2 dx0 = add2(x2.x, o.nx), dx1 = add2(x2.y, o.nx);
+    const f32x2 dy0 = add2(y2.x, o.ny), dy1 = add2(y2.y, o.ny);
+    const f32x2 dz0 = add2(z2.x, o.nz), dz1 = add2(z2.y, o.nz);
+    const f32x2 r0 = fma2(dx0, dx0, fma2(dy0, dy0, fma2(dz0, dz0, o.nh)));
+    const f32x2 r1 = fma2(dx1, dx1, fma2(dy1, dy1, fma2(dz1, dz1, o.nh)));
+    m = __funnelshift_l((uint32_t)r0, m, 1);  // the sign bit of r^2 - h2: set = within
+    m = __funnelshift_l((uint32_t)(r0 >> 32), m, 1);
+    m = __funnelshift_l((uint32_t)r1, m, 1);
+    m = __funnelshift_l((uint32_t)(r1 >> 32), m, 1);
+  }
+  // slots of the groups outside the piece: before its first, after its last
+  m &= 0xffffffffu >> (32 - 4 * (g1 - g0) + (first & 3));
+  m &= 0xffffffffu << (4 * g1 - end);
+  last = 4 * g1 - 1;
+  return m;
+}
+
+// Replaces the pieces in `words` by their non-empty hit words (mask, last).
 FS_DEV int scan_words(const ScanXyz& q, float4 xi, float h2, uint2* words, int nthr, int np) {
-  const f32x2 nx = pack2(-xi.x, -xi.x), ny = pack2(-xi.y, -xi.y), nz = pack2(-xi.z, -xi.z);
-  const f32x2 nh = pack2(-h2, -h2);
+  const ScanQuery o(xi, h2);
   int nw = 0;
   for (int k = 0; k < np; ++k) {
     const uint2 piece = words[k * nthr];
-    const uint32_t g0 = piece.x >> 2, g1 = (piece.y + 3) >> 2;  // groups of four candidates
-    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(q.g) + (size_t)g0 * 3;
-    uint32_t m = 0;
-#pragma unroll 2  // two groups of loads in flight (density time with 1: +1 to 3 %, with 4: up to +7 %)
-    for (uint32_t i = g0; i < g1; ++i, p += 3) {
-      const ulonglong2 x2 = __ldg(p), y2 = __ldg(p + 1), z2 = __ldg(p + 2);
-      const f32x2 dx0 = add2(x2.x, nx), dx1 = add2(x2.y, nx);
-      const f32x2 dy0 = add2(y2.x, ny), dy1 = add2(y2.y, ny);
-      const f32x2 dz0 = add2(z2.x, nz), dz1 = add2(z2.y, nz);
-      const f32x2 r0 = fma2(dx0, dx0, fma2(dy0, dy0, fma2(dz0, dz0, nh)));
-      const f32x2 r1 = fma2(dx1, dx1, fma2(dy1, dy1, fma2(dz1, dz1, nh)));
-      m = __funnelshift_l((uint32_t)r0, m, 1);  // the sign bit of r^2 - h2: set = within
-      m = __funnelshift_l((uint32_t)(r0 >> 32), m, 1);
-      m = __funnelshift_l((uint32_t)r1, m, 1);
-      m = __funnelshift_l((uint32_t)(r1 >> 32), m, 1);
-    }
-    // slots of the groups outside the piece: before its first, after its last
-    m &= 0xffffffffu >> (32 - 4 * (g1 - g0) + (piece.x & 3));
-    m &= 0xffffffffu << (4 * g1 - piece.y);
+    uint32_t last;
+    const uint32_t m = scan_word(q, o, piece.x, piece.y, last);
     if (m) {
-      words[nw * nthr] = make_uint2(m, 4 * g1 - 1);
+      words[nw * nthr] = make_uint2(m, last);
       ++nw;
     }
   }
@@ -366,7 +381,7 @@ FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restri
   while (live) {
     int nw = 0;
     if (scan) {
-      const int np = scan_pieces<COUNT>(g, xs, s, xi, h, inactive, words, nthr, pos, live, ncand);
+      const int np = scan_pieces<COUNT, kWords>(g, xs, s, xi, h, inactive, words, nthr, pos, live, ncand);
       nw = scan_words(q, xi, h2rec * kScanSlack, words, nthr, np);
     } else {
       live = false;
@@ -534,11 +549,13 @@ FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, const fl
 // Every kernel of a context and particle count takes the same G.
 constexpr int kGroupList = 128;  // hits of a particle held in shared memory between two visits
 
+constexpr int kGroupRows = 9;    // rows of a usual query, each scanned by one lane
+
 // Shared memory of a recording launch: one thread per particle keeps kWords
-// words at stride `threads`, a group its words and kGroupList hits.
+// words at stride `threads`, a group kGroupRows pieces and kGroupList hits.
 inline size_t scan_smem(int threads, int group) {
-  const size_t words = sizeof(uint2) * kWords;
-  return group == 1 ? words * threads : (words + sizeof(int32_t) * kGroupList) * (threads / group);
+  return group == 1 ? sizeof(uint2) * kWords * threads
+                    : (sizeof(uint2) * kGroupRows + sizeof(int32_t) * kGroupList) * (threads / group);
 }
 
 // K floats a pair contributes; the zero value changes no sum.  K = 0: the
@@ -603,93 +620,129 @@ FS_DEV void group_visit(const float4* __restrict__ rec, int s, float4 xi, float 
   }
 }
 
+// The rows of a usual query (up to 3 x 3 rows of one slot range each, at most
+// two pieces a row): lane l of the group gets rows l, l + G, ... as [f, e),
+// empty where there is none.  False where the query is none of the usual ones;
+// f and e are then not to be used.
+template <int G, int N>
+FS_DEV bool group_rows(const GridDev& g, float4 xi, float h, int (&f)[N], int (&e)[N]) {
+  const WorldDev* W = g.worlds ? g.worlds + world_index(world_of(xi), g.nworlds) : nullptr;
+  const QueryBox b = W ? query_box_world(g, *W, xi.x, xi.y, xi.z, h) : query_box_hash(g, xi.x, xi.y, xi.z, h);
+  const int nx = b.x1 - b.x0 + 1, ny = b.y1 - b.y0 + 1, nz = b.z1 - b.z0 + 1;
+  int c0 = b.x0;
+  bool plain = nx > 0 && ny <= 3 && nz <= 3;
+  if (!W) {
+    const int xa = b.x0 + (1 << 20);
+    c0 = g.mask_x >= 0 ? (xa & g.mask_x) : xa % g.dim_x;
+    plain = plain && xa >= 0 && c0 + nx <= g.dim_x && min(b.y0, b.z0) >= -(1 << 20);
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const int r = (int)(threadIdx.x & (G - 1)) + k * G, z = (r * 11) >> 5, y = r - 3 * z;
+    f[k] = e[k] = 0;
+    if (plain && r < kGroupRows && z < nz && y < ny) {
+      const int row = W ? W->base + ((b.z0 + z) * W->dims[1] + b.y0 + y) * W->dims[0]
+                        : (wrap_axis(b.z0 + z, g.dim_z, g.mask_z) * g.dim_y + wrap_axis(b.y0 + y, g.dim_y, g.mask_y)) *
+                              g.dim_x;
+      f[k] = __ldg(g.off + row + c0);
+      e[k] = __ldg(g.off + row + c0 + nx);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) plain = plain && e[k] - (f[k] & ~3) <= 64;
+  return plain;
+}
+
 // scan_visit by the G lanes of a group (`on` and `reuse` are the same in all
 // of them; `on` = false: the particle takes no part).  All lanes of the warp
-// call it together.
+// call it together.  Each lane scans whole rows (other queries: pieces cut by
+// scan_pieces), the hits get their places in visiting order from a scan of
+// the lanes' counts, and group_visit takes them from shared memory.
 template <int G, bool WITH_SELF, bool COUNT, bool REUSE, int K, class Load, class Term, class Acc>
 FS_DEV int group_scan(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
                       float h2rec, float h2m, const NbrList& L, void* smem, bool on, int reuse, Load&& load,
                       Term&& term, Acc&& acc) {
-  constexpr int kIt = kWords * 8 / G;      // groups of four candidates per lane between two visits
-  constexpr int kPk = (kIt + 3) / 4;       // their hit counts, a byte each
+  constexpr int N = (kGroupRows + G - 1) / G;  // rows per lane
   const int lane = threadIdx.x & (G - 1), grp = threadIdx.x / G;
-  uint2* const words = (uint2*)smem + grp * kWords;
-  int32_t* const list = (int32_t*)((uint2*)smem + (blockDim.x / G) * kWords) + grp * kGroupList;
+  uint2* const pieces = (uint2*)smem + grp * kGroupRows;
+  int32_t* const list = (int32_t*)((uint2*)smem + (blockDim.x / G) * kGroupRows) + grp * kGroupList;
   int32_t* const row = L.idx + (int64_t)s * kNbMax;
   const bool inactive = COUNT && L.ctl->inactive;
-  const float h2 = h2rec * kScanSlack;
-  const f32x2 nx = pack2(-xi.x, -xi.x), ny = pack2(-xi.y, -xi.y), nz = pack2(-xi.z, -xi.z), nh = pack2(-h2, -h2);
+  const ScanQuery o(xi, h2rec * kScanSlack);
   const bool scan = on && (!REUSE || reuse < 0);
+  int f[N], e[N];
+  const bool usual = group_rows<G>(g, xi, h, f, e);
+  // the whole group takes the usual way, or none of it
+  const unsigned votes = __ballot_sync(0xffffffffu, usual) >> (threadIdx.x & (32 - G));
+  const bool plain = (votes & (unsigned)((1ull << G) - 1)) == (unsigned)((1ull << G) - 1);
   ScanPos pos{INT32_MIN, 0, 0, -1};
   bool live = on;
   int n = 0, ncand = 0;
   while (__any_sync(0xffffffffu, live)) {
-    int np = 0;
-    if (live && scan)
-      np = scan_pieces<COUNT>(g, xs, s, xi, h, inactive, words, 1, pos, live, ncand);  // all lanes write the same
-    __syncwarp();
-    uint32_t hit[(kIt + 7) / 8] = {}, pk[kPk] = {};  // four hit bits a round; their counts
+    const bool now = live && scan, again = REUSE && live && !scan;  // (other groups of the warp may go on)
+    if (now && !plain) {
+      int nc = 0;
+      const int np = scan_pieces<COUNT, kGroupRows>(g, xs, s, xi, h, inactive, pieces, 1, pos, live, nc);
+      if (lane == 0) ncand += nc;
+      // every lane has written the same pieces
 #pragma unroll
-    for (int i = 0; i < kIt; ++i) {
-      const int slot = i * G + lane, piece = slot >> 3;
-      uint32_t nib = 0;
-      if (piece < np) {
-        const uint2 w = words[piece];
-        const uint32_t gi = (w.x >> 2) + (slot & 7);
-        if (gi < (w.y + 3) >> 2) {
-          const ulonglong2* p = reinterpret_cast<const ulonglong2*>(q.g) + (size_t)gi * 3;
-          const ulonglong2 x2 = __ldg(p), y2 = __ldg(p + 1), z2 = __ldg(p + 2);
-          const f32x2 dx0 = add2(x2.x, nx), dx1 = add2(x2.y, nx);
-          const f32x2 dy0 = add2(y2.x, ny), dy1 = add2(y2.y, ny);
-          const f32x2 dz0 = add2(z2.x, nz), dz1 = add2(z2.y, nz);
-          const f32x2 r0 = fma2(dx0, dx0, fma2(dy0, dy0, fma2(dz0, dz0, nh)));
-          const f32x2 r1 = fma2(dx1, dx1, fma2(dy1, dy1, fma2(dz1, dz1, nh)));
-          nib = ((uint32_t)r0 >> 31) | ((uint32_t)(r0 >> 63) << 1) | (((uint32_t)r1 >> 31) << 2) |
-                ((uint32_t)(r1 >> 63) << 3);
-          const int f = (int)w.x - (int)(4 * gi), e = (int)w.y - (int)(4 * gi);  // the piece within this group
-          if (f > 0) nib &= 0xfu << f;
-          if (e < 4) nib &= (1u << e) - 1u;
+      for (int k = 0; k < N; ++k) {
+        const bool in = lane + k * G < np;
+        f[k] = in ? (int)pieces[lane + k * G].x : 0;
+        e[k] = in ? (int)pieces[lane + k * G].y : 0;
+      }
+    } else {
+      live = false;
+    }
+    static_assert(N <= 3, "hits of the rounds, ten bits each");
+    uint32_t w[N][2], last[N][2], cnt = 0;  // hit words; hits of the rounds
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      if (COUNT && now && plain) {
+        if (inactive) {
+          for (int t = f[k]; t < e[k]; ++t) ncand += (t != s) ? (__float_as_int(__ldg(&xs[t].w)) & PF_ACTIVE) : 0;
+        } else {
+          ncand += (e[k] - f[k]) - ((s >= f[k] && s < e[k]) ? 1 : 0);
         }
       }
-      hit[i >> 3] |= nib << (4 * (i & 7));
-      pk[i >> 2] += (uint32_t)__popc(nib) << (8 * (i & 3));
+      const int mid = min(e[k], (f[k] & ~3) + 32);
+      w[k][0] = w[k][1] = last[k][0] = last[k][1] = 0;
+      if (now && f[k] < mid) w[k][0] = scan_word(q, o, f[k], mid, last[k][0]);
+      if (now && mid < e[k]) w[k][1] = scan_word(q, o, mid, e[k], last[k][1]);
+      cnt |= (uint32_t)(__popc(w[k][0]) + __popc(w[k][1])) << (10 * k);
     }
-    // hits before this lane's in each round, and in all lanes
-    uint32_t tot[kPk];
+    // hits before this lane's in each round, and in all lanes (at most 9 rows of 64: ten bits)
+    const uint32_t own = cnt;
 #pragma unroll
-    for (int k = 0; k < kPk; ++k) {
-      const uint32_t own = pk[k];
-#pragma unroll
-      for (int o = 1; o < G; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, pk[k], o, G);
-        if (lane >= o) pk[k] += v;
-      }
-      tot[k] = __shfl_sync(0xffffffffu, pk[k], G - 1, G);
-      pk[k] -= own;
+    for (int d = 1; d < G; d <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, cnt, d, G);
+      if (lane >= d) cnt += v;
     }
+    const uint32_t tot = __shfl_sync(0xffffffffu, cnt, G - 1, G);
+    cnt -= own;
     int nb = 0;
 #pragma unroll
-    for (int i = 0; i < kIt; ++i) nb += (tot[i >> 2] >> (8 * (i & 3))) & 0xff;
-    if (REUSE && live && !scan) nb = reuse;
+    for (int k = 0; k < N; ++k) nb += (int)((tot >> (10 * k)) & 1023);
+    if (again) nb = reuse;
     const int nbmax = __reduce_max_sync(0xffffffffu, nb);
     for (int w0 = 0; w0 < nbmax; w0 += kGroupList) {
-      if (REUSE && live && !scan) {
+      if (again) {
         for (int k = lane; k < kGroupList && w0 + k < nb; k += G) list[k] = row[w0 + k];
       } else {
         int base = 0;
 #pragma unroll
-        for (int i = 0; i < kIt; ++i) {
-          uint32_t m = (hit[i >> 3] >> (4 * (i & 7))) & 0xf;
-          int o = base + ((pk[i >> 2] >> (8 * (i & 3))) & 0xff);
-          base += (tot[i >> 2] >> (8 * (i & 3))) & 0xff;
-          if (m) {
-            const int slot = i * G + lane;
-            const int t = (int)(((words[slot >> 3].x >> 2) + (slot & 7)) * 4);
-            for (; m; m &= m - 1, ++o) {
-              const int v = t + __ffs(m) - 1;
-              if (o >= w0 && o < w0 + kGroupList) {
-                list[o - w0] = v;
-                if (n + o < kNbMax) row[n + o] = v;
+        for (int k = 0; k < N; ++k) {
+          int p = base + (int)((cnt >> (10 * k)) & 1023);
+          base += (int)((tot >> (10 * k)) & 1023);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            for (uint32_t m = w[k][u]; m; ++p) {
+              const uint32_t hi = 31 - __clz(m);
+              m ^= 1u << hi;
+              const int t = (int)(last[k][u] - hi);
+              if (p >= w0 && p < w0 + kGroupList) {
+                list[p - w0] = t;
+                if (n + p < kNbMax) row[n + p] = t;
               }
             }
           }
@@ -701,10 +754,9 @@ FS_DEV int group_scan(const GridDev& g, const ScanXyz& q, const float4* __restri
       __syncwarp();
     }
     n += nb;
-    if (!scan) live = false;
   }
   if (scan && lane == 0) L.cnt[s] = n <= kNbMax ? n : kNbMax + 1;
-  return ncand;
+  return COUNT ? group_sum<G>(ncand) : 0;
 }
 
 // The two neighbour sums of the passes, for one thread (G = 1) or a group of

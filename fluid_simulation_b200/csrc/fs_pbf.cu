@@ -20,6 +20,9 @@
 // the 401,856-particle dam break than the compiler's own choice (56
 // registers with spills) and than an 85-register budget.
 #define FS_NB_BOUNDS_PBF __launch_bounds__(kNbBlockMax, 1024 / kNbBlockMax)
+// The scanning kernels with several lanes per particle need 80 registers (PBF
+// frame at 19,997 particles with 64 and spills: 701 us, with 80: 630).
+#define FS_SCAN_BOUNDS_PBF __launch_bounds__(kNbBlockMax, G == 1 ? 4 : 3)
 
 namespace fs {
 
@@ -91,7 +94,7 @@ struct PbfGather {
 // vout[s] = ((x_pred - x_in) / max(dt, 1e-8), m / max(rho, 1e-6)), v_pred
 // for non-dynamic particles.
 template <int G>
-__global__ void FS_NB_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, int64_t n, const float4* __restrict__ xs,
+__global__ void FS_SCAN_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, int64_t n, const float4* __restrict__ xs,
                                            float4* __restrict__ vs, const float* __restrict__ mv,
                                            const float* __restrict__ ms, float h, float skin, float* rho,
                                            const float4* __restrict__ xin, float dt, float4* __restrict__ vout) {
@@ -247,7 +250,7 @@ struct LambdaArgs {
 // reproduces the scan's pair sequence exactly.  Particles failing (b), and
 // every particle when (a) fails, scan the grid.
 template <int G>
-__global__ void FS_NB_BOUNDS_PBF k_lambda(LambdaArgs a) {
+__global__ void FS_SCAN_BOUNDS_PBF k_lambda(LambdaArgs a) {
   extern __shared__ uint2 smem[];
   grid_begin();
   lists_recorded(a.L);

@@ -51,7 +51,7 @@ struct DensityArgs {
 // resident warps) a launch at 4,194,304 particles takes 1.44 ms, at 64 1.00,
 // at 48 1.07.  Before the word scan (scan_words) it took 1.63.
 template <int G>
-__global__ void __launch_bounds__(kNbBlockMax, 4) k_wcsph_density(DensityArgs a) {
+__global__ void __launch_bounds__(kNbBlockMax, G == 1 ? 4 : 3) k_wcsph_density(DensityArgs a) {
   extern __shared__ uint2 smem[];
   grid_begin();
   if (clock_idle(a.clock)) return;

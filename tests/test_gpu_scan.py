@@ -130,12 +130,14 @@ def test_particles_of_another_mass_far_away_change_no_bit(kind, n, cuda_device):
         assert torch.equal(t[:n], mixed[name][:n]), name
 
 
-@pytest.mark.parametrize("total", [4999, 5001, 14000, 14001, 36000, 36001])
+@pytest.mark.parametrize("total", [4999, 6000, 6001, 14000, 14001, 38000, 38001])
 @pytest.mark.parametrize("kind", ["wcsph", "dfsph", "pbf"])
-def test_lanes_per_particle_change_no_bit(kind, total, cuda_device):
+@pytest.mark.parametrize("corners", [((-0.55, -0.55, 0.02), (-0.2, -0.2, 0.02)),
+                                     ((-0.07, -0.07, 0.02), (0.15, 0.15, 0.02))])  # around x = y = 0: wide rows, wraps
+def test_lanes_per_particle_change_no_bit(kind, total, corners, cuda_device):
     n = 2500
-    x, v = block(n, (-0.55, -0.55, 0.02), 1)
-    x2, v2 = block(total - n, (-0.2, -0.2, 0.02), 2)
+    x, v = block(n, corners[0], 1)
+    x2, v2 = block(total - n, corners[1], 2)
 
     mass = 1000.0 * SP ** 3
     alone = run_step(kind, x, v, mass, cuda_device)
