@@ -132,58 +132,34 @@ struct AdjGather {
   }
 };
 
-// d (c d) / d(d) applied to ab:  rb = c ab + (ab . d) dc/dd, and the
-// velocity adjoint ub of the pair, for the term of a_i with neighbour j.
-struct PairAdj {
-  float3 rb, ub;
-  float pb_sum;  // coefficient of (P_i + P_j):  -m_j gs (ab . d)
-  float nub;     // d/d nu_i
-  float rb_j;    // d/d R_j
-};
-
-FS_DEV PairAdj pair_adjoint(const Cubic& K, float h, float particle_radius, float3 d, float r2, float3 u, float3 ab,
-                            float nu_i, float coh_i, float m_j, float R_j, float Psum) {
-  PairAdj o;
-  float r, rinv;
-  r_and_inv(r2, r, rinv);
-  const float q = r * K.inv_h;
-  // gs(r) and its derivative d gs / dr (Cubic.grad_scale)
-  float gs = 0.f, dgs = 0.f;
-  if (r > 1.0e-5f && q <= 1.f) {
-    if (q <= 0.5f) {
-      gs = K.g_in * fmaf(3.f, q, -2.f);
-      dgs = K.g_in * 3.f * K.inv_h;
-    } else {
-      const float t = 1.f - q;
-      gs = K.g_out * t * t * rinv;
-      dgs = K.g_out * (-2.f * t * K.inv_h * rinv - t * t * rinv * rinv);
+// What both sides of a pair share: gs(r) and its derivative (Cubic.grad_scale),
+// 1 / (r^2 + 0.01 h^2), the cohesion weight W(max(r, r_p)) and its derivative
+// in r (0 unless needed).
+struct PairGeometry {
+  float rinv, gs, dgs, den, w, dw;
+  FS_DEV PairGeometry(const Cubic& K, float h, float particle_radius, float r2, bool cohesion) {
+    float r;
+    r_and_inv(r2, r, rinv);
+    const float q = r * K.inv_h;
+    gs = dgs = w = dw = 0.f;
+    if (r > 1.0e-5f && q <= 1.f) {
+      if (q <= 0.5f) {
+        gs = K.g_in * fmaf(3.f, q, -2.f);
+        dgs = K.g_in * 3.f * K.inv_h;
+      } else {
+        const float t = 1.f - q;
+        gs = K.g_out * t * t * rinv;
+        dgs = K.g_out * (-2.f * t * K.inv_h * rinv - t * t * rinv * rinv);
+      }
+    }
+    den = 1.0f / (r2 + 0.01f * (h * h));
+    if (cohesion) {
+      const float s = fmaxf(r, particle_radius);
+      w = K.w(s);
+      if (r > particle_radius && s > 1.0e-5f) dw = K.grad_scale(s, 1.0f / s) * s;
     }
   }
-  const float eps = 0.01f * (h * h);
-  const float den = 1.0f / (r2 + eps);
-  const float ud = u.x * d.x + u.y * d.y + u.z * d.z;
-  const float kv = 10.f * nu_i * m_j * R_j;
-  const float visc = kv * ud * den;
-  const float A = visc - m_j * Psum;
-  // cohesion -coh_i m_j W(s) with s = max(r, r_p)
-  const float s = fmaxf(r, particle_radius);
-  const float wc = coh_i * m_j * K.w(s);
-  float dwc = 0.f;  // d wc / dr
-  if (coh_i != 0.f && r > particle_radius && s > 1.0e-5f) dwc = coh_i * m_j * K.grad_scale(s, 1.0f / s) * s;
-  const float c = A * gs - wc;
-  const float abd = ab.x * d.x + ab.y * d.y + ab.z * d.z;
-  // dc/dd = gs dA/dd + (A dgs - dwc) d / r
-  //   dA/dd = kv (u den - 2 ud d den^2)
-  const float radial = (A * dgs - dwc) * rinv - 2.f * kv * ud * den * den * gs;
-  const float tang = kv * den * gs;
-  o.rb = make_float3(c * ab.x + abd * (tang * u.x + radial * d.x), c * ab.y + abd * (tang * u.y + radial * d.y),
-                     c * ab.z + abd * (tang * u.z + radial * d.z));
-  o.ub = make_float3(abd * tang * d.x, abd * tang * d.y, abd * tang * d.z);
-  o.pb_sum = -m_j * gs * abd;
-  o.nub = abd * gs * 10.f * m_j * R_j * ud * den;
-  o.rb_j = abd * gs * 10.f * nu_i * m_j * ud * den;
-  return o;
-}
+};
 
 // G lanes per particle add up their own pairs' terms, then the lanes' sums
 // (the adjoint's sums have no order to keep).
@@ -192,6 +168,22 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
   extern __shared__ uint2 smem[];
   grid_begin();
   lists_recorded(a.L);
+  struct Neighbour {
+    float4 v, ab;
+    float2 PR;
+    float nu, coh;
+  };
+  auto fetch = [&](int t) {
+    return Neighbour{__ldg(a.vs + t), __ldg(a.ab + t), __ldg(a.sc2 + t), __ldg(a.nu + t), __ldg(a.coh + t)};
+  };
+  // with one thread per particle four neighbours are in flight: their records
+  // would not fit the registers, and load when their terms need them
+  auto load = [&](int t) {
+    if constexpr (G > 1)
+      return fetch(t);
+    else
+      return 0;
+  };
   for_groups<G>(a.n, [&](int64_t s, bool live, bool lead) {
     const float4 xk = a.xs[s];
     const int32_t i = a.g.perm[s];
@@ -212,33 +204,47 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
     const float h2m = a.h * a.h * kSupportMargin;
     float Pb = 0.f, Rb = 0.f, nub = 0.f;
     scan_sum<G, false, false, false, 0>(
-        a.g, a.q, a.xs, (int)s, xk, a.h, h2m, h2m, a.L, smem, on, -1, [](int) { return 0; },
-        [&](int t, float4 xj, int) {
+        a.g, a.q, a.xs, (int)s, xk, a.h, h2m, h2m, a.L, smem, on, -1, load,
+        [&](int t, float4 xj, const auto& p) {
           const float3 d = make_float3(xk.x - xj.x, xk.y - xj.y, xk.z - xj.z);
           const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
           if (r2 == 0.f) return Terms<0>{};  // the forward skips coincident pairs
-          const float4 vj = __ldg(a.vs + t);
-          const float2 PRj = __ldg(a.sc2 + t);
-          const float3 u = make_float3(vk.x - vj.x, vk.y - vj.y, vk.z - vj.z);
-          const float Psum = PRk.x + PRj.x;
-          if (pfk & PF_DYNAMIC) {  // term of a_k with neighbour j
-            const PairAdj o = pair_adjoint(K, a.h, a.particle_radius, d, r2, u, abk, nu_k, coh_k, vj.w, PRj.y, Psum);
-            xb = make_float3(xb.x + o.rb.x, xb.y + o.rb.y, xb.z + o.rb.z);
-            vb = make_float3(vb.x + o.ub.x, vb.y + o.ub.y, vb.z + o.ub.z);
-            Pb += o.pb_sum;
-            nub += o.nub;
-          }
-          if (pf_of(xj) & PF_DYNAMIC) {  // term of a_j with neighbour k: d_jk = -d, u_jk = -u
-            const float4 abj4 = __ldg(a.ab + t);
-            const float3 abj = make_float3(abj4.x, abj4.y, abj4.z);
-            const float3 dn = make_float3(-d.x, -d.y, -d.z), un = make_float3(-u.x, -u.y, -u.z);
-            const PairAdj o = pair_adjoint(K, a.h, a.particle_radius, dn, r2, un, abj, __ldg(a.nu + t),
-                                           __ldg(a.coh + t), m_k, PRk.y, Psum);
-            xb = make_float3(xb.x - o.rb.x, xb.y - o.rb.y, xb.z - o.rb.z);
-            vb = make_float3(vb.x - o.ub.x, vb.y - o.ub.y, vb.z - o.ub.z);
-            Pb += o.pb_sum;
-            Rb += o.rb_j;
-          }
+          Neighbour nb;
+          if constexpr (G > 1)
+            nb = p;
+          else
+            nb = fetch(t);
+          // The two terms of the pair, of a_k (weights ab_k) and of a_j (weights
+          // ab_j, d_jk = -d, u_jk = -u), share their geometry and directions:
+          //   c = A gs - coh m W with A = kv ud den - m Psum, kv = 10 nu m R
+          //   d(c d)/dd . ab = c ab + (ab . d) (tang u + radial d)
+          // (evaluated side by side, they took twice the operations; ab is 0
+          // for a particle that is not dynamic)
+          const float3 u = make_float3(vk.x - nb.v.x, vk.y - nb.v.y, vk.z - nb.v.z);
+          const float m_j = nb.v.w;
+          const PairGeometry P(K, a.h, a.particle_radius, r2, coh_k != 0.f || nb.coh != 0.f);
+          const float ud = fmaf(u.x, d.x, fmaf(u.y, d.y, u.z * d.z)), udd = ud * P.den;
+          const float abk_d = fmaf(abk.x, d.x, fmaf(abk.y, d.y, abk.z * d.z));
+          const float abj_d = fmaf(nb.ab.x, d.x, fmaf(nb.ab.y, d.y, nb.ab.z * d.z));
+          const float Psum = PRk.x + nb.PR.x;
+          const float visc_k = 10.f * m_j * nb.PR.y, visc_j = 10.f * m_k * PRk.y;  // kv / nu
+          const float kv_k = nu_k * visc_k, kv_j = nb.nu * visc_j;
+          const float A_k = fmaf(kv_k, udd, -m_j * Psum), A_j = fmaf(kv_j, udd, -m_k * Psum);
+          const float g_k = coh_k * m_j, g_j = nb.coh * m_k;
+          const float c_k = fmaf(A_k, P.gs, -g_k * P.w), c_j = fmaf(A_j, P.gs, -g_j * P.w);
+          const float curl = 2.f * udd * P.den * P.gs;
+          const float radial_k = fmaf(fmaf(A_k, P.dgs, -g_k * P.dw), P.rinv, -kv_k * curl);
+          const float radial_j = fmaf(fmaf(A_j, P.dgs, -g_j * P.dw), P.rinv, -kv_j * curl);
+          const float S = P.den * P.gs * fmaf(abk_d, kv_k, -abj_d * kv_j);
+          const float T = fmaf(abk_d, radial_k, -abj_d * radial_j);
+          xb.x += fmaf(c_k, abk.x, fmaf(-c_j, nb.ab.x, fmaf(S, u.x, T * d.x)));
+          xb.y += fmaf(c_k, abk.y, fmaf(-c_j, nb.ab.y, fmaf(S, u.y, T * d.y)));
+          xb.z += fmaf(c_k, abk.z, fmaf(-c_j, nb.ab.z, fmaf(S, u.z, T * d.z)));
+          vb = make_float3(fmaf(S, d.x, vb.x), fmaf(S, d.y, vb.y), fmaf(S, d.z, vb.z));
+          Pb = fmaf(P.gs, fmaf(m_k, abj_d, -m_j * abk_d), Pb);
+          const float gu = P.gs * udd;
+          nub = fmaf(abk_d * visc_k, gu, nub);
+          Rb = fmaf(-abj_d * (10.f * nb.nu * m_k), gu, Rb);
           return Terms<0>{};
         },
         [](const Terms<0>&) {});
