@@ -85,6 +85,8 @@ struct fs_context {
   float built_inv = 0.f;
   cudaStream_t last_stream = nullptr;
 
+  char* arena = nullptr;  // the one allocation that holds the arrays below (worlds' tables apart)
+
   // grid build
   int32_t* key = nullptr;        // [cap] cell key of original particle i
   int32_t* slot = nullptr;       // [cap] arrival slot inside the cell
