@@ -319,17 +319,22 @@ __device__ void block_reduce_store(double v, long long c, double* part, int64_t*
   }
 }
 
-// last-block-done: returns true in exactly one block, after every block's partial is visible
+// last-block-done: returns true in exactly one block, after every block's
+// partial is visible (thread 0 has stored it and fences; what the other
+// threads wrote need not be visible before the end of the kernel)
 __device__ bool last_block(uint32_t* ticket) {
   __shared__ bool am_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) am_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    am_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
   __syncthreads();
   if (am_last) __threadfence();
   return am_last;
 }
 
+// 64 registers: with 80, 73 us a launch at 401,856 particles, with 48 79,
+// against 65.
 template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, 4) k_rate(RateArgs a) {
   grid_begin();
@@ -481,10 +486,11 @@ struct CorrectArgs {
   int nworlds;
 };
 
-// Four resident 256-thread blocks per SM: a 64-register budget (the compiler
-// otherwise settles at 48 registers and spills; 3.7 % faster measured).
+// A pair gathers one 16-byte record, so that 40 registers and 48 resident warps
+// hold more of them in flight than 56 and 36: 47.6 -> 44.5 us a launch at
+// 401,856 particles (32 registers: 66).  Several lanes per particle want 64.
 template <int G>
-__global__ void __launch_bounds__(kNbBlockMax, 4) k_correct(CorrectArgs a) {
+__global__ void __launch_bounds__(kNbBlockMax, G == 1 ? 6 : 4) k_correct(CorrectArgs a) {
   grid_begin();
   if (a.ctrl && a.ctrl->done) return;
   if (clock_idle(a.clock)) return;

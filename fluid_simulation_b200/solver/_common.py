@@ -13,6 +13,11 @@ from ..newton_shim import HashGrid, ModelBuilder, Model, vec3
 
 def ptr(t, name, dtype=torch.float32, cols=None, n=None, device=None, optional=False):
     """Device pointer of a contiguous tensor after checking dtype/shape/device."""
+    # a step makes some twenty-five of these checks: the usual, valid argument first
+    if (type(t) is torch.Tensor and t.dtype is dtype and t.is_contiguous()
+            and (device is None or t.device == device)
+            and (n is None or t.shape == ((n, cols) if cols else (n,)))):
+        return t.data_ptr()
     if t is None:
         if optional:
             return None
