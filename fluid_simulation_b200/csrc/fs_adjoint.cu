@@ -203,7 +203,7 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
     const Cubic K(a.h);
     const float h2m = a.h * a.h * kSupportMargin;
     float Pb = 0.f, Rb = 0.f, nub = 0.f;
-    scan_sum<G, false, false, false, 0>(
+    scan_sum<G, false, false, false, true, 0>(
         a.g, a.q, a.xs, (int)s, xk, a.h, h2m, h2m, a.L, smem, on, -1, load,
         [&](int t, float4 xj, const auto& p) {
           const float3 d = make_float3(xk.x - xj.x, xk.y - xj.y, xk.z - xj.z);

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kNbBlockMax, 3) k_density_factor(DensFactorArg
     const Cubic K(a.h);
     float rho = 0.f, sgx = 0.f, sgy = 0.f, sgz = 0.f, sq = 0.f;
     // the candidate count (no distance test, solver_dfsph.py:163-164) comes from the scan
-    const int cnt = scan_sum<G, true, true, false, 5>(
+    const int cnt = scan_sum<G, true, true, false, false, 5>(
         a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, -1,
         [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(a.ms + t)); },
         [&](int t, float4 xj, const float2& mm) {  // (rest_density * volume, mass)

@@ -362,7 +362,14 @@ FS_DEV int scan_words(const ScanXyz& q, float4 xi, float h2, uint2* words, int n
 // pairs are still all visited here.  REUSE: a particle with reuse >= 0 visits
 // the `reuse` entries its list already holds instead of scanning (in the same
 // loop: lanes that scan and lanes that reuse share the warp's pair math).
-template <bool WITH_SELF, bool COUNT = false, bool REUSE = false, class Load, class Pair>
+// KEEP_SELF = false leaves the particle itself out of its list, for the passes
+// that sum over the others: one entry in 30 less to gather.  The DFSPH
+// iterations read a list 34 times a substep (rate 64.8 -> 63.2 us, correct
+// 43.6 -> 42.6 at 401,856 particles), a PBF lambda's is read once (delta 44.0
+// -> 42.5).  The WCSPH density keeps it: what recording costs there (999 ->
+// 1015 us at 4M) the force pass only just gives back (708 -> 695).  The bound
+// on a list counts the particle either way.
+template <bool WITH_SELF, bool COUNT, bool REUSE, bool KEEP_SELF, class Load, class Pair>
 FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
                       float h2rec, float h2m, const NbrList& L, uint2* smem, Load&& load, Pair&& pair,
                       int reuse = -1) {
@@ -414,7 +421,26 @@ FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restri
       }
       const float4 x0 = __ldg(xs + t0), x1 = __ldg(xs + t1), x2 = __ldg(xs + t2), x3 = __ldg(xs + t3);
       const auto p0 = load(t0), p1 = load(t1), p2 = load(t2), p3 = load(t3);
-      if (!scan) {
+      if (!KEEP_SELF && scan) {
+        const bool r0 = t0 != s, r1 = t1 != s, r2 = t2 != s, r3 = t3 != s;  // a slot that was not popped is s
+        int32_t* o = col + (int64_t)n * L.stride;
+        if (n + 4 <= kNbMax) {
+          *o = t0;
+          if (r0) o += L.stride;
+          if (r1) *o = t1, o += L.stride;
+          if (r2) *o = t2, o += L.stride;
+          if (r3) *o = t3;
+          n += (int)r0 + (int)r1 + (int)r2 + (int)r3;
+        } else {
+          const int tt[4] = {t0, t1, t2, t3};
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (tt[k] != s) {
+              if (n < kNbMax) col[(int64_t)n * L.stride] = tt[k];
+              ++n;
+            }
+        }
+      } else if (!scan) {
       } else if (n + 4 <= kNbMax) {
         int32_t* const o = col + (int64_t)n * L.stride;
         o[0] = t0;
@@ -428,14 +454,14 @@ FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restri
         for (int k = 0; k < 4; ++k)
           if (kk[k] && n + k < kNbMax) col[(int64_t)(n + k) * L.stride] = tt[k];
       }
-      n += (int)k0 + (int)k1 + (int)k2 + (int)k3;
+      if (KEEP_SELF || !scan) n += (int)k0 + (int)k1 + (int)k2 + (int)k3;
       one(t0, x0, p0);
       if (k1) one(t1, x1, p1);
       if (k2) one(t2, x2, p2);
       if (k3) one(t3, x3, p3);
     }
   }
-  if (scan) L.cnt[s] = n <= kNbMax ? n : kNbMax + 1;
+  if (scan) L.cnt[s] = n + !KEEP_SELF <= kNbMax ? n : kNbMax + 1;
   return ncand;
 }
 
@@ -475,9 +501,16 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, const float4*
       one(t2, x2);
       one(t3, x3);
     }
-    for (; k < n; ++k) {
-      const int t0 = entry(k);
-      one(t0, __ldg(rec + t0));
+    // the last one to three together: one after the other each waited a latency
+    // (DFSPH rate 66.1 -> 64.8 us, PBF delta 45.8 -> 44.0 at 401,856 particles,
+    // WCSPH force 719 -> 708 at 4M)
+    if (k < n) {
+      const bool k1 = k + 1 < n, k2 = k + 2 < n;
+      const int t0 = entry(k), t1 = k1 ? entry(k + 1) : s, t2 = k2 ? entry(k + 2) : s;
+      const float4 x0 = __ldg(rec + t0), x1 = __ldg(rec + t1), x2 = __ldg(rec + t2);
+      one(t0, x0);
+      if (k1) one(t1, x1);
+      if (k2) one(t2, x2);
     }
   } else {
     scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { pair(t, __ldg(rec + t)); });
@@ -521,10 +554,14 @@ FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, const fl
       one(t2, x2, p2);
       one(t3, x3, p3);
     }
-    for (; k < n; ++k) {
-      const int t0 = entry(k);
-      const float4 x0 = __ldg(rec + t0);
-      one(t0, x0, load(t0));
+    if (k < n) {
+      const bool k1 = k + 1 < n, k2 = k + 2 < n;
+      const int t0 = entry(k), t1 = k1 ? entry(k + 1) : s, t2 = k2 ? entry(k + 2) : s;
+      const float4 x0 = __ldg(rec + t0), x1 = __ldg(rec + t1), x2 = __ldg(rec + t2);
+      const auto p0 = load(t0), p1 = load(t1), p2 = load(t2);
+      one(t0, x0, p0);
+      if (k1) one(t1, x1, p1);
+      if (k2) one(t2, x2, p2);
     }
   } else {
     scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { pair(t, __ldg(rec + t), load(t)); });
@@ -766,13 +803,13 @@ FS_DEV int group_scan(const GridDev& g, const ScanXyz& q, const float4* __restri
 //             or rescans where there is none; LAZY: load(t) only after the
 //             distance test (G = 1), where the early load costs registers
 // A particle with on = false takes no part.
-template <int G, bool WITH_SELF, bool COUNT, bool REUSE, int K, class Load, class Term, class Acc>
+template <int G, bool WITH_SELF, bool COUNT, bool REUSE, bool KEEP_SELF, int K, class Load, class Term, class Acc>
 FS_DEV int scan_sum(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
                     float h2rec, float h2m, const NbrList& L, void* smem, bool on, int reuse, Load&& load, Term&& term,
                     Acc&& acc) {
   if constexpr (G == 1) {
     if (!on) return 0;
-    return scan_visit<WITH_SELF, COUNT, REUSE>(
+    return scan_visit<WITH_SELF, COUNT, REUSE, KEEP_SELF>(
         g, q, xs, s, xi, h, h2rec, h2m, L, (uint2*)smem, load,
         [&](int t, float4 xj, const auto& p) { acc(term(t, xj, p)); }, reuse);
   } else {

@@ -109,7 +109,7 @@ __global__ void FS_SCAN_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, in
     const Poly6Spiky K(h);
     const bool on = live && (pf_of(xi) & PF_ACTIVE);
     const float hr = h * (1.0f + skin);
-    scan_sum<G, true, false, false, 2>(
+    scan_sum<G, true, false, false, true, 2>(
         g, q, xs, (int)s, xi, h, hr * hr * kSupportMargin, h2m, L, smem, on, -1, [&](int t) { return __ldg(mv + t); },
         [&](int t, float4 xj, const float& m) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -274,7 +274,7 @@ __global__ void FS_SCAN_BOUNDS_PBF k_lambda(LambdaArgs a) {
       const unsigned b = __ballot_sync(full, reuse && lead);
       if ((int)(threadIdx.x & 31) == __ffs(full) - 1) atomicAdd(a.g.tile_stats + 2, (unsigned long long)__popc(b));
     }
-    scan_sum<G, true, false, true, 5>(
+    scan_sum<G, true, false, true, false, 5>(
         a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, reuse ? listed : -1,
         mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;

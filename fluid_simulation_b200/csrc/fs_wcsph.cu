@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kNbBlockMax, G == 1 ? 4 : 3) k_wcsph_density(D
     const float h2m = a.h * a.h * kSupportMargin;
     const Cubic K(a.h);
     float acc = 0.f;
-    scan_sum<G, true, false, false, 2>(
+    scan_sum<G, true, false, false, true, 2>(
         a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, -1, [&](int t) { return __ldg(a.mv + t); },
         [&](int t, float4 xj, const float& m) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;

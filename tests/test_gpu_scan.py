@@ -144,3 +144,21 @@ def test_lanes_per_particle_change_no_bit(kind, total, corners, cuda_device):
     both = run_step(kind, np.concatenate([x, x2]), np.concatenate([v, v2]), mass, cuda_device)
     for name, t in alone.items():
         assert torch.equal(t, both[name][:n]), name
+
+
+@pytest.mark.parametrize("m", [2, 4, 5, 188, 189, 190, 191, 192, 193, 194, 197])
+@pytest.mark.parametrize("kind", ["wcsph", "dfsph", "pbf"])
+def test_full_lists_of_one_lane_change_no_bit(kind, m, cuda_device):
+    """m particles that all see each other, around the 192 entries a list holds (the particle itself counts), alone
+    with 16 lanes each and with so many others that each has one."""
+    rng = np.random.default_rng(m)
+    d = rng.normal(size=(m, 3))
+    r = 0.45 * H * rng.uniform(0.0, 1.0, (m, 1)) ** (1.0 / 3.0)
+    x = (d / np.linalg.norm(d, axis=1, keepdims=True) * r + (-0.45, -0.45, 0.2)).astype(np.float32)
+    v = rng.normal(0.0, 0.1, x.shape).astype(np.float32)
+    x2, v2 = block(38100, (-0.07, -0.07, 0.02), 2)
+    mass = 1000.0 * SP ** 3
+    alone = run_step(kind, x, v, mass, cuda_device)
+    both = run_step(kind, np.concatenate([x, x2]), np.concatenate([v, v2]), mass, cuda_device)
+    for name, t in alone.items():
+        assert torch.equal(t.view(torch.int32), both[name][:m].view(torch.int32)), name
