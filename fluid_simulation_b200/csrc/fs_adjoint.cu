@@ -203,7 +203,7 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
     const Cubic K(a.h);
     const float h2m = a.h * a.h * kSupportMargin;
     float Pb = 0.f, Rb = 0.f, nub = 0.f;
-    scan_sum<G, false, false, false, true, 0>(
+    scan_sum<G, false, false, false, kExact, 0>(
         a.g, a.q, a.xs, (int)s, xk, a.h, h2m, h2m, a.L, smem, on, -1, load,
         [&](int t, float4 xj, const auto& p) {
           const float3 d = make_float3(xk.x - xj.x, xk.y - xj.y, xk.z - xj.z);
@@ -299,7 +299,7 @@ __global__ void FS_NB_BOUNDS k_adj_density(AdjArgs a) {
     const float mv_k = a.mv[s];
     const Cubic K(a.h);
     float3 xb = lead ? make_float3(xr.x, xr.y, xr.z) : make_float3(0.f, 0.f, 0.f);
-    list_sum<G, false, false, true, 0>(
+    list_sum<G, false, false, true, true, 0>(
         a.g, a.xs, a.xs, (int)s, xk, a.h, a.h * a.h * kSupportMargin, a.L, lists_usable(a.L), on,
         [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.xr[t].w)); },
         [&](int t, float4 xj, const float2& j) {

@@ -362,14 +362,24 @@ FS_DEV int scan_words(const ScanXyz& q, float4 xi, float h2, uint2* words, int n
 // pairs are still all visited here.  REUSE: a particle with reuse >= 0 visits
 // the `reuse` entries its list already holds instead of scanning (in the same
 // loop: lanes that scan and lanes that reuse share the warp's pair math).
-// KEEP_SELF = false leaves the particle itself out of its list, for the passes
-// that sum over the others: one entry in 30 less to gather.  The DFSPH
-// iterations read a list 34 times a substep (rate 64.8 -> 63.2 us, correct
-// 43.6 -> 42.6 at 401,856 particles), a PBF lambda's is read once (delta 44.0
-// -> 42.5).  The WCSPH density keeps it: what recording costs there (999 ->
-// 1015 us at 4M) the force pass only just gives back (708 -> 695).  The bound
-// on a list counts the particle either way.
-template <bool WITH_SELF, bool COUNT, bool REUSE, bool KEEP_SELF, class Load, class Pair>
+// LIST: what the list holds beside the pairs within h2rec.  kAll: the particle
+// itself too, and the few candidates that the scan takes past the radius;
+// kOthers: not itself; kExact: neither, only what passes the test at h2m, so
+// that its readers gather nothing in vain and test nothing again.  Which is
+// best depends on the readers, since the stores of kExact wait for the
+// positions (at 401,856 particles and, WCSPH, 4M):
+//                       kAll              kOthers           kExact
+//   DFSPH density       118.2 us          117.8             118.2
+//     17 rate, correct  64.8, 43.6        63.2, 42.6        60.4, 41.5
+//   WCSPH density       999 us            1015              1024
+//     force             708               695               669
+//   PBF lambda          109.9 us          109.1             113.5
+//     delta             44.0              42.4              39.4
+// The PBF density's list is visited again with the particle itself: kAll.
+// The bound on a list counts the particle in any case.
+enum ListOf { kAll, kOthers, kExact };
+
+template <bool WITH_SELF, bool COUNT, bool REUSE, ListOf LIST, class Load, class Pair>
 FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
                       float h2rec, float h2m, const NbrList& L, uint2* smem, Load&& load, Pair&& pair,
                       int reuse = -1) {
@@ -380,10 +390,14 @@ FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restri
   bool live = true;
   int n = 0, ncand = 0;
   int32_t* const col = L.idx + s;
-  auto one = [&](int t, float4 xj, const auto& p) {
+  auto within = [&](float4 xj) {
     const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    if (fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, xj.w))) <= h2m && (WITH_SELF || t != s)) pair(t, xj, p);
+    return fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, xj.w))) <= h2m;
   };
+  auto one = [&](int t, float4 xj, const auto& p) {
+    if (within(xj) && (WITH_SELF || t != s)) pair(t, xj, p);
+  };
+  static_assert(!REUSE || LIST != kExact, "a list that is visited again holds more");
   const bool scan = !REUSE || reuse < 0;
   while (live) {
     int nw = 0;
@@ -421,47 +435,71 @@ FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restri
       }
       const float4 x0 = __ldg(xs + t0), x1 = __ldg(xs + t1), x2 = __ldg(xs + t2), x3 = __ldg(xs + t3);
       const auto p0 = load(t0), p1 = load(t1), p2 = load(t2), p3 = load(t3);
-      if (!KEEP_SELF && scan) {
-        const bool r0 = t0 != s, r1 = t1 != s, r2 = t2 != s, r3 = t3 != s;  // a slot that was not popped is s
+      if constexpr (LIST == kExact) {
+        k0 = within(x0), k1 = k1 && within(x1), k2 = k2 && within(x2), k3 = k3 && within(x3);
+        const int tt[4] = {t0, t1, t2, t3};
+        const bool rr[4] = {k0 && t0 != s, k1 && t1 != s, k2 && t2 != s, k3 && t3 != s};
         int32_t* o = col + (int64_t)n * L.stride;
         if (n + 4 <= kNbMax) {
-          *o = t0;
-          if (r0) o += L.stride;
-          if (r1) *o = t1, o += L.stride;
-          if (r2) *o = t2, o += L.stride;
-          if (r3) *o = t3;
-          n += (int)r0 + (int)r1 + (int)r2 + (int)r3;
-        } else {
-          const int tt[4] = {t0, t1, t2, t3};
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (tt[k] != s) {
-              if (n < kNbMax) col[(int64_t)n * L.stride] = tt[k];
+          for (int e = 0; e < 4; ++e)
+            if (rr[e]) *o = tt[e], o += L.stride;
+          n += (int)rr[0] + (int)rr[1] + (int)rr[2] + (int)rr[3];
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (rr[e]) {
+              if (n < kNbMax) col[(int64_t)n * L.stride] = tt[e];
               ++n;
             }
         }
-      } else if (!scan) {
-      } else if (n + 4 <= kNbMax) {
-        int32_t* const o = col + (int64_t)n * L.stride;
-        o[0] = t0;
-        if (k1) o[L.stride] = t1;
-        if (k2) o[2 * L.stride] = t2;
-        if (k3) o[3 * L.stride] = t3;
+        if (k0 && (WITH_SELF || t0 != s)) pair(t0, x0, p0);
+        if (k1 && (WITH_SELF || t1 != s)) pair(t1, x1, p1);
+        if (k2 && (WITH_SELF || t2 != s)) pair(t2, x2, p2);
+        if (k3 && (WITH_SELF || t3 != s)) pair(t3, x3, p3);
       } else {
-        const int tt[4] = {t0, t1, t2, t3};
-        const bool kk[4] = {k0, k1, k2, k3};
+        if (LIST == kOthers && scan) {
+          const bool r0 = t0 != s, r1 = t1 != s, r2 = t2 != s, r3 = t3 != s;  // a slot that was not popped is s
+          int32_t* o = col + (int64_t)n * L.stride;
+          if (n + 4 <= kNbMax) {
+            *o = t0;
+            if (r0) o += L.stride;
+            if (r1) *o = t1, o += L.stride;
+            if (r2) *o = t2, o += L.stride;
+            if (r3) *o = t3;
+            n += (int)r0 + (int)r1 + (int)r2 + (int)r3;
+          } else {
+            const int tt[4] = {t0, t1, t2, t3};
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (kk[k] && n + k < kNbMax) col[(int64_t)(n + k) * L.stride] = tt[k];
+            for (int e = 0; e < 4; ++e)
+              if (tt[e] != s) {
+                if (n < kNbMax) col[(int64_t)n * L.stride] = tt[e];
+                ++n;
+              }
+          }
+        } else if (!scan) {
+        } else if (n + 4 <= kNbMax) {
+          int32_t* const o = col + (int64_t)n * L.stride;
+          o[0] = t0;
+          if (k1) o[L.stride] = t1;
+          if (k2) o[2 * L.stride] = t2;
+          if (k3) o[3 * L.stride] = t3;
+        } else {
+          const int tt[4] = {t0, t1, t2, t3};
+          const bool kk[4] = {k0, k1, k2, k3};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (kk[e] && n + e < kNbMax) col[(int64_t)(n + e) * L.stride] = tt[e];
+        }
+        if (LIST == kAll || !scan) n += (int)k0 + (int)k1 + (int)k2 + (int)k3;
+        one(t0, x0, p0);
+        if (k1) one(t1, x1, p1);
+        if (k2) one(t2, x2, p2);
+        if (k3) one(t3, x3, p3);
       }
-      if (KEEP_SELF || !scan) n += (int)k0 + (int)k1 + (int)k2 + (int)k3;
-      one(t0, x0, p0);
-      if (k1) one(t1, x1, p1);
-      if (k2) one(t2, x2, p2);
-      if (k3) one(t3, x3, p3);
     }
   }
-  if (scan) L.cnt[s] = n + !KEEP_SELF <= kNbMax ? n : kNbMax + 1;
+  if (scan) L.cnt[s] = n + (LIST != kAll) <= kNbMax ? n : kNbMax + 1;
   return ncand;
 }
 
@@ -476,11 +514,22 @@ FS_DEV void scan_grid(const GridDev& g, const float4* __restrict__ xs, int s, fl
   });
 }
 
+// One entry of a list, past L1, which the neighbours' data fill (the lists
+// stay in L2): DFSPH rate 63.1 -> 62.2 us, correct 42.7 -> 42.1 at 401,856
+// particles.
+FS_DEV int32_t ld_list(const int32_t* p) {
+  int32_t v;
+  asm("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
 // Visits the neighbours of slot s within h2m through its recorded list when
 // lists_ok and the list did not overflow, else by rescanning the grid.
 // rec: the record gathered with each neighbour, its position and one value
-// (xs itself, or a pass's own); pair(t, rec[t]).
-template <bool WITH_SELF, class Pair>
+// (xs itself, or a pass's own); pair(t, rec[t]).  EXACT: a kExact list, whose
+// entries need no test (with one: rate 62.2 instead of 60.4 us, WCSPH force
+// 695 instead of 669).
+template <bool WITH_SELF, bool EXACT, class Pair>
 FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s, float4 xi,
                   float h, float h2m, const NbrList& L, bool lists_ok, Pair&& pair) {
   const int n = lists_ok ? __ldg(L.cnt + s) : kNbMax + 1;
@@ -490,7 +539,7 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, const float4*
     auto entry = [&](int k) { return __ldg(col + (int64_t)k * L.stride); };
     auto one = [&](int t, float4 xj) {
       const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-      if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= h2m && (WITH_SELF || t != s)) pair(t, xj);
+      if (EXACT || (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= h2m && (WITH_SELF || t != s))) pair(t, xj);
     };
     int k = 0;
     for (; k + 3 < n; k += 4) {  // four independent gathers in flight
@@ -530,19 +579,19 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, const float4*
 // lists at most one later pass reads again (delta, non-pressure, XSPH:
 // 1.304 -> 1.287 ms per substep at 401,856 particles); the DFSPH iteration
 // passes, which read the same lists 34 times a substep, were slower with it.
-template <bool WITH_SELF, bool EVICT_FIRST = false, class Load, class Pair>
+template <bool WITH_SELF, bool EVICT_FIRST, bool EXACT, class Load, class Pair>
 FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s,
                        float4 xi, float h, float h2m, const NbrList& L, bool lists_ok, Load&& load, Pair&& pair) {
   const int n = lists_ok ? __ldg(L.cnt + s) : kNbMax + 1;
   const bool use = n <= kNbMax;
   auto one = [&](int t, float4 xj, const auto& p) {
     const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-    if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= h2m && (WITH_SELF || t != s)) pair(t, xj, p);
+    if (EXACT || (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= h2m && (WITH_SELF || t != s))) pair(t, xj, p);
   };
   if (use) {
     const int32_t* col = L.idx + s;
     auto entry = [&](int k) {
-      return EVICT_FIRST ? __ldcs(col + (int64_t)k * L.stride) : __ldg(col + (int64_t)k * L.stride);
+      return EVICT_FIRST ? __ldcs(col + (int64_t)k * L.stride) : ld_list(col + (int64_t)k * L.stride);
     };
     int k = 0;
     for (; k + 3 < n; k += 4) {
@@ -803,13 +852,13 @@ FS_DEV int group_scan(const GridDev& g, const ScanXyz& q, const float4* __restri
 //             or rescans where there is none; LAZY: load(t) only after the
 //             distance test (G = 1), where the early load costs registers
 // A particle with on = false takes no part.
-template <int G, bool WITH_SELF, bool COUNT, bool REUSE, bool KEEP_SELF, int K, class Load, class Term, class Acc>
+template <int G, bool WITH_SELF, bool COUNT, bool REUSE, ListOf LIST, int K, class Load, class Term, class Acc>
 FS_DEV int scan_sum(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
                     float h2rec, float h2m, const NbrList& L, void* smem, bool on, int reuse, Load&& load, Term&& term,
                     Acc&& acc) {
   if constexpr (G == 1) {
     if (!on) return 0;
-    return scan_visit<WITH_SELF, COUNT, REUSE, KEEP_SELF>(
+    return scan_visit<WITH_SELF, COUNT, REUSE, LIST>(
         g, q, xs, s, xi, h, h2rec, h2m, L, (uint2*)smem, load,
         [&](int t, float4 xj, const auto& p) { acc(term(t, xj, p)); }, reuse);
   } else {
@@ -818,16 +867,16 @@ FS_DEV int scan_sum(const GridDev& g, const ScanXyz& q, const float4* __restrict
   }
 }
 
-template <int G, bool WITH_SELF, bool EVICT_FIRST, bool LAZY, int K, class Load, class Term, class Acc>
+template <int G, bool WITH_SELF, bool EVICT_FIRST, bool LAZY, bool EXACT, int K, class Load, class Term, class Acc>
 FS_DEV void list_sum(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s, float4 xi,
                      float h, float h2m, const NbrList& L, bool lists_ok, bool on, Load&& load, Term&& term,
                      Acc&& acc) {
   if constexpr (G == 1) {
     if (!on) return;
     if constexpr (LAZY)
-      visit<WITH_SELF>(g, xs, rec, s, xi, h, h2m, L, lists_ok, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
+      visit<WITH_SELF, EXACT>(g, xs, rec, s, xi, h, h2m, L, lists_ok, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
     else
-      visit_with<WITH_SELF, EVICT_FIRST>(g, xs, rec, s, xi, h, h2m, L, lists_ok, load,
+      visit_with<WITH_SELF, EVICT_FIRST, EXACT>(g, xs, rec, s, xi, h, h2m, L, lists_ok, load,
                                          [&](int t, float4 xj, const auto& p) { acc(term(t, xj, p)); });
   } else {
     const int n = !on ? 0 : (lists_ok ? __ldg(L.cnt + s) : kNbMax + 1);

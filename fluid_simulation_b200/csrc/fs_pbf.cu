@@ -109,7 +109,7 @@ __global__ void FS_SCAN_BOUNDS_PBF k_density(GridDev g, NbrList L, ScanXyz q, in
     const Poly6Spiky K(h);
     const bool on = live && (pf_of(xi) & PF_ACTIVE);
     const float hr = h * (1.0f + skin);
-    scan_sum<G, true, false, false, true, 2>(
+    scan_sum<G, true, false, false, kAll, 2>(
         g, q, xs, (int)s, xi, h, hr * hr * kSupportMargin, h2m, L, smem, on, -1, [&](int t) { return __ldg(mv + t); },
         [&](int t, float4 xj, const float& m) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -176,7 +176,7 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
     const Poly6Spiky K(a.h);
     float ax = 0.f, ay = 0.f, az = 0.f;
     const bool on = live && dyn && (gamma != 0.f || mu != 0.f);
-    list_sum<G, false, true, false, 4>(
+    list_sum<G, false, true, false, false, 4>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), on,
         [&](int t) { return Neighbour{__ldg(a.vs + t), mass(t)}; },
         [&](int t, float4 xj, const Neighbour& j) {
@@ -274,7 +274,7 @@ __global__ void FS_SCAN_BOUNDS_PBF k_lambda(LambdaArgs a) {
       const unsigned b = __ballot_sync(full, reuse && lead);
       if ((int)(threadIdx.x & 31) == __ffs(full) - 1) atomicAdd(a.g.tile_stats + 2, (unsigned long long)__popc(b));
     }
-    scan_sum<G, true, false, true, false, 5>(
+    scan_sum<G, true, false, true, kOthers, 5>(
         a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, reuse ? listed : -1,
         mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -358,7 +358,7 @@ __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
     const bool scorr = a.scorr_k != 0.f && !(a.w_dq <= 1.0e-6f);
     const float inv_wdq = scorr ? 1.0f / a.w_dq : 0.f;
     float dx_ = 0.f, dy_ = 0.f, dz_ = 0.f;
-    list_sum<G, false, true, false, 4>(
+    list_sum<G, false, true, false, false, 4>(
         a.g, a.xs, a.rec, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn, mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -430,7 +430,7 @@ __global__ void FS_NB_BOUNDS_PBF k_xsph_final(XsphArgs a) {
     const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const Poly6Spiky K(a.h);
     float cx = 0.f, cy = 0.f, cz = 0.f;
-    list_sum<G, false, true, false, 4>(
+    list_sum<G, false, true, false, false, 4>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn && a.c > 0.f, [&](int t) { return __ldg(a.vel + t); },
         [&](int t, float4 xj, const float4& vj) {

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kNbBlockMax, G == 1 ? 4 : 3) k_wcsph_density(D
     const float h2m = a.h * a.h * kSupportMargin;
     const Cubic K(a.h);
     float acc = 0.f;
-    scan_sum<G, true, false, false, true, 2>(
+    scan_sum<G, true, false, false, kExact, 2>(
         a.g, a.q, a.xs, (int)s, xi, a.h, h2m, h2m, a.L, smem, on, -1, [&](int t) { return __ldg(a.mv + t); },
         [&](int t, float4 xj, const float& m) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -128,7 +128,7 @@ __global__ void FS_NB_BOUNDS k_wcsph_force(ForceArgs a) {
       float4 v;
       float2 r;  // (p_j / rho_j^2, 1 / rho_j)
     };
-    list_sum<G, false, false, true, 4>(
+    list_sum<G, false, false, true, true, 4>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn, [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(a.sc2 + t)}; },
         [&](int t, float4 xj, const Neighbour& j) {
