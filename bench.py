@@ -55,38 +55,41 @@ sys.path.insert(0, ROOT)
 # vec3 = 12 B).  Per substep: PBF 728 B, WCSPH 180 B, DFSPH 328 B + 116 B per
 # density iteration + 108 B per divergence iteration.  PBF's final density
 # pass also does the velocity update (44 B), so its two density launches
-# average 28 + 44 / 2 B.
+# average 28 + 44 / 2 B; its predict (60 B) and DFSPH's integrate (36 B, in
+# one of two builds) run in the grid build's first kernel (B_ALG_IN_BUILD).
 B_ALG = {
     "grid_build": 48, "pbf_predict": 60, "pbf_density": 50, "pbf_accel": 72, "pbf_lambda": 40, "pbf_delta": 56,
     "pbf_velocity": 44, "pbf_xsph": 64, "wcsph_density": 40, "wcsph_force": 92, "dfsph_density_factor": 36,
     "dfsph_accel": 76, "dfsph_rate": 60, "dfsph_correct": 56, "dfsph_integrate": 36, "dfsph_final": 48,
 }
+B_ALG_IN_BUILD = {"pbf": 60, "dfsph": 18}
 PUBLISHED_PBF = 401856 * 4 / 0.06464700849610381   # particle-substeps/s, RTX 4090 (performance_summary.json)
 # DRAM bytes (read + write) per particle per launch, cold cache, from the
-# ncu captures summarised under profiles/: PBF lambda, the mean of one
-# substep's four launches at 401,856 particles (the first reuses the density
-# pass's lists and reads them back, 79.64 MB; the three scanning ones 38.2
-# MB each); WCSPH at 524,288 particles.
-TRAFFIC_PER_PARTICLE = {"pbf_lambda": 48.91e6 / 401856, "dfsph_rate": 68.17e6 / 401856,
-                        "dfsph_density_factor": 36.86e6 / 401856, "wcsph_density": 62.30e6 / 524288,
-                        "wcsph_force": 94.48e6 / 524288}
+# ncu captures summarised in profiles/launches_current.md: PBF lambda, the
+# mean of one substep's four launches at 401,856 particles (the first reuses
+# the density pass's lists and reads them back, 82.4 MB; the three scanning
+# ones 25.5 MB each); DFSPH rate, the mean of four; WCSPH at 524,288 particles.
+TRAFFIC_PER_PARTICLE = {"pbf_lambda": 39.75e6 / 401856, "dfsph_rate": 79.26e6 / 401856,
+                        "dfsph_density_factor": 27.57e6 / 401856, "wcsph_density": 54.41e6 / 524288,
+                        "wcsph_force": 107.57e6 / 524288}
 TRAFFIC_SOURCE = {
-    "pbf_lambda": "ncu, mean of one substep's 4 launches at 401,856 particles (profiles/pbf_dam_401856.md)",
-    "dfsph_rate": "ncu, one launch at 401,856 particles (profiles/dfsph_dam_401856.md)",
-    "dfsph_density_factor": "ncu, one launch at 401,856 particles (profiles/dfsph_dam_401856.md)",
-    "wcsph_density": "ncu at 524,288 particles (profiles/wcsph_bcc_524k.md), scaled by the particle count",
-    "wcsph_force": "ncu at 524,288 particles (profiles/wcsph_bcc_524k.md), scaled by the particle count",
+    "pbf_lambda": "ncu, mean of one substep's 4 launches at 401,856 particles (profiles/launches_current.md)",
+    "dfsph_rate": "ncu, launches at 401,856 particles (profiles/launches_current.md)",
+    "dfsph_density_factor": "ncu, launches at 401,856 particles (profiles/launches_current.md)",
+    "wcsph_density": "ncu at 524,288 particles (profiles/launches_current.md), scaled by the particle count",
+    "wcsph_force": "ncu at 524,288 particles (profiles/launches_current.md), scaled by the particle count",
 }
-# Warp instructions per particle per launch from the ncu captures of the
-# PBF, WCSPH and DFSPH workloads (PBF lambda: the mean of 36.33 M for the
-# reusing launch and 90.41 M for each scanning one; PBF delta: the mean of
-# its captured launches).  The neighbour passes are bound by instruction issue, so the bench reports
+# Warp instructions per particle per launch from the same captures (PBF
+# lambda: the mean of 45.42 M for the reusing launch and 76.9 M for each
+# scanning one; the others: the mean of their captured launches).  The
+# neighbour passes are bound on chip, by L1 data cycles, gather latency and
+# issue together, so the bench reports
 # the issue rate beside the HBM roofline.  Issue peak = 148 SMs x 4
 # schedulers x 1 warp instruction per cycle at the SM clock sampled during
 # the timed region.
-WARP_INST_PER_PARTICLE = {"pbf_lambda": 76.89e6 / 401856, "pbf_delta": 24.32e6 / 401856,
-                          "wcsph_density": 126.16e6 / 524288, "wcsph_force": 49.30e6 / 524288,
-                          "dfsph_density_factor": 92.02e6 / 401856, "dfsph_rate": 26.87e6 / 401856}
+WARP_INST_PER_PARTICLE = {"pbf_lambda": 69.06e6 / 401856, "pbf_delta": 25.74e6 / 401856,
+                          "wcsph_density": 103.93e6 / 524288, "wcsph_force": 61.30e6 / 524288,
+                          "dfsph_density_factor": 77.27e6 / 401856, "dfsph_rate": 28.14e6 / 401856}
 FALLBACK_HBM_GBS = 6650.0
 SUBSTEP_DT = {"pbf": 1.0 / 240.0, "dfsph": 1.0 / 240.0}
 
@@ -855,7 +858,9 @@ def measure_workload(name, dev, flush, steps, warmup, args, world=1, clocks_gpu=
             passes[pname] = dict(ms_total=round(ms[p], 4), launches=int(cnt[p]), ms_avg=round(ms[p] / cnt[p], 5))
     dom = max(passes, key=lambda k: passes[k]["ms_total"])
     peak, peak_kind = measured_peak()
-    bpl = B_ALG.get(dom, 0) * n
+    in_build = B_ALG_IN_BUILD.get(name.split("_")[0], 0)
+    per_launch = {k: (B_ALG.get(k, 0) + (in_build if k == "grid_build" else 0)) * n for k in passes}
+    bpl = per_launch[dom]
     achieved = bpl / (passes[dom]["ms_avg"] * 1e-3) / 1e9
     traffic = TRAFFIC_PER_PARTICLE.get(dom)
     roofline = dict(bound="hbm", kernel=dom, achieved=round(achieved, 1), peak=peak, unit="GB/s",
@@ -874,7 +879,7 @@ def measure_workload(name, dev, flush, steps, warmup, args, world=1, clocks_gpu=
                                  source="warp instructions per particle from the committed ncu capture"
                                  + ("" if name.startswith("pbf") or name.startswith("dfsph") or name.endswith("524k")
                                     else " of the 524,288-particle lattice, scaled by the particle count"))
-    bytes_per_step = sum(B_ALG.get(k, 0) * n * v["launches"] for k, v in passes.items()) / Kp
+    bytes_per_step = sum(per_launch[k] * v["launches"] for k, v in passes.items()) / Kp
     gbs = bytes_per_step / (step_ms / K * 1e-3) / 1e9
     step_roofline = dict(algorithmic_bytes_per_step=bytes_per_step, achieved_gbs=round(gbs, 1),
                          frac=round(gbs / peak, 4))

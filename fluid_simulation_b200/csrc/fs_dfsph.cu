@@ -333,8 +333,8 @@ __device__ bool last_block(uint32_t* ticket) {
   return am_last;
 }
 
-// 64 registers: with 80, 73 us a launch at 401,856 particles, with 48 79,
-// against 65.
+// 64 registers: 60.4 us a launch at 401,856 particles, with 48 68.0, with 40
+// 89 (with 80, of lists that were still tested: 73 against 65).
 template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, 4) k_rate(RateArgs a) {
   grid_begin();
@@ -488,7 +488,8 @@ struct CorrectArgs {
 
 // A pair gathers one 16-byte record, so that 40 registers and 48 resident warps
 // hold more of them in flight than 56 and 36: 47.6 -> 44.5 us a launch at
-// 401,856 particles (32 registers: 66).  Several lanes per particle want 64.
+// 401,856 particles (32 registers: 66; without the list's tests 41.4, with 48
+// registers the same).  Several lanes per particle want 64.
 template <int G>
 __global__ void __launch_bounds__(kNbBlockMax, G == 1 ? 6 : 4) k_correct(CorrectArgs a) {
   grid_begin();
