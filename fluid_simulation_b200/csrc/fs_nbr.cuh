@@ -1,6 +1,6 @@
 // Neighbour loops of the per-particle passes.
 //
-// One thread per cell-sorted slot.  Only ~15 % of a particle's 27-cell grid
+// One thread per cell-sorted slot (several in small scenes).  Only ~15 % of a particle's 27-cell grid
 // candidates (the reference's hash_grid_query set) lie inside the support,
 // and every pass of a substep after the first reuses the same grid.  The
 // first pass over a grid therefore scans the candidates (scan_visit) and
@@ -355,7 +355,7 @@ FS_DEV int scan_words(const ScanXyz& q, float4 xi, float h2, uint2* words, int n
 }
 
 // Records the list of slot s (candidates within the radius whose square is
-// h2rec, in visiting order, self included) and calls pair(t, xj, payload) for
+// h2rec, in visiting order; LIST says which) and calls pair(t, xj, payload) for
 // those that pass visit_with's test at h2m, in the same order; load(t) is
 // issued together with the position gather.  Returns the DFSPH candidate
 // count when COUNT.  More than kNbMax entries mark the list overflowed; the
