@@ -74,8 +74,8 @@ struct AdjArgs {
   const float4* vs;    // (v, mass)
   const float* mv;     // rest_density * volume
   const float2* sc2;   // (P, R)
-  const float* nu;     // viscosity, cell order
-  const float* coh;    // surface_tension / mass, cell order
+  const float* nu;     // viscosity, cell order (0: does not move)
+  const float* coh;    // surface_tension / mass, cell order (0: does not move)
   float4* ab;          // (ab, 0), cell order
   float4* xr;          // (xb partial, rhob), cell order
   const float* xin;    // step input positions, original order
@@ -120,10 +120,14 @@ struct AdjGather {
     mv[s] = rd * (mass / fmaxf(rd, 1.0e-6f));
     const float r = a.rho[i];
     sc2[s] = make_float2(a.pressure[i] / fmaxf(r * r, 1.0e-6f), 1.0f / fmaxf(r, 1.0e-6f));
-    nu[s] = m.viscosity[i];
-    coh[s] = m.surface_tension[i] / mass;
+    // A particle that does not move has no terms of its own.  Its coefficients
+    // are 0 as its ab is, so that the products of the two are 0: without mass,
+    // surface_tension / mass is not finite.
+    const bool dyn = pf & PF_DYNAMIC;
+    nu[s] = dyn ? m.viscosity[i] : 0.f;
+    coh[s] = dyn ? m.surface_tension[i] / mass : 0.f;
     float3 ab = make_float3(0.f, 0.f, 0.f);
-    if (pf & PF_DYNAMIC) {
+    if (dyn) {
       float3 xb, vb;
       integrate_adjoint(walls_of(a.walls, a.g, w), x, v, ld3(a.accel, i), a.dt, ld3(a.xbo, i), ld3(a.vbo, i), xb, vb,
                         ab);
@@ -218,8 +222,8 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
           // ab_j, d_jk = -d, u_jk = -u), share their geometry and directions:
           //   c = A gs - coh m W with A = kv ud den - m Psum, kv = 10 nu m R
           //   d(c d)/dd . ab = c ab + (ab . d) (tang u + radial d)
-          // (evaluated side by side, they took twice the operations; ab is 0
-          // for a particle that is not dynamic)
+          // (evaluated side by side, they took twice the operations; ab, nu and
+          // coh are 0 for a particle that is not dynamic)
           const float3 u = make_float3(vk.x - nb.v.x, vk.y - nb.v.y, vk.z - nb.v.z);
           const float m_j = nb.v.w;
           const PairGeometry P(K, a.h, a.particle_radius, r2, coh_k != 0.f || nb.coh != 0.f);
