@@ -155,11 +155,18 @@ __global__ void __launch_bounds__(kRankThreads) k_rank(int64_t n, const int32_t*
   }
 }
 
-// fs_grid.cu: argument checks and the arguments of the first launch; the scan
-// and the scatter; the context's note of the finished build.
-int grid_prepare(fs_context* c, int64_t n, float radius, const int32_t* world, const fs_frame_clock* clock, KeyArgs* a);
-void grid_scan_scatter(fs_context* c, int64_t n, cudaStream_t st, const fs_frame_clock* clock);
-int grid_finish(fs_context* c, int64_t n, float radius, cudaStream_t st);
+// fs_grid.cu: argument checks, the arguments of the first launch and the
+// context's note that a build has begun; the scan and the scatter; the note of
+// the finished build (launched: what its launches returned).
+//
+// Each launch of a build writes where the one before it says: with the offsets
+// of an earlier build, or with counts that a scan has not cleared, the scatter
+// would write past its array.  So the first launch that fails ends the build,
+// and the next build clears the counts before it counts.
+int grid_prepare(fs_context* c, int64_t n, float radius, cudaStream_t st, const int32_t* world,
+                 const fs_frame_clock* clock, KeyArgs* a);
+cudaError_t grid_scan_scatter(fs_context* c, int64_t n, cudaStream_t st, const fs_frame_clock* clock);
+int grid_finish(fs_context* c, int64_t n, float radius, cudaStream_t st, cudaError_t launched);
 
 // Builds the grid of n > 0 positions of the Key functor and gathers into cell
 // order.  world: particle_world (required by batched contexts).  clock
@@ -168,14 +175,15 @@ template <class Key, class Gather>
 int grid_build(fs_context* c, int64_t n, float radius, cudaStream_t st, const int32_t* world,
                const fs_frame_clock* clock, const Key& source, const Gather& gather) {
   KeyArgs a;
-  int rc = grid_prepare(c, n, radius, world, clock, &a);
+  int rc = grid_prepare(c, n, radius, st, world, clock, &a);
   if (rc) return rc;
   PassScope ps_(c, P_GRID, st, 4);
-  launch(k_cell_keys<Key>, blocks_for(n), kBlock, sizeof(int32_t) * a.ntiles, st, n, source, a);
-  grid_scan_scatter(c, n, st, clock);
-  launch(k_rank<Gather>, blocks_for(n, kRankThreads), kRankThreads, 0, st, n, c->key, c->cell_off, c->tmp_ids, c->perm, gather,
-                                                               clock);
-  return grid_finish(c, n, radius, st);
+  cudaError_t e = launch(k_cell_keys<Key>, blocks_for(n), kBlock, sizeof(int32_t) * a.ntiles, st, n, source, a);
+  if (!e) e = grid_scan_scatter(c, n, st, clock);
+  if (!e)
+    e = launch(k_rank<Gather>, blocks_for(n, kRankThreads), kRankThreads, 0, st, n, c->key, c->cell_off, c->tmp_ids,
+               c->perm, gather, clock);
+  return grid_finish(c, n, radius, st, e);
 }
 
 }  // namespace fs

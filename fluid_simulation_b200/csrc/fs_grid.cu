@@ -219,8 +219,8 @@ GridDev grid_view(const fs_context* c) {
   return g;
 }
 
-int grid_prepare(fs_context* c, int64_t n, float radius, const int32_t* world, const fs_frame_clock* clock,
-                 KeyArgs* a) {
+int grid_prepare(fs_context* c, int64_t n, float radius, cudaStream_t st, const int32_t* world,
+                 const fs_frame_clock* clock, KeyArgs* a) {
   if (n < 0 || !(radius > 0.f)) return set_error(FS_ERR_INVALID, "grid_build: bad arguments");
   if (c->worlds && n > 0 && !world)
     return set_error(FS_ERR_INVALID, "grid_build: a batched context needs particle_world");
@@ -239,22 +239,35 @@ int grid_prepare(fs_context* c, int64_t n, float radius, const int32_t* world, c
   a->status = c->status;
   a->ctl = (ListCtl*)c->nb_ctl;
   a->clock = clock;
+  c->built_n = -1;  // until this build is done there is none
+  if (c->counting) {  // the one before ended half-way
+    int rc = check_cuda(cudaMemsetAsync(c->cell_count, 0, sizeof(int32_t) * (c->ncell + 1), st), "memset cell counts");
+    if (!rc)
+      rc = check_cuda(cudaMemsetAsync(c->scan_part, 0, sizeof(int32_t) * a->ntiles * tile_copies_max(a->ntiles), st),
+                      "memset tile sums");
+    if (rc) return rc;
+  }
+  c->counting = true;
   return FS_OK;
 }
 
-void grid_scan_scatter(fs_context* c, int64_t n, cudaStream_t st, const fs_frame_clock* clock) {
+cudaError_t grid_scan_scatter(fs_context* c, int64_t n, cudaStream_t st, const fs_frame_clock* clock) {
   // ncell + 1 buckets: the cells, then the non-finite positions
   const int64_t nbucket = c->ncell + 1;
   const int nb = scan_blocks(nbucket), copies = tile_copies(nb, n);
-  launch(k_scan, nb, kScanThreads, 0, st, c->cell_count, nbucket, c->scan_part, copies, c->cell_off, clock);
-  if (n > 0)
-    launch(k_scatter, blocks_for(n), kBlock, 0, st, n, c->key, c->slot, c->cell_off, c->tmp_ids, c->scan_part,
-                                                    nb * copies, clock);
+  cudaError_t e =
+      launch(k_scan, nb, kScanThreads, 0, st, c->cell_count, nbucket, c->scan_part, copies, c->cell_off, clock);
+  if (!e && n > 0)
+    e = launch(k_scatter, blocks_for(n), kBlock, 0, st, n, c->key, c->slot, c->cell_off, c->tmp_ids, c->scan_part,
+               nb * copies, clock);
+  return e;
 }
 
-int grid_finish(fs_context* c, int64_t n, float radius, cudaStream_t st) {
-  int rc = launch_check("grid_build");
+int grid_finish(fs_context* c, int64_t n, float radius, cudaStream_t st, cudaError_t launched) {
+  int rc = launch_check("grid_build");  // (clears the error that `launched` names)
+  if (launched) rc = check_cuda(launched, "grid_build");
   if (rc) return rc;
+  c->counting = false;
   c->built_n = n;
   c->built_inv = 1.0f / radius;
   c->last_stream = st;
@@ -267,13 +280,13 @@ static int grid_build_positions(fs_context* c, const float* x, int64_t n, float 
   if (n > 0 && !x) return set_error(FS_ERR_INVALID, "grid_build: bad arguments");
   if (n > 0) return grid_build(c, n, radius, st, world, nullptr, KeyPositions{x}, NoGather{});
   KeyArgs a;
-  int rc = grid_prepare(c, n, radius, world, nullptr, &a);
+  int rc = grid_prepare(c, n, radius, st, world, nullptr, &a);
   if (rc) return rc;
   PassScope ps_(c, P_GRID, st, 1);
   rc = check_cuda(cudaMemsetAsync(c->nb_ctl, 0, sizeof(ListCtl), st), "memset list control");
   if (rc) return rc;
-  grid_scan_scatter(c, 0, st, nullptr);  // the counts are zero: so are the offsets
-  return grid_finish(c, n, radius, st);
+  // the counts are zero: so are the offsets
+  return grid_finish(c, n, radius, st, grid_scan_scatter(c, 0, st, nullptr));
 }
 
 }  // namespace fs

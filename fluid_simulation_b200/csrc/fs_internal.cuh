@@ -82,6 +82,7 @@ struct fs_context {
   fs_grid_config grid{};
   int64_t ncell = 0;
   int64_t built_n = -1;      // n of the last grid build, -1 = none
+  bool counting = false;     // a build has begun and not ended: its counts may not be cleared
   float built_inv = 0.f;
   cudaStream_t last_stream = nullptr;
 
@@ -236,8 +237,10 @@ __device__ __forceinline__ int64_t thread_id() {
   return (int64_t)blockIdx.x * blockDim.x + threadIdx.x + zero;
 }
 
+// A failure is returned, and stays for launch_check().
 template <class... P, class... A>
-inline void launch(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st, A&&... args) {
+inline cudaError_t launch(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
+                          A&&... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -248,7 +251,7 @@ inline void launch(void (*kernel)(P...), unsigned blocks, unsigned threads, size
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);  // a failure stays for launch_check()
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
 }
 
 // Grid-stride loop over cell-sorted slots: thread k of a grid of G threads
