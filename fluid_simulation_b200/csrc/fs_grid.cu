@@ -400,6 +400,7 @@ int fs_context_create_worlds(fs_context** out, int64_t capacity, const fs_world_
   if (!rc)
     rc = check_cuda(cudaMemset(c->dfsph_worlds, 0, sizeof(DfsphWorld) * 2 * nworlds),
                     "fs_context_create_worlds: memset");
+  if (!rc) rc = check_cuda(cudaStreamSynchronize(cudaStreamLegacy), "fs_context_create_worlds: synchronize");
   delete[] host;
   if (rc) {
     fs_context_destroy(c);

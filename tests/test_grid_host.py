@@ -1,6 +1,7 @@
 """Host side of the grid build and of context creation, on a CUDA runtime that
 runs nothing (fake_cudart.cpp): a launch that fails ends the build, and the
-next build starts from cleared counts."""
+next build starts from cleared counts; a context is handed out when all that
+was cleared and copied for it is done."""
 
 import ctypes as C
 import os
@@ -33,7 +34,8 @@ def lib(tmp_path_factory):
                            os.path.join(build.CSRC, "fs_grid.cu"), str(stub), os.path.join(HERE, "fake_cudart.cpp")])
     lib = C.CDLL(str(out))
     lib.fake_calls.restype = C.c_char_p
-    for name in ("fs_context_create", "fs_context_destroy", "fs_grid_build", "fs_grid_tables", "fs_last_error_string"):
+    for name in ("fs_context_create", "fs_context_create_worlds", "fs_context_destroy", "fs_grid_build", "fs_grid_tables",
+                 "fs_last_error_string"):
         getattr(lib, name).restype, getattr(lib, name).argtypes = _lib.SIGNATURES[name]
     return lib
 
@@ -99,3 +101,19 @@ def test_a_refused_build_changes_nothing(lib, ctx):
     assert lib.fs_grid_build(ctx, None, 100, 0.1, None) == _lib.FS_ERR_INVALID
     assert calls(lib) == []
     assert lib.fs_grid_tables(ctx, None, None, None, None, None) == _lib.FS_OK
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_a_new_context_waits_for_its_clearing(lib, batched):
+    """The legacy stream's clears and copies: a caller's stream need not wait for them."""
+    p = C.c_void_p()
+    if batched:
+        box = _lib.WorldBox()
+        box.dims[:] = [4, 4, 4]
+        rc = lib.fs_context_create_worlds(C.byref(p), 1000, C.byref(box), 1, 0)
+    else:
+        rc = lib.fs_context_create(C.byref(p), 1000, C.byref(_lib.GridConfig(16, 16, 16, 0)), 0)
+    assert rc == _lib.FS_OK
+    lines = calls(lib)
+    lib.fs_context_destroy(p)
+    assert [ln for ln in lines if ln.startswith("memset")] and lines[-1] == "synchronize"
