@@ -33,7 +33,7 @@ constexpr int kCacheSlots = 64;  // CUDA contexts whose scratch address is cache
 
 struct NoAllocScratch {
   int32_t key[kNoAllocMaxParticles];   // cell key per original particle
-  int32_t slot[kNoAllocMaxParticles];  // arrival slot inside its cell; then the crowded-cell sort's second buffer
+  int32_t slot[kNoAllocMaxParticles];  // arrival slot inside its cell
   int32_t tmp[kNoAllocMaxParticles];   // ids, unordered inside cells
   int32_t perm[kNoAllocMaxParticles];  // sorted slot -> original id
   int32_t count[kNoAllocCells + 1];    // occupancy (cleared by every call); the last bucket: non-finite positions
@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(kSortThreads) k_na_big_sort(NoAllocScratch* sc
   for (int b = blockIdx.x; b < nbig; b += gridDim.x) {
     const int32_t c = sc->big_cells[b];
     const int32_t a = sc->off[c], len = sc->off[c + 1] - a;
-    const int32_t* sorted = block_sort_ids(sc->tmp + a, sc->slot + a, len, id_bits(n), sort_smem);
-    for (int k = threadIdx.x; k < len; k += blockDim.x) na_gather(sc, a + k, sorted[k], m, x);
+    block_sort_ids(sc->tmp + a, sc->perm + a, len, n, sort_smem);
+    for (int k = threadIdx.x; k < len; k += blockDim.x) na_gather(sc, a + k, sc->perm[a + k], m, x);
     __syncthreads();
   }
 }
