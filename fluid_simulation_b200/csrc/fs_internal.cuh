@@ -634,9 +634,10 @@ FS_DEV int particle_pf(const int32_t* flags, const int32_t* mask, int64_t i) {
 }
 
 // The scan copy of the positions (ScanXyz in fs_nbr.cuh): groups of four
-// slots, x[4], y[4], z[4].  An inactive particle lies at kScanFar: its squared
-// distance overflows to +inf.
-constexpr float kScanFar = 1.0e30f;
+// slots, x[4], y[4], z[4].  An inactive particle lies at x = +inf: its squared
+// distance is +inf.  It is alone there: an active one whose x is not finite,
+// which is within reach of nothing either, lies at -inf.
+constexpr uint32_t kScanInactive = 0x7f800000u, kScanNonFinite = 0xff800000u;
 struct ScanOut {
   float* g;
   ListCtl* ctl;  // notes of the gather (may be null)
@@ -644,7 +645,7 @@ struct ScanOut {
 FS_DEV void scan_put(const ScanOut& q, int64_t s, float3 p, bool active) {
   if (!active && q.ctl) q.ctl->inactive = 1;
   float* o = q.g + (s >> 2) * 12 + (s & 3);
-  o[0] = active ? p.x : kScanFar;
+  o[0] = !active ? __uint_as_float(kScanInactive) : isfinite(p.x) ? p.x : __uint_as_float(kScanNonFinite);
   o[4] = p.y;
   o[8] = p.z;
 }

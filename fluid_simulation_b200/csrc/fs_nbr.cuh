@@ -136,7 +136,7 @@ struct Masses {
 
 // The coordinates of the cell-order particles for the grid scans: groups of
 // four slots, x[4], y[4], z[4] (48 bytes, 16-byte aligned); an inactive
-// particle lies far outside any support (kScanFar).
+// particle lies outside any support (kScanInactive).
 struct ScanXyz {
   const float* g;
 };
@@ -197,11 +197,11 @@ struct ScanPos {
 // (for_each_range's ranges) and cut into pieces of at most 32 candidates
 // (counted from the 16-byte group that holds the first), to words[k * nthr]
 // as (first, end), from pos on until CAP pieces are written or the query
-// is exhausted (live = false); returns their number.  COUNT adds the active
-// candidates other than s (no distance test) to ncand.
+// is exhausted (live = false); returns their number.  COUNT adds the
+// candidates other than s (no distance test, inactive ones too) to ncand.
 template <bool COUNT, int CAP>
-FS_DEV int scan_pieces(const GridDev& g, const float4* __restrict__ xs, int s, float4 xi, float h, bool inactive,
-                       uint2* words, int nthr, ScanPos& pos, bool& live, int& ncand) {
+FS_DEV int scan_pieces(const GridDev& g, int s, float4 xi, float h, uint2* words, int nthr, ScanPos& pos, bool& live,
+                       int& ncand) {
   const WorldDev* W = g.worlds ? g.worlds + world_index(world_of(xi), g.nworlds) : nullptr;
   const QueryBox b = W ? query_box_world(g, *W, xi.x, xi.y, xi.z, h) : query_box_hash(g, xi.x, xi.y, xi.z, h);
   const int nx = b.x1 - b.x0 + 1;
@@ -215,13 +215,7 @@ FS_DEV int scan_pieces(const GridDev& g, const float4* __restrict__ xs, int s, f
     nseg = slow ? nx : (nx > len1 ? 2 : 1);  // a run that wraps modulo dim_x splits in two
   }
   int nw = 0;
-  auto count = [&](int a, int e) {
-    if (inactive) {
-      for (int k = a; k < e; ++k) ncand += (k != s) ? (__float_as_int(__ldg(&xs[k].w)) & PF_ACTIVE) : 0;
-    } else {
-      ncand += (e - a) - ((s >= a && s < e) ? 1 : 0);
-    }
-  };
+  auto count = [&](int a, int e) { ncand += (e - a) - ((s >= a && s < e) ? 1 : 0); };
   const int ny = b.y1 - b.y0 + 1, nz = b.z1 - b.z0 + 1;
   if (pos.z == INT32_MIN) {
     pos.z = b.z0, pos.y = b.y0;
@@ -314,10 +308,16 @@ struct ScanQuery {
 
 // The hit word of the piece [first, end), not empty, at most 32 slots from the
 // group of four that holds the first: bit b set = slot last - b is within.
-FS_DEV uint32_t scan_word(const ScanXyz& q, const ScanQuery& o, uint32_t first, uint32_t end, uint32_t& last) {
+// INACTIVE: ninactive is the number of inactive particles in the piece, three
+// more operations a candidate (DFSPH's density pass, whose candidates are
+// counted; with their flags read one by one it took 152 us at 401,856
+// particles, one of them inactive, for 107 with none; now 109, at 10 % 153 -> 107).
+template <bool INACTIVE = false>
+FS_DEV uint32_t scan_word(const ScanXyz& q, const ScanQuery& o, uint32_t first, uint32_t end, uint32_t& last,
+                          int* ninactive = nullptr) {
   const uint32_t g0 = first >> 2, g1 = (end + 3) >> 2;
   const ulonglong2* p = reinterpret_cast<const ulonglong2*>(q.g) + (size_t)g0 * 3;
-  uint32_t m = 0;
+  uint32_t m = 0, far = 0;
 #pragma unroll 2  // two groups of loads in flight (density time with 1: +1 to 3 %, with 4: up to +7 %)
   for (uint32_t i = g0; i < g1; ++i, p += 3) {
     const ulonglong2 x2 = __ldg(p), y2 = __ldg(p + 1), z2 = __ldg(p + 2);
@@ -330,22 +330,32 @@ FS_DEV uint32_t scan_word(const ScanXyz& q, const ScanQuery& o, uint32_t first, 
     m = __funnelshift_l((uint32_t)(r0 >> 32), m, 1);
     m = __funnelshift_l((uint32_t)r1, m, 1);
     m = __funnelshift_l((uint32_t)(r1 >> 32), m, 1);
+    if (INACTIVE) {
+      // x = +inf (kScanInactive, no active particle's): the sum's sign bit is
+      // set for it and for negative x
+      auto mark = [&](uint32_t x) { far = __funnelshift_l((x + 0x00800000u) & ~x, far, 1); };
+      mark((uint32_t)x2.x), mark((uint32_t)(x2.x >> 32)), mark((uint32_t)x2.y), mark((uint32_t)(x2.y >> 32));
+    }
   }
-  // slots of the groups outside the piece: before its first, after its last
-  m &= 0xffffffffu >> (32 - 4 * (g1 - g0) + (first & 3));
-  m &= 0xffffffffu << (4 * g1 - end);
+  // without the slots of the groups outside the piece: before its first, after its last
+  const uint32_t in = (0xffffffffu >> (32 - 4 * (g1 - g0) + (first & 3))) & (0xffffffffu << (4 * g1 - end));
+  if (INACTIVE) *ninactive = __popc(far & in);
   last = 4 * g1 - 1;
-  return m;
+  return m & in;
 }
 
-// Replaces the pieces in `words` by their non-empty hit words (mask, last).
-FS_DEV int scan_words(const ScanXyz& q, float4 xi, float h2, uint2* words, int nthr, int np) {
+// Replaces the pieces in `words` by their non-empty hit words (mask, last);
+// INACTIVE takes the inactive candidates from ncand.
+template <bool INACTIVE>
+FS_DEV int scan_words(const ScanXyz& q, float4 xi, float h2, uint2* words, int nthr, int np, int& ncand) {
   const ScanQuery o(xi, h2);
   int nw = 0;
   for (int k = 0; k < np; ++k) {
     const uint2 piece = words[k * nthr];
     uint32_t last;
-    const uint32_t m = scan_word(q, o, piece.x, piece.y, last);
+    int ninactive = 0;
+    const uint32_t m = scan_word<INACTIVE>(q, o, piece.x, piece.y, last, &ninactive);
+    if (INACTIVE) ncand -= ninactive;
     if (m) {
       words[nw * nthr] = make_uint2(m, last);
       ++nw;
@@ -402,8 +412,9 @@ FS_DEV int scan_visit(const GridDev& g, const ScanXyz& q, const float4* __restri
   while (live) {
     int nw = 0;
     if (scan) {
-      const int np = scan_pieces<COUNT, kWords>(g, xs, s, xi, h, inactive, words, nthr, pos, live, ncand);
-      nw = scan_words(q, xi, h2rec * kScanSlack, words, nthr, np);
+      const int np = scan_pieces<COUNT, kWords>(g, s, xi, h, words, nthr, pos, live, ncand);
+      nw = COUNT && inactive ? scan_words<COUNT>(q, xi, h2rec * kScanSlack, words, nthr, np, ncand)
+                             : scan_words<false>(q, xi, h2rec * kScanSlack, words, nthr, np, ncand);
     } else {
       live = false;
     }
@@ -768,7 +779,7 @@ FS_DEV int group_scan(const GridDev& g, const ScanXyz& q, const float4* __restri
     const bool now = live && scan, again = REUSE && live && !scan;  // (other groups of the warp may go on)
     if (now && !plain) {
       int nc = 0;
-      const int np = scan_pieces<COUNT, kGroupRows>(g, xs, s, xi, h, inactive, pieces, 1, pos, live, nc);
+      const int np = scan_pieces<COUNT, kGroupRows>(g, s, xi, h, pieces, 1, pos, live, nc);
       if (lane == 0) ncand += nc;
       // every lane has written the same pieces
 #pragma unroll
@@ -784,17 +795,18 @@ FS_DEV int group_scan(const GridDev& g, const ScanXyz& q, const float4* __restri
     uint32_t w[N][2], last[N][2], cnt = 0;  // hit words; hits of the rounds
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-      if (COUNT && now && plain) {
-        if (inactive) {
-          for (int t = f[k]; t < e[k]; ++t) ncand += (t != s) ? (__float_as_int(__ldg(&xs[t].w)) & PF_ACTIVE) : 0;
-        } else {
-          ncand += (e[k] - f[k]) - ((s >= f[k] && s < e[k]) ? 1 : 0);
-        }
-      }
+      if (COUNT && now && plain) ncand += (e[k] - f[k]) - ((s >= f[k] && s < e[k]) ? 1 : 0);
       const int mid = min(e[k], (f[k] & ~3) + 32);
       w[k][0] = w[k][1] = last[k][0] = last[k][1] = 0;
-      if (now && f[k] < mid) w[k][0] = scan_word(q, o, f[k], mid, last[k][0]);
-      if (now && mid < e[k]) w[k][1] = scan_word(q, o, mid, e[k], last[k][1]);
+      auto word = [&](int first, int end, uint32_t& at) {
+        if (!(COUNT && inactive)) return scan_word(q, o, first, end, at);
+        int ninactive;
+        const uint32_t m = scan_word<true>(q, o, first, end, at, &ninactive);
+        ncand -= ninactive;
+        return m;
+      };
+      if (now && f[k] < mid) w[k][0] = word(f[k], mid, last[k][0]);
+      if (now && mid < e[k]) w[k][1] = word(mid, e[k], last[k][1]);
       cnt |= (uint32_t)(__popc(w[k][0]) + __popc(w[k][1])) << (10 * k);
     }
     // hits before this lane's in each round, and in all lanes (at most 9 rows of 64: ten bits)
