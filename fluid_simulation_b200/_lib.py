@@ -119,6 +119,7 @@ SIGNATURES = {
     "fs_dfsph_nonpressure_predict": (C.c_int, [P, C.POINTER(Model), P, P, P, F, F, F, P, P, P]),
     "fs_pbf_predict": (C.c_int, [P, C.POINTER(Model), P, P, C.POINTER(PbfParams), P, P, P]),
     "fs_context_get_tuning": (C.c_int, [P, C.POINTER(Tuning)]),
+    "fs_lanes_per_particle": (I32, [I64]),
     "fs_context_cells": (I64, [P]),
     "fs_grid_build_worlds": (C.c_int, [P, P, P, I64, F, P]),
     "fs_grid_candidates_worlds": (C.c_int, [P, P, P, I64, F, P, P, P, P]),

@@ -6,7 +6,9 @@ much of that latency is hidden.  Three knobs of a context (``fs_tuning``)
 move that balance:
 
   block_size            threads per block (64, 128, 256)
-  particles_per_thread  cell-sorted particles each thread walks (1, 2, 4)
+  particles_per_thread  cell-sorted particles each thread walks (1, 2, 4);
+                        left at 1 in small scenes, where several lanes
+                        share a particle
   cell_ratio            grid cell width / h (WCSPH only: 1 or 0.5)
 
 (a fourth, ``list_skin``, the skin of PBF's first density lists that lets
@@ -58,12 +60,14 @@ def set_tuning(ctx, tuning: Tuning) -> None:
     _lib.check(_lib.load().fs_context_set_tuning(ctx, C.byref(t)), "fs_context_set_tuning")
 
 
-def candidates(solver_kind: str, batched: bool = False):
-    """Every tuning worth timing for a solver ('wcsph', 'dfsph', 'pbf'),
-    the default first (it wins ties)."""
+def candidates(solver_kind: str, batched: bool = False, lanes: int = 1):
+    """Every tuning worth timing for a solver ('wcsph', 'dfsph', 'pbf') whose
+    kernels give a particle ``lanes`` lanes, the default first (it wins
+    ties)."""
+    per_thread = PARTICLES_PER_THREAD if lanes == 1 else (1,)
     ratios = (1.0, 0.5) if solver_kind == "wcsph" and not batched else (1.0,)
     out = [Tuning(*DEFAULT)]
-    for b, p, r in itertools.product(BLOCK_SIZES, PARTICLES_PER_THREAD, ratios):
+    for b, p, r in itertools.product(BLOCK_SIZES, per_thread, ratios):
         t = Tuning(b, p, r)
         if t not in out:
             out.append(t)
@@ -92,7 +96,8 @@ def autotune(solver, state, dt: float, steps: int = 3, repeats: int = 2, timer=N
     model = solver.model
     grid = model.particle_grid
     ctx = grid._ctx
-    cands = candidates(_kind(solver), batched=isinstance(grid, WorldGrid))
+    cands = candidates(_kind(solver), batched=isinstance(grid, WorldGrid),
+                       lanes=_lib.load().fs_lanes_per_particle(model.particle_count))
     if timer is None:
         timer = _device_timer(solver, state, dt, steps, repeats)
     times = {}

@@ -441,6 +441,8 @@ int fs_context_get_tuning(const fs_context* c, fs_tuning* t) {
   return FS_OK;
 }
 
+int32_t fs_lanes_per_particle(int64_t n) { return nb_group(n); }
+
 int32_t fs_context_worlds(const fs_context* c) { return c ? c->nworlds : -1; }
 int64_t fs_context_cells(const fs_context* c) { return c ? c->ncell : -1; }
 

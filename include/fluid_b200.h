@@ -155,7 +155,9 @@ int64_t fs_context_capacity(const fs_context* ctx);
  * the autotuner (fluid_simulation_b200.autotune) from measured substeps.
  *   block_size            threads per block: 64, 128 (default) or 256
  *   particles_per_thread  1 (default), 2 or 4: each thread walks that many
- *                         cell-sorted particles (grid-stride)
+ *                         cell-sorted particles (grid-stride); no effect
+ *                         where several lanes share a particle
+ *                         (fs_lanes_per_particle)
  *   cell_ratio            WCSPH grid cell width / h: 1 (default, the
  *                         reference's grid: candidates in its order) or 0.5
  *                         (125 half-width cells per query instead of 27;
@@ -179,6 +181,10 @@ typedef struct {
 } fs_tuning;
 int fs_context_set_tuning(fs_context* ctx, const fs_tuning* tuning);
 int fs_context_get_tuning(const fs_context* ctx, fs_tuning* tuning);
+
+/* Lanes that share a particle in the substeps' neighbour kernels of a model
+ * of n particles: 16, 8 or 4 in small scenes, 1 in others. */
+int32_t fs_lanes_per_particle(int64_t n);
 
 /* `grid.build(points, radius)` (solver_wcsph.py:456, solver_dfsph.py:624,783,
  * solver_pbf.py:737,858): cell keys, stable sort by cell, cell ranges. */
