@@ -58,9 +58,9 @@ sys.path.insert(0, ROOT)
 # average 28 + 44 / 2 B; its predict (60 B) and DFSPH's integrate (36 B, in
 # one of two builds) run in the grid build's first kernel (B_ALG_IN_BUILD).
 B_ALG = {
-    "grid_build": 48, "pbf_predict": 60, "pbf_density": 50, "pbf_accel": 72, "pbf_lambda": 40, "pbf_delta": 56,
-    "pbf_velocity": 44, "pbf_xsph": 64, "wcsph_density": 40, "wcsph_force": 92, "dfsph_density_factor": 36,
-    "dfsph_accel": 76, "dfsph_rate": 60, "dfsph_correct": 56, "dfsph_integrate": 36, "dfsph_final": 48,
+    "grid_build": 48, "pbf_density": 50, "pbf_accel": 72, "pbf_lambda": 40, "pbf_delta": 56, "pbf_xsph": 64,
+    "wcsph_density": 40, "wcsph_force": 92, "dfsph_density_factor": 36, "dfsph_accel": 76, "dfsph_rate": 60,
+    "dfsph_correct": 56, "dfsph_final": 48,
 }
 B_ALG_IN_BUILD = {"pbf": 60, "dfsph": 18}
 PUBLISHED_PBF = 401856 * 4 / 0.06464700849610381   # particle-substeps/s, RTX 4090 (performance_summary.json)

@@ -25,9 +25,9 @@
 namespace fs {
 
 // Partial-sum slots for the residual reductions: one per block of the
-// smallest block size that launches them (64 threads, up to 32 lanes a
-// particle: two particles a block).
-int reduction_blocks(int64_t n) { return blocks_for(n > 0 ? n : 1, 2); }
+// smallest block size that launches them (64 threads, up to 16 lanes a
+// particle: four particles a block).
+int reduction_blocks(int64_t n) { return blocks_for(n > 0 ? n : 1, 4); }
 
 // gather of fs_wcsph.cu reused here
 __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
@@ -656,7 +656,8 @@ int run_rate(fs_context* c, const fs_model* m, int mode, int it, float h, float 
   a.term = per_world ? c->sc1b : nullptr;
   if (per_world && !m->particle_world) return set_error(FS_ERR_INVALID, "dfsph rate: a batched context needs particle_world");
   const int group = use_lists ? nb_group(a.n) : 1;  // no list: each thread rescans
-  if (ctrl && !per_world && nb_blocks(c, a.n * group) > reduction_blocks(c->capacity))
+  const int64_t blocks = group > 1 ? (a.n * group + c->nb_block - 1) / c->nb_block : nb_blocks(c, a.n);
+  if (ctrl && !per_world && blocks > reduction_blocks(c->capacity))
     return set_error(FS_ERR_INVALID, "dfsph rate: reduction buffer too small");
   {
     PassScope ps_(c, P_DFSPH_RATE, st, per_world ? 2 : 1);
@@ -726,10 +727,6 @@ int run_density_factor(fs_context* c, const fs_model* m, float h, int min_nb, fl
 }  // namespace fs
 
 using namespace fs;
-
-extern "C" {
-
-}  // extern "C"
 
 namespace fs {
 namespace {

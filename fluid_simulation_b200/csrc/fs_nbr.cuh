@@ -105,8 +105,6 @@ FS_DEV bool exact_lt_h(float r2_any, float dx, float dy, float dz, float h, floa
 // 1.1 % after 500), and each overflowing particle rescans the grid in every
 // pass at those positions, its whole warp with it.
 constexpr int kNbMax = 192;
-// Entry offsets k * stride (k < kNbMax) fit 32 bits up to this stride (capacity).
-constexpr int64_t kListStride32Max = 0xffffffffLL / kNbMax;
 
 // The mass that the pair terms read for each neighbour.  Particles of one
 // fluid mostly share one: the gather notes whether they do (ListCtl), and then
