@@ -15,8 +15,8 @@
 // What bounds it: at small counts the launches and the 16.8 MB that the scan
 // of 128^3 cells moves through L2, at large ones the scattered accesses of
 // keys and rank.  B200, predict + build + gather of a PBF substep: 35 + 9 + 7
-// us in eleven launches before, 25 in these four at 4,079 particles; 45 + 19 +
-// 13 and 54 at 401,856.
+// us in eleven launches before, 22 in these four at 4,079 particles; 45 + 19 +
+// 13 and 48 at 401,856.
 #pragma once
 
 #include "fs_nbr.cuh"

@@ -180,19 +180,29 @@ NbrList nbr_list(const fs_context* c) {
 }
 
 // Lanes per particle: as many as fill the GPU (148 SMs hold 151,552 threads of
-// these kernels), fewer where the sums, which every lane of a group repeats,
-// outweigh the shorter chain.  Substep times in us, B200:
-//   particles        4,000   7,500   14,000   30,000   38,000   46,000
-//   PBF    1 lane      218     221      227      239      269      273
-//          4 lanes     132     135      145      218      263      294
-//          8 lanes     104     115      135      253      299      353
-//         16 lanes      93     129      177      322      394      460
-//   DFSPH  1 lane      495     513      536      556      587      599
-//          4 lanes     301     311      328      446      521      644
-//          8 lanes     278     296      346      579      657      804
-//         16 lanes     265     325      481      792      962    1,119
-// (WCSPH and its adjoint cross over at the same sizes; two lanes are slower
-// than one or four throughout, but for DFSPH between 38,000 and 50,000.)
+// these kernels), fewer where what every lane of a group repeats (the ordered
+// sums; in the adjoint, which adds up per lane, the particle's own data and the
+// reduction of nine sums) outweighs the shorter chain.  One rule for all
+// methods, as the lists' layout hangs on it; they cross over at much the same
+// sizes.  B200, us a substep, in a replayed frame of four (backward: in a
+// segment of ten):
+//   particles          4,000  7,500 14,000 20,000 30,000 38,000 46,000
+//   PBF       1 lane     282    297    304    312    321    326    336
+//             4          185    196    206    221    254    276    309
+//             8          150    160    180    224    274    313    365
+//            16          130    154    213    257    346    422    485
+//   DFSPH     1          589    694    855    981  1,205  1,214  1,165
+//             4          363    421    514    606    794    795    804
+//             8          332    385    487    587    767    844    958
+//            16          297    362    556    729  1,006  1,181  1,357
+//   WCSPH     1         44.7   49.4   51.2   52.3   53.9   56.5   57.9
+//             4         32.9   35.2   37.2   39.4   47.5   54.8   59.2
+//             8         29.1   31.5   34.8   45.0   53.2   60.3   69.3
+//            16         27.6   33.5   40.3   49.7   64.1   74.3   85.6
+//   backward  1         64.5   66.7   69.5   70.0   73.1   76.5   80.6
+//             4         40.6   42.7   46.2   55.4   65.5   68.9   81.4
+//             8         35.3   39.2   50.4   58.1   72.8   81.9   94.1
+//            16         32.2   41.2   52.8   67.3   86.6  101.1  117.3
 int nb_group(int64_t n) { return n <= 6000 ? 16 : n <= 14000 ? 8 : n <= 38000 ? 4 : 1; }
 
 ScanXyz scan_xyz(const fs_context* c) { return ScanXyz{c->sxyz}; }

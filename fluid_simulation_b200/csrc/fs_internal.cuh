@@ -108,8 +108,7 @@ struct fs_context {
   float* sc1 = nullptr;   // per-slot scalar (kappa / lambda)
   float* sc1b = nullptr;  // per-slot scalar (second)
   float* mass = nullptr;  // per-slot mass
-  float4* rec = nullptr;  // per-slot (x, y, z, value): kappa / rho for the DFSPH correction, lambda for PBF's delta,
-                          // p / rho^2 for the WCSPH force
+  float4* rec = nullptr;  // per-slot (x, y, z, value): kappa / rho for the DFSPH correction, lambda for PBF's delta
   float* xo_tmp = nullptr;  // [cap*3] original-order scratch positions (PBF x_pred)
   float* vo_tmp = nullptr;  // [cap*3] original-order scratch velocities (PBF v_pred)
 
@@ -124,7 +123,7 @@ struct fs_context {
   bool stats_on = false;                     // count them (fs_list_stats_enable)
 
   // neighbour lists (fs_nbr.cuh)
-  int32_t* nb_idx = nullptr;     // [kNbMax][cap]
+  int32_t* nb_idx = nullptr;     // [kNbMax][cap]; several lanes a particle: [cap][kNbMax]
   int32_t* nb_cnt = nullptr;     // [cap]
   void* nb_ctl = nullptr;        // ListCtl
 
