@@ -305,7 +305,7 @@ __global__ void FS_NB_BOUNDS k_adj_density(AdjArgs a) {
     const float mv_k = a.mv[s];
     const Cubic K(a.h);
     float3 xb = lead ? make_float3(xr.x, xr.y, xr.z) : make_float3(0.f, 0.f, 0.f);
-    list_sum<G, false, false, true, true, 0>(
+    list_sum<G, false, false, true, true, 0, kAhead>(
         a.g, a.xs, a.xs, (int)s, xk, a.h, a.h * a.h * kSupportMargin, a.L, lists_usable(a.L), on,
         [&](int t) { return make_float2(__ldg(a.mv + t), __ldg(&a.xr[t].w)); },
         [&](int t, float4 xj, const float2& j) {

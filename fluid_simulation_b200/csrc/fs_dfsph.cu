@@ -173,7 +173,7 @@ __global__ void FS_NB_BOUNDS k_accel_predict(AccelArgs a) {
       float4 v;
       float rho;
     };
-    list_sum<G, false, false, true, true, 4>(
+    list_sum<G, false, false, true, true, 4, kAhead>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn, [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(&a.sc2[t].x)}; },
         [&](int t, float4 xj, const Neighbour& j) {
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kNbBlockMax, 4) k_rate(RateArgs a) {
     float d = 0.f;
     const float4 vi = make_float4(a.xv[s].w, a.vyz[s].x, a.vyz[s].y, 0.f);
     const Cubic K(a.h);
-    list_sum<G, false, false, false, true, 2>(
+    list_sum<G, false, false, false, true, 2, kAhead>(
         a.g, a.xs, a.xv, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && !over && (pf & PF_ACTIVE), [&](int t) { return Neighbour{__ldg(a.vyz + t), mass(t)}; },
         [&](int t, float4 xj, const Neighbour& j) {
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(kNbBlockMax, G == 1 ? 6 : 4) k_correct(Correct
     const Cubic K(a.h);
     const float ci = a.rec[s].w;
     float dvx = 0.f, dvy = 0.f, dvz = 0.f;
-    list_sum<G, false, false, false, true, 4>(
+    list_sum<G, false, false, false, true, 4, kRecords>(
         a.g, a.xs, a.rec, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && !over && dyn, mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;

@@ -523,6 +523,41 @@ FS_DEV void scan_grid(const GridDev& g, const float4* __restrict__ xs, int s, fl
   });
 }
 
+// The same for lists that overflowed: pair(t, rec[t]), by RESCAN
+//   kGrid     scan_grid, then the record
+//   kRecords  the positions from the records that the pairs gather anyway; a
+//             hit's flag is read only where some particle is inactive
+//   kAhead    and the next record loads while one is tested
+// DFSPH substep with lists that all overflow (four spacings to the support,
+// about 250 neighbours), in ms at 61,740 and 401,856 particles: 15.9, 34.3;
+// 14.4, 31.1; 13.2, 33.2; kAhead but in the correction, which is short of
+// registers, 13.4, 31.0.  kGrid where that cost the ordinary path: WCSPH's force
+// 1 %, PBF's passes 0.4 % of a substep of 100,003 particles, several lanes per
+// particle 0.4 % at 4,079.
+enum Rescan { kGrid, kRecords, kAhead };
+
+template <bool WITH_SELF, Rescan RESCAN, class Pair>
+FS_DEV void rescan(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s, float4 xi,
+                   float h, float h2m, const NbrList& L, Pair&& pair) {
+  if constexpr (RESCAN == kGrid) {
+    scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { pair(t, __ldg(rec + t)); });
+  } else {
+    const bool inactive = L.ctl->inactive != 0;
+    for_each_range(g, world_of(xi), xi.x, xi.y, xi.z, h, [&](int a, int e) {
+      if (a >= e) return;
+      float4 next = __ldg(rec + a);
+      for (int t = a; t < e; ++t) {
+        const float4 xj = RESCAN == kAhead ? next : __ldg(rec + t);
+        if (RESCAN == kAhead && t + 1 < e) next = __ldg(rec + t + 1);
+        const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
+        if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= h2m && (WITH_SELF || t != s) &&
+            (!inactive || (pf_of(__ldg(xs + t)) & PF_ACTIVE)))
+          pair(t, xj);
+      }
+    });
+  }
+}
+
 // One entry of a list, past L1, which the neighbours' data fill (the lists
 // stay in L2): DFSPH rate 63.1 -> 62.2 us, correct 42.7 -> 42.1 at 401,856
 // particles.
@@ -538,7 +573,7 @@ FS_DEV int32_t ld_list(const int32_t* p) {
 // (xs itself, or a pass's own); pair(t, rec[t]).  EXACT: a kExact list, whose
 // entries need no test (with one: rate 62.2 instead of 60.4 us, WCSPH force
 // 695 instead of 669).
-template <bool WITH_SELF, bool EXACT, class Pair>
+template <bool WITH_SELF, bool EXACT, Rescan RESCAN, class Pair>
 FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s, float4 xi,
                   float h, float h2m, const NbrList& L, bool lists_ok, Pair&& pair) {
   const int n = lists_ok ? __ldg(L.cnt + s) : kNbMax + 1;
@@ -571,7 +606,7 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, const float4*
       if (k2) one(t2, x2);
     }
   } else {
-    scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { pair(t, __ldg(rec + t)); });
+    rescan<WITH_SELF, RESCAN>(g, xs, rec, s, xi, h, h2m, L, pair);
   }
 }
 
@@ -588,7 +623,7 @@ FS_DEV void visit(const GridDev& g, const float4* __restrict__ xs, const float4*
 // lists at most one later pass reads again (delta, non-pressure, XSPH:
 // 1.304 -> 1.287 ms per substep at 401,856 particles); the DFSPH iteration
 // passes, which read the same lists 34 times a substep, were slower with it.
-template <bool WITH_SELF, bool EVICT_FIRST, bool EXACT, class Load, class Pair>
+template <bool WITH_SELF, bool EVICT_FIRST, bool EXACT, Rescan RESCAN, class Load, class Pair>
 FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s,
                        float4 xi, float h, float h2m, const NbrList& L, bool lists_ok, Load&& load, Pair&& pair) {
   const int n = lists_ok ? __ldg(L.cnt + s) : kNbMax + 1;
@@ -622,7 +657,7 @@ FS_DEV void visit_with(const GridDev& g, const float4* __restrict__ xs, const fl
       if (k2) one(t2, x2, p2);
     }
   } else {
-    scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { pair(t, __ldg(rec + t), load(t)); });
+    rescan<WITH_SELF, RESCAN>(g, xs, rec, s, xi, h, h2m, L, [&](int t, float4 xj) { pair(t, xj, load(t)); });
   }
 }
 
@@ -860,7 +895,8 @@ FS_DEV int group_scan(const GridDev& g, const ScanXyz& q, const float4* __restri
 //   scan_sum  scans the grid and records the list (scan_visit, group_scan)
 //   list_sum  iterates the recorded list (visit, visit_with, group_visit),
 //             or rescans where there is none; LAZY: load(t) only after the
-//             distance test (G = 1), where the early load costs registers
+//             distance test (G = 1), where the early load costs registers;
+//             RESCAN with one thread per particle (several: kGrid)
 // A particle with on = false takes no part.
 template <int G, bool WITH_SELF, bool COUNT, bool REUSE, ListOf LIST, int K, class Load, class Term, class Acc>
 FS_DEV int scan_sum(const GridDev& g, const ScanXyz& q, const float4* __restrict__ xs, int s, float4 xi, float h,
@@ -877,16 +913,17 @@ FS_DEV int scan_sum(const GridDev& g, const ScanXyz& q, const float4* __restrict
   }
 }
 
-template <int G, bool WITH_SELF, bool EVICT_FIRST, bool LAZY, bool EXACT, int K, class Load, class Term, class Acc>
+template <int G, bool WITH_SELF, bool EVICT_FIRST, bool LAZY, bool EXACT, int K, Rescan RESCAN, class Load,
+          class Term, class Acc>
 FS_DEV void list_sum(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s, float4 xi,
                      float h, float h2m, const NbrList& L, bool lists_ok, bool on, Load&& load, Term&& term,
                      Acc&& acc) {
   if constexpr (G == 1) {
     if (!on) return;
     if constexpr (LAZY)
-      visit<WITH_SELF, EXACT>(g, xs, rec, s, xi, h, h2m, L, lists_ok, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
+      visit<WITH_SELF, EXACT, RESCAN>(g, xs, rec, s, xi, h, h2m, L, lists_ok, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
     else
-      visit_with<WITH_SELF, EVICT_FIRST, EXACT>(g, xs, rec, s, xi, h, h2m, L, lists_ok, load,
+      visit_with<WITH_SELF, EVICT_FIRST, EXACT, RESCAN>(g, xs, rec, s, xi, h, h2m, L, lists_ok, load,
                                          [&](int t, float4 xj, const auto& p) { acc(term(t, xj, p)); });
   } else {
     const int n = !on ? 0 : (lists_ok ? __ldg(L.cnt + s) : kNbMax + 1);
@@ -894,7 +931,7 @@ FS_DEV void list_sum(const GridDev& g, const float4* __restrict__ xs, const floa
     const int32_t* const row = L.idx + (int64_t)s * kNbMax;
     group_visit<G, WITH_SELF, K>(rec, s, xi, h2m, over ? 0 : n, [&](int k) { return __ldg(row + k); }, load, term, acc);
     if (over && (K > 0 || (threadIdx.x & (G - 1)) == 0))  // each lane adds up the whole sum (K = 0: the first)
-      scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { acc(term(t, __ldg(rec + t), load(t))); });
+      rescan<WITH_SELF, kGrid>(g, xs, rec, s, xi, h, h2m, L, [&](int t, float4 xj) { acc(term(t, xj, load(t))); });
   }
 }
 

@@ -176,7 +176,7 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
     const Poly6Spiky K(a.h);
     float ax = 0.f, ay = 0.f, az = 0.f;
     const bool on = live && dyn && (gamma != 0.f || mu != 0.f);
-    list_sum<G, false, true, false, false, 4>(
+    list_sum<G, false, true, false, false, 4, kGrid>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), on,
         [&](int t) { return Neighbour{__ldg(a.vs + t), mass(t)}; },
         [&](int t, float4 xj, const Neighbour& j) {
@@ -358,7 +358,7 @@ __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
     const bool scorr = a.scorr_k != 0.f && !(a.w_dq <= 1.0e-6f);
     const float inv_wdq = scorr ? 1.0f / a.w_dq : 0.f;
     float dx_ = 0.f, dy_ = 0.f, dz_ = 0.f;
-    list_sum<G, false, true, false, false, 4>(
+    list_sum<G, false, true, false, false, 4, kGrid>(
         a.g, a.xs, a.rec, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn, mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -430,7 +430,7 @@ __global__ void FS_NB_BOUNDS_PBF k_xsph_final(XsphArgs a) {
     const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const Poly6Spiky K(a.h);
     float cx = 0.f, cy = 0.f, cz = 0.f;
-    list_sum<G, false, true, false, false, 4>(
+    list_sum<G, false, true, false, false, 4, kGrid>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn && a.c > 0.f, [&](int t) { return __ldg(a.vel + t); },
         [&](int t, float4 xj, const float4& vj) {

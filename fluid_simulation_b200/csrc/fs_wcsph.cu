@@ -128,7 +128,7 @@ __global__ void FS_NB_BOUNDS k_wcsph_force(ForceArgs a) {
       float4 v;
       float2 r;  // (p_j / rho_j^2, 1 / rho_j)
     };
-    list_sum<G, false, false, true, true, 4>(
+    list_sum<G, false, false, true, true, 4, kGrid>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn, [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(a.sc2 + t)}; },
         [&](int t, float4 xj, const Neighbour& j) {
