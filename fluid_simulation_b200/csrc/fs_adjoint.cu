@@ -292,7 +292,7 @@ __global__ void FS_NB_BOUNDS k_adj_force(AdjArgs a) {
   });
 }
 
-// 40 registers, the compiler's choice, with 32 bytes of spills (12 with several
+// The compiler takes 64 registers (40 and 12 bytes of spills with several
 // lanes); no other budget was measured.
 template <int G>
 __global__ void FS_NB_BOUNDS k_adj_density(AdjArgs a) {
