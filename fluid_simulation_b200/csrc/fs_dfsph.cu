@@ -489,9 +489,10 @@ struct CorrectArgs {
 // A pair gathers one 16-byte record, so that 40 registers and 48 resident warps
 // hold more of them in flight than 56 and 36: 47.6 -> 44.5 us a launch at
 // 401,856 particles (32 registers: 66; without the list's tests 41.4, with 48
-// registers the same).  Several lanes per particle want 64.
-template <int G>
-__global__ void __launch_bounds__(kNbBlockMax, G == 1 ? 6 : 4) k_correct(CorrectArgs a) {
+// registers the same).  It spills 52 bytes at 40; the compiler takes 61.  Several
+// lanes per particle want 64, and so does the pass without lists (kAhead).
+template <int G, Rescan RESCAN = kRecords>
+__global__ void __launch_bounds__(kNbBlockMax, G == 1 && RESCAN == kRecords ? 6 : 4) k_correct(CorrectArgs a) {
   grid_begin();
   if (a.ctrl && a.ctrl->done) return;
   if (clock_idle(a.clock)) return;
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(kNbBlockMax, G == 1 ? 6 : 4) k_correct(Correct
     const Cubic K(a.h);
     const float ci = a.rec[s].w;
     float dvx = 0.f, dvy = 0.f, dvz = 0.f;
-    list_sum<G, false, false, false, true, 4, kRecords>(
+    list_sum<G, false, false, false, true, 4, RESCAN>(
         a.g, a.xs, a.rec, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && !over && dyn, mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -541,13 +542,22 @@ __global__ void k_kappa_ratio(int64_t n, const float* __restrict__ kappa, const 
   if (s < n) rec[s] = make_float4(xs[s].x, xs[s].y, xs[s].z, kappa[s] / fmaxf(sc2[s].x, 1.0e-6f));
 }
 
-// (x, y, z, v_x) and (v_y, v_z) of gathered positions and velocities (separate passes)
-__global__ void k_pack_velocity(int64_t n, const float4* __restrict__ xs, const float4* __restrict__ vs,
-                                float4* __restrict__ xv, float2* __restrict__ vyz) {
+// What a rate or correction that runs by itself reads, in cell order: positions
+// and masses, (x, y, z, v_x) and (v_y, v_z), and with kappa the correction's
+// record (x, y, z, kappa / max(rho, 1e-6)).
+__global__ void k_gather_velocity(int64_t n, const int32_t* __restrict__ perm, fs_model m, const float* __restrict__ x,
+                                  const float* __restrict__ v, const float* __restrict__ rho,
+                                  const float* __restrict__ kappa, float4* __restrict__ xs, ScanOut q,
+                                  float* __restrict__ ms, float4* __restrict__ xv, float2* __restrict__ vyz,
+                                  float4* __restrict__ rec, uint32_t* status, int nworlds) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  xv[s] = make_float4(xs[s].x, xs[s].y, xs[s].z, vs[s].x);
-  vyz[s] = make_float2(vs[s].y, vs[s].z);
+  const int32_t i = perm[s];
+  gather_common_slot<false>(s, i, m, x, nullptr, xs, q, nullptr, nullptr, ms, status, nworlds);
+  const float3 p = ld3(x, i), u = ld3(v, i);
+  xv[s] = make_float4(p.x, p.y, p.z, u.x);
+  vyz[s] = make_float2(u.y, u.z);
+  if (kappa) rec[s] = make_float4(p.x, p.y, p.z, kappa[i] / fmaxf(rho[i], 1.0e-6f));
 }
 
 // The second half's gather: what the neighbour loops read, v* packed for them.
@@ -694,7 +704,10 @@ int run_correct(fs_context* c, const fs_model* m, float h, float dt, const float
   a.nworlds = c->nworlds;
   {
     PassScope ps_(c, P_DFSPH_CORRECT, st);
-    FS_NB_LAUNCH(k_correct, c, a.n, use_lists ? nb_group(a.n) : 1, st, false, a);
+    if (use_lists)
+      FS_NB_LAUNCH(k_correct, c, a.n, nb_group(a.n), st, false, a);
+    else  // each thread rescans
+      launch(k_correct<1, kAhead>, nb_blocks(c, a.n), c->nb_block, 0, st, a);
   }
   return launch_check("dfsph correct");
 }
@@ -973,7 +986,8 @@ int fs_dfsph_nonpressure_predict(fs_context* c, const fs_model* m, const float* 
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t n = m->n;
-  k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs, c->mv, c->mass, c->status, c->nworlds);
+  k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, no_scan(c), c->vs, nullptr, c->mass,
+                                                    c->status, c->nworlds);
   k_gather_pair<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, rho, nullptr, c->sc2);
   AccelArgs aa;
   aa.g = grid_view(c);
@@ -1004,8 +1018,9 @@ int fs_dfsph_divergence(fs_context* c, const fs_model* m, const float* x, const 
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_dfsph_divergence: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs2, nullptr, c->mass, c->status, c->nworlds);
-  k_pack_velocity<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->xs, c->vs2, c->xs2, (float2*)c->vo_tmp);
+  k_gather_velocity<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v, nullptr, nullptr, c->xs, no_scan(c),
+                                                         c->mass, c->xs2, (float2*)c->vo_tmp, nullptr, c->status,
+                                                         c->nworlds);
   // rho/factor are not needed for the rate itself (mode 1 reads them only for kappa, which is discarded)
   if (cudaMemsetAsync(c->sc2, 0, sizeof(float2) * m->n, st) != cudaSuccess)
     return set_error(FS_ERR_CUDA, "fs_dfsph_divergence: memset");
@@ -1019,14 +1034,11 @@ int fs_dfsph_correct(fs_context* c, const fs_model* m, const float* x, float* v_
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_dfsph_correct: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v_star, c->xs, scan_out(c), c->vs2, nullptr,
-                                                       c->mass, c->status, c->nworlds);
-  k_pack_velocity<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->xs, c->vs2, c->xs2, (float2*)c->vo_tmp);
-  k_gather_pair<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, rho, nullptr, c->sc2);
-  launch(k_gather_scalar, blocks_for(m->n), kBlock, 0, st, m->n, c->perm, kappa, c->sc1, nullptr);
   {
     PassScope ps_(c, P_GATHER, st);
-    launch(k_kappa_ratio, blocks_for(m->n), kBlock, 0, st, m->n, c->sc1, c->sc2, c->xs, c->rec);
+    k_gather_velocity<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x, v_star, rho, kappa, c->xs, no_scan(c),
+                                                           c->mass, c->xs2, (float2*)c->vo_tmp, c->rec, c->status,
+                                                           c->nworlds);
   }
   return run_correct(c, m, h, dt, c->sc1, c->rec, nullptr, v_star, nullptr, st, false);
 }

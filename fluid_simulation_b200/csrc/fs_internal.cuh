@@ -641,20 +641,25 @@ struct ScanOut {
   float* g;
   ListCtl* ctl;  // notes of the gather (may be null)
 };
-FS_DEV void scan_put(const ScanOut& q, int64_t s, float3 p, bool active) {
+FS_DEV void scan_note(const ScanOut& q, bool active) {
   if (!active && q.ctl) q.ctl->inactive = 1;
+}
+FS_DEV void scan_put(const ScanOut& q, int64_t s, float3 p, bool active) {
+  scan_note(q, active);
   float* o = q.g + (s >> 2) * 12 + (s & 3);
   o[0] = !active ? __uint_as_float(kScanInactive) : isfinite(p.x) ? p.x : __uint_as_float(kScanNonFinite);
   o[4] = p.y;
   o[8] = p.z;
 }
 ScanOut scan_out(const fs_context* c);
+inline ScanOut no_scan(const fs_context* c) { return ScanOut{nullptr, (ListCtl*)c->nb_ctl}; }
 
 // Slot s (particle i = perm[s]) of the cell-order copies that the neighbour
 // loops read: xs = (x, flags + world), ms = mass when ms, vs = (v, mass) when vs, and
 // mv = rest_density * volume with volume = mass / max(rest_density, 1e-6)
 // (compute_particle_volume, solver_wcsph.py:110-116) when mv.  A world index
-// past the model's worlds raises FS_STATUS_BOUNDS.
+// past the model's worlds raises FS_STATUS_BOUNDS.  SCAN: the scan copy too.
+template <bool SCAN = true>
 FS_DEV void gather_common_slot(int64_t s, int32_t i, const fs_model& m, const float* __restrict__ x,
                                const float* __restrict__ v, float4* __restrict__ xs, const ScanOut& q,
                                float4* __restrict__ vs, float* __restrict__ mv, float* __restrict__ ms,
@@ -664,7 +669,10 @@ FS_DEV void gather_common_slot(int64_t s, int32_t i, const fs_model& m, const fl
   // batched contexts carry the world in the flags word (queries stay in it)
   const int w = (nworlds > 0 && m.particle_world) ? world_index(m.particle_world[i], nworlds) : 0;
   xs[s] = make_float4(p.x, p.y, p.z, pack_pf(pf, w));
-  scan_put(q, s, p, (pf & PF_ACTIVE) != 0);
+  if (SCAN)
+    scan_put(q, s, p, (pf & PF_ACTIVE) != 0);
+  else
+    scan_note(q, (pf & PF_ACTIVE) != 0);
   const float mass = m.particle_mass[i];
   if (ms) {
     ms[s] = mass;

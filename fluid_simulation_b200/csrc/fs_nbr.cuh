@@ -523,23 +523,29 @@ FS_DEV void scan_grid(const GridDev& g, const float4* __restrict__ xs, int s, fl
   });
 }
 
-// The same for lists that overflowed: pair(t, rec[t]), by RESCAN
-//   kGrid     scan_grid, then the record
-//   kRecords  the positions from the records that the pairs gather anyway; a
-//             hit's flag is read only where some particle is inactive
-//   kAhead    and the next record loads while one is tested
+// The same for lists that overflowed and passes that run by themselves, without
+// lists: pair(t, rec[t]), by RESCAN
+//   kPositions  scan_grid (the record is the position: rec = xs)
+//   kGrid       scan_grid, then the record
+//   kRecords    the positions from the records that the pairs gather anyway; a
+//               hit's flag is read only where some particle is inactive
+//   kAhead      and the next record loads while one is tested
 // DFSPH substep with lists that all overflow (four spacings to the support,
-// about 250 neighbours), in ms at 61,740 and 401,856 particles: 15.9, 34.3;
-// 14.4, 31.1; 13.2, 33.2; kAhead but in the correction, which is short of
-// registers, 13.4, 31.0.  kGrid where that cost the ordinary path: WCSPH's force
+// about 250 neighbours), in ms at 61,740 and 401,856 particles: kGrid 15.9,
+// 34.3; kRecords 14.4, 31.1; kAhead 13.2, 33.2; kAhead but in the correction,
+// which is short of registers there, 13.4, 31.0.  Passes by themselves at 401,856:
+// PBF's delta 221 us with kGrid, 178 with kAhead, DFSPH's correction 200, 175.
+// kPositions and kGrid where the others cost the path with lists: WCSPH's force
 // 1 %, PBF's passes 0.4 % of a substep of 100,003 particles, several lanes per
 // particle 0.4 % at 4,079.
-enum Rescan { kGrid, kRecords, kAhead };
+enum Rescan { kPositions, kGrid, kRecords, kAhead };
 
 template <bool WITH_SELF, Rescan RESCAN, class Pair>
 FS_DEV void rescan(const GridDev& g, const float4* __restrict__ xs, const float4* __restrict__ rec, int s, float4 xi,
                    float h, float h2m, const NbrList& L, Pair&& pair) {
-  if constexpr (RESCAN == kGrid) {
+  if constexpr (RESCAN == kPositions) {
+    scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, pair);
+  } else if constexpr (RESCAN == kGrid) {
     scan_grid<WITH_SELF>(g, xs, s, xi, h, h2m, [&](int t, float4) { pair(t, __ldg(rec + t)); });
   } else {
     const bool inactive = L.ctl->inactive != 0;

@@ -176,7 +176,7 @@ __global__ void FS_NB_BOUNDS_PBF k_accel_apply(AccelArgs a) {
     const Poly6Spiky K(a.h);
     float ax = 0.f, ay = 0.f, az = 0.f;
     const bool on = live && dyn && (gamma != 0.f || mu != 0.f);
-    list_sum<G, false, true, false, false, 4, kGrid>(
+    list_sum<G, false, true, false, false, 4, kPositions>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L), on,
         [&](int t) { return Neighbour{__ldg(a.vs + t), mass(t)}; },
         [&](int t, float4 xj, const Neighbour& j) {
@@ -342,7 +342,7 @@ FS_DEV float pow_uint(float x, int n) {
   return r;
 }
 
-template <int G>
+template <int G, Rescan RESCAN = kGrid>
 __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
   grid_begin();
   // an integral exponent 1..8 (the class default is 4) takes pow_uint
@@ -358,7 +358,7 @@ __global__ void FS_NB_BOUNDS_PBF k_delta(DeltaArgs a) {
     const bool scorr = a.scorr_k != 0.f && !(a.w_dq <= 1.0e-6f);
     const float inv_wdq = scorr ? 1.0f / a.w_dq : 0.f;
     float dx_ = 0.f, dy_ = 0.f, dz_ = 0.f;
-    list_sum<G, false, true, false, false, 4, kGrid>(
+    list_sum<G, false, true, false, false, 4, RESCAN>(
         a.g, a.xs, a.rec, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn, mass, [&](int t, float4 xj, const float& mj) {
           const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
@@ -430,7 +430,7 @@ __global__ void FS_NB_BOUNDS_PBF k_xsph_final(XsphArgs a) {
     const bool dyn = pf_of(xi) & PF_DYNAMIC;
     const Poly6Spiky K(a.h);
     float cx = 0.f, cy = 0.f, cz = 0.f;
-    list_sum<G, false, true, false, false, 4, kGrid>(
+    list_sum<G, false, true, false, false, 4, kPositions>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn && a.c > 0.f, [&](int t) { return __ldg(a.vel + t); },
         [&](int t, float4 xj, const float4& vj) {
@@ -716,7 +716,7 @@ int fs_pbf_delta(fs_context* c, const fs_model* m, const float* x_pred, const fl
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_pbf_delta: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, x_pred, c->xs, scan_out(c), c->vs, nullptr,
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, x_pred, c->xs, no_scan(c), c->vs, nullptr,
                                                        c->mass, c->status, c->nworlds);
   k_gather_lambda_rec<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, pbf_lambda, c->xs, c->rec);
   DeltaArgs da;
@@ -738,7 +738,7 @@ int fs_pbf_delta(fs_context* c, const fs_model* m, const float* x_pred, const fl
   da.delta_p = delta_p;
   da.xs_out = nullptr;
   da.q = ScanOut{};
-  launch(k_delta<1>, nb_blocks(c, m->n), c->nb_block, 0, st, da);  // no list: each thread rescans
+  launch(k_delta<1, kAhead>, nb_blocks(c, m->n), c->nb_block, 0, st, da);  // no list: each thread rescans
   return launch_check("fs_pbf_delta");
 }
 
@@ -749,7 +749,7 @@ int fs_pbf_xsph(fs_context* c, const fs_model* m, const float* x_pred, const flo
   if (c->built_n != m->n) return set_error(FS_ERR_NOGRID, "fs_pbf_xsph: build the grid first");
   DeviceGuard dg(c->device);
   cudaStream_t st = (cudaStream_t)stream;
-  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, v_in, c->xs, scan_out(c), c->vs2, nullptr,
+  k_gather_common<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, *m, x_pred, v_in, c->xs, no_scan(c), c->vs2, nullptr,
                                                        c->mass, c->status, c->nworlds);
   k_gather_lambda<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->perm, rho, c->sc1);
   k_rho_ratio<<<blocks_for(m->n), kBlock, 0, st>>>(m->n, c->sc1, c->vs2);

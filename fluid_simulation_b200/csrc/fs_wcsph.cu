@@ -22,7 +22,10 @@ __global__ void k_gather_common(int64_t n, const int32_t* __restrict__ perm, fs_
                                 uint32_t* status, int nworlds) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  gather_common_slot(s, perm[s], m, x, v, xs, q, vs, mv, ms, status, nworlds);
+  if (q.g)
+    gather_common_slot(s, perm[s], m, x, v, xs, q, vs, mv, ms, status, nworlds);
+  else  // of a pass that does not scan
+    gather_common_slot<false>(s, perm[s], m, x, v, xs, q, vs, mv, ms, status, nworlds);
 }
 
 // ------------------------------------------------------------- density ----
@@ -128,7 +131,7 @@ __global__ void FS_NB_BOUNDS k_wcsph_force(ForceArgs a) {
       float4 v;
       float2 r;  // (p_j / rho_j^2, 1 / rho_j)
     };
-    list_sum<G, false, false, true, true, 4, kGrid>(
+    list_sum<G, false, false, true, true, 4, kPositions>(
         a.g, a.xs, a.xs, (int)s, xi, a.h, a.h * a.h * kSupportMargin, a.L, a.use_lists && lists_usable(a.L),
         live && dyn, [&](int t) { return Neighbour{__ldg(a.vs + t), __ldg(a.sc2 + t)}; },
         [&](int t, float4 xj, const Neighbour& j) {
@@ -197,7 +200,8 @@ int wcsph_gather(fs_context* c, const fs_model* m, const float* x, const float* 
   const int64_t n = m->n;
   {
     PassScope ps_(c, P_GATHER, st);
-    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, scan_out(c), c->vs, c->mv, c->mass, c->status, c->nworlds);
+    k_gather_common<<<blocks_for(n), kBlock, 0, st>>>(n, c->perm, *m, x, v, c->xs, no_scan(c), c->vs, c->mv, nullptr,
+                                                      c->status, c->nworlds);
   }
   return launch_check("wcsph gather");
 }
